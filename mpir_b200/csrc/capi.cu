@@ -232,8 +232,6 @@ struct StreamGuard {
   }
 };
 
-void invert_diag_blocks(const Plan &P, Numeric &F, cudaStream_t s);
-
 }  // namespace mpir
 
 using namespace mpir;
@@ -424,7 +422,7 @@ static int qdldl_solve_phases(int64_t n, const int64_t *Lp, const int64_t *Li, c
                                 cudaMemcpyHostToDevice, c->s));
       MPIR_CUDA(cudaMemcpyAsync(c->F->Dinv.as<void>(), dv.data(), n * sizeof(float),
                                 cudaMemcpyHostToDevice, c->s));
-      invert_diag_blocks(*c->P, *c->F, c->s);
+      flow_invert(*c->P, *c->F, c->s);
       c->F->trim();  // the solves read L, Dinv and the block inverses only
       c->ws = std::make_unique<SolveWorkspace>();
       c->ws->allocate(*c->P);

@@ -60,8 +60,10 @@ inline void launch(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem,
 struct StepDesc {
   int64_t panel;
   int64_t uofs;
-  int64_t linv;       // nbk x nbk inverse of the unit-lower diagonal block,
-                      // column-major with leading dimension kNB
+  int64_t linv;       // inverse of the unit-lower diagonal block, column-major
+                      // with leading dimension kNB and nbk columns rounded up
+                      // to 32 (zeros past nbk), among those
+                      // of the step (they are read by its panel solve only)
   int32_t h, w, kb, nbk;
   int32_t col0;       // permuted index of the front's first column
   int32_t trsm_tile0; // first TRSM row tile of this desc within the step
@@ -76,41 +78,11 @@ struct StepDesc {
   int32_t pk_wt;
 };
 
-// One large front in the triangular solves.  The forward solve of a level
-// runs one CTA per row block of 128 rows of each front (first the diagonal
-// row blocks of all fronts, front-major, then the off-diagonal ones); the
-// backward solve one CTA per 128-row chunk of the
-// off-diagonal rows (partial sums for all columns) and then one CTA per
-// column block (front-major, last block first).  CTAs take their work in
-// ticket order, so every block they wait for belongs to an earlier ticket.
-struct SolveFront {
-  int64_t panel;   // panel offset (h x w, column-major)
-  int64_t zofs;    // front vector in the solve workspace (h doubles)
-  int64_t linv;    // float64 inverse of diagonal block 0 (block b at + b kNB^2)
-  int64_t part;    // backward chunk partials (chunks x w doubles)
-  int64_t rows;    // the front's row index set at srows[rows ..]
-  int64_t gptr;    // row i's child contributions: zbuf[gsrc[e]] for e in
-                   // gp[gptr + i] .. gp[gptr + i + 1], in child order
-  int32_t h, w, nb;
-  int32_t col0;    // permuted index of the front's first column
-  int32_t n;       // order of the whole system (stride of the ready copies)
-  int32_t chunk0, chunks;  // backward chunk CTAs
-  int32_t own0;    // first backward column-block CTA
-};
-
-// One work item of the ticketed solve launches: a copy of its front's
-// descriptor and its row block (forward) or column block (backward), so a CTA
-// reads one record after taking its ticket.
-struct SolveItem {
-  SolveFront f;
-  int32_t    r;
-  int32_t    pad;
-};
-
 // Packed copy of a large front's L for the tensor-core updates.  Rows are
 // renumbered so that the off-diagonal rows start on a 128-row boundary:
 // packed row p = r for r < w, p = Wt + (r - w) for r >= w, Wt = w rounded up
-// to 128.  Row tile t (packed rows 128t .. 128t+127) holds the columns in
+// to 128 (0 for w <= 128: a front of one block step has no operands among its
+// own rows, and keeps the others only).  Row tile t (packed rows 128t .. 128t+127) holds the columns in
 // K-groups of 4; K-group g of row tile t is 2048 contiguous bytes at float
 // offset pk + (t * G + g) * 512, in the tensor cores' K-major core-matrix
 // layout without swizzle (packed row m of the tile at byte 16m, its 4 columns
@@ -208,11 +180,8 @@ constexpr int kSmallThreads = 256;
 constexpr int kDiagThreads  = 512;
 constexpr int kGemmThreads  = 256;
 constexpr int kEaChunk      = 8;     // parent columns per extend-add CTA
-constexpr int kSolveRows = 128;        // rows per forward-solve CTA
-constexpr int kSolveChunk = 128;       // rows per backward-solve CTA
-constexpr int kSolveThreads = 512;     // 4 column quarters x 128 rows
-// Fronts of at most this width and height are solved by one warp each
-// (column by column); larger ones by the SolveFront launches.
+// Fronts of at most this width and height are solved by one warp each, larger
+// ones by a CTA or several (flow.cuh).
 constexpr int kWarpSolveW = 32;
 constexpr int kWarpSolveH = 256;
 

@@ -7,6 +7,7 @@
 #include <vector>
 
 #include "common.cuh"
+#include "flow.cuh"
 #include "symbolic.hpp"
 
 namespace mpir {
@@ -105,16 +106,6 @@ struct LevelPlan {
   std::vector<Step> steps;
   // update matrices of the level's large fronts, after their last step
   int32_t u_begin = 0, u_count = 0, u_tiles = 0, u_rtiles = 0, u_convs = 0;
-  // Solve: large fronts' gather list = large list; small fronts handled by
-  // one warp each; large fronts by the SolveFront launches: fronts
-  // [sf_begin, sf_begin + sf_count), forward CTAs, backward chunk CTAs and
-  // backward column-block CTAs.
-  int32_t sf_begin = 0, sf_count = 0;
-  int32_t sw_begin = 0, sw_count = 0;  // warp-solved fronts (swarp list)
-  int32_t fwd_items = 0, bwd_chunk_items = 0, bwd_owner_items = 0;
-  // Offsets of the level's work items (Plan::fwd_item, own_item) and of its
-  // chunk -> front map (front index within the level).
-  int64_t fwd_map0 = 0, chunk_map0 = 0, own_map0 = 0;
 };
 
 // Everything the kernels need about one analysed pattern.
@@ -122,28 +113,26 @@ class Plan {
  public:
   Symbolic               S;
   std::vector<LevelPlan> levels;
-  int64_t                linv_elems = 0;
+  int64_t                linv_elems = 0;  // diagonal-block inverses of one step (floats)
   int64_t                nnz_full   = 0;
   int64_t                ndesc      = 0;  // step descriptors in total
-  int64_t                spart_elems = 0; // backward chunk partials (doubles)
-  // Solve synchronisation words (2 tickets per level) and whether any front
-  // takes the ticketed block kernels; reset before every solve.
-  int64_t                nblock_fronts = 0, sync_elems = 0;
   double                 update_flops = 0, trsm_flops = 0, panel_read_bytes = 0;
   // Pattern arrays on the device.
   DeviceBuffer amap, arow, acol, diag_pos, Kp, Kj, Ksrc;
   DeviceBuffer sfirst, srowptr, srows, srel, slofs, uofs, zofs, child_ptr,
       child_list, perm;
   DeviceBuffer ea_chunks, ea_hits;  // EaChunk / EaHit, see LevelPlan::ea_begin
-  DeviceBuffer small_list, large_list, steps, ea_tasks, linv_ofs_d, gemm_probs,
-      solve_fronts, swarp_list, sblock_list, gp, gsrc, fwd_item, chunk_map, own_item;
+  DeviceBuffer small_list, large_list, steps, ea_tasks, gemm_probs;
+  // Triangular solves (flow.cuh): warp-solved fronts, the work items of the two
+  // directions, the strips of the block inverses, the rows' child contributions.
+  DeviceBuffer flow_warp, flow_fwd, flow_bwd, flow_inv, flow_gfirst, flow_gmore;
+  int32_t      nflow_fwd = 0, nflow_bwd = 0, nflow_inv = 0;
+  int64_t      flow_part_elems = 0, flow_inv_elems = 0, flow_wpanel_total = 0;
+  bool warp_solved(int64_t J) const { return S.w(J) <= kWarpSolveW && S.h(J) <= kWarpSolveH; }
+  void build_flow();
   int64_t      ws_elems = 0;  // split-K partial tiles (floats)
   int64_t      bconv_elems = 0;  // converted B operands of the largest launch (floats)
   std::vector<int32_t> h_small, h_large;
-  // Solve lists: fronts solved by one warp, fronts with a SolveFront entry
-  // (same order as the SolveFront array).
-  std::vector<int32_t> h_swarp, h_sblock;
-  std::vector<int64_t> linv_ofs;  // per supernode, -1 for small fronts
   // Packed fronts (PackedFront) of the large fronts: float offsets of the
   // packed rows and of the packed pivots per supernode (-1 for small
   // fronts), and the totals.
@@ -167,16 +156,18 @@ class Plan {
     std::vector<EaTask>     tasks;
     std::vector<EaChunk>    chunks;
     std::vector<EaHit>      hits;
-    std::vector<int32_t>    chunk_map;
     std::vector<GemmProb>   probs;
-    std::vector<SolveFront> sfronts;
-    std::vector<int64_t>    gp, gsrc;
-    std::vector<SolveItem>  fwd_item, own_item;
+    std::vector<FlowFront>   flow_warp;
+    std::vector<FlowItem>    flow_fwd, flow_bwd;
+    std::vector<FlowInvDesc> flow_inv;
+    std::vector<int2>        flow_gfirst;
+    std::vector<int32_t>     flow_gmore;
   } host_;
   bool is_large(int64_t J) const { return S.h(J) > kSmallFront; }
   // Packed-front geometry (PackedFront): first packed row of the
   // off-diagonal rows, K-groups per row tile, row tiles.
-  int64_t pk_wt(int64_t J) const { return (S.w(J) + 127) / 128 * 128; }
+  // (Of a front of one block step only the off-diagonal rows are operands.)
+  int64_t pk_wt(int64_t J) const { return S.w(J) <= kNB ? 0 : (S.w(J) + 127) / 128 * 128; }
   int64_t pk_groups(int64_t J) const { return (S.w(J) + 31) / 32 * 8; }
   int64_t pk_tiles(int64_t J) const { return (pk_wt(J) + S.h(J) - S.w(J) + 127) / 128; }
 };
@@ -184,10 +175,9 @@ class Plan {
 // Numeric factor of one value set on a plan.
 class Numeric {
  public:
-  // linv: float32 inverses of the diagonal blocks (the factor's panel solve);
-  // linv64: the same inverses in float64 (the triangular solves), column-major;
-  // linv64t: row-major copy of linv64 (the backward solve).
-  DeviceBuffer panel, uarena, linv, linv64, linv64t, D, Dinv, status, ws;
+  // inv64: float64 inverses of the diagonal super-blocks, wpanel: the float64
+  // panels of the warp-solved fronts (the triangular solves, flow.cuh).
+  DeviceBuffer panel, uarena, inv64, wpanel, D, Dinv, status, ws;
   // Packed fronts for the tensor-core updates: rows (pack) and pivots
   // (packd: D, then sign(D) sqrt|D|, Plan::pd_elems floats each).
   DeviceBuffer pack, packd;
@@ -196,7 +186,8 @@ class Numeric {
   DeviceBuffer panel16;
   int          store_prec = 1;
   int          solve_prec() const { return panel16.bytes() ? store_prec : 1; }
-  // B operands converted ahead of the 3xTF32 updates (GemmProb::bc).
+  // B operands converted ahead of the 3xTF32 updates (GemmProb::bc); and, from
+  // a step's diagonal blocks to its panel solve, those blocks' float32 inverses.
   DeviceBuffer bconv;
   DeviceBuffer AD, Axs, Kval, Korig, Ax;
   double       eps_uf = 0;
@@ -247,6 +238,10 @@ class Numeric {
                  bool *nonfinite = nullptr) const;
 };
 
+// What the triangular solves read of a factor beyond its panels: the float64
+// inverses of the diagonal blocks and the panels of the warp-solved fronts
+// (solve.cu), once per factorization.
+void flow_invert(const Plan &P, Numeric &F, cudaStream_t s);
 // Tensor-core GemmProb updates from the packed fronts (mode 0 bfloat16,
 // 1 3xTF32, 2 float16).  packs = the sign(D) sqrt|D| array.
 void launch_gemm_tc(int mode, const GemmProb *probs, int nprob, int tiles, const float *pack,

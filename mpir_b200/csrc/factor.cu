@@ -451,6 +451,7 @@ __global__ void __launch_bounds__(kDiagThreads)
 #pragma unroll 4
   for (int m = 0; m < 32; m++) {
     const int j = c + 4 * m;
+    if (j >= n32) break;
     Lv[ri + j * kNB] = (ri < n && j < n && ri / 32 >= j / 32) ? Xs[ri * LD + j] : 0.0f;
   }
 }
@@ -801,49 +802,6 @@ __global__ void __launch_bounds__(256)
     if (at[v] >= 0) C[at[v]] = cv[v] - a[v];
 }
 
-// Inverses, in float64, of the unit-lower diagonal blocks of the large
-// fronts, for the triangular solves: run once after a factorization (off its
-// critical path), and for a factor supplied by the caller (the QDLDL_solve
-// entry point).
-__global__ void __launch_bounds__(kDiagThreads)
-    k_invert_blocks(const StepDesc *descs, const float *panel, double *linv64,
-                    double *linv64t) {
-  extern __shared__ double smd[];
-  constexpr int            LD = kNB + 1;
-  double                  *X  = smd;
-  float                   *F  = reinterpret_cast<float *>(smd + kNB * LD);
-  const StepDesc           d  = descs[blockIdx.x];
-  const int                n  = d.nbk;
-  const int64_t            h  = d.h;
-  const int                tid = threadIdx.x, bd = blockDim.x;
-  const float             *P   = panel + d.panel + d.kb + (int64_t)d.kb * h;
-  for (int idx = tid; idx < n * n; idx += bd) {
-    const int i = idx % n, j = idx / n;
-    F[i * LD + j] = i > j ? P[i + (int64_t)j * h] : 0.0f;
-    X[i * LD + j] = i == j ? 1.0 : 0.0;
-  }
-  __syncthreads();
-  // Step k subtracts L[i][k] X[k][j] from X[i][j] for all i > k, j <= k:
-  // thread (i, g) = (tid % kNB, tid / kNB) takes row i and the columns
-  // j = g, g + 4, ... (every entry gets its terms in increasing k).
-  static_assert(kDiagThreads == 4 * kNB, "invert thread mapping");
-  const int ri = tid % kNB, g = tid / kNB;
-  for (int k = 0; k < n; k++) {
-    if (ri > k && ri < n) {
-      const double f = static_cast<double>(F[ri * LD + k]);
-      for (int j = g; j <= k; j += 4) X[ri * LD + j] -= f * X[k * LD + j];
-    }
-    __syncthreads();
-  }
-  double *Ld = linv64 + d.linv, *Lt = linv64t + d.linv;
-  for (int idx = tid; idx < kNB * kNB; idx += bd) {
-    const int    i = idx % kNB, j = idx / kNB;
-    const double v = (i < n && j < n) ? X[i * LD + j] : 0.0;
-    Ld[i + j * kNB] = v;
-    Lt[i * kNB + j] = v;
-  }
-}
-
 // The panels rounded to bfloat16 (bf != 0) or float16 for the solves of the
 // 16-bit tiers: L is stored in the tier's type and the solves read half the
 // bytes (their arithmetic stays float64).
@@ -860,17 +818,6 @@ __global__ void k_panel_to16(int64_t n, const float *in, uint16_t *out, int bf) 
   }
 }
 
-void invert_diag_blocks(const Plan &P, Numeric &F, cudaStream_t s) {
-  if (P.ndesc == 0) return;
-  const int smem = kNB * (kNB + 1) * (sizeof(double) + sizeof(float));
-  MPIR_CUDA(cudaFuncSetAttribute(k_invert_blocks,
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-  launch(k_invert_blocks, static_cast<unsigned>(P.ndesc), kDiagThreads, smem, s,
-         P.steps.as<StepDesc>(), F.panel.as<float>(), F.linv64.as<double>(),
-         F.linv64t.as<double>());
-  MPIR_CHECK_LAUNCH();
-}
-
 // ---------------------------------------------------------------------------
 // Plan construction.
 
@@ -879,16 +826,7 @@ void Plan::build(Symbolic &&sym, cudaStream_t s, bool upload) {
   const int64_t ns = S.ns;
   nnz_full         = static_cast<int64_t>(S.Kj.size());
   // Persistent Linv storage for the large fronts.
-  linv_ofs.assign(ns, -1);
   linv_elems   = 0;
-  spart_elems  = 0;
-  nblock_fronts = 0;
-  h_swarp.clear();
-  h_sblock.clear();
-  std::vector<int64_t> gp_h, gsrc_h;
-  std::vector<int32_t>   chunk_map_h;
-  std::vector<SolveItem> fwd_item_h, own_item_h;
-  std::vector<SolveFront> sfronts;
   update_flops = 0;
   trsm_flops   = 0;
   pk_ofs.assign(ns, -1);
@@ -896,8 +834,6 @@ void Plan::build(Symbolic &&sym, cudaStream_t s, bool upload) {
   pk_elems = pd_elems = 0;
   for (int64_t J = 0; J < ns; J++)
     if (is_large(J)) {
-      linv_ofs[J] = linv_elems;
-      linv_elems += ((S.w(J) + kNB - 1) / kNB) * (int64_t)kNB * kNB;
       pk_ofs[J] = pk_elems;
       pk_elems += pk_tiles(J) * pk_groups(J) * PackedFront::kGroupFloats;
       pd_ofs[J] = pd_elems;
@@ -1074,13 +1010,14 @@ void Plan::build(Symbolic &&sym, cudaStream_t s, bool upload) {
     for (int64_t kb = 0; kb < maxw; kb += kNB) {
       LevelPlan::Step st{static_cast<int32_t>(descs.size()), 0, 0, 0,
                          static_cast<int32_t>(probs.size()), 0, 0, 0, 0};
+      int64_t linv_top = 0;
       for (int32_t q = L.large_begin; q < L.large_begin + L.large_count; q++) {
         const int64_t J = h_large[q], w = S.w(J), h = S.h(J);
         if (w <= kb) continue;
         StepDesc d;
         d.panel  = S.slofs[J];
         d.uofs   = S.uofs[J];
-        d.linv   = linv_ofs[J] + (kb / kNB) * (int64_t)kNB * kNB;
+        d.linv   = linv_top;
         d.h      = static_cast<int32_t>(h);
         d.w      = static_cast<int32_t>(w);
         d.kb     = static_cast<int32_t>(kb);
@@ -1121,89 +1058,13 @@ void Plan::build(Symbolic &&sym, cudaStream_t s, bool upload) {
         d.pk_wt        = static_cast<int32_t>(pk_wt(J));
         descs.push_back(d);
         st.count++;
+        linv_top += (d.nbk + 31) / 32 * 32 * (int64_t)kNB;
+        linv_elems = std::max(linv_elems, linv_top);
       }
       st.ll_count = static_cast<int32_t>(probs.size()) - st.ll_begin;
       finish_launch(st.ll_begin, st.ll_count, st.ll_tiles, st.ll_rtiles, st.ll_convs);
       L.steps.push_back(st);
     }
-    // Solve work of the level: narrow, short fronts one warp each, the rest
-    // through SolveFront entries.
-    L.sw_begin = static_cast<int32_t>(h_swarp.size());
-    L.sf_begin = static_cast<int32_t>(sfronts.size());
-    for (int32_t q = L.small_begin; q < L.small_begin + L.small_count; q++)
-      h_swarp.push_back(h_small[q]);
-    int64_t spart = 0;
-    for (int32_t q = L.large_begin; q < L.large_begin + L.large_count; q++) {
-      const int64_t J = h_large[q], w = S.w(J), h = S.h(J);
-      if (w <= kWarpSolveW && h <= kWarpSolveH) {
-        h_swarp.push_back(J);
-        continue;
-      }
-      h_sblock.push_back(J);
-      SolveFront    f{};
-      // Child contributions per row, in child order (the forward solve adds
-      // them in this order).
-      f.rows = S.srowptr[J];
-      f.gptr = static_cast<int64_t>(gp_h.size());
-      {
-        std::vector<int64_t> cnt(h + 1, 0);
-        for (int64_t c = S.child_ptr[J]; c < S.child_ptr[J + 1]; c++) {
-          const int64_t C = S.child_list[c], wc = S.w(C), rc = S.h(C) - wc;
-          for (int64_t a = 0; a < rc; a++) cnt[S.srel[S.srowptr[C] + wc + a] + 1]++;
-        }
-        for (int64_t i = 0; i < h; i++) cnt[i + 1] += cnt[i];
-        const int64_t base = static_cast<int64_t>(gsrc_h.size());
-        for (int64_t i = 0; i <= h; i++) gp_h.push_back(base + cnt[i]);
-        gsrc_h.resize(base + cnt[h]);
-        for (int64_t c = S.child_ptr[J]; c < S.child_ptr[J + 1]; c++) {
-          const int64_t C = S.child_list[c], wc = S.w(C), rc = S.h(C) - wc;
-          for (int64_t a = 0; a < rc; a++)
-            gsrc_h[base + cnt[S.srel[S.srowptr[C] + wc + a]]++] = S.zofs[C] + wc + a;
-        }
-      }
-      f.panel  = S.slofs[J];
-      f.zofs   = S.zofs[J];
-      f.linv   = linv_ofs[J];
-      f.h      = static_cast<int32_t>(h);
-      f.w      = static_cast<int32_t>(w);
-      f.nb     = static_cast<int32_t>((w + kNB - 1) / kNB);
-      f.col0   = static_cast<int32_t>(S.sfirst[J]);
-      f.n      = static_cast<int32_t>(S.n);
-      nblock_fronts++;
-      L.fwd_items += static_cast<int32_t>((h + kNB - 1) / kNB);
-      f.chunks = static_cast<int32_t>((h - w + kNB - 1) / kNB);
-      f.chunk0 = L.bwd_chunk_items;
-      L.bwd_chunk_items += f.chunks;
-      f.part   = spart;
-      spart += static_cast<int64_t>(f.chunks) * w;
-      f.own0   = L.bwd_owner_items;
-      L.bwd_owner_items += f.nb;
-      sfronts.push_back(f);
-    }
-    L.sf_count  = static_cast<int32_t>(sfronts.size()) - L.sf_begin;
-    // Item -> front maps of the level's solve launches.
-    L.fwd_map0   = static_cast<int64_t>(fwd_item_h.size());
-    L.chunk_map0 = static_cast<int64_t>(chunk_map_h.size());
-    L.own_map0   = static_cast<int64_t>(own_item_h.size());
-    // Forward: every front's diagonal row blocks first (their chains start
-    // together), then the off-diagonal row blocks, which wait on them.
-    for (int32_t q = 0; q < L.sf_count; q++) {
-      const SolveFront &f = sfronts[L.sf_begin + q];
-      for (int32_t i = 0; i < f.nb; i++) fwd_item_h.push_back(SolveItem{f, i, 0});
-    }
-    for (int32_t q = 0; q < L.sf_count; q++) {
-      const SolveFront &f = sfronts[L.sf_begin + q];
-      for (int32_t i = f.nb; i < (f.h + kNB - 1) / kNB; i++)
-        fwd_item_h.push_back(SolveItem{f, i, 0});
-    }
-    // Backward: each front's column blocks, last first.
-    for (int32_t q = 0; q < L.sf_count; q++) {
-      const SolveFront &f = sfronts[L.sf_begin + q];
-      for (int32_t i = 0; i < f.chunks; i++) chunk_map_h.push_back(q);
-      for (int32_t i = 0; i < f.nb; i++) own_item_h.push_back(SolveItem{f, f.nb - 1 - i, 0});
-    }
-    L.sw_count  = static_cast<int32_t>(h_swarp.size()) - L.sw_begin;
-    spart_elems = std::max(spart_elems, spart);
     L.u_begin = static_cast<int32_t>(probs.size());
     for (int32_t q = L.large_begin; q < L.large_begin + L.large_count; q++) {
       const int64_t J = h_large[q], w = S.w(J), h = S.h(J), r = h - w;
@@ -1235,7 +1096,6 @@ void Plan::build(Symbolic &&sym, cudaStream_t s, bool upload) {
     const double w = static_cast<double>(S.w(J)), h = static_cast<double>(S.h(J));
     panel_read_bytes += 4.0 * (w * h - w * (w - 1) / 2);
   }
-  sync_elems = 2 * static_cast<int64_t>(levels.size());
   // The host arrays stay with the plan, so an evicted plan can go back to
   // the device without being built again.
   host_.descs       = std::move(descs);
@@ -1243,12 +1103,7 @@ void Plan::build(Symbolic &&sym, cudaStream_t s, bool upload) {
   host_.chunks      = std::move(chunks_h);
   host_.hits        = std::move(hits_h);
   host_.probs       = std::move(probs);
-  host_.sfronts     = std::move(sfronts);
-  host_.gp          = std::move(gp_h);
-  host_.gsrc        = std::move(gsrc_h);
-  host_.fwd_item    = std::move(fwd_item_h);
-  host_.chunk_map   = std::move(chunk_map_h);
-  host_.own_item    = std::move(own_item_h);
+  build_flow();
   if (upload) upload_all(s);
 }
 
@@ -1258,8 +1113,8 @@ size_t Plan::upload_bytes() const {
          b(S.sfirst) + b(S.srowptr) + b(S.srows) + b(S.srel) + b(S.slofs) + b(S.uofs) +
          b(S.zofs) + b(S.child_ptr) + b(S.child_list) + b(S.perm) + b(h_small) + b(h_large) +
          b(host_.descs) + b(host_.tasks) + b(host_.chunks) + b(host_.hits) + b(host_.probs) +
-         b(linv_ofs) + b(host_.sfronts) + b(h_swarp) + b(h_sblock) + b(host_.gp) +
-         b(host_.gsrc) + b(host_.fwd_item) + b(host_.chunk_map) + b(host_.own_item);
+         b(host_.flow_warp) + b(host_.flow_fwd) + b(host_.flow_bwd) + b(host_.flow_inv) +
+         b(host_.flow_gfirst) + b(host_.flow_gmore);
 }
 
 void Plan::upload_all(cudaStream_t s) {
@@ -1288,15 +1143,12 @@ void Plan::upload_all(cudaStream_t s) {
   ea_chunks  = upload(host_.chunks, s);
   ea_hits    = upload(host_.hits, s);
   gemm_probs = upload(host_.probs, s);
-  linv_ofs_d = upload(linv_ofs, s);
-  solve_fronts = upload(host_.sfronts, s);
-  swarp_list   = upload(h_swarp, s);
-  sblock_list  = upload(h_sblock, s);
-  gp           = upload(host_.gp, s);
-  gsrc         = upload(host_.gsrc, s);
-  fwd_item     = upload(host_.fwd_item, s);
-  chunk_map    = upload(host_.chunk_map, s);
-  own_item     = upload(host_.own_item, s);
+  flow_warp    = upload(host_.flow_warp, s);
+  flow_fwd     = upload(host_.flow_fwd, s);
+  flow_bwd     = upload(host_.flow_bwd, s);
+  flow_inv     = upload(host_.flow_inv, s);
+  flow_gfirst  = upload(host_.flow_gfirst, s);
+  flow_gmore   = upload(host_.flow_gmore, s);
   MPIR_CUDA(cudaStreamSynchronize(s));
   upload_ms = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
   on_device = true;
@@ -1306,8 +1158,8 @@ void Plan::release_device() {
   for (DeviceBuffer *d :
        {&amap, &arow, &acol, &diag_pos, &Kp, &Kj, &Ksrc, &sfirst, &srowptr, &srows, &srel,
         &slofs, &uofs, &zofs, &child_ptr, &child_list, &perm, &ea_chunks, &ea_hits, &small_list,
-        &large_list, &steps, &ea_tasks, &linv_ofs_d, &gemm_probs, &solve_fronts, &swarp_list,
-        &sblock_list, &gp, &gsrc, &fwd_item, &chunk_map, &own_item})
+        &large_list, &steps, &ea_tasks, &gemm_probs, &flow_warp, &flow_fwd,
+        &flow_bwd, &flow_inv, &flow_gfirst, &flow_gmore})
     d->release();
   on_device = false;
 }
@@ -1320,8 +1172,10 @@ void Numeric::allocate(const Plan &P) {
     panel16.resize(std::max<int64_t>(S.panel_elems, 1) * 2);
   else
     panel16.release();
-  linv64.resize(std::max<int64_t>(P.linv_elems, 1) * sizeof(double));
-  linv64t.resize(std::max<int64_t>(P.linv_elems, 1) * sizeof(double));
+  // Positions of the inverses that no column of a front has stay zero.
+  wpanel.resize(std::max<int64_t>(P.flow_wpanel_total, 1) * sizeof(double));
+  inv64.resize(std::max<int64_t>(P.flow_inv_elems, 1) * sizeof(double));
+  device_zero(inv64.as<void>(), inv64.bytes());
   D.resize(std::max<int64_t>(S.n, 1) * sizeof(float));
   Dinv.resize(std::max<int64_t>(S.n, 1) * sizeof(float));
   status.resize(sizeof(FactorStatus));
@@ -1339,11 +1193,10 @@ void Numeric::ensure_scratch(const Plan &P) {
   const Symbolic &S = P.S;
   if (!panel.bytes()) panel.resize(std::max<int64_t>(S.panel_elems, 1) * sizeof(float));
   uarena.resize(std::max<int64_t>(S.uarena_elems, 1) * sizeof(float));
-  linv.resize(std::max<int64_t>(P.linv_elems, 1) * sizeof(float));
   ws.resize(std::max<int64_t>(P.ws_elems, 1) * sizeof(float));
   // Packed fronts: positions that hold no value of L are never written and
   // stay zero from here on.
-  bconv.resize(std::max<int64_t>(P.bconv_elems, 1) * sizeof(float));
+  bconv.resize(std::max<int64_t>(std::max(P.bconv_elems, P.linv_elems), 1) * sizeof(float));
   pack.resize(std::max<int64_t>(P.pk_elems, 1) * sizeof(float));
   packd.resize(std::max<int64_t>(2 * P.pd_elems, 1) * sizeof(float));
   device_zero(pack.as<void>(), pack.bytes());
@@ -1355,7 +1208,7 @@ void Numeric::ensure_scratch(const Plan &P) {
 
 void Numeric::trim() {
   release_graph();
-  for (DeviceBuffer *b : {&uarena, &linv, &ws, &bconv, &pack, &packd, &Axs, &Ax}) b->release();
+  for (DeviceBuffer *b : {&uarena, &ws, &bconv, &pack, &packd, &Axs, &Ax}) b->release();
   if (panel16.bytes()) panel.release();  // the solves read the 16-bit copy
   has_scratch = false;
 }
@@ -1363,15 +1216,15 @@ void Numeric::trim() {
 size_t Numeric::bytes_for(const Plan &P, int store_prec) {
   const Symbolic &S  = P.S;
   auto            at = [](int64_t e, size_t b) { return std::max<int64_t>(e, 1) * b; };
-  return at(S.panel_elems, store_prec == 1 ? 4 : 6) + at(S.uarena_elems, 4) + at(P.linv_elems, 4) +
-         2 * at(P.linv_elems, 8) + at(P.ws_elems, 4) + at(P.bconv_elems, 4) +
+  return at(S.panel_elems, store_prec == 1 ? 4 : 6) + at(S.uarena_elems, 4) +
+         at(P.flow_inv_elems, 8) + at(P.flow_wpanel_total, 8) + at(P.ws_elems, 4) + at(std::max(P.bconv_elems, P.linv_elems), 4) +
          at(P.pk_elems, 4) + at(2 * P.pd_elems, 4) + 2 * at(S.n, 4) + sizeof(FactorStatus) +
          at(S.n, 8) + 2 * at(S.nnz, 8) + 2 * at(P.nnz_full, 8);
 }
 
 size_t Numeric::device_bytes() const {
   size_t b = 0;
-  for (const DeviceBuffer *d : {&panel, &panel16, &uarena, &linv, &linv64, &linv64t, &D, &Dinv, &status,
+  for (const DeviceBuffer *d : {&panel, &panel16, &uarena, &inv64, &wpanel, &D, &Dinv, &status,
                                 &ws, &pack, &packd, &bconv, &AD, &Axs, &Kval, &Korig, &Ax})
     b += d->bytes();
   return b;
@@ -1382,8 +1235,8 @@ size_t Plan::device_bytes() const {
   for (const DeviceBuffer *d :
        {&amap, &arow, &acol, &diag_pos, &Kp, &Kj, &Ksrc, &sfirst, &srowptr, &srows, &srel,
         &slofs, &uofs, &zofs, &child_ptr, &child_list, &perm, &ea_chunks, &ea_hits, &small_list,
-        &large_list, &steps, &ea_tasks, &linv_ofs_d, &gemm_probs, &solve_fronts, &swarp_list,
-        &sblock_list, &gp, &gsrc, &fwd_item, &chunk_map, &own_item})
+        &large_list, &steps, &ea_tasks, &gemm_probs, &flow_warp, &flow_fwd,
+        &flow_bwd, &flow_inv, &flow_gfirst, &flow_gmore})
     b += d->bytes();
   return b;
 }
@@ -1547,18 +1400,18 @@ void Numeric::run(const Plan &P, const double *d_Ax, double eps, cudaStream_t s)
       const StepDesc *dd = P.steps.as<StepDesc>() + stp.begin;
       gemm(stp.ll_begin, stp.ll_count, stp.ll_tiles, stp.ll_rtiles, stp.ll_convs);
       kt.begin(kKcDiag, s);
-      launch(k_diag_block, stp.count, kDiagThreads, diag_smem, s, dd, pan, linv.as<float>(),
+      launch(k_diag_block, stp.count, kDiagThreads, diag_smem, s, dd, pan, bconv.as<float>(),
              D.as<float>(), Dinv.as<float>(), packd.as<float>(),
              packd.as<float>() + P.pd_elems, st);
       kt.end(s);
       if (stp.trsm_tiles > 0) {
         kt.begin(kKcTrsm, s);
         if (trsm_tc)
-          launch_trsm_tc(dd, stp.count, stp.trsm_tiles, pan, linv.as<float>(), Dinv.as<float>(),
+          launch_trsm_tc(dd, stp.count, stp.trsm_tiles, pan, bconv.as<float>(), Dinv.as<float>(),
                          pack.as<float>(), st, s);
         else
           launch(k_step_gemm<true>, stp.trsm_tiles, kGemmThreads, trsm_smem, s, dd, stp.count,
-                 pan, ua, linv.as<float>(), Dinv.as<float>(), pack.as<float>());
+                 pan, ua, bconv.as<float>(), Dinv.as<float>(), pack.as<float>());
         kt.end(s);
       }
     }
@@ -1568,7 +1421,7 @@ void Numeric::run(const Plan &P, const double *d_Ax, double eps, cudaStream_t s)
   }
   // Float64 inverses of the diagonal blocks for the triangular solves.
   kt.begin(kKcDiag, s);
-  invert_diag_blocks(P, *this, s);
+  flow_invert(P, *this, s);
   kt.end(s);
   if (panel16.bytes() && S.panel_elems) {
     kt.begin(kKcScatter, s);

@@ -121,8 +121,8 @@ void Solver::adopt(std::shared_ptr<Plan> P) {
 
 size_t Solver::device_bytes() const {
   size_t b = num_.device_bytes();
-  for (const DeviceBuffer *d : {&ws_.zbuf, &ws_.part, &ws_.sync, &ws_.ready, &ws_.err, &ws_.xbuf,
-                                &mws_.zbuf, &mws_.part, &mws_.sync, &mws_.ready, &mws_.err,
+  for (const DeviceBuffer *d : {&ws_.vals, &ws_.sync, &ws_.err,
+                                &mws_.vals, &mws_.sync, &mws_.err,
                                 &vec_.part, &vec_.count, &vec_.infbits, &vecb_.part, &vecb_.count,
                                 &vecb_.infbits, &V_, &bs_, &bp_, &ADp_, &x_, &r_, &t_, &d_, &hd_,
                                 &y_, &hb_, &hx_, &bV_, &bbs_, &bbp_, &bx_, &br_, &bt_, &bd_, &bhd_,
@@ -136,8 +136,7 @@ size_t Solver::bytes_for(const Plan &P, int64_t gmres_iter, int width, int uf) {
   const int64_t m  = std::max<int64_t>(std::min(gmres_iter, n), 1);
   size_t        b  = Numeric::bytes_for(P, uf == kBF16 ? 2 : uf == kF16 ? 3 : 1);
   // single-vector workspace and vectors
-  b += (std::max<int64_t>(P.S.z_elems, 1) + std::max<int64_t>(P.spart_elems, 1) +
-        static_cast<int64_t>(kReadyCopies) * n + n) * sizeof(double);
+  b += SolveWorkspace::bytes_for(P);
   b += (m + 1 + 10) * n * sizeof(double) + 2048 * sizeof(double);
   if (width > 1) {
     b += MultiSolveWorkspace::bytes_for(P, width);
@@ -264,7 +263,7 @@ void Solver::precond_gmres(const double *b, double *res, Report &st) {
   read(&rho, 0, 1);
   if (rho < tol) return;
   MPIR_CUDA(cudaMemcpyAsync(V, b, n * sizeof(double), cudaMemcpyDeviceToDevice, s));
-  ldlt_solve_graph(P, num_, V, ws_, s, own_stream_);
+  ldlt_solve(P, num_, V, ws_, s);
   st.precond_applies++;
   vec_.mgs_pass(V, nullptr, nullptr, nullptr, 1, hd, s);
   read(&rho, 0, 1);
@@ -280,7 +279,7 @@ void Solver::precond_gmres(const double *b, double *res, Report &st) {
     double *vk = V + k * n, *w = V + (k + 1) * n;
     vec_.spmv(Kp, Kj, Kv, vk, w, s);
     st.spmv_count++;
-    ldlt_solve_graph(P, num_, w, ws_, s, own_stream_);
+    ldlt_solve(P, num_, w, ws_, s);
     st.precond_applies++;
     double *hn = hd + (m + 2);  // normav
     vec_.mgs_pass(w, nullptr, nullptr, nullptr, 1, hn, s);
@@ -491,7 +490,7 @@ int Solver::luir_device(const double *d_b, double *d_x, int maxiter, Report *rep
   vec_.rhs_in(P.perm.as<int64_t>(), num_.AD.as<double>(), d_b, bs, ADp, bp_.as<double>(), s);
   MPIR_CUDA(cudaMemcpyAsync(x, bs, n * sizeof(double), cudaMemcpyDeviceToDevice, s));
   vec_.round_to(uf, x, s);
-  ldlt_solve_graph(P, num_, x, ws_, s, own_stream_);
+  ldlt_solve(P, num_, x, ws_, s);
   st.precond_applies++;
   vec_.round_to(uf, x, s);
   const double eps = eps_of(kF64);
@@ -512,7 +511,7 @@ int Solver::luir_device(const double *d_b, double *d_x, int maxiter, Report *rep
     }
     vec_.scale(r, 1.0 / rn, r, s);
     vec_.round_to(uf, r, s);
-    ldlt_solve_graph(P, num_, r, ws_, s, own_stream_);
+    ldlt_solve(P, num_, r, ws_, s);
     st.precond_applies++;
     vec_.round_to(uf, r, s);
     vec_.ir_update(r, rn, x, s, ADp);

@@ -32,8 +32,8 @@ size_t Solver::batch_growth(int width) const {
                       2048 * width * sizeof(double);
   size_t have = 0;
   for (const DeviceBuffer *d : {&bV_, &bbs_, &bbp_, &bx_, &br_, &bt_, &bd_, &bhd_, &by_, &bfac_,
-                                &bact_, &bkq_, &bin_, &bout_, &bpre_, &mws_.zbuf, &mws_.part,
-                                &mws_.sync, &mws_.ready, &mws_.err, &mws_.xbuf, &vecb_.part,
+                                &bact_, &bkq_, &bin_, &bout_, &bpre_, &mws_.vals,
+                                &mws_.sync, &mws_.err, &vecb_.part,
                                 &vecb_.count, &vecb_.infbits})
     have += d->bytes();
   return want > have ? want - have : 0;
@@ -84,7 +84,7 @@ void Solver::ensure_batch(int width) {
 }
 
 void Solver::multi_apply(double *block) {
-  ldlt_solve_multi_graph(*plan_, num_, block, bw_, mws_, stream_, own_stream_);
+  ldlt_solve_multi(*plan_, num_, block, bw_, mws_, stream_);
 }
 
 void Solver::precond_device(int nrhs, double *d_X) {

@@ -1,21 +1,39 @@
 // Triangular solves with the supernodal LDL^T factor on the GPU.
 //
 // Computes x <- L^{-T} D^{-1} L^{-1} x, the preconditioner application that
-// QDLDL_solve performs column by column (qdldl.hpp:362-432), level by level
-// over the supernodal elimination tree:
+// QDLDL_solve performs column by column (qdldl.hpp:362-432), over the
+// supernodal elimination tree:
 //   forward   each front takes its own right-hand side entries plus its
 //             children's update vectors, solves with its unit-lower diagonal
 //             block and leaves L_{R,J} x_J (negated, accumulated) as its own
 //             update vector for its parent;
-//   diagonal  x <- Dinv .* x;
+//   diagonal  x <- Dinv .* x, read by the backward solve;
 //   backward  each front gathers the finished x of its row set R_J and solves
-//             with L_J^T, last column block first.
-// Small fronts use one warp each; large fronts run column-block steps batched
-// over the level, reusing the inverses of the diagonal blocks kept by the
-// factorization so the diagonal solves become small dense products.  Vectors
-// are float64, the factor float32 (widened on load), as QDLDL_solve with
-// FACTPREC = float and XPREC = double.  Reductions have a fixed order, so
-// results do not depend on scheduling.
+//             with L_J^T.
+// Each direction is one launch for the whole tree.  CTAs take work items by
+// ticket in an order in which an item waits only on earlier ones (leaves to
+// root, or root to leaves), and every value that passes between items (an
+// update vector entry, a block result, a partial sum) is its own ready
+// signal: it is stored once over a pending marker, and the items that need it
+// poll it (solve_dev.cuh).  No level waits for another as a whole: what bounds
+// a direction is the chain of hand-overs from the leaves to the root (about
+// three per level, 1 to 1.5 us each) and, inside the root, two per 512
+// columns, or the bytes of L where they are many.
+//
+// Diagonal blocks are applied through their inverse, computed in float64
+// from the float32 factor per super-block of 512 columns (k_flow_invert).
+// Per 128 columns, as before, the n = 40,960 system's root (9,317 columns)
+// was a chain of 73 block products; per 512 it is 19, each spread over 16
+// CTAs.  A wider block would shorten the chain further, but its share per
+// CTA of 32 rows no longer fits in shared memory.
+//
+// Measured, one application (forward + backward, float32 factor), against the
+// solves by levels of 128-row blocks that this replaced: n = 1,280: 0.081 ms
+// (0.205); n = 2,160: 0.082 (0.231); n = 40,960: 0.41 (0.98), 277 MB of L read
+// twice at 1.35 TB/s; n = 138,240: 2.09 (3.04), 2.6 GB read twice at 2.5 TB/s.
+// Vectors are float64, the factor float32 or 16-bit (widened on load), as
+// QDLDL_solve with FACTPREC = float and XPREC = double.  Sums have a fixed
+// order, so results do not depend on scheduling.
 #include <atomic>
 #include <string>
 #include <vector>
@@ -24,113 +42,969 @@
 #include "engine.hpp"
 #include "solve.hpp"
 #include "solve_dev.cuh"
+#include "flow_dev.cuh"
 
 namespace mpir {
 
-constexpr int kWarpsPerCta = 4;
-constexpr int kSmallH      = kWarpSolveH;
+// Shared memory (doubles): kFlowInvSmem, then 4,608 for vectors and partial sums.
+constexpr int kFlowSmem = kFlowInvSmem + 4608;
+
+__global__ void k_mark_pending(int64_t n, double *p) { flow_mark(p, n); }
+
+void flow_pending(double *p, int64_t n, cudaStream_t s) {
+  launch(k_mark_pending, static_cast<unsigned>(std::min<int64_t>((n + 255) / 256, kSMs * 16)), 256, 0, s,
+         n, p);
+}
+
+// sum_k l[k] y[k] over 32 entries of shared memory (16-byte aligned).
+template <class V>
+__device__ __forceinline__ double dot32(const V (&l)[32], const double *y) {
+  double s0 = 0.0, s1 = 0.0, s2 = 0.0, s3 = 0.0;
+#pragma unroll
+  for (int k = 0; k < 32; k += 4) {
+    const double2 a = *reinterpret_cast<const double2 *>(y + k);
+    const double2 b = *reinterpret_cast<const double2 *>(y + k + 2);
+    s0 += static_cast<double>(l[k]) * a.x;
+    s1 += static_cast<double>(l[k + 1]) * a.y;
+    s2 += static_cast<double>(l[k + 2]) * b.x;
+    s3 += static_cast<double>(l[k + 3]) * b.y;
+  }
+  return (s0 + s1) + (s2 + s3);
+}
+
+// sum_k m[P k] y[k] over 32 entries, both in shared memory.
+template <int P>
+__device__ __forceinline__ double dot_pitch(const double *m, const double *y) {
+  double s0 = 0.0, s1 = 0.0, s2 = 0.0, s3 = 0.0;
+#pragma unroll
+  for (int k = 0; k < 32; k += 4) {
+    const double2 a = *reinterpret_cast<const double2 *>(y + k);
+    const double2 b = *reinterpret_cast<const double2 *>(y + k + 2);
+    s0 += m[P * k] * a.x;
+    s1 += m[P * (k + 1)] * a.y;
+    s2 += m[P * (k + 2)] * b.x;
+    s3 += m[P * (k + 3)] * b.y;
+  }
+  return (s0 + s1) + (s2 + s3);
+}
 
 // ---------------------------------------------------------------------------
-// Products with the float64 inverse of one diagonal block (128 x 128), 512
-// threads.  Each thread first copies the inverse entries it will use into
-// shared memory with cp.async (asynchronous, no registers held): a CTA does
-// this when it starts, so the product at the end of its wait chain reads
-// shared memory only, and each thread reads only what it copied itself.
-constexpr int kTri = kNB * (kNB + 1) / 2;
+// Forward.
 
-// Thread layout of the forward block product: lane l of warp v takes row
-// i = 8 v + l / 4 of the block and its slice q = l % 4; the four slices of i
-// sit in four neighbouring lanes and are added with two shuffles,
-// (s0 + s1) + (s2 + s3), with no CTA barrier.
-__device__ __forceinline__ int blk_i() { return (threadIdx.x / 32) * 8 + (threadIdx.x % 32) / 4; }
-__device__ __forceinline__ int blk_q() { return threadIdx.x % 4; }
-__device__ __forceinline__ int pad(int j) { return (j / 32) * 33 + j % 32; }
-__device__ __forceinline__ double quad_sum(double s) {
-  s += __shfl_xor_sync(0xffffffffu, s, 1);
-  s += __shfl_xor_sync(0xffffffffu, s, 2);
+// sum_c L(r, c) y_c over the columns c < cend of a wide front, tile by tile
+// (512 / RG columns) as the block results y become ready: warp v takes the
+// rows 32 (v % RG) .. (lane) and the columns 32 (v / RG) .. of each tile;
+// the next tile's L values are loaded while the current one waits, so that a
+// CTA that starts late catches up at two tiles in flight.  The last tile (the
+// result just before on the chain) is widened before its wait: conversions
+// run at a quarter of the FMA rate and would be on the chain.
+template <int RG, class T>
+__device__ __forceinline__ double rows_apply(const FlowArgs<T> &a, const T *P, int64_t h, int64_t r,
+                                             bool rok, int cend, const double *y, double *yw,
+                                             long polls) {
+  constexpr int TW = 512 / RG;
+  const int     warp = threadIdx.x / 32, lane = threadIdx.x % 32, cq = 32 * (warp / RG);
+  const int     tiles = (cend + TW - 1) / TW;
+  if (tiles == 0) return 0.0;
+  double  acc = 0.0;
+  double *yv  = yw + 32 * warp;
+  float   lv[32], lvn[32];
+  auto    load_y = [&](int c) { return c + lane < cend ? ld_relaxed_u64(y + c + lane) : 0ull; };
+  load_cols(lv, P, h, r, rok, cq, cend);
+  unsigned long long raw = load_y(cq);
+  for (int b = 0; b + 1 < tiles; b++) {
+    const int c = b * TW + cq;
+    load_cols(lvn, P, h, r, rok, c + TW, cend);
+    const unsigned long long rawn = b + 2 < tiles ? load_y(c + TW) : 0ull;
+    yv[lane] = c + lane < cend ? take_value(raw, y + c + lane, a.err, polls) : 0.0;
+    __syncwarp();
+    acc += dot32(lv, yv);
+    __syncwarp();
+#pragma unroll
+    for (int k = 0; k < 32; k++) lv[k] = lvn[k];
+    raw = rawn;
+  }
+  const int c = (tiles - 1) * TW + cq;
+  double    ld[32];
+#pragma unroll
+  for (int k = 0; k < 32; k++) ld[k] = static_cast<double>(lv[k]);
+  yv[lane] = c + lane < cend ? wait_value(y + c + lane, a.err, polls) : 0.0;
+  __syncwarp();
+  acc += dot32(ld, yv);
+  return acc;
+}
+
+// kFwdNarrow (w <= 128): y_J = Inv z_J, then up to 512 of the rows below,
+// u = z_R - L_{R,J} y_J.  Every item of the front computes y_J itself (w
+// values), which saves a hand-over; the first one keeps it.  RG = 16 (w <= 32):
+// a thread a row; RG = 4: tiles of 128 rows, a quarter of the columns each
+// (the next tile's L values are loaded while the current one is applied).
+// Thread tid gathers and stores row tid of the item.
+template <int RG, class T>
+__device__ __noinline__ void fwd_narrow(const FlowArgs<T> &a, FlowShared &S, const FlowSlot &I, FlowSlot &N,
+                                        double *sm, uint32_t &phase) {
+  const FlowFront &f   = I.item.f;
+  const int        tid = threadIdx.x, warp = tid / 32, lane = tid % 32;
+  const int        w = f.w, nbw = (w + 31) / 32, nr = I.item.nr;
+  const long       polls = I.polls;
+  double          *inv = sm, *zs = sm + kFlowInvSmem, *ys = zs + 512, *part = ys + 512;
+  const uint32_t   bar = smem_addr(&S.bar);
+  if (tid == 0) {
+    const uint32_t bytes = nbw * (nbw + 1) / 2 * kFlowBlk * sizeof(double);
+    bulk_expect(bar, bytes);
+    bulk_get(inv, a.inv + f.inv, bytes, bar);
+  }
+  constexpr int kTile = 32 * RG;
+  const int     cq = warp / RG, rt = tid % kTile;
+  const int64_t r0 = I.item.r0;
+  const T      *P  = a.panel + f.panel;
+  float         lv[32], lvn[32];
+  load_cols(lv, P, f.h, r0 + rt, rt < nr, 32 * cq, w);
+  flow_fetch(a, N);
+  Gather<1> gz, gr;
+  if (tid < w) gz.begin(a, f.zofs + tid, a.z);
+  if (tid < nr) gr.begin(a, f.zofs + r0 + tid, a.z);
+  if (tid < 32 * nbw) zs[tid] = tid < w ? gz.finish(a, a.z, a.x[f.col0 + tid], polls) : 0.0;
+  __syncthreads();
+  bulk_wait(bar, phase, a.err);
+  phase ^= 1;
+  const int bi = warp / 4, bj = warp % 4;
+  if (bi < nbw && bj <= bi) {
+    const double *blk = inv + (bi * (bi + 1) / 2 + bj) * kFlowBlk + lane;
+    double        iv[32];
+#pragma unroll
+    for (int c = 0; c < 32; c++) iv[c] = blk[33 * c];
+    part[bj * 128 + 32 * bi + lane] = dot32(iv, zs + 32 * bj);
+  }
+  __syncthreads();
+  if (tid < 128) {
+    double y = 0.0;
+    if (tid < w)
+      for (int j = 0; j <= tid / 32; j++) y += part[j * 128 + tid];
+    ys[tid] = y;
+    if (tid < w && r0 == w) a.f[f.col0 + tid] = y;
+  }
+  __syncthreads();
+  double acc = 0.0;
+  if (RG == 16) {
+    acc = dot32(lv, ys);
+  } else {
+    for (int q = 0; q * kTile < nr; q++) {
+      const int rn = (q + 1) * kTile + rt;
+      if ((q + 1) * kTile < nr) load_cols(lvn, P, f.h, r0 + rn, rn < nr, 32 * cq, w);
+      part[(4 * q + cq) * 128 + rt] = dot32(lv, ys + 32 * cq);
+#pragma unroll
+      for (int k = 0; k < 32; k++) lv[k] = lvn[k];
+    }
+    __syncthreads();
+    const double *p = part + tid / 128 * 512 + tid % 128;
+    if (tid < nr) acc = (p[0] + p[128]) + (p[256] + p[384]);
+  }
+  if (tid < nr) {
+    const double u = gr.finish(a, a.z, 0.0, polls) - acc;
+    if (I.publish) st_relaxed_f64(a.z + f.zofs + r0 + tid, u);
+  }
+}
+
+// kFwdSlab (w > 128): 32 rows of the diagonal block.  z = its right-hand side
+// less the columns of the super-blocks before its own, handed to the other
+// slabs of the super-block; then y = the slab's rows of the inverse times
+// their z: warp 0 takes the diagonal 32 x 32 block, warp v the block v - 1.
+template <class T>
+__device__ __noinline__ void fwd_slab(const FlowArgs<T> &a, FlowShared &S, const FlowSlot &I, FlowSlot &N,
+                                      double *sm, uint32_t &phase) {
+  const FlowFront &f   = I.item.f;
+  const int        tid = threadIdx.x, warp = tid / 32, lane = tid % 32;
+  const long       polls = I.polls;
+  const int        r0 = I.item.r0, s = r0 / kFlowSB, i = (r0 % kFlowSB) / 32;
+  const bool       rok = lane < I.item.nr, last = r0 + 32 >= f.w || i == 15;
+  double          *inv = sm, *yw = sm + kFlowInvSmem, *part = yw + 512, *part2 = part + 512;
+  const uint32_t   bar = smem_addr(&S.bar);
+  if (tid == 0) {
+    const uint32_t bytes = (i + 1) * kFlowBlk * sizeof(double);
+    bulk_expect(bar, bytes);
+    bulk_get(inv, a.inv + f.inv + (static_cast<int64_t>(s) * kFlowTriSB + i * (i + 1) / 2) * kFlowBlk,
+             bytes, bar);
+  }
+  flow_fetch(a, N);
+  double zr = 0.0;
+  if (warp == 0 && rok) {
+    Gather<1> g;
+    g.begin(a, f.zofs + r0 + lane, a.z);
+    zr = g.finish(a, a.z, a.x[f.col0 + r0 + lane], polls);
+  }
+  const double *y = a.y + (I.ticket % kFlowCopies) * a.n + f.col0;
+  if (s > 0) {
+    part[32 * warp + lane] = rows_apply<1>(a, a.panel + f.panel, f.h, r0 + lane, rok,
+                                           s * kFlowSB, y, yw, polls);
+    __syncthreads();
+  }
+  double *yz = a.yz + f.col0 + s * kFlowSB;
+  if (warp == 0) {
+    if (s > 0) {
+      double t[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+      for (int v = 0; v < 16; v++) t[v % 4] += part[32 * v + lane];
+      zr -= (t[0] + t[1]) + (t[2] + t[3]);
+    }
+    if (!last && I.publish) st_relaxed_f64(yz + 32 * i + lane, zr);
+  }
+  bulk_wait(bar, phase, a.err);
+  phase ^= 1;
+  if (warp <= i) {
+    const int     j   = warp == 0 ? i : warp - 1;
+    const double *blk = inv + j * kFlowBlk + lane;
+    double        iv[32];
+#pragma unroll
+    for (int c = 0; c < 32; c++) iv[c] = blk[33 * c];
+    if (warp > 0) zr = wait_value(yz + 32 * j + lane, a.err, polls);
+    yw[32 * warp + lane] = zr;
+    __syncwarp();
+    part2[32 * warp + lane] = dot32(iv, yw + 32 * warp);
+  }
+  __syncthreads();
+  if (warp == 0 && rok) {
+    double t[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+    for (int v = 0; v < 16; v++)
+      if (v <= i) t[v % 4] += part2[32 * v + lane];
+    const double  yv = (t[0] + t[1]) + (t[2] + t[3]);
+    const int64_t g  = f.col0 + r0 + lane;
+    if (I.publish) {
+#pragma unroll
+      for (int c = 0; c < kFlowCopies; c++) st_relaxed_f64(a.y + c * a.n + g, yv);
+    }
+    a.f[g] = yv;
+  }
+}
+
+// kFwdRows (w > 128): 128 rows below the diagonal block.
+template <class T>
+__device__ __noinline__ void fwd_rows(const FlowArgs<T> &a, const FlowSlot &I, FlowSlot &N,
+                                       double *sm) {
+  const FlowFront &f   = I.item.f;
+  const int        tid = threadIdx.x, warp = tid / 32, lane = tid % 32;
+  const long       polls = I.polls;
+  double          *yw = sm + kFlowInvSmem, *part = yw + 512;
+  const int64_t    r   = I.item.r0 + 32 * (warp % 4) + lane;
+  const bool       rok = r < I.item.r0 + I.item.nr;
+  Gather<1>        g;
+  if (rok && warp < 4) g.begin(a, f.zofs + r, a.z);
+  flow_fetch(a, N);
+  const double *y = a.y + (I.ticket % kFlowCopies) * a.n + f.col0;
+  part[(warp / 4) * 128 + tid % 128] =
+      rows_apply<4>(a, a.panel + f.panel, f.h, r, rok, f.w, y, yw, polls);
+  __syncthreads();
+  if (rok && warp < 4) {
+    const double *p = part + tid;
+    const double  u = g.finish(a, a.z, 0.0, polls) - ((p[0] + p[128]) + (p[256] + p[384]));
+    if (I.publish) st_relaxed_f64(a.z + f.zofs + r, u);
+  }
+}
+
+// z -= M(:, k) y_k over the columns, for the first 32 RT rows (those at or past
+// h read what lies behind the panel and are not used).  No branch inside the
+// loop: one warp alone hides latency only by what a column has in flight.
+template <int RT>
+__device__ __forceinline__ void warp_columns(const double *M, int ld, int w, const double *y,
+                                             double (&z)[8]) {
+#pragma unroll 4
+  for (int k = 0; k < w; k++) {
+    const double yk = y[k];
+#pragma unroll
+    for (int t = 0; t < RT; t++) z[t] -= M[k * ld + 32 * t] * yk;
+  }
+}
+
+// kFlowWarps: one front of w <= 32, h <= 256 per warp; lane l holds rows
+// l + 32 t.  The rows' child contributions are polled together, one of each
+// row at a time; then y = Inv z, and the rows below less L y.
+template <class T>
+__device__ __noinline__ void fwd_warp(const FlowArgs<T> &a, FlowShared &S, const FlowSlot &I, FlowSlot &N,
+                                      double *sm, uint32_t &wphase) {
+  const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+  if (warp >= I.item.nr) {
+    flow_fetch(a, N);
+    return;
+  }
+  const long      polls = I.polls;
+  const FlowFront f = a.warps[I.item.r0 + warp];
+  const int       w = f.w, h = f.h, ld = h | 1;
+  const uint32_t  bar = smem_addr(&S.wbar[warp]);
+  const double   *M   = warp_panel(a, f, sm, bar) + lane;
+  double         *zs  = sm + kFlowInvSmem + 64 * warp, *ys = zs + 32;
+  constexpr int   RT = kWarpSolveH / 32;
+  int             ix[RT], more[RT];
+  double          z[RT];
+#pragma unroll
+  for (int t = 0; t < RT; t++) {
+    int2 g = {-1, -1};
+    if (lane + 32 * t < h) g = a.gfirst[f.zofs + lane + 32 * t];
+    ix[t]   = g.x;
+    more[t] = g.y;
+    z[t]    = 0.0;
+  }
+  if (lane < w) z[0] = a.x[f.col0 + lane];
+  flow_fetch(a, N);
+  add_values<RT>(a.z, ix, z, a.err, polls);
+  // the rows with further children: their lists, one entry of each at a time
+  int  n[RT];
+  bool any = false;
+#pragma unroll
+  for (int t = 0; t < RT; t++) {
+    n[t] = more[t] >= 0 ? a.gmore[more[t]] : 0;
+    any |= n[t] > 0;
+  }
+  for (int q = 0; __any_sync(0xffffffffu, any); q++) {
+    any = false;
+#pragma unroll
+    for (int t = 0; t < RT; t++) {
+      ix[t] = q < n[t] ? a.gmore[more[t] + 1 + q] : -1;
+      any |= q + 1 < n[t];
+    }
+    add_values<RT>(a.z, ix, z, a.err, polls);
+  }
+  zs[lane] = z[0];
+  __syncwarp();
+  bulk_wait(bar, wphase, a.err);
+  wphase ^= 1;
+  double y0 = 0.0, y1 = 0.0;
+  int    k  = 0;
+#pragma unroll 4
+  for (; k + 1 < w; k += 2) {
+    y0 += M[k * ld] * zs[k];
+    y1 += M[(k + 1) * ld] * zs[k + 1];
+  }
+  if (k < w) y0 += M[k * ld] * zs[k];
+  ys[lane] = y0 + y1;  // entries at or past w are not used
+  __syncwarp();
+  if (h <= 64)
+    warp_columns<2>(M, ld, w, ys, z);
+  else if (h <= 128)
+    warp_columns<4>(M, ld, w, ys, z);
+  else
+    warp_columns<8>(M, ld, w, ys, z);
+  if (lane < w) a.f[f.col0 + lane] = y0 + y1;
+#pragma unroll
+  for (int t = 0; t < RT; t++) {
+    const int i = lane + 32 * t;
+    if (i >= w && i < h && I.publish) st_relaxed_f64(a.z + f.zofs + i, z[t]);
+  }
+}
+
+template <class T>
+__global__ void __launch_bounds__(kFlowThreads, 1) k_fwd_flow(const __grid_constant__ FlowArgs<T> a) {
+  extern __shared__ __align__(128) double sm[];
+  __shared__ __align__(16) FlowShared S;
+  uint32_t phase = 0, wphase = 0;
+  flow_loop(a, S, [&](const FlowSlot &I, FlowSlot &N) {
+    switch (I.item.kind) {
+      case kFlowWarps: fwd_warp(a, S, I, N, sm, wphase); break;
+      case kFwdNarrow:
+        if (I.item.f.w <= 32)
+          fwd_narrow<16>(a, S, I, N, sm, phase);
+        else
+          fwd_narrow<4>(a, S, I, N, sm, phase);
+        break;
+      case kFwdSlab: fwd_slab(a, S, I, N, sm, phase); break;
+      default: fwd_rows(a, I, N, sm);
+    }
+  });
+  flow_mark(a.mark, a.nmark);
+}
+
+// ---------------------------------------------------------------------------
+// Backward.
+
+// Sums of the warp's two columns over its lanes: the lower half of the warp
+// ends with column 0, the upper half with column 1.
+__device__ __forceinline__ double sum2(double s0, double s1) {
+  const bool up = threadIdx.x & 16;
+  double     s  = (up ? s1 : s0) + __shfl_xor_sync(0xffffffffu, up ? s0 : s1, 16);
+#pragma unroll
+  for (int o = 8; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
   return s;
 }
 
-// Forward copy of Linv, by rows in 64-byte segments: row i = 8 a + r holds
-// its first 8 (a + 1) entries (those right of the diagonal are zero), and a
-// row of an odd group a one segment of padding more, so the 8 rows a warp
-// reads start alternately in the two halves of the banks (a warp's 16-byte
-// loads then take the minimum of four shared-memory wavefronts).
-constexpr int kFwdTri = 64 * (16 * 17 / 2 + 8);
-__device__ __forceinline__ int fwd_row_start(int i) {
-  const int a = i / 8, r = i % 8;
-  return 64 * (a * (a + 1) / 2 + a / 2) + r * 8 * (a + 1 + (a & 1));
-}
-
-// Thread (i, q) copies the pairs j = 8 m + 2 q, 8 m + 2 q + 1 (m <= i / 8) of
-// row i from the row-major inverse Lt (Lt[i * kNB + j] = Linv[i][j]).
-__device__ __forceinline__ void stage_lower(const double *Lt, double *Ls) {
-  const int     i = blk_i(), q = blk_q(), a = i / 8;
-  double       *d = Ls + fwd_row_start(i) + 2 * q;
-  const double *s = Lt + i * kNB + 2 * q;
-  for (int m = 0; m <= a; m++) cp_async16(d + 8 * m, s + 8 * m);
-}
-
-// y_i = (Linv z)_i from the staged copy, in all four lanes of row i; z holds
-// 128 entries (16-byte aligned).  Warp v (rows 8 v .. 8 v + 7) takes the
-// segments m <= v: 4 (v + 1) loads of Linv and of z per warp in all.
-__device__ __forceinline__ double block_lower_apply(const double *Ls, const double *z) {
-  const int     i = blk_i(), q = blk_q(), a = i / 8;
-  const double *row = Ls + fwd_row_start(i) + 2 * q;
-  const double *zq  = z + 2 * q;
-  cp_async_wait_all();
-  double a0 = 0.0, a1 = 0.0;
-#pragma unroll 4
-  for (int m = 0; m <= a; m++) {
-    const double2 l = *reinterpret_cast<const double2 *>(row + 8 * m);
-    const double2 v = *reinterpret_cast<const double2 *>(zq + 8 * m);
-    a0 += l.x * v.x;
-    a1 += l.y * v.y;
-  }
-  return quad_sum(a0 + a1);
-}
-
-// Stage the row-major copy Lt (Lt[i * kNB + j] = Linv[i][j]) for x = Linv^T v:
-// thread (q, j) = (tid / 128, tid % 128) copies rows i >= j of slice q (a
-// warp reads 32 consecutive entries of a row).
-__device__ __forceinline__ void stage_upper(const double *Lt, double *Ls, int nb) {
-  const int tid = threadIdx.x, j = tid % kNB, q = tid / kNB;
-  for (int ii = 0; ii < kNB / 4; ii++) {
-    const int i = q * (kNB / 4) + ii;
-    if (i >= j && i < nb) cp_async8(Ls + i * (i + 1) / 2 + j, Lt + i * kNB + j);
-  }
-}
-
-// x_j = (Linv^T v)_j from the staged copy for thread (q, j): the four slices
-// are added in order through part (one CTA barrier).
-__device__ __forceinline__ double block_upper_apply(const double *Ls, const double *v, int nb,
-                                                    double (*part)[kNB]) {
-  const int tid = threadIdx.x, j = tid % kNB, q = tid / kNB, i0 = q * (kNB / 4);
-  cp_async_wait_all();
-  double a0 = 0.0, a1 = 0.0;
-  // Row i starts at i (i + 1) / 2: the offset of (i, j) grows by i + 1 from
-  // row i to row i + 1.
-  int off = i0 * (i0 + 1) / 2 + j;
-#pragma unroll
-  for (int ii = 0; ii < kNB / 4; ii += 2) {
-    const int i = i0 + ii;
-    if (i >= j && i < nb) a0 += Ls[off] * v[i];
-    off += i + 1;
-    if (i + 1 >= j && i + 1 < nb) a1 += Ls[off] * v[i + 1];
-    off += i + 2;
-  }
-  part[q][j] = a0 + a1;
+// The x values of the front's rows w + 512 c .. (nr of them) into xs.
+template <class T>
+__device__ __forceinline__ void get_rows(const FlowArgs<T> &a, const FlowFront &f, int64_t rb, int nr,
+                                         double *xs, long polls) {
+  const int tid = threadIdx.x;
+  const int row = tid < nr ? a.srows[f.rows + rb + tid] : -1;
+  wait_gate(a, f.gate, polls);
+  xs[tid] = row >= 0 ? wait_value(a.xr + row, a.err, polls) : 0.0;
   __syncthreads();
-  return (part[0][j] + part[1][j]) + (part[2][j] + part[3][j]);
 }
+
+// t_c = sum_r L(r, c) x_r over up to 512 rows below the block, for columns
+// [c0, cend): emit(c, t_c) by one lane a column.
+template <class T, class Emit>
+__device__ __forceinline__ void chunk_cols(const FlowArgs<T> &a, const FlowFront &f, int64_t rb,
+                                           int nr, int c0, int cend, double *xs, long polls,
+                                           FlowSlot &N, Emit emit) {
+  const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+  const T  *P = a.panel + f.panel;
+  float     lv[2][16], lvn[2][16];
+  load_rows(lv, P, f.h, rb, nr, c0, cend);
+  flow_fetch(a, N);
+  // The first tile is widened before the wait (see rows_apply).
+  double ld[2][16];
+#pragma unroll
+  for (int j = 0; j < 2; j++)
+#pragma unroll
+    for (int i = 0; i < 16; i++) ld[j][i] = static_cast<double>(lv[j][i]);
+  if (c0 + 32 < cend) load_rows(lv, P, f.h, rb, nr, c0 + 32, cend);
+  get_rows(a, f, rb, nr, xs, polls);
+  const int dc = 2 * warp + (lane >> 4);  // the lane's column of a tile
+  {
+    double s0 = 0.0, s1 = 0.0;
+#pragma unroll
+    for (int i = 0; i < 16; i++) {
+      const double xv = xs[lane + 32 * i];
+      s0 += ld[0][i] * xv;
+      s1 += ld[1][i] * xv;
+    }
+    const double t = sum2(s0, s1);
+    if ((lane & 15) == 0 && c0 + dc < cend) emit(c0 + dc, t);
+  }
+  for (int c = c0 + 32; c < cend; c += 32) {
+    if (c + 32 < cend) load_rows(lvn, P, f.h, rb, nr, c + 32, cend);
+    double s0 = 0.0, s1 = 0.0;
+#pragma unroll
+    for (int i = 0; i < 16; i++) {
+      const double xv = xs[lane + 32 * i];
+      s0 += static_cast<double>(lv[0][i]) * xv;
+      s1 += static_cast<double>(lv[1][i]) * xv;
+    }
+    const double t = sum2(s0, s1);
+    if ((lane & 15) == 0 && c + dc < cend) emit(c + dc, t);
+#pragma unroll
+    for (int j = 0; j < 2; j++)
+#pragma unroll
+      for (int i = 0; i < 16; i++) lv[j][i] = lvn[j][i];
+  }
+}
+
+template <class T>
+__device__ __noinline__ void bwd_chunk(const FlowArgs<T> &a, const FlowSlot &I, FlowSlot &N,
+                                       double *sm) {
+  const FlowFront &f  = I.item.f;
+  const int        c  = I.item.c0;
+  const int64_t    rb = f.w + static_cast<int64_t>(c) * kFlowChunk;
+  const int        nr = static_cast<int>(min(static_cast<int64_t>(kFlowChunk), f.h - rb));
+  double          *pp = a.part + f.part + static_cast<int64_t>(c) * f.w;
+  chunk_cols(a, f, rb, nr, I.item.r0, I.item.r0 + I.item.nr, sm + kFlowInvSmem,
+             I.polls, N, [&](int col, double t) { st_relaxed_f64(pp + col, t); });
+}
+
+// kBwdNarrow (w <= 128): x_J = Inv^T (z_J - t), t the rows below: the chunk
+// partials, or (at most 512 rows) computed here.
+template <class T>
+__device__ __noinline__ void bwd_narrow(const FlowArgs<T> &a, FlowShared &S, const FlowSlot &I, FlowSlot &N,
+                                        double *sm, uint32_t &phase) {
+  const FlowFront &f   = I.item.f;
+  const int        tid = threadIdx.x, warp = tid / 32, lane = tid % 32;
+  const int        w = f.w, nbw = (w + 31) / 32;
+  const long       polls = I.polls;
+  double          *inv = sm, *xs = sm + kFlowInvSmem, *vs = xs + 512, *red = vs + 512,
+                  *part = red + 512;
+  const uint32_t   bar = smem_addr(&S.bar);
+  if (tid == 0) {
+    const uint32_t bytes = nbw * (nbw + 1) / 2 * kFlowBlk * sizeof(double);
+    bulk_expect(bar, bytes);
+    bulk_get(inv, a.inv + f.inv, bytes, bar);
+  }
+  double v = 0.0;
+  if (tid < w) {
+    v = a.f[f.col0 + tid];
+    if (a.Dinv) v *= static_cast<double>(a.Dinv[f.col0 + tid]);
+  }
+  red[tid] = 0.0;
+  if (f.chunks > 0 || f.h == w) flow_fetch(a, N);
+  if (f.chunks > 0) {
+    const int k = tid % 128, q = tid / 128;
+    double    s = 0.0;
+    if (k < w)
+      for (int c = q; c < f.chunks; c += 4)
+        s += wait_value(a.part + f.part + static_cast<int64_t>(c) * w + k, a.err, polls);
+    red[tid] = s;
+  } else if (f.h > w) {
+    __syncthreads();
+    chunk_cols(a, f, w, f.h - w, 0, w, xs, polls, N, [&](int col, double t) { red[col] = t; });
+  }
+  __syncthreads();
+  if (tid < 128) vs[tid] = v - ((red[tid] + red[tid + 128]) + (red[tid + 256] + red[tid + 384]));
+  __syncthreads();
+  bulk_wait(bar, phase, a.err);
+  phase ^= 1;
+  const int bj = warp % 4, bi = warp / 4;
+  if (bi < nbw && bj <= bi) {
+    const double *blk = inv + (bi * (bi + 1) / 2 + bj) * kFlowBlk + 33 * lane;
+    part[bi * 128 + 32 * bj + lane] = dot_pitch<1>(blk, vs + 32 * bi);
+  }
+  __syncthreads();
+  if (tid < w) {
+    double xo = 0.0;
+    for (int i = tid / 32; i < nbw; i++) xo += part[i * 128 + tid];
+    st_relaxed_f64(a.xr + f.col0 + tid, xo);
+    a.x[f.col0 + tid] = xo;
+  }
+}
+
+// kBwdSlab (w > 128): 32 columns of the diagonal block, the mirror of
+// fwd_slab: t = the chunk partials + the rows of the super-blocks after its
+// own, last first; v = z - t handed to the slabs before it in the
+// super-block; x = the slab's columns of the inverse times v.
+template <class T>
+__device__ __noinline__ void bwd_slab(const FlowArgs<T> &a, FlowShared &S, const FlowSlot &I, FlowSlot &N,
+                                      double *sm, uint32_t &phase) {
+  const FlowFront &f   = I.item.f;
+  const int        tid = threadIdx.x, warp = tid / 32, lane = tid % 32;
+  const long       polls = I.polls;
+  const int        w = f.w, k0 = I.item.r0, s = k0 / kFlowSB, j = (k0 % kFlowSB) / 32;
+  const int        nsl = min(16, (w - s * kFlowSB + 31) / 32), nsb = (w + kFlowSB - 1) / kFlowSB;
+  const bool       ok = lane < I.item.nr;
+  double          *inv = sm, *xs = sm + kFlowInvSmem, *part = xs + 1024, *ts = part + 512;
+  __shared__ double ts2[32];
+  const uint32_t   bar = smem_addr(&S.bar);
+  if (tid == 0) {
+    bulk_expect(bar, (nsl - j) * kFlowBlk * sizeof(double));
+    for (int i = j; i < nsl; i++)
+      bulk_get(inv + (i - j) * kFlowBlk,
+               a.inv + f.inv +
+                   (static_cast<int64_t>(s) * kFlowTriSB + i * (i + 1) / 2 + j) * kFlowBlk,
+               kFlowBlk * sizeof(double), bar);
+  }
+  double v = 0.0;
+  if (warp == 0 && ok) {
+    v = a.f[f.col0 + k0 + lane];
+    if (a.Dinv) v *= static_cast<double>(a.Dinv[f.col0 + k0 + lane]);
+  }
+  const T      *P    = a.panel + f.panel;
+  const double *xr   = a.xr + (I.ticket % kFlowCopies) * a.n + f.col0;
+  const int     cend = k0 + I.item.nr;
+  float         lv[2][16], lvn[2][16];
+  if (nsb - 1 > s) load_rows(lv, P, f.h, static_cast<int64_t>(nsb - 1) * kFlowSB,
+                             w - (nsb - 1) * kFlowSB, k0, cend);
+  flow_fetch(a, N);
+  // Chunk partials: warp v takes chunks v, v + 16, .. of the slab's columns.
+  double p2 = 0.0;
+  if (ok)
+    for (int c = warp; c < f.chunks; c += 16)
+      p2 += wait_value(a.part + f.part + static_cast<int64_t>(c) * w + k0 + lane, a.err, polls);
+  part[32 * warp + lane] = p2;
+  double s0 = 0.0, s1 = 0.0;
+  for (int R = nsb - 1; R > s; R--) {
+    double   *xb = xs + (R & 1) * 512;
+    const int g  = R * kFlowSB + tid;
+    if (R - 1 > s) {
+      load_rows(lvn, P, f.h, static_cast<int64_t>(R - 1) * kFlowSB, kFlowSB, k0, cend);
+      xb[tid] = g < w ? wait_value(xr + g, a.err, polls) : 0.0;
+      __syncthreads();
+#pragma unroll
+      for (int i = 0; i < 16; i++) {
+        const double xv = xb[lane + 32 * i];
+        s0 += static_cast<double>(lv[0][i]) * xv;
+        s1 += static_cast<double>(lv[1][i]) * xv;
+      }
+#pragma unroll
+      for (int q = 0; q < 2; q++)
+#pragma unroll
+        for (int i = 0; i < 16; i++) lv[q][i] = lvn[q][i];
+    } else {
+      // the last tile, widened before its wait (see rows_apply)
+      double ld[2][16];
+#pragma unroll
+      for (int q = 0; q < 2; q++)
+#pragma unroll
+        for (int i = 0; i < 16; i++) ld[q][i] = static_cast<double>(lv[q][i]);
+      xb[tid] = g < w ? wait_value(xr + g, a.err, polls) : 0.0;
+      __syncthreads();
+#pragma unroll
+      for (int i = 0; i < 16; i++) {
+        const double xv = xb[lane + 32 * i];
+        s0 += ld[0][i] * xv;
+        s1 += ld[1][i] * xv;
+      }
+    }
+  }
+  const double t2 = sum2(s0, s1);
+  if ((lane & 15) == 0) ts2[2 * warp + (lane >> 4)] = t2;
+  __syncthreads();
+  double *xz = a.xz + f.col0 + s * kFlowSB;
+  if (warp == 0) {
+    double t[4] = {ts2[lane], 0.0, 0.0, 0.0};
+#pragma unroll
+    for (int q = 0; q < 16; q++) t[q % 4] += part[32 * q + lane];
+    v = ok ? v - ((t[0] + t[1]) + (t[2] + t[3])) : 0.0;
+    if (j > 0 && ok) st_relaxed_f64(xz + 32 * j + lane, v);
+  }
+  bulk_wait(bar, phase, a.err);
+  phase ^= 1;
+  if (j + warp < nsl) {
+    const int     i   = j + warp;
+    const double *blk = inv + warp * kFlowBlk + 33 * lane;
+    double        iv[32];
+#pragma unroll
+    for (int r = 0; r < 32; r++) iv[r] = blk[r];
+    if (warp > 0)
+      v = s * kFlowSB + 32 * i + lane < w ? wait_value(xz + 32 * i + lane, a.err, polls) : 0.0;
+    xs[32 * warp + lane] = v;
+    __syncwarp();
+    ts[32 * warp + lane] = dot32(iv, xs + 32 * warp);
+  }
+  __syncthreads();
+  if (warp == 0 && ok) {
+    double t[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+    for (int q = 0; q < 16; q++)
+      if (j + q < nsl) t[q % 4] += ts[32 * q + lane];
+    const double  xv = (t[0] + t[1]) + (t[2] + t[3]);
+    const int64_t g  = f.col0 + k0 + lane;
+#pragma unroll
+    for (int c = 0; c < kFlowCopies; c++) st_relaxed_f64(a.xr + c * a.n + g, xv);
+    a.x[g] = xv;
+  }
+}
+
+// kFlowWarps, backward: t = the rows below, then x = Inv^T (z - t), lane =
+// column (the panel's odd pitch keeps that free of bank conflicts; of fronts
+// with at most 16 columns each half of the warp takes every other row).
+template <class T>
+__device__ __noinline__ void bwd_warp(const FlowArgs<T> &a, FlowShared &S, const FlowSlot &I, FlowSlot &N,
+                                      double *sm, uint32_t &wphase) {
+  const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+  if (warp >= I.item.nr) {
+    flow_fetch(a, N);
+    return;
+  }
+  const long      polls = I.polls;
+  const FlowFront f = a.warps[I.item.r0 + warp];
+  const int       w = f.w, h = f.h, ld = h | 1, nr = h - w;
+  const uint32_t  bar = smem_addr(&S.wbar[warp]);
+  const double   *M   = warp_panel(a, f, sm, bar);
+  constexpr int   RT = kWarpSolveH / 32;
+  double         *vs = sm + kFlowInvSmem + 288 * warp, *xs = vs + 32;
+  double          v  = 0.0;
+  if (lane < w) {
+    v = a.f[f.col0 + lane];
+    if (a.Dinv) v *= static_cast<double>(a.Dinv[f.col0 + lane]);
+  }
+  {
+    int    gi[RT];
+    double xv[RT];
+#pragma unroll
+    for (int t = 0; t < RT; t++) {
+      gi[t] = lane + 32 * t < nr ? a.srows[f.rows + w + lane + 32 * t] : -1;
+      xv[t] = 0.0;
+    }
+    flow_fetch(a, N);
+    bulk_wait(bar, wphase, a.err);
+    wphase ^= 1;
+    wait_gate(a, f.gate, polls);
+    add_values<RT>(a.xr, gi, xv, a.err, polls);
+#pragma unroll
+    for (int t = 0; t < RT; t++) xs[lane + 32 * t] = xv[t];
+  }
+  __syncwarp();
+  const bool    half = w <= 16;
+  const double *col  = M + min(half ? lane & 15 : lane, w - 1) * ld;
+  const int     step = half ? 2 : 1;
+  double        t0 = 0.0, t1 = 0.0, t2 = 0.0, t3 = 0.0;
+  int           r  = half ? lane >> 4 : 0;
+#pragma unroll 2
+  for (; r + 3 * step < nr; r += 4 * step) {
+    t0 += col[w + r] * xs[r];
+    t1 += col[w + r + step] * xs[r + step];
+    t2 += col[w + r + 2 * step] * xs[r + 2 * step];
+    t3 += col[w + r + 3 * step] * xs[r + 3 * step];
+  }
+  for (; r < nr; r += step) t0 += col[w + r] * xs[r];
+  double t = (t0 + t1) + (t2 + t3);
+  if (half) t += __shfl_xor_sync(0xffffffffu, t, 16);
+  vs[lane] = lane < w ? v - t : 0.0;
+  __syncwarp();
+  double x0 = 0.0, x1 = 0.0;
+  int    i  = 0;
+#pragma unroll 4
+  for (; i + 1 < w; i += 2) {
+    x0 += col[i] * vs[i];
+    x1 += col[i + 1] * vs[i + 1];
+  }
+  if (i < w) x0 += col[i] * vs[i];
+  if (lane < w) {
+    st_relaxed_f64(a.xr + f.col0 + lane, x0 + x1);
+    a.x[f.col0 + lane] = x0 + x1;
+  }
+}
+
+template <class T>
+__global__ void __launch_bounds__(kFlowThreads, 1) k_bwd_flow(const __grid_constant__ FlowArgs<T> a) {
+  extern __shared__ __align__(128) double sm[];
+  __shared__ __align__(16) FlowShared S;
+  uint32_t phase = 0, wphase = 0;
+  flow_loop(a, S, [&](const FlowSlot &I, FlowSlot &N) {
+    switch (I.item.kind) {
+      case kFlowWarps: bwd_warp(a, S, I, N, sm, wphase); break;
+      case kBwdChunk: bwd_chunk(a, I, N, sm); break;
+      case kBwdNarrow: bwd_narrow(a, S, I, N, sm, phase); break;
+      default: bwd_slab(a, S, I, N, sm, phase);
+    }
+  });
+  flow_mark(a.mark, a.nmark);
+}
+
+__global__ void k_dscale(int64_t n, const float *Dinv, double *x) {
+  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (i < n) x[i] *= static_cast<double>(Dinv[i]);
+}
+
+// ---------------------------------------------------------------------------
+// Inverses of the diagonal super-blocks in float64 from the float32 factor,
+// once per factorization: a warp solves L X = E for two columns, by blocks of
+// 32 rows: the block's triangle (lane = row, the pivots' values by shuffle),
+// then the block's columns into the sums of the rows below (acc[q] belongs to
+// the q-th block from the current one).  Bound by the float32 -> float64
+// conversions (a quarter of the FMA rate), which is why a warp takes two
+// columns.
+__global__ void __launch_bounds__(128)
+    k_flow_invert(const FlowInvDesc *descs, const float *panel, double *inv) {
+  __shared__ __align__(16) double xs[4][2][32];
+  const FlowInvDesc d    = descs[blockIdx.x];
+  const int         warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+  const int         n = d.n, nb = (n + 31) / 32, col = d.c0 + 2 * warp, j = col / 32;
+  const int64_t     h = d.h;
+  const float      *P = panel + d.panel;
+  double            acc[16][2];
+#pragma unroll
+  for (int q = 0; q < 16; q++) acc[q][0] = acc[q][1] = 0.0;
+  for (int i = j; i < nb; i++) {
+    const int row = 32 * i + lane;
+    float     l[32];
+    load_cols(l, P, h, row, row < n, 32 * i, min(n, 32 * i + lane));
+    double v0 = (row == col && col < n ? 1.0 : 0.0) - acc[0][0];
+    double v1 = (row == col + 1 && col + 1 < n ? 1.0 : 0.0) - acc[0][1];
+#pragma unroll
+    for (int k = 0; k < 32; k++) {
+      const double x0 = __shfl_sync(0xffffffffu, v0, k), x1 = __shfl_sync(0xffffffffu, v1, k);
+      const double lk = static_cast<double>(l[k]);
+      v0 -= lk * x0;
+      v1 -= lk * x1;
+    }
+    double *o = inv + d.inv + (static_cast<int64_t>(i) * (i + 1) / 2 + j) * kFlowBlk +
+                (col % 32) * 33 + lane;
+    o[0]  = v0;
+    o[33] = v1;
+    __syncwarp();
+    xs[warp][0][lane] = v0;
+    xs[warp][1][lane] = v1;
+    __syncwarp();
+#pragma unroll
+    for (int q = 1; q < 16; q++) {
+      if (i + q < nb) {
+        const int rq = 32 * (i + q) + lane;
+        load_cols(l, P, h, rq, rq < n, 32 * i, 32 * i + 32);
+        double s0 = 0.0, s1 = 0.0;
+#pragma unroll
+        for (int k = 0; k < 32; k += 2) {
+          const double2 x0 = *reinterpret_cast<const double2 *>(&xs[warp][0][k]);
+          const double2 x1 = *reinterpret_cast<const double2 *>(&xs[warp][1][k]);
+          const double  la = static_cast<double>(l[k]), lb = static_cast<double>(l[k + 1]);
+          s0 += la * x0.x;
+          s1 += la * x1.x;
+          s0 += lb * x0.y;
+          s1 += lb * x1.y;
+        }
+        acc[q][0] += s0;
+        acc[q][1] += s1;
+      }
+    }
+#pragma unroll
+    for (int q = 0; q < 15; q++) {
+      acc[q][0] = acc[q + 1][0];
+      acc[q][1] = acc[q + 1][1];
+    }
+  }
+}
+
+// Panels of the warp-solved fronts in float64, the w x w triangle replaced by
+// its inverse (zeros above the diagonal), columns h | 1 apart: one warp per
+// front, lane = column of the inverse.  A conversion takes a lone warp 24
+// cycles (measured, against 2 for an FMA): for a front of 256 x 32 that was
+// 3 us of each solve; and with the inverse the block solve is a sum, not a
+// chain of w steps.
+__global__ void __launch_bounds__(128)
+    k_flow_wpanel(const FlowFront *fronts, int count, const float *panel, double *wpanel) {
+  __shared__ float ls[4][32][33];
+  const int warp = threadIdx.x / 32, lane = threadIdx.x % 32, q = 4 * blockIdx.x + warp;
+  if (q >= count) return;
+  const FlowFront f = fronts[q];
+  const int       w = f.w, h = f.h, ld = h | 1;
+  const float    *P = panel + f.panel;
+  double         *M = wpanel + f.inv;
+  for (int k = 0; k < w; k++) {
+    for (int i = w + lane; i < h; i += 32) M[k * ld + i] = static_cast<double>(P[i + k * h]);
+    ls[warp][lane][k] = lane > k && lane < w ? P[lane + k * h] : 0.0f;
+  }
+  __syncwarp();
+  double x[32];
+#pragma unroll
+  for (int i = 0; i < 32; i++) {
+    double s = i == lane ? 1.0 : 0.0;
+    if (i < w) {
+#pragma unroll
+      for (int k = 0; k < i; k++) s -= static_cast<double>(ls[warp][i][k]) * x[k];
+      if (lane < w) M[lane * ld + i] = s;
+    }
+    x[i] = s;
+  }
+}
+
+void flow_invert(const Plan &P, Numeric &F, cudaStream_t s) {
+  if (!P.host_.flow_warp.empty())
+    launch(k_flow_wpanel, static_cast<unsigned>((P.host_.flow_warp.size() + 3) / 4), 128, 0, s,
+           static_cast<const FlowFront *>(P.flow_warp.as<FlowFront>()),
+           static_cast<int>(P.host_.flow_warp.size()), static_cast<const float *>(F.panel.as<float>()),
+           F.wpanel.as<double>());
+  if (P.nflow_inv == 0) return;
+  launch(k_flow_invert, static_cast<unsigned>(P.nflow_inv), 128, 0, s,
+         static_cast<const FlowInvDesc *>(P.flow_inv.as<FlowInvDesc>()),
+         static_cast<const float *>(F.panel.as<float>()), F.inv64.as<double>());
+  MPIR_CHECK_LAUNCH();
+}
+
+// ---------------------------------------------------------------------------
+namespace {
+// The handed-over values in one buffer: the forward solve's, then the
+// backward solve's (each side is marked pending as a whole).
+struct FlowBuffers {
+  int64_t fwd, bwd;
+  explicit FlowBuffers(const Plan &P)
+      : fwd(P.S.z_elems + (kFlowCopies + 1) * P.S.n),
+        bwd(P.flow_part_elems + (kFlowCopies + 1) * P.S.n) {}
+};
+}  // namespace
+
+size_t SolveWorkspace::bytes_for(const Plan &P) {
+  const FlowBuffers b(P);
+  return (b.fwd + b.bwd + P.S.n) * sizeof(double) + 4 * sizeof(int32_t) + sizeof(SolveCtl);
+}
+
+void SolveWorkspace::allocate(const Plan &P) {
+  const FlowBuffers b(P);
+  vals.resize(std::max<int64_t>(b.fwd + b.bwd + P.S.n, 1) * sizeof(double));
+  sync.resize(4 * sizeof(int32_t));
+  device_zero(sync.as<void>(), sync.bytes());
+  err.resize(sizeof(SolveCtl));
+  device_zero(err.as<void>(), sizeof(SolveCtl));
+  fwd_pending = bwd_pending = false;
+}
+
+template <class T>
+static void ldlt_solve_t(const Plan &P, const Numeric &F, const T *pan, double *x,
+                         SolveWorkspace &ws, cudaStream_t s, int phases) {
+  const int64_t n = P.S.n;
+  if (n == 0) return;
+  KernelTimer      &kt = kernel_timer();
+  const FlowBuffers b(P);
+  double           *fv = ws.vals.as<double>(), *bv = fv + b.fwd;
+  FlowArgs<T> a{};
+  a.warps = P.flow_warp.as<FlowFront>();
+  a.panel = pan;
+  a.inv   = F.inv64.as<double>();
+  a.wpanel = F.wpanel.as<double>();
+  a.gfirst = P.flow_gfirst.as<int2>();
+  a.gmore  = P.flow_gmore.as<int32_t>();
+  a.srows = P.srows.as<int32_t>();
+  a.n     = n;
+  a.x     = x;
+  a.f     = (phases & kForward) ? bv + b.bwd : x;
+  a.z     = fv;
+  a.y     = a.z + P.S.z_elems;
+  a.yz    = a.y + kFlowCopies * n;
+  a.part  = bv;
+  a.xr    = a.part + P.flow_part_elems;
+  a.xz    = a.xr + kFlowCopies * n;
+  a.err   = ws.err.as<int32_t>();
+  static std::atomic<bool> attr{false};
+  constexpr int            smem = kFlowSmem * sizeof(double);
+  if (!attr) {
+    MPIR_CUDA(cudaFuncSetAttribute(k_fwd_flow<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    MPIR_CUDA(cudaFuncSetAttribute(k_bwd_flow<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    attr = true;
+  }
+  kt.begin(kKcSolveFwd, s);
+  if (phases & kForward) {
+    if (!ws.fwd_pending) flow_pending(fv, b.fwd, s);
+    a.items  = P.flow_fwd.as<FlowItem>();
+    a.nitems = P.nflow_fwd;
+    a.mark   = bv;
+    a.nmark  = b.bwd;
+    a.ticket = ws.sync.as<int32_t>();
+    launch(k_fwd_flow<T>, std::min(P.nflow_fwd, kSMs), kFlowThreads, smem, s, a);
+    ws.fwd_pending = false;
+    ws.bwd_pending = true;
+  }
+  if (!(phases & kBackward) && (phases & kForward))
+    MPIR_CUDA(cudaMemcpyAsync(x, a.f, n * sizeof(double), cudaMemcpyDeviceToDevice, s));
+  // The backward solve reads f .* Dinv as its right-hand side.
+  if ((phases & kDiagonal) && !(phases & kBackward))
+    launch(k_dscale, static_cast<unsigned>((n + 255) / 256), 256, 0, s, n, F.Dinv.as<float>(), x);
+  kt.end(s);
+  MPIR_CHECK_LAUNCH();
+  if (!(phases & kBackward)) return;
+  kt.begin(kKcSolveBwd, s);
+  if (!ws.bwd_pending) flow_pending(bv, b.bwd, s);
+  a.items  = P.flow_bwd.as<FlowItem>();
+  a.nitems = P.nflow_bwd;
+  a.mark   = fv;
+  a.nmark  = b.fwd;
+  a.Dinv   = (phases & kDiagonal) ? F.Dinv.as<float>() : nullptr;
+  a.ticket = ws.sync.as<int32_t>() + 1;
+  launch(k_bwd_flow<T>, std::min(P.nflow_bwd, kSMs), kFlowThreads, smem, s, a);
+  ws.bwd_pending = false;
+  ws.fwd_pending = true;
+  kt.end(s);
+  MPIR_CHECK_LAUNCH();
+}
+
+void ldlt_solve(const Plan &P, const Numeric &F, double *x, SolveWorkspace &ws,
+                cudaStream_t s, int phases) {
+  switch (F.solve_prec()) {
+    case 2:
+      ldlt_solve_t(P, F, F.panel16.as<__nv_bfloat16>(), x, ws, s, phases);
+      break;
+    case 3:
+      ldlt_solve_t(P, F, F.panel16.as<__half>(), x, ws, s, phases);
+      break;
+    default:
+      ldlt_solve_t(P, F, F.panel.as<float>(), x, ws, s, phases);
+  }
+}
+
+// ---------------------------------------------------------------------------
+// QDLDL_solve without device allocation.
+//
+// For callers that cannot call cudaMalloc: processes whose device memory is
+// reserved up front and handed out entirely by their own pooling allocator,
+// and loops that cannot take cudaMalloc's implicit device-wide
+// synchronisation.  All
+// device data of this entry point (the supernodal layout of L, the factor
+// values, Dinv, the fronts' update vectors and x) is packed into the one
+// file-scope array below, of fixed size, that every GPU holds once this
+// library is loaded.  Only factors whose supernodal fronts have at most
+// kSmallFront rows are taken (the warp-per-front kernels; no diagonal-block
+// inverses), and the packed data must fit the array.
+constexpr int kWarpsPerCta = 4;
+constexpr int kSmallH      = kWarpSolveH;
 
 // Forward
-template <class T>
 __global__ void __launch_bounds__(32 * kWarpsPerCta)
     k_fwd_small(const int32_t *list, int count, const int64_t *sfirst,
                 const int64_t *srowptr, const int64_t *slofs,
                 const int64_t *child_ptr, const int32_t *child_list,
-                const int32_t *srel, const int64_t *zofs, const T *panel,
+                const int32_t *srel, const int64_t *zofs, const float *panel,
                 double *x, double *zbuf) {
   __shared__ double zs[kWarpsPerCta][kSmallH];
   const int         warp = threadIdx.x / 32, lane = threadIdx.x % 32;
@@ -154,7 +1028,7 @@ __global__ void __launch_bounds__(32 * kWarpsPerCta)
   }
   // Columns four at a time; the next four columns' entries of this lane's
   // rows (lane + 32 t) are loaded while the current four are applied.
-  const T      *P  = panel + slofs[J];
+  const float  *P  = panel + slofs[J];
   constexpr int RT = kSmallH / 32;
   float         cur[4][RT], nxt[4][RT];
   auto          load4 = [&](float (*buf)[RT], int k0) {
@@ -163,7 +1037,7 @@ __global__ void __launch_bounds__(32 * kWarpsPerCta)
 #pragma unroll
       for (int t = 0; t < RT; t++) {
         const int k = k0 + u, i = lane + 32 * t;
-        buf[u][t]   = (k < w && i > k && i < h) ? to_f(P[i + (int64_t)k * h]) : 0.0f;
+        buf[u][t]   = (k < w && i > k && i < h) ? P[i + (int64_t)k * h] : 0.0f;
       }
   };
   load4(cur, 0);
@@ -193,221 +1067,11 @@ __global__ void __launch_bounds__(32 * kWarpsPerCta)
   }
 }
 
-
-// Waits for this lane's entries p[lane + 32 i] (i < 4) of a block result, the
-// entries at or past lim reading as 0; each round polls all four at once.
-__device__ __forceinline__ void wait_block4(const double *p, int lim, double (&v)[4],
-                                            int32_t *err, long polls) {
-  const int lane = threadIdx.x % 32;
-  unsigned  need = 0;
-#pragma unroll
-  for (int i = 0; i < 4; i++) {
-    v[i] = 0.0;
-    if (lane + 32 * i < lim) need |= 1u << i;
-  }
-  for (long it = 0; need != 0 && it < polls; it++) {
-    unsigned long long raw[4];
-#pragma unroll
-    for (int i = 0; i < 4; i++) raw[i] = (need >> i & 1u) ? ld_relaxed_u64(p + lane + 32 * i) : 0ull;
-#pragma unroll
-    for (int i = 0; i < 4; i++)
-      if ((need >> i & 1u) && raw[i] != kPending) {
-        v[i] = __longlong_as_double(static_cast<long long>(raw[i]));
-        need &= ~(1u << i);
-      }
-    if ((it & 63) == 63) {
-      if (*reinterpret_cast<volatile int32_t *>(err) != 0) return;
-      __nanosleep(32);
-    }
-  }
-  if (need != 0) atomicExch(err, 1);
-}
-
-// The value at p from a load issued ahead (raw) when that load already saw
-// it, else the wait for it.
-__device__ __forceinline__ double take_value(unsigned long long raw, const double *p,
-                                             int32_t *err, long polls) {
-  return raw != kPending ? __longlong_as_double(static_cast<long long>(raw))
-                         : wait_value(p, err, polls);
-}
-
-__global__ void k_mark_pending(int64_t n, double *ready) {
-  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (i < n) reinterpret_cast<unsigned long long *>(ready)[i] = kPending;
-}
-
-
-
-// Forward solve of the large fronts of one level: one CTA per 128-row block
-// R of a front.  z_R -= L_{R,b} y_b for the column blocks b left of R, in
-// order, each as soon as y_b is ready: thread (q, i) = (tid / 128,
-// tid % 128) takes row i and the columns 32 q .. 32 q + 31 of each tile (a
-// warp's loads are one 128-byte column segment), loads its L values before
-// the wait, and each lane waits for its own entry of y_b in the ready buffer
-// (no CTA barrier per tile); the four slices are added in order at the end.
-// A diagonal row block then solves y_R = Linv_R z_R into x and the ready
-// buffer (block product with warp-local slices, see blk_i); rows at or past
-// w are the front's update vector for its parent.
-template <class T>
-__global__ void __launch_bounds__(kSolveThreads, 1)
-    k_fwd_fronts(const SolveItem *items, const T *panel, const double *linv64t, const int64_t *gp,
-                 const int64_t *gsrc, double *x, double *zbuf, int32_t *tickets,
-                 double *ready, int32_t *err) {
-  extern __shared__ __align__(16) double tri[];  // kFwdTri doubles: the staged Linv_R
-  __shared__ __align__(16) double ys[kNB];
-  __shared__ double ys2[4 * 33];
-  __shared__ double yw[kSolveThreads / 32][32];
-  __shared__ double part[4][kNB];
-  // Thread 0 takes the CTA's ticket (the order in which CTAs take their work,
-  // so every block a CTA waits for belongs to an earlier ticket) and copies
-  // the item's record into shared memory: the code after the tile loop (on
-  // the chain of diagonal blocks) reads the descriptor again, and from global
-  // memory that took a round trip past an L1 the tiles had flushed.
-  __shared__ SolveFront sF;
-  __shared__ int        sR, sItem;
-  __shared__ long       sPolls;
-  __shared__ bool       sPublish;
-  if (threadIdx.x == 0) {
-    const int it = atomicAdd(tickets, 1);
-    sItem        = it;
-    sF           = items[it].f;
-    sR           = items[it].r;
-    const volatile SolveCtl *c = reinterpret_cast<const volatile SolveCtl *>(err);
-    sPolls       = poll_limit(c->poll_log2);
-    sPublish     = c->withhold != it + 1;
-  }
-  __syncthreads();
-  const int         item = sItem;
-  const SolveFront &F    = sF;
-  const int         R    = sR;
-  const long        polls = sPolls;
-  if (R < F.nb)
-    stage_lower(linv64t + F.linv + static_cast<int64_t>(R) * kNB * kNB, tri);
-  const int     tid = threadIdx.x, rr = tid % kNB, qq = tid / kNB;
-  const int     warp = tid / 32, lane = tid % 32;
-  const int64_t h = F.h;
-  const int     w = F.w;
-  const int64_t r = static_cast<int64_t>(R) * kNB + rr;
-  const T      *P  = panel + F.panel;
-  const int64_t n  = F.n;
-  const double *yr = ready + ((item * 16 + threadIdx.x / 32) % kReadyCopies) * n + F.col0;
-  const int     tiles = min(R, F.nb);
-  // Right-hand side of this row: its entry of x (rows < w), then the
-  // children's update vectors in child order.
-  __shared__ double zs[kNB];
-  if (qq == 0) {
-    double zr = 0.0;
-    if (r < h) {
-      zr = r < w ? x[F.col0 + r] : 0.0;
-      for (int64_t e = gp[F.gptr + r]; e < gp[F.gptr + r + 1]; e++) zr += zbuf[gsrc[e]];
-    }
-    zs[rr] = zr;
-  }
-  double acc = 0.0;
-  // The next tile's L values are loaded while the current one waits for y_b
-  // and is applied: two tiles in flight, so a CTA that starts late (when an
-  // earlier one leaves its SM) catches up on the tiles already available at
-  // about twice the rate of one tile at a time.
-  float lv[32], lvn[32];
-  auto  load_tile = [&](float (&dst)[32], int b) {
-    const int c0 = b * kNB + qq * 32;
-#pragma unroll
-    for (int k = 0; k < 32; k++)
-      dst[k] = (r < h && c0 + k < w) ? to_f(__ldg(P + r + static_cast<int64_t>(c0 + k) * h)) : 0.0f;
-  };
-  // The lane's entry of y_b is loaded ahead with the tile's L values too;
-  // only an entry that was still pending then is waited for.
-  auto load_y = [&](int b) {
-    const int c0 = b * kNB + qq * 32;
-    return c0 + lane < w ? ld_relaxed_u64(yr + c0 + lane) : 0ull;
-  };
-  unsigned long long yv = 0ull, yvn = 0ull;
-  cp_async_wait_all();
-  if (tiles > 0) {
-    load_tile(lv, 0);
-    yv = load_y(0);
-  }
-  // The last tile's block result is the one just before this block on the
-  // chain: the first warp of each column quarter waits for the quarter's 32
-  // entries and shares them with the quarter's other three warps through a
-  // named barrier (each warp waiting for its own copy saw them up to 2 us
-  // apart, and the CTA could only go on with the last).
-  __shared__ double ylast[kNB];
-  for (int b = 0; b + 1 < tiles; b++) {
-    const int c0 = b * kNB + qq * 32;
-    load_tile(lvn, b + 1);
-    if (b + 2 < tiles) yvn = load_y(b + 1);
-    yw[warp][lane] = c0 + lane < w ? take_value(yv, yr + c0 + lane, err, polls) : 0.0;
-    __syncwarp();
-#pragma unroll
-    for (int k = 0; k < 32; k++) acc += static_cast<double>(lv[k]) * yw[warp][k];
-    __syncwarp();
-#pragma unroll
-    for (int k = 0; k < 32; k++) lv[k] = lvn[k];
-    yv = yvn;
-  }
-  if (tiles > 0) {
-    // The last tile: its L values are widened before the wait (float to
-    // double conversions run at a quarter of the FMA rate; done after the
-    // wait, by all 16 warps, they took about 0.5 us of the chain).
-    const int c0 = (tiles - 1) * kNB + qq * 32;
-    double    ld[32];
-#pragma unroll
-    for (int k = 0; k < 32; k++) ld[k] = static_cast<double>(lv[k]);
-    if (warp % 4 == 0)
-      ylast[qq * 32 + lane] =
-          c0 + lane < w ? wait_value(ready + ((item + qq) % kReadyCopies) * n + F.col0 + c0 + lane,
-                                     err, polls)
-                        : 0.0;
-    asm volatile("bar.sync %0, %1;" ::"r"(1 + qq), "r"(kNB) : "memory");
-#pragma unroll
-    for (int k = 0; k < 32; k++) acc += ld[k] * ylast[qq * 32 + k];
-  }
-  part[qq][rr] = acc;
-  __syncthreads();
-  double z = 0.0;
-  if (qq == 0 && r < h) z = zs[rr] - ((part[0][rr] + part[1][rr]) + (part[2][rr] + part[3][rr]));
-  if (R < F.nb) {
-    const int nbk = min(kNB, w - R * kNB);
-    if (qq == 0) ys[rr] = rr < nbk ? z : 0.0;
-    __syncthreads();
-    const double y  = block_lower_apply(tri, ys);
-    const int    iy = blk_i();
-    if (blk_q() == 0 && iy < nbk && sPublish) {
-      const int64_t j = F.col0 + R * kNB + iy;
-#pragma unroll
-      for (int c = 0; c < kReadyCopies; c++) st_relaxed_f64(ready + c * n + j, y);
-      x[j] = y;
-    }
-    if ((R + 1) * kNB > w && h > w) {
-      // Rows of this block at or past w: their product with the block.
-      if (blk_q() == 0) ys2[pad(iy)] = iy < nbk ? y : 0.0;
-      __syncthreads();
-      double a2 = 0.0;
-      if (r >= w && r < h)
-        for (int k = qq * 32; k < min(nbk, qq * 32 + 32); k++)
-          a2 += static_cast<double>(to_f(P[r + static_cast<int64_t>(R * kNB + k) * h])) * ys2[pad(k)];
-      part[qq][rr] = a2;
-      __syncthreads();
-      if (qq == 0 && r >= w && r < h)
-        z -= (part[0][rr] + part[1][rr]) + (part[2][rr] + part[3][rr]);
-    }
-  }
-  if (qq == 0 && r >= w && r < h) zbuf[F.zofs + r] = z;
-}
-
-__global__ void k_dscale(int64_t n, const float *Dinv, double *x) {
-  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (i < n) x[i] *= static_cast<double>(Dinv[i]);
-}
-
-// ---------------------------------------------------------------------------
 // Backward
-template <class T>
 __global__ void __launch_bounds__(32 * kWarpsPerCta)
     k_bwd_small(const int32_t *list, int count, const int64_t *sfirst,
                 const int64_t *srowptr, const int32_t *srows,
-                const int64_t *slofs, const T *panel, double *x) {
+                const int64_t *slofs, const float *panel, double *x) {
   __shared__ double zs[kWarpsPerCta][kSmallH];
   const int         warp = threadIdx.x / 32, lane = threadIdx.x % 32;
   const int         idx  = blockIdx.x * kWarpsPerCta + warp;
@@ -422,7 +1086,7 @@ __global__ void __launch_bounds__(32 * kWarpsPerCta)
   __syncwarp();
   // Columns four at a time from the last; the next four columns' entries of
   // this lane's rows (lane + 32 t) are loaded while the current four are used.
-  const T      *P  = panel + slofs[J];
+  const float  *P  = panel + slofs[J];
   constexpr int RT = kSmallH / 32;
   float         cur[4][RT], nxt[4][RT];
   auto          load4 = [&](float (*buf)[RT], int k0) {  // columns k0, k0-1, ..
@@ -431,7 +1095,7 @@ __global__ void __launch_bounds__(32 * kWarpsPerCta)
 #pragma unroll
       for (int t = 0; t < RT; t++) {
         const int k = k0 - u, i = lane + 32 * t;
-        buf[u][t]   = (k >= 0 && i > k && i < h) ? to_f(P[i + (int64_t)k * h]) : 0.0f;
+        buf[u][t]   = (k >= 0 && i > k && i < h) ? P[i + (int64_t)k * h] : 0.0f;
       }
   };
   load4(cur, w - 1);
@@ -460,378 +1124,6 @@ __global__ void __launch_bounds__(32 * kWarpsPerCta)
   for (int i = lane; i < w; i += 32) x[f + i] = z[i];
 }
 
-
-// Backward solve, off-diagonal rows: CTA c takes rows w + 128c .. of one
-// front and writes t_k = sum_r L_{r,k} z_r for every column k of the front
-// (warp per column, rows over the lanes, shuffle reduction) to its partials.
-template <class T>
-__global__ void __launch_bounds__(kSolveThreads)
-    k_bwd_chunks(const SolveFront *fr, const int32_t *fmap, const T *panel,
-                 const int32_t *srows,
-                 const double *x, double *part) {
-  __shared__ double zr[kNB];
-  const SolveFront  F = fr[fmap[blockIdx.x]];
-  const int         c = blockIdx.x - F.chunk0;
-  const int         tid = threadIdx.x, warp = tid / 32, lane = tid % 32;
-  const int64_t     h = F.h, w = F.w;
-  const int64_t     r0 = w + static_cast<int64_t>(c) * kNB;
-  const int         nr = static_cast<int>(h - r0 < kNB ? h - r0 : kNB);
-  if (tid < kNB) zr[tid] = tid < nr ? x[srows[F.rows + r0 + tid]] : 0.0;
-  __syncthreads();
-  const T      *P  = panel + F.panel + r0;
-  double       *pp = part + F.part + static_cast<int64_t>(c) * w;
-  constexpr int kWarps = kSolveThreads / 32;
-#pragma unroll 2
-  for (int64_t k = warp; k < w; k += kWarps) {
-    const T     *col = P + k * h;
-    double       s   = 0.0;
-#pragma unroll
-    for (int i = 0; i < 4; i++) {
-      const int rr = lane + 32 * i;
-      if (rr < nr) s += static_cast<double>(to_f(__ldg(col + rr))) * zr[rr];
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    if (lane == 0) pp[k] = s;
-  }
-}
-
-// Backward solve, column blocks of the large fronts of one level: one CTA
-// per column block b (last first).  t = (sum of the chunk partials, in chunk
-// order) + (sum over the row blocks R > b of the diagonal part, last first,
-// each as soon as x_R is in the ready buffer); then x_b = Linv_b^T (z_b - t)
-// into x and the ready buffer.  In a tile, warp v takes the block's columns
-// 8v .. 8v+7 and the lanes the rows.
-template <class T>
-__global__ void __launch_bounds__(kSolveThreads, 1)
-    k_bwd_fronts(const SolveItem *items, const T *panel,
-                 const double *linv64t,
-                 double *x, const double *part, int32_t *tickets,
-                 double *ready, int32_t *err) {
-  extern __shared__ double tri[];  // kTri doubles: the staged Linv_b^T
-  __shared__ double v[kNB];
-  __shared__ double ts[kNB];
-  __shared__ double red[4][kNB];
-  // Ticket and item record as in k_fwd_fronts.
-  __shared__ SolveFront sF;
-  __shared__ int        sB, sItem;
-  __shared__ long       sPolls;
-  if (threadIdx.x == 0) {
-    const int it = atomicAdd(tickets, 1);
-    sItem        = it;
-    sF           = items[it].f;
-    sB           = items[it].r;
-    sPolls       = poll_limit(reinterpret_cast<const volatile SolveCtl *>(err)->poll_log2);
-  }
-  __syncthreads();
-  const int         item = sItem;
-  const SolveFront &F    = sF;
-  const int         b    = sB;
-  const long        polls = sPolls;
-  stage_upper(linv64t + F.linv + static_cast<int64_t>(b) * kNB * kNB, tri,
-              min(kNB, F.w - b * kNB));
-  const int         tid = threadIdx.x, warp = tid / 32, lane = tid % 32;
-  const int64_t     h = F.h;
-  const int         w = F.w;
-  const int         nbk = min(kNB, w - b * kNB);
-  // This block's right-hand side, read now (not on the chain at the end).
-  if (tid < nbk) v[tid] = x[F.col0 + b * kNB + tid];
-  const T          *P   = panel + F.panel;
-  const int64_t     n   = F.n;
-  const double     *xr  = ready + ((item * 16 + threadIdx.x / 32) % kReadyCopies) * n + F.col0;
-  {
-    // Chunk partials of column k (no wait needed): thread (q, k) adds chunks
-    // q, q + 4, ...; the four sums are added in order below.
-    const int k = tid % kNB, q = tid / kNB;
-    double    s = 0.0;
-    if (k < nbk)
-      for (int c = q; c < F.chunks; c += 4)
-        s += part[F.part + static_cast<int64_t>(c) * w + b * kNB + k];
-    red[q][k] = s;
-  }
-  double acc[8];
-#pragma unroll
-  for (int j = 0; j < 8; j++) acc[j] = 0.0;
-  // Tile R (the warp's columns 8 warp + j, rows lane + 32 i of row block R);
-  // the next tile (R - 1) is loaded while the current one waits for x_R and
-  // is applied, as in the forward solve.
-  float lv[8][4], lvn[8][4];
-  auto  load_tile = [&](float (&dst)[8][4], int R) {
-    const int64_t rb   = static_cast<int64_t>(R) * kNB;
-    const int     rows = min(kNB, w - R * kNB);
-#pragma unroll
-    for (int j = 0; j < 8; j++) {
-      const int c = warp * 8 + j;
-#pragma unroll
-      for (int i = 0; i < 4; i++) {
-        const int rr = lane + 32 * i;
-        dst[j][i]    = (c < nbk && rr < rows)
-                           ? to_f(__ldg(P + rb + rr + static_cast<int64_t>(b * kNB + c) * h))
-                           : 0.0f;
-      }
-    }
-  };
-  // The last tile (R = b + 1) is the block just before this one on the
-  // chain: one warp waits for all of x_R and shares it (as in the forward).
-  __shared__ double xlast[kNB];
-  if (F.nb - 1 > b) load_tile(lv, F.nb - 1);
-  for (int R = F.nb - 1; R > b + 1; R--) {
-    const int64_t rb   = static_cast<int64_t>(R) * kNB;
-    const int     rows = min(kNB, w - R * kNB);
-    load_tile(lvn, R - 1);
-#pragma unroll
-    for (int i = 0; i < 4; i++) {
-      const int    rr = lane + 32 * i;
-      const double zv = rr < rows ? wait_value(xr + rb + rr, err, polls) : 0.0;
-#pragma unroll
-      for (int j = 0; j < 8; j++) acc[j] += static_cast<double>(lv[j][i]) * zv;
-    }
-#pragma unroll
-    for (int j = 0; j < 8; j++)
-#pragma unroll
-      for (int i = 0; i < 4; i++) lv[j][i] = lvn[j][i];
-  }
-  if (F.nb - 1 > b) {
-    // The last tile (R = b + 1): its L values are widened before the wait,
-    // as in the forward solve.
-    const int64_t rb   = static_cast<int64_t>(b + 1) * kNB;
-    const int     rows = min(kNB, w - (b + 1) * kNB);
-    double        ld[8][4];
-#pragma unroll
-    for (int j = 0; j < 8; j++)
-#pragma unroll
-      for (int i = 0; i < 4; i++) ld[j][i] = static_cast<double>(lv[j][i]);
-    if (warp == 0) {
-      double xv[4];
-      wait_block4(ready + (item % kReadyCopies) * n + F.col0 + rb, rows, xv, err, polls);
-#pragma unroll
-      for (int i = 0; i < 4; i++) xlast[lane + 32 * i] = xv[i];
-    }
-    __syncthreads();
-#pragma unroll
-    for (int i = 0; i < 4; i++) {
-      const double zv = xlast[lane + 32 * i];
-#pragma unroll
-      for (int j = 0; j < 8; j++) acc[j] += ld[j][i] * zv;
-    }
-  }
-  // Sums of the warp's 8 columns over its 32 lanes: the usual butterfly
-  // (partners lane ^ 16, ^ 8, ^ 4, ^ 2, ^ 1), but at each of the first three
-  // levels a lane keeps half of its columns and sends the other half, so it
-  // takes 4 + 2 + 1 + 1 + 1 shuffles instead of 8 x 5 (the same additions in
-  // the same order).  Lane l ends with column (l >> 2) & 7.
-  {
-    const unsigned full = 0xffffffffu;
-    double         s4[4], s2[2];
-    const bool     b4 = lane & 16, b3 = lane & 8, b2 = lane & 4;
-#pragma unroll
-    for (int u = 0; u < 4; u++) {
-      const double keep = b4 ? acc[u + 4] : acc[u], send = b4 ? acc[u] : acc[u + 4];
-      s4[u] = keep + __shfl_xor_sync(full, send, 16);
-    }
-#pragma unroll
-    for (int u = 0; u < 2; u++) {
-      const double keep = b3 ? s4[u + 2] : s4[u], send = b3 ? s4[u] : s4[u + 2];
-      s2[u] = keep + __shfl_xor_sync(full, send, 8);
-    }
-    double s = (b2 ? s2[1] : s2[0]) + __shfl_xor_sync(full, b2 ? s2[0] : s2[1], 4);
-    s += __shfl_xor_sync(full, s, 2);
-    s += __shfl_xor_sync(full, s, 1);
-    if ((lane & 3) == 0) ts[warp * 8 + ((lane >> 2) & 7)] = s;
-  }
-  __syncthreads();
-  if (tid < nbk)
-    v[tid] = v[tid] - (((red[0][tid] + red[1][tid]) + (red[2][tid] + red[3][tid])) + ts[tid]);
-  __syncthreads();
-  // Lt[i * kNB + j] = Linv[i][j]
-  const double xb = block_upper_apply(tri, v, nbk, red);
-  if (tid < nbk) {
-    const int64_t j = F.col0 + b * kNB + tid;
-#pragma unroll
-    for (int c = 0; c < kReadyCopies; c++) st_relaxed_f64(ready + c * n + j, xb);
-    x[j] = xb;
-  }
-}
-
-// ---------------------------------------------------------------------------
-void SolveWorkspace::allocate(const Plan &P) {
-  release_graph();
-  zbuf.resize(std::max<int64_t>(P.S.z_elems, 1) * sizeof(double));
-  part.resize(std::max<int64_t>(P.spart_elems, 1) * sizeof(double));
-  sync.resize(std::max<int64_t>(P.sync_elems, 1) * sizeof(int32_t));
-  ready.resize(std::max<int64_t>(kReadyCopies * P.S.n, 1) * sizeof(double));
-  err.resize(sizeof(SolveCtl));
-  device_zero(err.as<void>(), sizeof(SolveCtl));
-  xbuf.resize(std::max<int64_t>(P.S.n, 1) * sizeof(double));
-}
-
-cudaStream_t SideStream::fork(cudaStream_t s) {
-  if (!st_) {
-    MPIR_CUDA(cudaStreamCreateWithFlags(&st_, cudaStreamNonBlocking));
-    MPIR_CUDA(cudaEventCreateWithFlags(&fork_, cudaEventDisableTiming));
-    MPIR_CUDA(cudaEventCreateWithFlags(&join_, cudaEventDisableTiming));
-  }
-  MPIR_CUDA(cudaEventRecord(fork_, s));
-  MPIR_CUDA(cudaStreamWaitEvent(st_, fork_, 0));
-  return st_;
-}
-
-void SideStream::join(cudaStream_t s) {
-  MPIR_CUDA(cudaEventRecord(join_, st_));
-  MPIR_CUDA(cudaStreamWaitEvent(s, join_, 0));
-}
-
-void SideStream::reset() {
-  if (st_) {
-    cudaStreamSynchronize(st_);
-    cudaStreamDestroy(st_);
-  }
-  if (fork_) cudaEventDestroy(fork_);
-  if (join_) cudaEventDestroy(join_);
-  st_   = nullptr;
-  fork_ = join_ = nullptr;
-}
-
-void SolveWorkspace::release_graph() {
-  if (graph) cudaGraphExecDestroy(graph);
-  graph = nullptr;
-}
-
-void ldlt_solve_graph(const Plan &P, const Numeric &F, double *x, SolveWorkspace &ws,
-                      cudaStream_t s, cudaStream_t capture_stream) {
-  const int64_t n = P.S.n;
-  if (n == 0) return;
-  if (kernel_timer().enabled) {  // per-class timing needs the plain launches
-    ldlt_solve(P, F, x, ws, s);
-    return;
-  }
-  if (!ws.graph) {
-    cudaGraph_t g = nullptr;
-    MPIR_CUDA(cudaStreamSynchronize(capture_stream));
-    MPIR_CUDA(cudaStreamBeginCapture(capture_stream, cudaStreamCaptureModeThreadLocal));
-    {
-      LaunchCapture cap;
-      ldlt_solve(P, F, ws.xbuf.as<double>(), ws, capture_stream);
-      ws.graph_launches = cap.count();
-    }
-    MPIR_CUDA(cudaStreamEndCapture(capture_stream, &g));
-    MPIR_CUDA(cudaGraphInstantiate(&ws.graph, g, 0));
-    cudaGraphDestroy(g);
-  }
-  MPIR_CUDA(cudaMemcpyAsync(ws.xbuf.as<void>(), x, n * sizeof(double), cudaMemcpyDeviceToDevice, s));
-  MPIR_CUDA(cudaGraphLaunch(ws.graph, s));
-  launch_add(ws.graph_launches);
-  MPIR_CUDA(cudaMemcpyAsync(x, ws.xbuf.as<void>(), n * sizeof(double), cudaMemcpyDeviceToDevice, s));
-}
-
-template <class T>
-static void ldlt_solve_t(const Plan &P, const Numeric &F, const T *pan, double *x,
-                         SolveWorkspace &ws, cudaStream_t s, int phases) {
-  const Symbolic &S  = P.S;
-  KernelTimer    &kt = kernel_timer();
-  if (S.n == 0) return;
-  const double *lvt = F.linv64t.as<double>();
-  double      *zbuf = ws.zbuf.as<double>();
-  const int    nl   = static_cast<int>(P.levels.size());
-  // Tickets (2 per level); the ready buffer is marked pending before each
-  // direction.
-  int32_t          *sync  = ws.sync.as<int32_t>();
-  double           *ready = ws.ready.as<double>();
-  int32_t          *err   = ws.err.as<int32_t>();
-  const SolveFront *sf    = P.solve_fronts.as<SolveFront>();
-  const bool        block = P.nblock_fronts > 0;
-  const int64_t     nready = kReadyCopies * S.n;
-  const unsigned    nmark  = static_cast<unsigned>((nready + 255) / 256);
-  if (block) MPIR_CUDA(cudaMemsetAsync(sync, 0, P.sync_elems * sizeof(int32_t), s));
-  if (block && (phases & kForward)) launch(k_mark_pending, nmark, 256, 0, s, nready, ready);
-  static std::atomic<bool> attr{false};
-  if (!attr) {
-    MPIR_CUDA(cudaFuncSetAttribute(k_fwd_fronts<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   static_cast<int>(kFwdTri * sizeof(double))));
-    MPIR_CUDA(cudaFuncSetAttribute(k_bwd_fronts<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   static_cast<int>(kTri * sizeof(double))));
-    attr = true;
-  }
-  kt.begin(kKcSolveFwd, s);
-  for (int t = 0; t < nl && (phases & kForward); t++) {
-    const LevelPlan &L    = P.levels[t];
-    const bool       both = L.sw_count > 0 && L.sf_count > 0;
-    cudaStream_t     ss   = both ? ws.side.fork(s) : s;  // warp fronts beside block fronts
-    if (L.sw_count > 0)
-      launch(k_fwd_small<T>, (L.sw_count + kWarpsPerCta - 1) / kWarpsPerCta, 32 * kWarpsPerCta, 0,
-             ss, P.swarp_list.as<int32_t>() + L.sw_begin, L.sw_count, P.sfirst.as<int64_t>(),
-             P.srowptr.as<int64_t>(), P.slofs.as<int64_t>(), P.child_ptr.as<int64_t>(),
-             P.child_list.as<int32_t>(), P.srel.as<int32_t>(), P.zofs.as<int64_t>(), pan, x,
-             zbuf);
-    if (L.sf_count > 0) {
-      launch(k_fwd_fronts<T>, L.fwd_items, kSolveThreads, kFwdTri * sizeof(double), s,
-             P.fwd_item.as<SolveItem>() + L.fwd_map0, pan, lvt, P.gp.as<int64_t>(),
-             P.gsrc.as<int64_t>(), x, zbuf, sync + 2 * t, ready, err);
-    }
-    if (both) ws.side.join(s);
-  }
-  if (phases & kDiagonal)
-    launch(k_dscale, static_cast<unsigned>((S.n + 255) / 256), 256, 0, s,
-           S.n, F.Dinv.as<float>(), x);
-  kt.end(s);
-  if (!(phases & kBackward)) return;
-  MPIR_CHECK_LAUNCH();
-  kt.begin(kKcSolveBwd, s);
-  if (block) launch(k_mark_pending, nmark, 256, 0, s, nready, ready);
-  for (int t = nl - 1; t >= 0; t--) {
-    const LevelPlan &L    = P.levels[t];
-    const bool       both = L.sw_count > 0 && L.sf_count > 0;
-    cudaStream_t     ss   = both ? ws.side.fork(s) : s;
-    if (L.sw_count > 0)
-      launch(k_bwd_small<T>, (L.sw_count + kWarpsPerCta - 1) / kWarpsPerCta, 32 * kWarpsPerCta, 0,
-             ss, P.swarp_list.as<int32_t>() + L.sw_begin, L.sw_count, P.sfirst.as<int64_t>(),
-             P.srowptr.as<int64_t>(), P.srows.as<int32_t>(), P.slofs.as<int64_t>(), pan, x);
-    if (L.sf_count > 0) {
-      if (L.bwd_chunk_items > 0)
-        launch(k_bwd_chunks<T>, L.bwd_chunk_items, kSolveThreads, 0, s, sf + L.sf_begin,
-               P.chunk_map.as<int32_t>() + L.chunk_map0, pan, P.srows.as<int32_t>(),
-               static_cast<const double *>(x),
-               ws.part.as<double>());
-      launch(k_bwd_fronts<T>, L.bwd_owner_items, kSolveThreads, kTri * sizeof(double), s,
-             P.own_item.as<SolveItem>() + L.own_map0, pan,
-             F.linv64t.as<double>(), x,
-             static_cast<const double *>(ws.part.as<double>()), sync + 2 * t + 1, ready, err);
-    }
-    if (both) ws.side.join(s);
-  }
-  kt.end(s);
-  MPIR_CHECK_LAUNCH();
-}
-
-
-void ldlt_solve(const Plan &P, const Numeric &F, double *x, SolveWorkspace &ws,
-                cudaStream_t s, int phases) {
-  switch (F.solve_prec()) {
-    case 2:
-      ldlt_solve_t(P, F, F.panel16.as<__nv_bfloat16>(), x, ws, s, phases);
-      break;
-    case 3:
-      ldlt_solve_t(P, F, F.panel16.as<__half>(), x, ws, s, phases);
-      break;
-    default:
-      ldlt_solve_t(P, F, F.panel.as<float>(), x, ws, s, phases);
-  }
-}
-
-
-// ---------------------------------------------------------------------------
-// QDLDL_solve without device allocation.
-//
-// For callers that cannot call cudaMalloc: processes whose device memory is
-// reserved up front and handed out entirely by their own pooling allocator,
-// and loops that cannot take cudaMalloc's implicit device-wide
-// synchronisation.  All
-// device data of this entry point (the supernodal layout of L, the factor
-// values, Dinv, the fronts' update vectors and x) is packed into the one
-// file-scope array below, of fixed size, that every GPU holds once this
-// library is loaded.  Only factors whose supernodal fronts have at most
-// kSmallFront rows are taken (the warp-per-front kernels; no diagonal-block
-// inverses), and the packed data must fit the array.
 namespace {
 constexpr size_t kNoAllocScratchBytes = size_t{32} << 20;  // 32 MiB
 constexpr int    kNoAllocMaxDevices   = 64;
@@ -954,14 +1246,14 @@ int qdldl_solve_noalloc(int64_t n, const int64_t *Lp, const int64_t *Li, const f
   const int      nl      = S.nlevels;
   for (int t = 0; t < nl; t++) {
     const int32_t cnt = static_cast<int32_t>(S.level_ptr[t + 1] - S.level_ptr[t]);
-    launch(k_fwd_small<float>, (cnt + kWarpsPerCta - 1) / kWarpsPerCta, 32 * kWarpsPerCta, 0, s,
+    launch(k_fwd_small, (cnt + kWarpsPerCta - 1) / kWarpsPerCta, 32 * kWarpsPerCta, 0, s,
            level + S.level_ptr[t], cnt, sfirst, srowptr, slofs, cptr, clist, srel, zofs, panel,
            xd, zbuf);
   }
   launch(k_dscale, static_cast<unsigned>((n + 255) / 256), 256, 0, s, n, dinv, xd);
   for (int t = nl - 1; t >= 0; t--) {
     const int32_t cnt = static_cast<int32_t>(S.level_ptr[t + 1] - S.level_ptr[t]);
-    launch(k_bwd_small<float>, (cnt + kWarpsPerCta - 1) / kWarpsPerCta, 32 * kWarpsPerCta, 0, s,
+    launch(k_bwd_small, (cnt + kWarpsPerCta - 1) / kWarpsPerCta, 32 * kWarpsPerCta, 0, s,
            level + S.level_ptr[t], cnt, sfirst, srowptr, srows, slofs, panel, xd);
   }
   MPIR_CHECK_LAUNCH();

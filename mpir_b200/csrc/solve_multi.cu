@@ -3,28 +3,22 @@
 // dimension n), the operation QDLDL_solve applies to one vector
 // (qdldl.hpp:417-432) and LUIR_QDLDL / PrecondGmres apply once per vector.
 //
-// The kernels follow the single-vector ones of solve.cu level by level and
-// reuse the same plan (the same fronts, work items, tickets and ready-value
-// hand-over), but every CTA applies each tile of L it loads to all NR
-// vectors: L moves from HBM once per application instead of NR times, and
-// the dependent round trips of a chain link (waiting for a block result,
-// the block product) are shared by the NR vectors.
+// The work items, their order and the hand-over of values are those of the
+// single-vector solves (solve.cu, flow.cuh): one launch a direction for the
+// whole tree.  Each item takes all NR vectors: L moves once per application
+// instead of NR times, and the hand-overs on the chain from the leaves to the
+// root are shared by the NR vectors.  Between items the NR values of an entry
+// lie side by side (entry i at NR i), so that a hand-over is NR / 2 loads of 16
+// bytes; in shared memory too, where a warp reads the same entry's values for
+// NR fused multiply-adds a value of L.
 //
-//   k_fwd_small_m / k_bwd_small_m  fronts solved by one warp, column by
-//                       column, each column applied to all vectors; per
-//                       vector the operations and their order are those of
-//                       k_fwd_small / k_bwd_small, so results are bitwise
-//                       the same as NR single solves;
-//   k_fwd_fronts_m      one CTA per 128-row block: row i by 4 column
-//                       quarters, the NR sums of each row in registers;
-//   k_bwd_chunks_m      partial sums of the off-diagonal rows per column;
-//   k_bwd_fronts_m      one CTA per column block; each tile of L is staged
-//                       through shared memory (coalesced loads by rows, read
-//                       by columns), thread (column, vector group) sums.
-// Block products use the float64 inverses of the diagonal blocks (staged as
-// a packed lower triangle).  Sums inside the large-front kernels run in
-// another order than in the single-vector kernels, so their results agree
-// with NR single solves to rounding.
+// What bounds it: below the root the chain of hand-overs, as for one vector;
+// in the wide fronts the float64 multiply-adds and the shared-memory reads that
+// feed them (an entry of L: NR FMAs and NR / 2 reads of 16 bytes a warp).
+// Measured, one application, against the solves by levels that this replaced:
+// 16 vectors at n = 20,480: 0.74 ms (2.73); 4 at n = 40,951: 0.45 ms (1.50).
+// Per vector the sums inside an item run in another order than in the
+// single-vector kernels, so results agree with NR single solves to rounding.
 #include <atomic>
 #include <algorithm>
 #include <type_traits>
@@ -33,605 +27,903 @@
 #include "engine.hpp"
 #include "solve.hpp"
 #include "solve_dev.cuh"
+#include "flow_dev.cuh"
 
 namespace mpir {
 
+void flow_pending(double *p, int64_t n, cudaStream_t s);
+
 namespace {
 
-constexpr int kTriM      = kNB * (kNB + 1) / 2;  // packed lower triangle of Linv
-constexpr int kSmallWarpsM = 2;                  // warps per CTA, small fronts
-constexpr int kLsPitch   = kNB + 1;              // staged tile row pitch (floats)
+constexpr int kMultiCopies = 2;  // copies of a wide front's block results
 
-// Copies of each block result in the ready buffer (see solve_dev.cuh).
-constexpr int kMultiCopies = 4;
+// Shared memory (doubles): kFlowInvSmem, then 9,216 for vectors and partial
+// sums (512 rows of 16 values, pitch 18).
+constexpr int kMultiBuf  = 512 * 18;
+constexpr int kMultiSmem = kFlowInvSmem + kMultiBuf;
 
-// Stage the lower triangle of the row-major inverse Lt (Lt[i * kNB + j] =
-// Linv[i][j]) packed by rows: (i, j <= i) at i (i + 1) / 2 + j.
-__device__ __forceinline__ void stage_tri_m(const double *Lt, double *Ls, int nb) {
-  const int tid = threadIdx.x, j = tid % kNB, q = tid / kNB;
-  for (int ii = 0; ii < kNB / 4; ii++) {
-    const int i = q * (kNB / 4) + ii;
-    if (i >= j && i < nb) cp_async8(Ls + i * (i + 1) / 2 + j, Lt + i * kNB + j);
-  }
+// Narrow fronts stage at most 10 blocks of the inverse; their vectors start
+// behind those.
+constexpr int kNarrowInv = 10 * kFlowBlk;
+
+struct alignas(16) V2 {
+  unsigned long long a, b;
+};
+__device__ __forceinline__ V2 ld_relaxed_2(const double *p) {
+  V2 v;
+  asm volatile("ld.relaxed.gpu.global.v2.b64 {%0, %1}, [%2];" : "=l"(v.a), "=l"(v.b) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ void st_relaxed_2(double *p, double a, double b) {
+  asm volatile("st.relaxed.gpu.global.v2.b64 [%0], {%1, %2};" ::"l"(p), "l"(__double_as_longlong(a)),
+               "l"(__double_as_longlong(b))
+               : "memory");
 }
 
-// Waits for the K entries p[k * stride] (k < K) of block results and stores
-// them to dst[k * dstride] (zeros for an inactive lane).  The entries are
-// polled in groups of at most 8 loads in flight.
+// Waits for K values side by side (16-byte aligned; none when !on) and adds
+// them to v; all that are pending are polled together.
 template <int K>
-__device__ __forceinline__ void wait_many(const double *p, int64_t stride, bool active,
-                                          double *dst, int dstride, int32_t *err, long polls) {
-  constexpr int G = K < 8 ? K : 8;
+__device__ __forceinline__ void add_entry(const double *p, bool on, double (&v)[K], int32_t *err,
+                                          long polls) {
+  unsigned need = on ? (1u << (K / 2)) - 1 : 0u;
+  for (long it = 0; need != 0; it++) {
+    V2 raw[K / 2];
 #pragma unroll
-  for (int k0 = 0; k0 < K; k0 += G) {
-    unsigned need = 0;
-#pragma unroll
-    for (int k = 0; k < G; k++) {
-      if (active) need |= 1u << k;
-      else dst[(k0 + k) * dstride] = 0.0;
+    for (int q = 0; q < K / 2; q++) {
+      raw[q] = V2{kPending, kPending};
+      if (need >> q & 1u) raw[q] = ld_relaxed_2(p + 2 * q);
     }
-    for (long it = 0; need != 0 && it < polls; it++) {
-      unsigned long long raw[G];
 #pragma unroll
-      for (int k = 0; k < G; k++)
-        raw[k] = (need >> k & 1u) ? ld_relaxed_u64(p + (k0 + k) * stride) : 0ull;
-#pragma unroll
-      for (int k = 0; k < G; k++)
-        if ((need >> k & 1u) && raw[k] != kPending) {
-          dst[(k0 + k) * dstride] = __longlong_as_double(static_cast<long long>(raw[k]));
-          need &= ~(1u << k);
-        }
-      if ((it & 63) == 63) {
-        if (*reinterpret_cast<volatile int32_t *>(err) != 0) return;
-        __nanosleep(32);
+    for (int q = 0; q < K / 2; q++)
+      if (raw[q].a != kPending && raw[q].b != kPending) {
+        v[2 * q] += __longlong_as_double(static_cast<long long>(raw[q].a));
+        v[2 * q + 1] += __longlong_as_double(static_cast<long long>(raw[q].b));
+        need &= ~(1u << q);
       }
-    }
-    if (need != 0) {
+    if (need != 0 && it >= polls) {
       atomicExch(err, 1);
       return;
     }
-  }
-}
-
-__global__ void k_mark_pending_m(int64_t count, double *ready) {
-  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (i < count) reinterpret_cast<unsigned long long *>(ready)[i] = kPending;
-}
-
-// X[:, k] .*= Dinv for every vector k < nr.
-__global__ void k_dscale_m(int64_t n, int nr, const float *Dinv, double *X) {
-  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (i >= n * nr) return;
-  X[i] *= static_cast<double>(Dinv[i % n]);
-}
-
-// ---------------------------------------------------------------------------
-// Fronts solved by one warp (w <= 32, h <= 256), forward.  z[k][i] is front
-// row i of vector k; per vector exactly the operations of k_fwd_small.
-template <int NR, class T>
-__global__ void __launch_bounds__(32 * kSmallWarpsM)
-    k_fwd_small_m(const int32_t *list, int count, const int64_t *sfirst,
-                  const int64_t *srowptr, const int64_t *slofs, const int64_t *child_ptr,
-                  const int32_t *child_list, const int32_t *srel, const int64_t *zofs,
-                  const T *panel, double *x, int64_t n, double *zbuf, int64_t zld) {
-  extern __shared__ __align__(16) double zsm[];  // [warps][NR][kWarpSolveH]
-  constexpr int H    = kWarpSolveH;
-  const int     warp = threadIdx.x / 32, lane = threadIdx.x % 32;
-  const int     idx  = blockIdx.x * kSmallWarpsM + warp;
-  if (idx >= count) return;
-  const int     J = list[idx];
-  const int64_t f = sfirst[J];
-  const int     w = static_cast<int>(sfirst[J + 1] - f);
-  const int     h = static_cast<int>(srowptr[J + 1] - srowptr[J]);
-  double       *z = zsm + static_cast<int64_t>(warp) * NR * H;
-  for (int k = 0; k < NR; k++)
-    for (int i = lane; i < h; i += 32) z[k * H + i] = i < w ? x[k * n + f + i] : 0.0;
-  __syncwarp();
-  for (int64_t c = child_ptr[J]; c < child_ptr[J + 1]; c++) {
-    const int      C  = child_list[c];
-    const int      wc = static_cast<int>(sfirst[C + 1] - sfirst[C]);
-    const int      rc = static_cast<int>(srowptr[C + 1] - srowptr[C]) - wc;
-    const int32_t *rl = srel + srowptr[C] + wc;
-    const int64_t  zc = zofs[C] + wc;
-    for (int k = 0; k < NR; k++)
-      for (int a = lane; a < rc; a += 32) z[k * H + rl[a]] += zbuf[k * zld + zc + a];
-    __syncwarp();
-  }
-  const T      *P  = panel + slofs[J];
-  constexpr int RT = H / 32;
-  float         cur[4][RT], nxt[4][RT];
-  auto          load4 = [&](float (*buf)[RT], int k0) {
-#pragma unroll
-    for (int u = 0; u < 4; u++)
-#pragma unroll
-      for (int t = 0; t < RT; t++) {
-        const int k = k0 + u, i = lane + 32 * t;
-        buf[u][t]   = (k < w && i > k && i < h) ? to_f(P[i + (int64_t)k * h]) : 0.0f;
-      }
-  };
-  load4(cur, 0);
-  for (int k0 = 0; k0 < w; k0 += 4) {
-    if (k0 + 4 < w) load4(nxt, k0 + 4);
-#pragma unroll
-    for (int u = 0; u < 4; u++) {
-      const int col = k0 + u;
-      if (col >= w) break;
-      for (int k = 0; k < NR; k++) {
-        double      *zk = z + k * H;
-        const double zc = zk[col];
-#pragma unroll
-        for (int t = 0; t < RT; t++) {
-          const int i = lane + 32 * t;
-          if (i > col && i < h) zk[i] -= static_cast<double>(cur[u][t]) * zc;
-        }
-      }
-      __syncwarp();
+    if ((it & 63) == 63) {
+      if (*reinterpret_cast<volatile int32_t *>(err) != 0) return;
+      __nanosleep(32);
     }
-#pragma unroll
-    for (int u = 0; u < 4; u++)
-#pragma unroll
-      for (int t = 0; t < RT; t++) cur[u][t] = nxt[u][t];
   }
-  const int64_t zo = zofs[J];
-  for (int k = 0; k < NR; k++)
-    for (int i = lane; i < h; i += 32) {
-      if (i < w) x[k * n + f + i] = z[k * H + i];
-      zbuf[k * zld + zo + i] = z[k * H + i];
-    }
 }
 
-// Backward counterpart of k_fwd_small_m (per vector the operations of
-// k_bwd_small).
-template <int NR, class T>
-__global__ void __launch_bounds__(32 * kSmallWarpsM)
-    k_bwd_small_m(const int32_t *list, int count, const int64_t *sfirst,
-                  const int64_t *srowptr, const int32_t *srows, const int64_t *slofs,
-                  const T *panel, double *x, int64_t n) {
-  extern __shared__ __align__(16) double zsm[];
-  constexpr int H    = kWarpSolveH;
-  const int     warp = threadIdx.x / 32, lane = threadIdx.x % 32;
-  const int     idx  = blockIdx.x * kSmallWarpsM + warp;
-  if (idx >= count) return;
-  const int      J  = list[idx];
-  const int64_t  f  = sfirst[J];
-  const int      w  = static_cast<int>(sfirst[J + 1] - f);
-  const int      h  = static_cast<int>(srowptr[J + 1] - srowptr[J]);
-  const int32_t *rw = srows + srowptr[J];
-  double        *z  = zsm + static_cast<int64_t>(warp) * NR * H;
-  for (int k = 0; k < NR; k++)
-    for (int i = lane; i < h; i += 32) z[k * H + i] = x[k * n + (i < w ? f + i : rw[i])];
-  __syncwarp();
-  const T      *P  = panel + slofs[J];
-  constexpr int RT = H / 32;
-  float         cur[4][RT], nxt[4][RT];
-  auto          load4 = [&](float (*buf)[RT], int k0) {
+// An entry's K values (zeros when !on) into shared memory.
+template <int K>
+__device__ __forceinline__ void get_entry(const double *p, bool on, double *dst, int32_t *err,
+                                          long polls) {
+  double v[K];
 #pragma unroll
-    for (int u = 0; u < 4; u++)
+  for (int k = 0; k < K; k++) v[k] = 0.0;
+  add_entry<K>(p, on, v, err, polls);
 #pragma unroll
-      for (int t = 0; t < RT; t++) {
-        const int k = k0 - u, i = lane + 32 * t;
-        buf[u][t]   = (k >= 0 && i > k && i < h) ? to_f(P[i + (int64_t)k * h]) : 0.0f;
-      }
-  };
-  load4(cur, w - 1);
-  for (int k0 = w - 1; k0 >= 0; k0 -= 4) {
-    if (k0 - 4 >= 0) load4(nxt, k0 - 4);
-#pragma unroll
-    for (int u = 0; u < 4; u++) {
-      const int col = k0 - u;
-      if (col < 0) break;
-      for (int k = 0; k < NR; k++) {
-        double *zk = z + k * H;
-        double  s  = 0.0;
-#pragma unroll
-        for (int t = 0; t < RT; t++) {
-          const int i = lane + 32 * t;
-          if (i > col && i < h) s += static_cast<double>(cur[u][t]) * zk[i];
-        }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-        if (lane == 0) zk[col] -= s;
-      }
-      __syncwarp();
-    }
-#pragma unroll
-    for (int u = 0; u < 4; u++)
-#pragma unroll
-      for (int t = 0; t < RT; t++) cur[u][t] = nxt[u][t];
-  }
-  for (int k = 0; k < NR; k++)
-    for (int i = lane; i < w; i += 32) x[k * n + f + i] = z[k * H + i];
+  for (int k = 0; k < K; k += 2) *reinterpret_cast<double2 *>(dst + k) = make_double2(v[k], v[k + 1]);
 }
 
-// ---------------------------------------------------------------------------
-// Forward, large fronts: one CTA per 128-row block R of a front (tickets as
-// in k_fwd_fronts).  Thread (qq, rr) = (tid / 128, tid % 128) takes row rr of
-// the block and columns 32 qq .. 32 qq + 31 of each tile; each lane waits
-// for its entry of y_b in all NR vectors, the warp shares them through
-// shared memory, and the row's NR sums stay in registers.
+// acc[k] += l y[k] for the NR values at y (shared memory, 16-byte aligned).
 template <int NR>
-constexpr int fwd_m_smem_doubles() {
-  return kTriM + 2 * NR * kNB + NR * 512;
+__device__ __forceinline__ void fma_entry(double l, const double *y, double (&acc)[NR]) {
+#pragma unroll
+  for (int q = 0; q < NR; q += 2) {
+    const double2 v = *reinterpret_cast<const double2 *>(y + q);
+    acc[q] += l * v.x;
+    acc[q + 1] += l * v.y;
+  }
 }
 
-template <int NR, class T>
-__global__ void __launch_bounds__(kSolveThreads, 1)
-    k_fwd_fronts_m(const SolveItem *items, const T *panel, const double *linv64t,
-                   const int64_t *gp, const int64_t *gsrc, double *x, double *zbuf,
-                   int64_t zld, int32_t *tickets, double *ready, int32_t *err) {
-  extern __shared__ __align__(16) double sm[];
-  double *tri = sm;                // packed lower Linv_R
-  double *zs  = tri + kTriM;       // [NR][kNB] right-hand side, then z
-  double *yb  = zs + NR * kNB;     // [NR][kNB] block result
-  double *S   = yb + NR * kNB;     // [16][NR][32] tile values, then [4][NR][kNB]
-  __shared__ SolveFront sF;
-  __shared__ int        sR, sItem;
-  __shared__ long       sPolls;
-  __shared__ bool       sPublish;
-  if (threadIdx.x == 0) {
-    const int it = atomicAdd(tickets, 1);
-    sItem        = it;
-    sF           = items[it].f;
-    sR           = items[it].r;
-    const volatile SolveCtl *c = reinterpret_cast<const volatile SolveCtl *>(err);
-    sPolls       = poll_limit(c->poll_log2);
-    sPublish     = c->withhold != it + 1;
+template <int NR>
+__device__ __forceinline__ void put_entry(double *dst, const double (&v)[NR]) {
+#pragma unroll
+  for (int k = 0; k < NR; k += 2) *reinterpret_cast<double2 *>(dst + k) = make_double2(v[k], v[k + 1]);
+}
+
+// ---------------------------------------------------------------------------
+// Forward.
+
+// acc += sum_c L(r, c) y_c over the columns c < cend of a wide front, tile by
+// tile as the block results become ready (rows_apply of solve.cu); own: the
+// warp's 32 NR doubles of shared memory.
+template <int RG, int NR, class T>
+__device__ __forceinline__ void rows_apply_m(const FlowArgs<T> &a, const T *P, int64_t h, int64_t r,
+                                             bool rok, int cend, const double *y, double *own,
+                                             double (&acc)[NR], long polls) {
+  constexpr int TW = 512 / RG;
+  const int     warp = threadIdx.x / 32, lane = threadIdx.x % 32, cq = 32 * (warp / RG);
+  float         lv[32], lvn[32];
+  load_cols(lv, P, h, r, rok, cq, cend);
+  for (int c = cq; c - cq < cend; c += TW) {
+    if (c - cq + TW < cend) load_cols(lvn, P, h, r, rok, c + TW, cend);
+    get_entry<NR>(y + static_cast<int64_t>(NR) * (c + lane), c + lane < cend, own + NR * lane, a.err, polls);
+    __syncwarp();
+#pragma unroll
+    for (int k = 0; k < 32; k++) fma_entry<NR>(static_cast<double>(lv[k]), own + NR * k, acc);
+    __syncwarp();
+#pragma unroll
+    for (int k = 0; k < 32; k++) lv[k] = lvn[k];
   }
-  __syncthreads();
-  const int         item  = sItem;
-  const SolveFront &F     = sF;
-  const int         R     = sR;
-  const long        polls = sPolls;
-  const int         tid = threadIdx.x, rr = tid % kNB, qq = tid / kNB;
-  const int         warp = tid / 32, lane = tid % 32;
-  const int64_t     h = F.h, n = F.n;
-  const int         w = F.w;
-  const int64_t     r = static_cast<int64_t>(R) * kNB + rr;
-  const T          *P = panel + F.panel;
-  if (R < F.nb) stage_tri_m(linv64t + F.linv + static_cast<int64_t>(R) * kNB * kNB, tri,
-                            min(kNB, w - R * kNB));
-  // Right-hand side rows: x (rows < w) plus the children's update vectors in
-  // child order; thread (qq, rr) fills vectors qq, qq + 4, ...
-  for (int k = qq; k < NR; k += 4) {
-    double zr = 0.0;
-    if (r < h) {
-      zr = r < w ? x[k * n + F.col0 + r] : 0.0;
-      for (int64_t e = gp[F.gptr + r]; e < gp[F.gptr + r + 1]; e++) zr += zbuf[k * zld + gsrc[e]];
-    }
-    zs[k * kNB + rr] = zr;
-  }
-  const int     copy  = (item * 16 + warp) % kMultiCopies;
-  const double *yr    = ready + static_cast<int64_t>(copy) * NR * n + F.col0;
-  const int     tiles = min(R, F.nb);
-  double        acc[NR];
+}
+
+// acc = the 32 x 32 block of the inverse at blk (entry (lane, c) at c * 33 +
+// lane) times the 32 entries at y.
+template <int NR>
+__device__ __forceinline__ void block_rows(const double *blk, const double *y, double (&acc)[NR]) {
 #pragma unroll
   for (int k = 0; k < NR; k++) acc[k] = 0.0;
-  // Each tile's L values are loaded before the wait for its block result,
-  // so the loads are in flight while the lane polls.
-  float   lv[32];
-  double *yw = S + warp * NR * 32;  // [NR][32]
-  for (int b = 0; b < tiles; b++) {
-    const int c0 = b * kNB + qq * 32;
-#pragma unroll
-    for (int k = 0; k < 32; k++)
-      lv[k] = (r < h && c0 + k < w) ? to_f(__ldg(P + r + static_cast<int64_t>(c0 + k) * h)) : 0.0f;
-    wait_many<NR>(yr + c0 + lane, n, c0 + lane < w, yw + lane, 32, err, polls);
-    __syncwarp();
-#pragma unroll
-    for (int kk = 0; kk < 32; kk++) {
-      const double l = static_cast<double>(lv[kk]);
-#pragma unroll
-      for (int k = 0; k < NR; k++) acc[k] += l * yw[k * 32 + kk];
-    }
-    __syncwarp();
+#pragma unroll 8
+  for (int c = 0; c < 32; c++) fma_entry<NR>(blk[33 * c], y + NR * c, acc);
+}
+
+template <int NR, class T>
+__device__ __noinline__ void fwd_slab_m(const FlowArgs<T> &a, FlowShared &S, const FlowSlot &I, FlowSlot &N,
+                                        double *sm, uint32_t &phase) {
+  const FlowFront &f   = I.item.f;
+  const int        tid = threadIdx.x, warp = tid / 32, lane = tid % 32;
+  const int        row = tid / NR, v = tid % NR;  // the thread's output, tid < 32 NR
+  const long       polls = I.polls;
+  const int        r0 = I.item.r0, s = r0 / kFlowSB, i = (r0 % kFlowSB) / 32;
+  const bool       mine = row < I.item.nr, last = r0 + 32 >= f.w || i == 15;
+  double          *inv = sm, *yw = sm + kFlowInvSmem, *own = yw + 32 * NR * warp;
+  const uint32_t   bar = smem_addr(&S.bar);
+  if (tid == 0) {
+    const uint32_t bytes = (i + 1) * kFlowBlk * sizeof(double);
+    bulk_expect(bar, bytes);
+    bulk_get(inv, a.inv + f.inv + (static_cast<int64_t>(s) * kFlowTriSB + i * (i + 1) / 2) * kFlowBlk,
+             bytes, bar);
   }
-  __syncthreads();  // every warp is done with its tile values: S becomes part
-  double *part = S;
+  flow_fetch(a, N);
+  double zr = 0.0;
+  if (mine) {
+    Gather<NR> g;
+    g.begin(a, f.zofs + r0 + row, a.z + v);
+    zr = g.finish(a, a.z + v, a.x[v * a.n + f.col0 + r0 + row], polls);
+  }
+  double acc[NR];
 #pragma unroll
-  for (int k = 0; k < NR; k++) part[(qq * NR + k) * kNB + rr] = acc[k];
+  for (int k = 0; k < NR; k++) acc[k] = 0.0;
+  if (s > 0) {
+    rows_apply_m<1, NR>(a, a.panel + f.panel, f.h, r0 + lane, lane < I.item.nr, s * kFlowSB,
+                        a.y + ((I.ticket % kMultiCopies) * a.n + f.col0) * NR, own, acc, polls);
+    put_entry<NR>(own + NR * lane, acc);
+    __syncthreads();
+    if (row < 32) {
+      double t[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+      for (int q = 0; q < 16; q++) t[q % 4] += yw[32 * NR * q + tid];
+      zr -= (t[0] + t[1]) + (t[2] + t[3]);
+    }
+    __syncthreads();
+  }
+  double *yz = a.yz + static_cast<int64_t>(NR) * (f.col0 + s * kFlowSB);
+  if (row < 32) {
+    if (!last && I.publish) st_relaxed_f64(yz + 32 * NR * i + tid, zr);
+    yw[tid] = zr;  // the diagonal block's, for warp 0
+  }
   __syncthreads();
-  for (int k = qq; k < NR; k += 4)
-    if (r < h) {
-      const double *p = part + k * kNB + rr;
-      zs[k * kNB + rr] -= (p[0] + p[NR * kNB]) + (p[2 * NR * kNB] + p[3 * NR * kNB]);
+  bulk_wait(bar, phase, a.err);
+  phase ^= 1;
+  if (warp <= i) {
+    const int j = warp == 0 ? i : warp - 1;
+    if (warp > 0) get_entry<NR>(yz + NR * (32 * j + lane), true, own + NR * lane, a.err, polls);
+    __syncwarp();
+    block_rows<NR>(inv + j * kFlowBlk + lane, own, acc);
+    __syncwarp();
+    put_entry<NR>(own + NR * lane, acc);
+  }
+  __syncthreads();
+  if (mine) {
+    double t[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+    for (int q = 0; q < 16; q++)
+      if (q <= i) t[q % 4] += yw[32 * NR * q + tid];
+    const double  y = (t[0] + t[1]) + (t[2] + t[3]);
+    const int64_t g = static_cast<int64_t>(NR) * (f.col0 + r0) + tid;
+    if (I.publish) {
+#pragma unroll
+      for (int c = 0; c < kMultiCopies; c++) st_relaxed_f64(a.y + c * a.n * NR + g, y);
     }
-  if (R < F.nb) {
-    const int nbk = min(kNB, w - R * kNB);
-    cp_async_wait_all();
-    __syncthreads();  // z complete, Linv_R staged
-    const int i = rr;
-    for (int k = qq; k < NR; k += 4) {
-      double y = 0.0;
-      if (i < nbk) {
-        const double *row = tri + i * (i + 1) / 2;
-        const double *zk  = zs + k * kNB;
-        double        a0 = 0.0, a1 = 0.0;
-        int           j = 0;
-        for (; j + 1 <= i; j += 2) {
-          a0 += row[j] * zk[j];
-          a1 += row[j + 1] * zk[j + 1];
-        }
-        if (j <= i) a0 += row[j] * zk[j];
-        y = a0 + a1;
-      }
-      yb[k * kNB + i] = y;
-      if (i < nbk && sPublish) {
-        const int64_t gj = F.col0 + static_cast<int64_t>(R) * kNB + i;
+    a.f[g] = y;
+  }
+}
+
+template <int NR, class T>
+__device__ __noinline__ void fwd_rows_m(const FlowArgs<T> &a, const FlowSlot &I, FlowSlot &N, double *sm) {
+  const FlowFront &f   = I.item.f;
+  const int        tid = threadIdx.x, warp = tid / 32, lane = tid % 32;
+  const long       polls = I.polls;
+  const int        r0 = I.item.r0, nr = I.item.nr;
+  double          *yw = sm + kFlowInvSmem, *own = yw + 32 * NR * warp;
+  const int        rl = 32 * (warp % 4) + lane;
+  flow_fetch(a, N);
+  double acc[NR];
 #pragma unroll
-        for (int c = 0; c < kMultiCopies; c++)
-          st_relaxed_f64(ready + (static_cast<int64_t>(c) * NR + k) * n + gj, y);
-        x[k * n + gj] = y;
-      }
-    }
-    if ((R + 1) * kNB > w && h > w) {
-      // Rows of this block at or past w: their product with the block.
-      __syncthreads();
-      if (r >= w && r < h) {
-        double a[NR / 4 > 0 ? NR / 4 : 1];
-        constexpr int KG = NR / 4 > 0 ? NR / 4 : 1;
+  for (int k = 0; k < NR; k++) acc[k] = 0.0;
+  rows_apply_m<4, NR>(a, a.panel + f.panel, f.h, r0 + rl, rl < nr, f.w,
+                      a.y + ((I.ticket % kMultiCopies) * a.n + f.col0) * NR, own, acc, polls);
+  put_entry<NR>(own + NR * lane, acc);
+  // Output e: row e / NR, vector e % NR; its column quarters are 4 warps apart.
+  constexpr int KO = NR / 4;
+  Gather<NR>    g[KO];
 #pragma unroll
-        for (int t = 0; t < KG; t++) a[t] = 0.0;
-        for (int k2 = 0; k2 < nbk; k2++) {
-          const double l = static_cast<double>(to_f(P[r + static_cast<int64_t>(R * kNB + k2) * h]));
+  for (int m = 0; m < KO; m++) {
+    const int e = tid + 512 * m;
+    if (e / NR < nr) g[m].begin(a, f.zofs + r0 + e / NR, a.z + e % NR);
+  }
+  __syncthreads();
 #pragma unroll
-          for (int t = 0; t < KG; t++) {
-            const int k = qq + 4 * t;
-            if (k < NR) a[t] += l * yb[k * kNB + k2];
-          }
-        }
-#pragma unroll
-        for (int t = 0; t < KG; t++) {
-          const int k = qq + 4 * t;
-          if (k < NR) zs[k * kNB + rr] -= a[t];
-        }
-      }
+  for (int m = 0; m < KO; m++) {
+    const int e = tid + 512 * m;
+    if (e / NR < nr) {
+      const double *p = yw + e;
+      const double  t = (p[0] + p[128 * NR]) + (p[256 * NR] + p[384 * NR]);
+      const double  u = g[m].finish(a, a.z + e % NR, 0.0, polls) - t;
+      if (I.publish) st_relaxed_f64(a.z + NR * (f.zofs + r0) + e, u);
     }
   }
-  if (r >= w && r < h)
-    for (int k = qq; k < NR; k += 4) zbuf[k * zld + F.zofs + r] = zs[k * kNB + rr];
+}
+
+template <int RG, int NR, class T>
+__device__ __noinline__ void fwd_narrow_m(const FlowArgs<T> &a, FlowShared &S, const FlowSlot &I,
+                                          FlowSlot &N, double *sm, uint32_t &phase) {
+  const FlowFront &f   = I.item.f;
+  const int        tid = threadIdx.x, warp = tid / 32, lane = tid % 32;
+  const int        w = f.w, nbw = (w + 31) / 32, nr = I.item.nr;
+  const long       polls = I.polls;
+  constexpr int    KO = NR / 4;
+  double          *inv = sm, *zs = sm + kNarrowInv, *ys = zs + 128 * NR, *part = ys + 128 * NR;
+  const uint32_t   bar = smem_addr(&S.bar);
+  if (tid == 0) {
+    const uint32_t bytes = nbw * (nbw + 1) / 2 * kFlowBlk * sizeof(double);
+    bulk_expect(bar, bytes);
+    bulk_get(inv, a.inv + f.inv, bytes, bar);
+  }
+  constexpr int kTile = 32 * RG;
+  const int     cq = warp / RG, rt = tid % kTile;
+  const int64_t r0 = I.item.r0;
+  const T      *P  = a.panel + f.panel;
+  float         lv[32], lvn[32];
+  load_cols(lv, P, f.h, r0 + rt, rt < nr, 32 * cq, w);
+  flow_fetch(a, N);
+  {
+    Gather<NR> g[KO];
+#pragma unroll
+    for (int m = 0; m < KO; m++) {
+      const int e = tid + 512 * m;
+      if (e < w * NR) g[m].begin(a, f.zofs + e / NR, a.z + e % NR);
+    }
+#pragma unroll
+    for (int m = 0; m < KO; m++) {
+      const int e = tid + 512 * m;
+      if (e < 128 * NR)
+        zs[e] = e < w * NR ? g[m].finish(a, a.z + e % NR, a.x[(e % NR) * a.n + f.col0 + e / NR], polls)
+                           : 0.0;
+    }
+  }
+  __syncthreads();
+  bulk_wait(bar, phase, a.err);
+  phase ^= 1;
+  {
+    // y = Inv z: thread (row tid % 128, vectors KO (tid / 128) ..)
+    const int i = tid % 128, vg = KO * (tid / 128), bi = i / 32;
+    double    y[KO];
+#pragma unroll
+    for (int k = 0; k < KO; k++) y[k] = 0.0;
+    if (bi < nbw)
+      for (int j = 0; j <= bi; j++) {
+        const double *blk = inv + (bi * (bi + 1) / 2 + j) * kFlowBlk + lane, *z = zs + 32 * NR * j + vg;
+#pragma unroll 8
+        for (int c = 0; c < 32; c++) {
+          const double l = blk[33 * c];
+#pragma unroll
+          for (int k = 0; k < KO; k++) y[k] += l * z[NR * c + k];
+        }
+      }
+#pragma unroll
+    for (int k = 0; k < KO; k++) {
+      ys[NR * i + vg + k] = i < w ? y[k] : 0.0;
+      if (i < w && r0 == w) a.f[static_cast<int64_t>(NR) * (f.col0 + i) + vg + k] = y[k];
+    }
+  }
+  __syncthreads();
+  for (int q = 0; q * kTile < nr; q++) {
+    const int rn = (q + 1) * kTile + rt;
+    if ((q + 1) * kTile < nr) load_cols(lvn, P, f.h, r0 + rn, rn < nr, 32 * cq, w);
+    double acc[NR];
+#pragma unroll
+    for (int k = 0; k < NR; k++) acc[k] = 0.0;
+#pragma unroll
+    for (int k = 0; k < 32; k++) fma_entry<NR>(static_cast<double>(lv[k]), ys + NR * (32 * cq + k), acc);
+    if (RG == 16) {
+      // one tile; the thread's row: its children's values, then the result
+      if (rt < nr) {
+        double u[NR];
+#pragma unroll
+        for (int k = 0; k < NR; k++) u[k] = 0.0;
+        const int2 g = a.gfirst[f.zofs + r0 + rt];
+        add_entry<NR>(a.z + static_cast<int64_t>(NR) * g.x, g.x >= 0, u, a.err, polls);
+        if (g.y >= 0)
+          for (int e = 1, n = a.gmore[g.y]; e <= n; e++)
+            add_entry<NR>(a.z + static_cast<int64_t>(NR) * a.gmore[g.y + e], true, u, a.err, polls);
+        if (I.publish) {
+          double *z = a.z + NR * (f.zofs + r0 + rt);
+#pragma unroll
+          for (int k = 0; k < NR; k += 2) st_relaxed_2(z + k, u[k] - acc[k], u[k + 1] - acc[k + 1]);
+        }
+      }
+    } else {
+      put_entry<NR>(part + NR * (128 * cq + rt), acc);
+      Gather<NR> g[KO];
+      const int  base = q * kTile * NR;  // output e of the item: row e / NR
+#pragma unroll
+      for (int m = 0; m < KO; m++) {
+        const int e = base + tid + 512 * m;
+        if (e / NR < nr) g[m].begin(a, f.zofs + r0 + e / NR, a.z + e % NR);
+      }
+      __syncthreads();
+#pragma unroll
+      for (int m = 0; m < KO; m++) {
+        const int e = base + tid + 512 * m;
+        if (e / NR < nr) {
+          const double *p = part + tid + 512 * m;
+          const double  t = (p[0] + p[128 * NR]) + (p[256 * NR] + p[384 * NR]);
+          const double  u = g[m].finish(a, a.z + e % NR, 0.0, polls) - t;
+          if (I.publish) st_relaxed_f64(a.z + NR * (f.zofs + r0) + e, u);
+        }
+      }
+      __syncthreads();
+    }
+#pragma unroll
+    for (int k = 0; k < 32; k++) lv[k] = lvn[k];
+  }
+}
+
+// The panels of an item's warp-solved fronts into shared memory: warp q starts
+// the copy of front q.
+template <class T>
+__device__ __forceinline__ void panels_get(const FlowArgs<T> &a, FlowShared &S, const FlowSlot &I,
+                                           double *sm) {
+  const int warp = threadIdx.x / 32;
+  if (warp < I.item.nr) warp_panel(a, a.warps[I.item.r0 + warp], sm, smem_addr(&S.wbar[warp]));
+}
+
+// kFlowWarps: two vectors of a front per warp, NR / 2 warps a front, 32 / NR
+// fronts at a time.
+template <int NR, class T>
+__device__ __noinline__ void fwd_warp_m(const FlowArgs<T> &a, FlowShared &S, const FlowSlot &I, FlowSlot &N,
+                                        double *sm, uint32_t &wphase) {
+  constexpr int WF = NR / 2, FR = 16 / WF, RT = kWarpSolveH / 32;
+  const int     warp = threadIdx.x / 32, lane = threadIdx.x % 32, vg = 2 * (warp % WF);
+  const long    polls = I.polls;
+  double       *zs = sm + kFlowInvSmem + 128 * warp, *ys = zs + 64;
+  panels_get(a, S, I, sm);
+  flow_fetch(a, N);
+  for (int q = warp / WF; q < I.item.nr; q += FR) {
+    const FlowFront f = a.warps[I.item.r0 + q];
+    const int       w = f.w, h = f.h, ld = h | 1;
+    const double   *M = sm + f.part / 8 + lane;
+    double          z[RT][2];
+    int2            g[RT];
+    bool            more = false;
+#pragma unroll
+    for (int t = 0; t < RT; t++) {
+      g[t] = make_int2(-1, -1);
+      if (lane + 32 * t < h) g[t] = a.gfirst[f.zofs + lane + 32 * t];
+      z[t][0] = z[t][1] = 0.0;
+      more |= g[t].y >= 0;
+    }
+    if (lane < w) {
+      z[0][0] = a.x[vg * a.n + f.col0 + lane];
+      z[0][1] = a.x[(vg + 1) * a.n + f.col0 + lane];
+    }
+    // first children of all rows, polled together
+    unsigned need = 0;
+#pragma unroll
+    for (int t = 0; t < RT; t++)
+      if (g[t].x >= 0) need |= 1u << t;
+    for (long it = 0; need != 0; it++) {
+      V2 raw[RT];
+#pragma unroll
+      for (int t = 0; t < RT; t++) {
+        raw[t] = V2{kPending, kPending};
+        if (need >> t & 1u) raw[t] = ld_relaxed_2(a.z + static_cast<int64_t>(NR) * g[t].x + vg);
+      }
+#pragma unroll
+      for (int t = 0; t < RT; t++)
+        if (raw[t].a != kPending && raw[t].b != kPending) {
+          z[t][0] += __longlong_as_double(static_cast<long long>(raw[t].a));
+          z[t][1] += __longlong_as_double(static_cast<long long>(raw[t].b));
+          need &= ~(1u << t);
+        }
+      if (need != 0 && it >= polls) {
+        atomicExch(a.err, 1);
+        break;
+      }
+      if ((it & 63) == 63) {
+        if (*reinterpret_cast<volatile int32_t *>(a.err) != 0) break;
+        __nanosleep(32);
+      }
+    }
+    if (more) {
+#pragma unroll
+      for (int t = 0; t < RT; t++)
+        if (g[t].y >= 0)
+          for (int e = 1, n = a.gmore[g[t].y]; e <= n; e++)
+            add_entry<2>(a.z + static_cast<int64_t>(NR) * a.gmore[g[t].y + e] + vg, true, z[t], a.err, polls);
+    }
+    put_entry<2>(zs + 2 * lane, z[0]);
+    __syncwarp();
+    bulk_wait(smem_addr(&S.wbar[q]), wphase >> q & 1u, a.err);
+    double y[2] = {0.0, 0.0};
+#pragma unroll 4
+    for (int k = 0; k < w; k++) fma_entry<2>(M[k * ld], zs + 2 * k, y);
+    put_entry<2>(ys + 2 * lane, y);  // entries at or past w are not used
+    __syncwarp();
+    if (lane < w) {
+      a.f[static_cast<int64_t>(NR) * (f.col0 + lane) + vg]     = y[0];
+      a.f[static_cast<int64_t>(NR) * (f.col0 + lane) + vg + 1] = y[1];
+    }
+#pragma unroll
+    for (int t = 0; t < RT; t++) {
+      if (32 * t >= h) break;
+      double u[2] = {0.0, 0.0};
+#pragma unroll 4
+      for (int k = 0; k < w; k++) fma_entry<2>(M[k * ld + 32 * t], ys + 2 * k, u);
+      const int i = lane + 32 * t;
+      if (i >= w && i < h && I.publish)
+        st_relaxed_2(a.z + NR * (f.zofs + i) + vg, z[t][0] - u[0], z[t][1] - u[1]);
+    }
+    __syncwarp();
+  }
+  // Barrier q is used once an item, whichever warps wait on it.
+  wphase ^= (1u << I.item.nr) - 1u;
+}
+
+template <int NR, class T>
+__global__ void __launch_bounds__(kFlowThreads, 1) k_fwd_flow_m(const __grid_constant__ FlowArgs<T> a) {
+  extern __shared__ __align__(128) double sm[];
+  __shared__ __align__(16) FlowShared S;
+  uint32_t phase = 0, wphase = 0;
+  flow_loop(a, S, [&](const FlowSlot &I, FlowSlot &N) {
+    switch (I.item.kind) {
+      case kFlowWarps: fwd_warp_m<NR>(a, S, I, N, sm, wphase); break;
+      case kFwdNarrow:
+        if (I.item.f.w <= 32)
+          fwd_narrow_m<16, NR>(a, S, I, N, sm, phase);
+        else
+          fwd_narrow_m<4, NR>(a, S, I, N, sm, phase);
+        break;
+      case kFwdSlab: fwd_slab_m<NR>(a, S, I, N, sm, phase); break;
+      default: fwd_rows_m<NR>(a, I, N, sm);
+    }
+  });
+  flow_mark(a.mark, a.nmark);
 }
 
 // ---------------------------------------------------------------------------
-// Backward, off-diagonal rows: CTA c takes rows w + 128 c .. of one front and
-// writes t_col = sum_r L_{r,col} x_r of every column for all NR vectors (warp
-// per column, rows over the lanes; per vector the sums of k_bwd_chunks).
-template <int NR, class T>
-__global__ void __launch_bounds__(kSolveThreads)
-    k_bwd_chunks_m(const SolveFront *fr, const int32_t *fmap, const T *panel,
-                   const int32_t *srows, const double *x, double *part, int64_t pld) {
-  __shared__ double zr[NR][kNB];
-  const SolveFront  F = fr[fmap[blockIdx.x]];
-  const int         c = blockIdx.x - F.chunk0;
-  const int         tid = threadIdx.x, warp = tid / 32, lane = tid % 32;
-  const int64_t     h = F.h, w = F.w, n = F.n;
-  const int64_t     r0 = w + static_cast<int64_t>(c) * kNB;
-  const int         nr = static_cast<int>(h - r0 < kNB ? h - r0 : kNB);
-  for (int e = tid; e < NR * kNB; e += kSolveThreads) {
-    const int k = e / kNB, i = e % kNB;
-    zr[k][i] = i < nr ? x[k * n + srows[F.rows + r0 + i]] : 0.0;
-  }
-  __syncthreads();
-  const T      *P  = panel + F.panel + r0;
-  constexpr int kWarps = kSolveThreads / 32;
-  for (int64_t col = warp; col < w; col += kWarps) {
-    const T     *cp = P + col * h;
-    double       l[4];
+// Backward.
+
+// Sums over the lanes of K values each (K = 8, 16 or 32): lane l returns the
+// sum of value l / (32 / K).  At each of the first levels a lane keeps half of
+// its values and sends the other half.
+template <int K>
+__device__ __forceinline__ double reduce_lanes(double (&v)[K]) {
+  const unsigned full = 0xffffffffu;
+  const int      lane = threadIdx.x % 32;
+  int            o    = 16;
 #pragma unroll
-    for (int i = 0; i < 4; i++) {
-      const int rr = lane + 32 * i;
-      l[i]         = rr < nr ? static_cast<double>(to_f(__ldg(cp + rr))) : 0.0;
+  for (int m = K / 2; m >= 1; m /= 2) {
+    const bool up = lane & o;
+#pragma unroll
+    for (int u = 0; u < m; u++) {
+      const double keep = up ? v[u + m] : v[u], send = up ? v[u] : v[u + m];
+      v[u] = keep + __shfl_xor_sync(full, send, o);
     }
-#pragma unroll
-    for (int k = 0; k < NR; k++) {
-      double s = 0.0;
-#pragma unroll
-      for (int i = 0; i < 4; i++)
-        if (lane + 32 * i < nr) s += l[i] * zr[k][lane + 32 * i];
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-      if (lane == 0) part[k * pld + F.part + static_cast<int64_t>(c) * w + col] = s;
-    }
+    o /= 2;
   }
+  for (; o >= 1; o /= 2) v[0] += __shfl_xor_sync(full, v[0], o);
+  return v[0];
 }
 
-// Backward, column blocks: one CTA per column block b (tickets as in
-// k_bwd_fronts).  Thread (c, g) = (tid % 128, tid / 128) takes column c of
-// the block and vectors g KG .. g KG + KG - 1.  Each tile of L (row block R
-// below the block, last first) is loaded into registers by rows (coalesced)
-// while the previous tile is applied, then stored to shared memory and read
-// by columns; the CTA waits for x_R of all vectors before applying tile R.
+// acc[NR j + k] += sum_i lv[j][i] x(lane + 32 i, k), the x values in shared
+// memory, a row every NR + 2 doubles (16-byte reads free of bank conflicts).
 template <int NR>
-constexpr int bwd_m_smem_doubles() {
-  return kTriM + (kNB * kLsPitch + 1) / 2 + 2 * NR * kNB;
-}
-
-template <int NR, class T>
-__global__ void __launch_bounds__(kSolveThreads, 1)
-    k_bwd_fronts_m(const SolveItem *items, const T *panel, const double *linv64t,
-                   double *x, const double *part, int64_t pld, int32_t *tickets,
-                   double *ready, int32_t *err) {
-  constexpr int KG = NR / 4;
-  extern __shared__ __align__(16) double sm[];
-  double *tri = sm;                                             // packed lower Linv_b
-  float  *Ls  = reinterpret_cast<float *>(tri + kTriM);         // [kNB][kLsPitch]
-  double *xs  = tri + kTriM + (kNB * kLsPitch + 1) / 2;         // [kNB][NR]
-  double *v   = xs + NR * kNB;                                  // [NR][kNB]
-  __shared__ SolveFront sF;
-  __shared__ int        sB, sItem;
-  __shared__ long       sPolls;
-  if (threadIdx.x == 0) {
-    const int it = atomicAdd(tickets, 1);
-    sItem        = it;
-    sF           = items[it].f;
-    sB           = items[it].r;
-    sPolls       = poll_limit(reinterpret_cast<const volatile SolveCtl *>(err)->poll_log2);
-  }
-  __syncthreads();
-  const int         item  = sItem;
-  const SolveFront &F     = sF;
-  const int         b     = sB;
-  const long        polls = sPolls;
-  const int         tid = threadIdx.x, c = tid % kNB, g = tid / kNB;
-  const int64_t     h = F.h, n = F.n;
-  const int         w = F.w;
-  const int         nbk = min(kNB, w - b * kNB);
-  stage_tri_m(linv64t + F.linv + static_cast<int64_t>(b) * kNB * kNB, tri, nbk);
-  // This block's right-hand side and the chunk partials of its columns.
-  double rhs[KG], acc[KG];
+__device__ __forceinline__ void tile_cols(const float (&lv)[2][16], const double *xs,
+                                          double (&acc)[2 * NR]) {
+  const int lane = threadIdx.x % 32;
+#pragma unroll 4
+  for (int i = 0; i < 16; i++) {
+    const double  l0 = static_cast<double>(lv[0][i]), l1 = static_cast<double>(lv[1][i]);
+    const double *x  = xs + (NR + 2) * (lane + 32 * i);
 #pragma unroll
-  for (int t = 0; t < KG; t++) {
-    const int k = g * KG + t;
-    rhs[t]      = c < nbk ? x[k * n + F.col0 + b * kNB + c] : 0.0;
-    double s    = 0.0;
-    if (c < nbk)
-      for (int ch = 0; ch < F.chunks; ch++)
-        s += part[k * pld + F.part + static_cast<int64_t>(ch) * w + b * kNB + c];
-    acc[t] = s;
-  }
-  const T     *P    = panel + F.panel;
-  const int    copy = (item * 16 + g) % kMultiCopies;
-  // Tile R: thread (rr, cg) = (tid % 128, tid / 128) loads row rr, columns
-  // 32 cg .. 32 cg + 31 of the block.
-  float     lr[32];
-  const int trr = tid % kNB, tcg = tid / kNB;
-  auto      load_tile = [&](int R) {
-    const int64_t rb   = static_cast<int64_t>(R) * kNB;
-    const int     rows = min(kNB, w - R * kNB);
-#pragma unroll
-    for (int k = 0; k < 32; k++) {
-      const int cc = tcg * 32 + k;
-      lr[k] = (trr < rows && cc < nbk)
-                  ? to_f(__ldg(P + rb + trr + static_cast<int64_t>(b * kNB + cc) * h))
-                  : 0.0f;
-    }
-  };
-  if (F.nb - 1 > b) load_tile(F.nb - 1);
-  for (int R = F.nb - 1; R > b; R--) {
-    const int rows = min(kNB, w - R * kNB);
-    // x_R of the KG vectors of this thread's group, row trr.
-    wait_many<KG>(ready + (static_cast<int64_t>(copy) * NR + tcg * KG) * n + F.col0 +
-                      static_cast<int64_t>(R) * kNB + trr,
-                  n, trr < rows, xs + trr * NR + tcg * KG, 1, err, polls);
-#pragma unroll
-    for (int k = 0; k < 32; k++) Ls[trr * kLsPitch + tcg * 32 + k] = lr[k];
-    __syncthreads();
-    if (R - 1 > b) load_tile(R - 1);
-    for (int rr = 0; rr < rows; rr++) {
-      const double l = static_cast<double>(Ls[rr * kLsPitch + c]);
-#pragma unroll
-      for (int t = 0; t < KG; t++) acc[t] += l * xs[rr * NR + g * KG + t];
-    }
-    __syncthreads();
-  }
-#pragma unroll
-  for (int t = 0; t < KG; t++) v[(g * KG + t) * kNB + c] = c < nbk ? rhs[t] - acc[t] : 0.0;
-  cp_async_wait_all();
-  __syncthreads();
-  // x_b = Linv_b^T v: x_c = sum_{i >= c} Linv[i][c] v_i.
-  const int i0 = c & ~31;
-#pragma unroll
-  for (int t = 0; t < KG; t++) {
-    const int     k  = g * KG + t;
-    const double *vk = v + k * kNB;
-    double        s  = 0.0;
-    for (int i = i0; i < nbk; i++)
-      if (i >= c) s += tri[i * (i + 1) / 2 + c] * vk[i];
-    if (c < nbk) {
-      const int64_t j = F.col0 + static_cast<int64_t>(b) * kNB + c;
-#pragma unroll
-      for (int cp = 0; cp < kMultiCopies; cp++)
-        st_relaxed_f64(ready + (static_cast<int64_t>(cp) * NR + k) * n + j, s);
-      x[k * n + j] = s;
+    for (int q = 0; q < NR; q += 2) {
+      const double2 v = *reinterpret_cast<const double2 *>(x + q);
+      acc[q] += l0 * v.x;
+      acc[q + 1] += l0 * v.y;
+      acc[NR + q] += l1 * v.x;
+      acc[NR + q + 1] += l1 * v.y;
     }
   }
 }
 
-template <int NR, class T>
-void set_smem_attrs() {
-  static std::atomic<bool> done{false};  // idempotent; set once per process
-  if (done) return;
-  MPIR_CUDA(cudaFuncSetAttribute(k_fwd_fronts_m<NR, T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 static_cast<int>(fwd_m_smem_doubles<NR>() * sizeof(double))));
-  MPIR_CUDA(cudaFuncSetAttribute(k_bwd_fronts_m<NR, T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 static_cast<int>(bwd_m_smem_doubles<NR>() * sizeof(double))));
-  const int small = static_cast<int>(kSmallWarpsM * NR * kWarpSolveH * sizeof(double));
-  MPIR_CUDA(cudaFuncSetAttribute(k_fwd_small_m<NR, T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 small));
-  MPIR_CUDA(cudaFuncSetAttribute(k_bwd_small_m<NR, T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 small));
-  done = true;
+// t(c, k) = sum_r L(r, c) x(r, k) over up to 512 rows below the block, for
+// columns [c0, cend): emit(c, k, t) by one lane a value.
+template <int NR, class T, class Emit>
+__device__ __forceinline__ void chunk_cols_m(const FlowArgs<T> &a, const FlowFront &f, int64_t rb, int nr,
+                                             int c0, int cend, double *xs, long polls, FlowSlot &N,
+                                             Emit emit) {
+  const int tid = threadIdx.x, warp = tid / 32, lane = tid % 32;
+  const T  *P = a.panel + f.panel;
+  float     lv[2][16];
+  load_rows(lv, P, f.h, rb, nr, c0, cend);
+  flow_fetch(a, N);
+  const int row = tid < nr ? a.srows[f.rows + rb + tid] : -1;
+  wait_gate(a, f.gate < 0 ? -1 : NR * f.gate, polls);
+  get_entry<NR>(a.xr + static_cast<int64_t>(NR) * row, row >= 0, xs + (NR + 2) * tid, a.err, polls);
+  __syncthreads();
+  for (int c = c0; c < cend; c += 32) {
+    double acc[2 * NR];
+#pragma unroll
+    for (int k = 0; k < 2 * NR; k++) acc[k] = 0.0;
+    tile_cols<NR>(lv, xs, acc);
+    if (c + 32 < cend) load_rows(lv, P, f.h, rb, nr, c + 32, cend);
+    const double t   = reduce_lanes<2 * NR>(acc);
+    constexpr int kL = 16 / NR;  // lanes a value
+    const int    e   = lane / kL, col = c + 2 * warp + e / NR;
+    if (lane % kL == 0 && col < cend) emit(col, e % NR, t);
+  }
 }
+
+template <int NR, class T>
+__device__ __noinline__ void bwd_chunk_m(const FlowArgs<T> &a, const FlowSlot &I, FlowSlot &N, double *sm) {
+  const FlowFront &f  = I.item.f;
+  const int        c  = I.item.c0;
+  const int64_t    rb = f.w + static_cast<int64_t>(c) * kFlowChunk;
+  const int        nr = static_cast<int>(min(static_cast<int64_t>(kFlowChunk), f.h - rb));
+  double          *pp = a.part + NR * (f.part + static_cast<int64_t>(c) * f.w);
+  chunk_cols_m<NR>(a, f, rb, nr, I.item.r0, I.item.r0 + I.item.nr, sm + kFlowInvSmem, I.polls, N,
+                   [&](int col, int k, double t) { st_relaxed_f64(pp + NR * col + k, t); });
+}
+
+// The sum of the chunk partials of output e (column e / NR, vector e % NR),
+// four polled at a time.
+template <int NR, class T>
+__device__ __forceinline__ double chunk_sum(const FlowArgs<T> &a, const FlowFront &f, int e, long polls) {
+  const double *p = a.part + NR * f.part + e;
+  const int64_t d = static_cast<int64_t>(NR) * f.w;
+  double        s = 0.0;
+  for (int c = 0; c < f.chunks; c += 4) {
+    unsigned long long raw[4];
+#pragma unroll
+    for (int u = 0; u < 4; u++) raw[u] = c + u < f.chunks ? ld_relaxed_u64(p + (c + u) * d) : 0ull;
+#pragma unroll
+    for (int u = 0; u < 4; u++)
+      if (c + u < f.chunks) s += take_value(raw[u], p + (c + u) * d, a.err, polls);
+  }
+  return s;
+}
+
+template <int NR, class T>
+__device__ __noinline__ void bwd_narrow_m(const FlowArgs<T> &a, FlowShared &S, const FlowSlot &I,
+                                          FlowSlot &N, double *sm, uint32_t &phase) {
+  const FlowFront &f   = I.item.f;
+  const int        tid = threadIdx.x, lane = tid % 32;
+  const int        w = f.w, nbw = (w + 31) / 32;
+  const long       polls = I.polls;
+  constexpr int    KO = NR / 4;
+  double          *inv = sm, *xs = sm + kNarrowInv, *vs = xs + 512 * (NR + 2);
+  const uint32_t   bar = smem_addr(&S.bar);
+  if (tid == 0) {
+    const uint32_t bytes = nbw * (nbw + 1) / 2 * kFlowBlk * sizeof(double);
+    bulk_expect(bar, bytes);
+    bulk_get(inv, a.inv + f.inv, bytes, bar);
+  }
+  // vs: the right-hand side less the rows below
+  double v[KO];
+#pragma unroll
+  for (int m = 0; m < KO; m++) {
+    const int e = tid + 512 * m;
+    v[m]        = 0.0;
+    if (e < w * NR) {
+      v[m] = a.f[static_cast<int64_t>(NR) * f.col0 + e];
+      if (a.Dinv) v[m] *= static_cast<double>(a.Dinv[f.col0 + e / NR]);
+    }
+  }
+  if (f.chunks > 0 || f.h == w) flow_fetch(a, N);
+  if (f.chunks == 0 && f.h > w) {
+    chunk_cols_m<NR>(a, f, w, f.h - w, 0, w, xs, polls, N,
+                     [&](int col, int k, double t) { vs[NR * col + k] = t; });
+    __syncthreads();
+  }
+#pragma unroll
+  for (int m = 0; m < KO; m++) {
+    const int e = tid + 512 * m;
+    if (e < w * NR && f.h > w) v[m] -= f.chunks > 0 ? chunk_sum<NR>(a, f, e, polls) : vs[e];
+  }
+  __syncthreads();
+#pragma unroll
+  for (int m = 0; m < KO; m++)
+    if (tid + 512 * m < 128 * NR) vs[tid + 512 * m] = v[m];
+  __syncthreads();
+  bulk_wait(bar, phase, a.err);
+  phase ^= 1;
+  // x = Inv^T v: thread (column tid % 128, vectors KO (tid / 128) ..)
+  const int i = tid % 128, vg = KO * (tid / 128), bj = i / 32;
+  double    x[KO];
+#pragma unroll
+  for (int k = 0; k < KO; k++) x[k] = 0.0;
+  for (int b = bj; b < nbw; b++) {
+    const double *blk = inv + (b * (b + 1) / 2 + bj) * kFlowBlk + 33 * lane, *z = vs + 32 * NR * b + vg;
+#pragma unroll 8
+    for (int r = 0; r < 32; r++) {
+      const double l = blk[r];
+#pragma unroll
+      for (int k = 0; k < KO; k++) x[k] += l * z[NR * r + k];
+    }
+  }
+  if (i < w) {
+#pragma unroll
+    for (int k = 0; k < KO; k++) {
+      st_relaxed_f64(a.xr + static_cast<int64_t>(NR) * (f.col0 + i) + vg + k, x[k]);
+      a.x[(vg + k) * a.n + f.col0 + i] = x[k];
+    }
+  }
+}
+
+template <int NR, class T>
+__device__ __noinline__ void bwd_slab_m(const FlowArgs<T> &a, FlowShared &S, const FlowSlot &I, FlowSlot &N,
+                                        double *sm, uint32_t &phase) {
+  const FlowFront &f   = I.item.f;
+  const int        tid = threadIdx.x, warp = tid / 32, lane = tid % 32;
+  const int        col = tid / NR, vv = tid % NR;  // the thread's output, tid < 32 NR
+  const long       polls = I.polls;
+  const int        w = f.w, k0 = I.item.r0, s = k0 / kFlowSB, j = (k0 % kFlowSB) / 32;
+  const int        nsl = min(16, (w - s * kFlowSB + 31) / 32), nsb = (w + kFlowSB - 1) / kFlowSB;
+  const bool       mine = col < I.item.nr;
+  double          *inv = sm, *xs = sm + kFlowInvSmem, *own = xs + 32 * NR * warp;
+  const uint32_t   bar = smem_addr(&S.bar);
+  if (tid == 0) {
+    bulk_expect(bar, (nsl - j) * kFlowBlk * sizeof(double));
+    for (int i = j; i < nsl; i++)
+      bulk_get(inv + (i - j) * kFlowBlk,
+               a.inv + f.inv +
+                   (static_cast<int64_t>(s) * kFlowTriSB + i * (i + 1) / 2 + j) * kFlowBlk,
+               kFlowBlk * sizeof(double), bar);
+  }
+  const T      *P    = a.panel + f.panel;
+  const double *xr   = a.xr + ((I.ticket % kMultiCopies) * a.n + f.col0) * NR;
+  const int     cend = k0 + I.item.nr;
+  float         lv[2][16];
+  if (nsb - 1 > s) load_rows(lv, P, f.h, static_cast<int64_t>(nsb - 1) * kFlowSB,
+                             w - (nsb - 1) * kFlowSB, k0, cend);
+  flow_fetch(a, N);
+  double v = 0.0;
+  if (mine) {
+    v = a.f[static_cast<int64_t>(NR) * (f.col0 + k0) + tid];
+    if (a.Dinv) v *= static_cast<double>(a.Dinv[f.col0 + k0 + col]);
+    if (f.chunks > 0) v -= chunk_sum<NR>(a, f, NR * k0 + tid, polls);
+  }
+  double acc[2 * NR];
+#pragma unroll
+  for (int k = 0; k < 2 * NR; k++) acc[k] = 0.0;
+  for (int R = nsb - 1; R > s; R--) {
+    const int g = R * kFlowSB + tid;
+    get_entry<NR>(xr + static_cast<int64_t>(NR) * g, g < w, xs + (NR + 2) * tid, a.err, polls);
+    __syncthreads();
+    tile_cols<NR>(lv, xs, acc);
+    if (R - 1 > s) load_rows(lv, P, f.h, static_cast<int64_t>(R - 1) * kFlowSB, kFlowSB, k0, cend);
+    __syncthreads();
+  }
+  // Sums of the warp's two columns, to the threads that own the outputs.
+  {
+    const double t   = reduce_lanes<2 * NR>(acc);
+    constexpr int kL = 16 / NR;
+    if (lane % kL == 0) xs[2 * NR * warp + lane / kL] = t;
+  }
+  __syncthreads();
+  if (col < 32) v -= xs[tid];
+  __syncthreads();
+  double *xz = a.xz + static_cast<int64_t>(NR) * (f.col0 + s * kFlowSB);
+  if (col < 32) {
+    if (!mine) v = 0.0;
+    if (j > 0 && mine) st_relaxed_f64(xz + 32 * NR * j + tid, v);
+    xs[tid] = v;  // the diagonal block's, for warp 0
+  }
+  __syncthreads();
+  bulk_wait(bar, phase, a.err);
+  phase ^= 1;
+  if (j + warp < nsl) {
+    const int i = j + warp;
+    if (warp > 0)
+      get_entry<NR>(xz + NR * (32 * i + lane), s * kFlowSB + 32 * i + lane < w, own + NR * lane, a.err,
+                    polls);
+    __syncwarp();
+    double o[NR];
+#pragma unroll
+    for (int k = 0; k < NR; k++) o[k] = 0.0;
+    const double *blk = inv + warp * kFlowBlk + 33 * lane;
+#pragma unroll 8
+    for (int r = 0; r < 32; r++) fma_entry<NR>(blk[r], own + NR * r, o);
+    __syncwarp();
+    put_entry<NR>(own + NR * lane, o);
+  }
+  __syncthreads();
+  if (mine) {
+    double t[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+    for (int q = 0; q < 16; q++)
+      if (j + q < nsl) t[q % 4] += xs[32 * NR * q + tid];
+    const double  x = (t[0] + t[1]) + (t[2] + t[3]);
+    const int64_t g = static_cast<int64_t>(NR) * (f.col0 + k0) + tid;
+#pragma unroll
+    for (int c = 0; c < kMultiCopies; c++) st_relaxed_f64(a.xr + c * a.n * NR + g, x);
+    a.x[vv * a.n + f.col0 + k0 + col] = x;
+  }
+}
+
+template <int NR, class T>
+__device__ __noinline__ void bwd_warp_m(const FlowArgs<T> &a, FlowShared &S, const FlowSlot &I, FlowSlot &N,
+                                        double *sm, uint32_t &wphase) {
+  constexpr int WF = NR / 2, FR = 16 / WF, RT = kWarpSolveH / 32;
+  const int     warp = threadIdx.x / 32, lane = threadIdx.x % 32, vg = 2 * (warp % WF);
+  const long    polls = I.polls;
+  double       *vs = sm + kFlowInvSmem + 576 * warp, *xs = vs + 64;
+  panels_get(a, S, I, sm);
+  flow_fetch(a, N);
+  for (int q = warp / WF; q < I.item.nr; q += FR) {
+    const FlowFront f = a.warps[I.item.r0 + q];
+    const int       w = f.w, h = f.h, ld = h | 1, nr = h - w;
+    double          v[2] = {0.0, 0.0};
+    if (lane < w) {
+      const double *p = a.f + static_cast<int64_t>(NR) * (f.col0 + lane) + vg;
+      const double  d = a.Dinv ? static_cast<double>(a.Dinv[f.col0 + lane]) : 1.0;
+      v[0]            = p[0] * d;
+      v[1]            = p[1] * d;
+    }
+    {
+      int    gi[RT];
+      double xv[RT][2];
+#pragma unroll
+      for (int t = 0; t < RT; t++) {
+        gi[t]    = lane + 32 * t < nr ? a.srows[f.rows + w + lane + 32 * t] : -1;
+        xv[t][0] = xv[t][1] = 0.0;
+      }
+      wait_gate(a, f.gate < 0 ? -1 : NR * f.gate, polls);
+      unsigned need = 0;
+#pragma unroll
+      for (int t = 0; t < RT; t++)
+        if (gi[t] >= 0) need |= 1u << t;
+      for (long it = 0; need != 0; it++) {
+        V2 raw[RT];
+#pragma unroll
+        for (int t = 0; t < RT; t++) {
+          raw[t] = V2{kPending, kPending};
+          if (need >> t & 1u) raw[t] = ld_relaxed_2(a.xr + static_cast<int64_t>(NR) * gi[t] + vg);
+        }
+#pragma unroll
+        for (int t = 0; t < RT; t++)
+          if (raw[t].a != kPending && raw[t].b != kPending) {
+            xv[t][0] = __longlong_as_double(static_cast<long long>(raw[t].a));
+            xv[t][1] = __longlong_as_double(static_cast<long long>(raw[t].b));
+            need &= ~(1u << t);
+          }
+        if (need != 0 && it >= polls) {
+          atomicExch(a.err, 1);
+          break;
+        }
+        if ((it & 63) == 63) {
+          if (*reinterpret_cast<volatile int32_t *>(a.err) != 0) break;
+          __nanosleep(32);
+        }
+      }
+#pragma unroll
+      for (int t = 0; t < RT; t++) put_entry<2>(xs + 2 * (lane + 32 * t), xv[t]);
+    }
+    __syncwarp();
+    bulk_wait(smem_addr(&S.wbar[q]), wphase >> q & 1u, a.err);
+    const bool    half = w <= 16;
+    const double *col  = sm + f.part / 8 + min(half ? lane & 15 : lane, w - 1) * ld;
+    const int     step = half ? 2 : 1;
+    double        t[2] = {0.0, 0.0};
+#pragma unroll 4
+    for (int r = half ? lane >> 4 : 0; r < nr; r += step) fma_entry<2>(col[w + r], xs + 2 * r, t);
+    if (half) {
+      t[0] += __shfl_xor_sync(0xffffffffu, t[0], 16);
+      t[1] += __shfl_xor_sync(0xffffffffu, t[1], 16);
+    }
+    v[0] = lane < w ? v[0] - t[0] : 0.0;
+    v[1] = lane < w ? v[1] - t[1] : 0.0;
+    put_entry<2>(vs + 2 * lane, v);
+    __syncwarp();
+    double x[2] = {0.0, 0.0};
+#pragma unroll 4
+    for (int i = 0; i < w; i++) fma_entry<2>(col[i], vs + 2 * i, x);
+    if (lane < w) {
+      st_relaxed_2(a.xr + static_cast<int64_t>(NR) * (f.col0 + lane) + vg, x[0], x[1]);
+      a.x[vg * a.n + f.col0 + lane]       = x[0];
+      a.x[(vg + 1) * a.n + f.col0 + lane] = x[1];
+    }
+    __syncwarp();
+  }
+  wphase ^= (1u << I.item.nr) - 1u;
+}
+
+template <int NR, class T>
+__global__ void __launch_bounds__(kFlowThreads, 1) k_bwd_flow_m(const __grid_constant__ FlowArgs<T> a) {
+  extern __shared__ __align__(128) double sm[];
+  __shared__ __align__(16) FlowShared S;
+  uint32_t phase = 0, wphase = 0;
+  flow_loop(a, S, [&](const FlowSlot &I, FlowSlot &N) {
+    switch (I.item.kind) {
+      case kFlowWarps: bwd_warp_m<NR>(a, S, I, N, sm, wphase); break;
+      case kBwdChunk: bwd_chunk_m<NR>(a, I, N, sm); break;
+      case kBwdNarrow: bwd_narrow_m<NR>(a, S, I, N, sm, phase); break;
+      default: bwd_slab_m<NR>(a, S, I, N, sm, phase);
+    }
+  });
+  flow_mark(a.mark, a.nmark);
+}
+
+// The handed-over values in one buffer, in entries of NR values.
+struct MultiBuffers {
+  int64_t fwd, bwd;
+  explicit MultiBuffers(const Plan &P)
+      : fwd(P.S.z_elems + (kMultiCopies + 1) * P.S.n),
+        bwd(P.flow_part_elems + (kMultiCopies + 1) * P.S.n) {}
+};
 
 template <int NR, class T>
 void solve_multi_nr(const Plan &P, const Numeric &F, const T *pan, double *X,
-                    MultiSolveWorkspace &ws, cudaStream_t s, int phases) {
-  const Symbolic &S  = P.S;
-  KernelTimer    &kt = kernel_timer();
-  set_smem_attrs<NR, T>();
-  const int64_t     n     = S.n;
-  const double     *lvt   = F.linv64t.as<double>();
-  double           *zbuf  = ws.zbuf.as<double>();
-  const int64_t     zld   = std::max<int64_t>(S.z_elems, 1);
-  const int64_t     pld   = std::max<int64_t>(P.spart_elems, 1);
-  int32_t          *sync  = ws.sync.as<int32_t>();
-  double           *ready = ws.ready.as<double>();
-  int32_t          *err   = ws.err.as<int32_t>();
-  const SolveFront *sf    = P.solve_fronts.as<SolveFront>();
-  const bool        block = P.nblock_fronts > 0;
-  const int64_t     nready = static_cast<int64_t>(kMultiCopies) * NR * n;
-  const unsigned    nmark  = static_cast<unsigned>((nready + 255) / 256);
-  const int         nl     = static_cast<int>(P.levels.size());
-  const size_t      small_smem = kSmallWarpsM * NR * kWarpSolveH * sizeof(double);
-  if (block) MPIR_CUDA(cudaMemsetAsync(sync, 0, P.sync_elems * sizeof(int32_t), s));
-  if (block && (phases & kForward)) launch(k_mark_pending_m, nmark, 256, 0, s, nready, ready);
-  kt.begin(kKcSolveFwd, s);
-  for (int t = 0; t < nl && (phases & kForward); t++) {
-    const LevelPlan &L    = P.levels[t];
-    const bool       both = L.sw_count > 0 && L.sf_count > 0;
-    cudaStream_t     ss   = both ? ws.side.fork(s) : s;  // warp fronts beside block fronts
-    if (L.sw_count > 0)
-      launch(k_fwd_small_m<NR, T>, (L.sw_count + kSmallWarpsM - 1) / kSmallWarpsM, 32 * kSmallWarpsM,
-             small_smem, ss, P.swarp_list.as<int32_t>() + L.sw_begin, L.sw_count,
-             P.sfirst.as<int64_t>(), P.srowptr.as<int64_t>(), P.slofs.as<int64_t>(),
-             P.child_ptr.as<int64_t>(), P.child_list.as<int32_t>(), P.srel.as<int32_t>(),
-             P.zofs.as<int64_t>(), pan, X, n, zbuf, zld);
-    if (L.sf_count > 0)
-      launch(k_fwd_fronts_m<NR, T>, L.fwd_items, kSolveThreads,
-             fwd_m_smem_doubles<NR>() * sizeof(double), s,
-             P.fwd_item.as<SolveItem>() + L.fwd_map0, pan, lvt, P.gp.as<int64_t>(),
-             P.gsrc.as<int64_t>(), X, zbuf, zld, sync + 2 * t, ready, err);
-    if (both) ws.side.join(s);
+                    MultiSolveWorkspace &ws, cudaStream_t s) {
+  const int64_t      n = P.S.n;
+  KernelTimer       &kt = kernel_timer();
+  const MultiBuffers b(P);
+  double            *fv = ws.vals.as<double>(), *bv = fv + NR * b.fwd;
+  FlowArgs<T>        a{};
+  a.warps  = P.flow_warp.as<FlowFront>();
+  a.panel  = pan;
+  a.inv    = F.inv64.as<double>();
+  a.wpanel = F.wpanel.as<double>();
+  a.gfirst = P.flow_gfirst.as<int2>();
+  a.gmore  = P.flow_gmore.as<int32_t>();
+  a.srows  = P.srows.as<int32_t>();
+  a.n      = n;
+  a.x      = X;
+  a.f      = bv + NR * b.bwd;
+  a.z      = fv;
+  a.y      = a.z + NR * P.S.z_elems;
+  a.yz     = a.y + NR * kMultiCopies * n;
+  a.part   = bv;
+  a.xr     = a.part + NR * P.flow_part_elems;
+  a.xz     = a.xr + NR * kMultiCopies * n;
+  a.err    = ws.err.as<int32_t>();
+  static std::atomic<bool> attr{false};  // idempotent; set once per process
+  constexpr int            smem = kMultiSmem * sizeof(double);
+  if (!attr) {
+    MPIR_CUDA(cudaFuncSetAttribute(k_fwd_flow_m<NR, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    MPIR_CUDA(cudaFuncSetAttribute(k_bwd_flow_m<NR, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    attr = true;
   }
-  if (phases & kDiagonal)
-    launch(k_dscale_m, static_cast<unsigned>((n * NR + 255) / 256), 256, 0, s, n, NR,
-           F.Dinv.as<float>(), X);
+  kt.begin(kKcSolveFwd, s);
+  if (!ws.fwd_pending) flow_pending(fv, NR * b.fwd, s);
+  a.items  = P.flow_fwd.as<FlowItem>();
+  a.nitems = P.nflow_fwd;
+  a.mark   = bv;
+  a.nmark  = NR * b.bwd;
+  a.ticket = ws.sync.as<int32_t>();
+  launch(k_fwd_flow_m<NR, T>, std::min(P.nflow_fwd, kSMs), kFlowThreads, smem, s, a);
   kt.end(s);
-  if (!(phases & kBackward)) return;
   MPIR_CHECK_LAUNCH();
   kt.begin(kKcSolveBwd, s);
-  if (block) launch(k_mark_pending_m, nmark, 256, 0, s, nready, ready);
-  for (int t = nl - 1; t >= 0; t--) {
-    const LevelPlan &L    = P.levels[t];
-    const bool       both = L.sw_count > 0 && L.sf_count > 0;
-    cudaStream_t     ss   = both ? ws.side.fork(s) : s;
-    if (L.sw_count > 0)
-      launch(k_bwd_small_m<NR, T>, (L.sw_count + kSmallWarpsM - 1) / kSmallWarpsM, 32 * kSmallWarpsM,
-             small_smem, ss, P.swarp_list.as<int32_t>() + L.sw_begin, L.sw_count,
-             P.sfirst.as<int64_t>(), P.srowptr.as<int64_t>(), P.srows.as<int32_t>(),
-             P.slofs.as<int64_t>(), pan, X, n);
-    if (L.sf_count > 0) {
-      if (L.bwd_chunk_items > 0)
-        launch(k_bwd_chunks_m<NR, T>, L.bwd_chunk_items, kSolveThreads, 0, s, sf + L.sf_begin,
-               P.chunk_map.as<int32_t>() + L.chunk_map0, pan, P.srows.as<int32_t>(),
-               static_cast<const double *>(X), ws.part.as<double>(), pld);
-      launch(k_bwd_fronts_m<NR, T>, L.bwd_owner_items, kSolveThreads,
-             bwd_m_smem_doubles<NR>() * sizeof(double), s,
-             P.own_item.as<SolveItem>() + L.own_map0, pan, lvt, X,
-             static_cast<const double *>(ws.part.as<double>()), pld, sync + 2 * t + 1, ready,
-             err);
-    }
-    if (both) ws.side.join(s);
-  }
+  a.items  = P.flow_bwd.as<FlowItem>();
+  a.nitems = P.nflow_bwd;
+  a.mark   = fv;
+  a.nmark  = NR * b.fwd;
+  a.Dinv   = F.Dinv.as<float>();
+  a.ticket = ws.sync.as<int32_t>() + 1;
+  launch(k_bwd_flow_m<NR, T>, std::min(P.nflow_bwd, kSMs), kFlowThreads, smem, s, a);
+  ws.fwd_pending = true;
   kt.end(s);
   MPIR_CHECK_LAUNCH();
 }
@@ -645,79 +937,38 @@ int multi_width(int nrhs) {
 }
 
 void MultiSolveWorkspace::allocate(const Plan &P, int width) {
-  const Symbolic &S = P.S;
-  nr = width;
-  graph.reset();
-  xbuf.resize(std::max<int64_t>(S.n, 1) * width * sizeof(double));
-  device_zero(xbuf.as<void>(), xbuf.bytes());
-  zbuf.resize(std::max<int64_t>(S.z_elems, 1) * width * sizeof(double));
-  part.resize(std::max<int64_t>(P.spart_elems, 1) * width * sizeof(double));
-  sync.resize(std::max<int64_t>(P.sync_elems, 1) * sizeof(int32_t));
-  ready.resize(std::max<int64_t>(static_cast<int64_t>(kMultiCopies) * width * S.n, 1) *
-               sizeof(double));
+  const MultiBuffers b(P);
+  nr          = width;
+  fwd_pending = false;
+  vals.resize(std::max<int64_t>((b.fwd + b.bwd + P.S.n) * width, 1) * sizeof(double));
+  sync.resize(4 * sizeof(int32_t));
+  device_zero(sync.as<void>(), sync.bytes());
   err.resize(sizeof(SolveCtl));
   device_zero(err.as<void>(), sizeof(SolveCtl));
 }
 
 size_t MultiSolveWorkspace::bytes_for(const Plan &P, int width) {
-  const Symbolic &S = P.S;
-  return (std::max<int64_t>(S.z_elems, 1) + std::max<int64_t>(P.spart_elems, 1) +
-          static_cast<int64_t>(kMultiCopies + 1) * S.n) *
-             width * sizeof(double) +
-         std::max<int64_t>(P.sync_elems, 1) * sizeof(int32_t) + sizeof(SolveCtl);
+  const MultiBuffers b(P);
+  return (b.fwd + b.bwd + P.S.n) * width * sizeof(double) + 4 * sizeof(int32_t) + sizeof(SolveCtl);
 }
 
 void ldlt_solve_multi(const Plan &P, const Numeric &F, double *X, int width,
-                      MultiSolveWorkspace &ws, cudaStream_t s, int phases) {
+                      MultiSolveWorkspace &ws, cudaStream_t s) {
   if (P.S.n == 0) return;
   if (ws.nr != width) throw std::logic_error("multi-vector workspace of another width");
   if (width != 4 && width != 8 && width != 16)
     throw std::invalid_argument("multi-vector solve width must be 4, 8 or 16");
   auto run = [&](auto *pan) {
     using T = std::remove_const_t<std::remove_pointer_t<decltype(pan)>>;
-    if (width == 4) solve_multi_nr<4, T>(P, F, pan, X, ws, s, phases);
-    if (width == 8) solve_multi_nr<8, T>(P, F, pan, X, ws, s, phases);
-    if (width == 16) solve_multi_nr<16, T>(P, F, pan, X, ws, s, phases);
+    if (width == 4) solve_multi_nr<4, T>(P, F, pan, X, ws, s);
+    if (width == 8) solve_multi_nr<8, T>(P, F, pan, X, ws, s);
+    if (width == 16) solve_multi_nr<16, T>(P, F, pan, X, ws, s);
   };
   switch (F.solve_prec()) {
     case 2: run(F.panel16.as<const __nv_bfloat16>()); break;
     case 3: run(F.panel16.as<const __half>()); break;
     default: run(F.panel.as<const float>());
   }
-}
-
-void ldlt_solve_multi_graph(const Plan &P, const Numeric &F, double *X, int width,
-                            MultiSolveWorkspace &ws, cudaStream_t s,
-                            cudaStream_t capture_stream) {
-  const int64_t n = P.S.n;
-  if (n == 0) return;
-  if (kernel_timer().enabled) {
-    ldlt_solve_multi(P, F, X, width, ws, s);
-    return;
-  }
-  if (!ws.graph.g) {
-    cudaGraph_t g = nullptr;
-    MPIR_CUDA(cudaStreamSynchronize(capture_stream));
-    MPIR_CUDA(cudaStreamBeginCapture(capture_stream, cudaStreamCaptureModeThreadLocal));
-    try {
-      LaunchCapture cap;
-      ldlt_solve_multi(P, F, ws.xbuf.as<double>(), width, ws, capture_stream);
-      ws.graph_launches = cap.count();
-    } catch (...) {
-      cudaStreamEndCapture(capture_stream, &g);
-      if (g) cudaGraphDestroy(g);
-      throw;
-    }
-    MPIR_CUDA(cudaStreamEndCapture(capture_stream, &g));
-    const cudaError_t e = cudaGraphInstantiate(&ws.graph.g, g, 0);
-    cudaGraphDestroy(g);
-    MPIR_CUDA(e);
-  }
-  const size_t bytes = static_cast<size_t>(n) * width * sizeof(double);
-  MPIR_CUDA(cudaMemcpyAsync(ws.xbuf.as<void>(), X, bytes, cudaMemcpyDeviceToDevice, s));
-  MPIR_CUDA(cudaGraphLaunch(ws.graph.g, s));
-  launch_add(ws.graph_launches);
-  MPIR_CUDA(cudaMemcpyAsync(X, ws.xbuf.as<void>(), bytes, cudaMemcpyDeviceToDevice, s));
 }
 
 }  // namespace mpir

@@ -745,14 +745,17 @@ __global__ void __launch_bounds__(256, 1)
   // Every global load of the CTA is issued before the first is used (one
   // memory latency instead of one per batch): A's two halves, and B = X
   // diag(Dinv) by thread (row n = m, K-groups gsel + 2 i, i < 16).
-  const int halves = nbk > 64 ? 2 : 1;
+  const int halves = nbk > 64 ? 2 : 1, nb32 = (nbk + 31) / 32 * 32;
   float     a[32], a1[32], xv[64];
   load_a(0, a);
   const float dv = m < nbk ? Dinv[static_cast<int64_t>(d.col0) + kb + m] : 0.0f;
 #pragma unroll
   for (int i = 0; i < 16; i++)
 #pragma unroll
-    for (int j = 0; j < 4; j++) xv[4 * i + j] = X[m + (4 * (gsel + 2 * i) + j) * kNB];
+    for (int j = 0; j < 4; j++) {
+      const int k = 4 * (gsel + 2 * i) + j;
+      xv[4 * i + j] = k < nb32 ? X[m + k * kNB] : 0.0f;
+    }
   if (halves == 2) load_a(1, a1);
 #pragma unroll
   for (int i = 0; i < 16; i++) {
