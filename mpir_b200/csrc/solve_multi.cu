@@ -12,11 +12,19 @@
 // bytes; in shared memory too, where a warp reads the same entry's values for
 // NR fused multiply-adds a value of L.
 //
+// Products with L and with the inverses run on the float64 matrix
+// instructions (m8n8k4): a warp takes 32 x 32 entries of L, each lane those of
+// its fragments, and a value of y from shared memory serves 8 multiply-adds a
+// lane.  With plain FMAs, a read of 16 bytes for every 2, the reads took most
+// of a wide front's time (16 vectors: 17 us per 512 columns of the root).
+//
 // What bounds it: below the root the chain of hand-overs, as for one vector;
-// in the wide fronts the float64 multiply-adds and the shared-memory reads that
-// feed them (an entry of L: NR FMAs and NR / 2 reads of 16 bytes a warp).
-// Measured, one application, against the solves by levels that this replaced:
-// 16 vectors at n = 20,480: 0.74 ms (2.73); 4 at n = 40,951: 0.45 ms (1.50).
+// in the wide fronts the float64 multiply-adds (512 x 32 x 16 take 2.2 us of an
+// SM, twice per 512 columns of the chain).
+// Measured, one application, against the solves by levels that these replaced
+// and, in between, the same items with plain FMAs: 16 vectors at n = 20,480:
+// 0.48 ms (2.73; 0.64 to 0.78), 8 at n = 40,960: 0.76 ms (3.00; 0.95), 4 at
+// n = 40,951: 0.44 ms (1.50; 0.44), for which half of each product is unused.
 // Per vector the sums inside an item run in another order than in the
 // single-vector kernels, so results agree with NR single solves to rounding.
 #include <atomic>
@@ -37,14 +45,22 @@ namespace {
 
 constexpr int kMultiCopies = 2;  // copies of a wide front's block results
 
-// Shared memory (doubles): kFlowInvSmem, then 9,216 for vectors and partial
-// sums (512 rows of 16 values, pitch 18).
-constexpr int kMultiBuf  = 512 * 18;
-constexpr int kMultiSmem = kFlowInvSmem + kMultiBuf;
+// Shared memory (doubles): kFlowInvSmem, then vectors and partial sums.  The
+// most is taken by the backward solve of a narrow front with its rows below: 10
+// blocks of the inverse, 512 + 128 + 256 entries of 16 values at a pitch of 18
+// (of 8 values at a pitch of 10: 512 + 128 + 512).
+constexpr int kMultiSmem = 10 * kFlowBlk + 896 * 18;
+static_assert(kMultiSmem >= kFlowInvSmem + 512 * 18, "16 warps' 32 entries behind the inverse blocks");
 
 // Narrow fronts stage at most 10 blocks of the inverse; their vectors start
 // behind those.
 constexpr int kNarrowInv = 10 * kFlowBlk;
+
+// In shared memory an entry's NR values lie every NR + 2 doubles where the lanes
+// of a warp read or write an entry each (16-byte accesses then go without bank
+// conflicts; at a pitch of NR = 16 each took 8 times as long).
+template <int NR>
+constexpr int kPitch = NR + 2;
 
 struct alignas(16) V2 {
   unsigned long long a, b;
@@ -61,13 +77,30 @@ __device__ __forceinline__ void st_relaxed_2(double *p, double a, double b) {
 }
 
 // Waits for K values side by side (16-byte aligned; none when !on) and adds
-// them to v; all that are pending are polled together.
+// them to v.  All are asked for at once; while they are pending, the last pair
+// alone is polled (an entry's values are stored together): with 16 vectors the
+// CTAs that wait on a wide front's newest results would otherwise poll 64 KB
+// each.
 template <int K>
 __device__ __forceinline__ void add_entry(const double *p, bool on, double (&v)[K], int32_t *err,
                                           long polls) {
   unsigned need = on ? (1u << (K / 2)) - 1 : 0u;
   for (long it = 0; need != 0; it++) {
     V2 raw[K / 2];
+    if (K > 2 && it > 0 && need >> (K / 2 - 1) != 0) {
+      const V2 g = ld_relaxed_2(p + K - 2);
+      if (g.a == kPending || g.b == kPending) {
+        if (it >= polls) {
+          atomicExch(err, 1);
+          return;
+        }
+        if ((it & 63) == 63) {
+          if (*reinterpret_cast<volatile int32_t *>(err) != 0) return;
+          __nanosleep(32);
+        }
+        continue;
+      }
+    }
 #pragma unroll
     for (int q = 0; q < K / 2; q++) {
       raw[q] = V2{kPending, kPending};
@@ -120,40 +153,160 @@ __device__ __forceinline__ void put_entry(double *dst, const double (&v)[NR]) {
   for (int k = 0; k < NR; k += 2) *reinterpret_cast<double2 *>(dst + k) = make_double2(v[k], v[k + 1]);
 }
 
+// A warp's 32 x NR result in fragments of the m8n8k4 product: c[o][n] holds, of
+// row (lane / 4) of octet o, the vectors 8 n + 2 (lane % 4) and the next (of 4
+// vectors half of the fragment is not used).
+template <int NR>
+struct Frag {
+  static constexpr int kN = NR < 8 ? 1 : NR / 8;
+  double               c[4][kN][2];
+  __device__ __forceinline__ void zero() {
+#pragma unroll
+    for (int o = 0; o < 4; o++)
+#pragma unroll
+      for (int n = 0; n < kN; n++) c[o][n][0] = c[o][n][1] = 0.0;
+  }
+  // The lane's values of the entry at p (8 vectors a fragment).
+  static __device__ __forceinline__ void get_b(double (&b)[kN], const double *p) {
+    const int v = threadIdx.x % 32 / 4;
+#pragma unroll
+    for (int n = 0; n < kN; n++) b[n] = p[8 * n + (NR < 8 ? v % 4 : v)];
+  }
+  __device__ __forceinline__ void mma(int o, double a, const double (&b)[kN]) {
+#pragma unroll
+    for (int n = 0; n < kN; n++)
+      asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+          : "+d"(c[o][n][0]), "+d"(c[o][n][1])
+          : "d"(a), "d"(b[n]));
+  }
+  // Row of octet o held by the lane: 8 o + lane / 4, or (kPerm) 4 (lane / 4) + o.
+  template <bool kPerm>
+  static __device__ __forceinline__ int row(int o) {
+    const int g = threadIdx.x % 32 / 4;
+    return kPerm ? 4 * g + o : 8 * o + g;
+  }
+  template <bool kPerm>
+  __device__ __forceinline__ void put(double *dst) const {
+    const int v = 2 * (threadIdx.x % 4);
+    if (NR < 8 && v >= 4) return;
+#pragma unroll
+    for (int o = 0; o < 4; o++)
+#pragma unroll
+      for (int n = 0; n < kN; n++)
+        *reinterpret_cast<double2 *>(dst + kPitch<NR> * row<kPerm>(o) + 8 * n + v) =
+            make_double2(c[o][n][0], c[o][n][1]);
+  }
+  __device__ __forceinline__ void add(const double *src) {
+    const int v = 2 * (threadIdx.x % 4);
+    if (NR < 8 && v >= 4) return;
+#pragma unroll
+    for (int o = 0; o < 4; o++)
+#pragma unroll
+      for (int n = 0; n < kN; n++) {
+        const double2 s =
+            *reinterpret_cast<const double2 *>(src + kPitch<NR> * row<false>(o) + 8 * n + v);
+        c[o][n][0] += s.x;
+        c[o][n][1] += s.y;
+      }
+  }
+};
+
+// Fragments of 32 x 32 entries of L: of L itself (rows rb .., columns c ..; row
+// 8 o + lane / 4, column 4 q + lane % 4 in d[8 o + q]), or of its transpose
+// (column 8 o + lane / 4, row 4 q + lane % 4).
+template <class T>
+__device__ __forceinline__ void load_frag(float (&d)[32], const T *P, int64_t h, int64_t rb, int64_t rend,
+                                          int c, int cend) {
+  const int     lane = threadIdx.x % 32;
+  const int64_t r    = rb + lane / 4;
+  const int     c0   = c + lane % 4;
+  const T      *p    = P + r + c0 * h;
+#pragma unroll
+  for (int q = 0; q < 8; q++)
+#pragma unroll
+    for (int o = 0; o < 4; o++)
+      d[8 * o + q] = (r + 8 * o < rend && c0 + 4 * q < cend) ? to_f(__ldg(p + 8 * o + 4 * q * h)) : 0.0f;
+}
+template <class T>
+__device__ __forceinline__ void load_frag_t(float (&d)[32], const T *P, int64_t h, int64_t rb, int64_t rend,
+                                            int c, int cend) {
+  const int     lane = threadIdx.x % 32;
+  const int64_t r    = rb + lane % 4;
+  const int     c0   = c + lane / 4;
+  const T      *p    = P + r + c0 * h;
+#pragma unroll
+  for (int o = 0; o < 4; o++)
+#pragma unroll
+    for (int q = 0; q < 8; q++)
+      d[8 * o + q] = (r + 4 * q < rend && c0 + 8 * o < cend) ? to_f(__ldg(p + 4 * q + 8 * o * h)) : 0.0f;
+}
+
+// f += (32 x 32 entries of L) times the 32 entries at y.
+template <int NR>
+__device__ __forceinline__ void mma_tile(Frag<NR> &f, const float (&d)[32], const double *y) {
+#pragma unroll
+  for (int q = 0; q < 8; q++) {
+    double b[Frag<NR>::kN];
+    Frag<NR>::get_b(b, y + kPitch<NR> * (4 * q + threadIdx.x % 4));
+#pragma unroll
+    for (int o = 0; o < 4; o++) f.mma(o, static_cast<double>(d[8 * o + q]), b);
+  }
+}
+
+// f = a 32 x 32 block of the inverse (entry (r, c) at 33 c + r) times the 32
+// entries at y; rows as Frag::row<true>, which keeps the lanes' reads of the
+// block free of bank conflicts.
+template <int NR>
+__device__ __forceinline__ void mma_inverse(Frag<NR> &f, const double *blk, const double *y) {
+  const int g = threadIdx.x % 32 / 4, k = threadIdx.x % 4;
+  f.zero();
+#pragma unroll
+  for (int q = 0; q < 8; q++) {
+    double b[Frag<NR>::kN];
+    Frag<NR>::get_b(b, y + kPitch<NR> * (4 * q + k));
+#pragma unroll
+    for (int o = 0; o < 4; o++) f.mma(o, blk[33 * (4 * q + k) + 4 * g + o], b);
+  }
+}
+// f += its transpose times the 32 entries at y (the block's rows are taken in
+// the order 16 (q / 4) + 4 k + q % 4, for the same reason).
+template <int NR>
+__device__ __forceinline__ void mma_inverse_t(Frag<NR> &f, const double *blk, const double *y) {
+  const int g = threadIdx.x % 32 / 4, k = threadIdx.x % 4;
+#pragma unroll
+  for (int q = 0; q < 8; q++) {
+    const int r = 16 * (q / 4) + 4 * k + q % 4;
+    double    b[Frag<NR>::kN];
+    Frag<NR>::get_b(b, y + kPitch<NR> * r);
+#pragma unroll
+    for (int o = 0; o < 4; o++) f.mma(o, blk[33 * (8 * o + g) + r], b);
+  }
+}
+
 // ---------------------------------------------------------------------------
 // Forward.
 
-// acc += sum_c L(r, c) y_c over the columns c < cend of a wide front, tile by
-// tile as the block results become ready (rows_apply of solve.cu); own: the
-// warp's 32 NR doubles of shared memory.
+// f += L(rb .., c) y_c over the columns c < cend of a wide front, tile by tile
+// as the block results become ready (rows_apply of solve.cu); own: the warp's
+// 32 entries of shared memory.
 template <int RG, int NR, class T>
-__device__ __forceinline__ void rows_apply_m(const FlowArgs<T> &a, const T *P, int64_t h, int64_t r,
-                                             bool rok, int cend, const double *y, double *own,
-                                             double (&acc)[NR], long polls) {
+__device__ __forceinline__ void rows_apply_m(const FlowArgs<T> &a, const T *P, int64_t h, int64_t rb,
+                                             int64_t rend, int cend, const double *y, double *own,
+                                             Frag<NR> &f, long polls) {
   constexpr int TW = 512 / RG;
   const int     warp = threadIdx.x / 32, lane = threadIdx.x % 32, cq = 32 * (warp / RG);
   float         lv[32], lvn[32];
-  load_cols(lv, P, h, r, rok, cq, cend);
+  load_frag(lv, P, h, rb, rend, cq, cend);
   for (int c = cq; c - cq < cend; c += TW) {
-    if (c - cq + TW < cend) load_cols(lvn, P, h, r, rok, c + TW, cend);
-    get_entry<NR>(y + static_cast<int64_t>(NR) * (c + lane), c + lane < cend, own + NR * lane, a.err, polls);
+    if (c - cq + TW < cend) load_frag(lvn, P, h, rb, rend, c + TW, cend);
+    get_entry<NR>(y + static_cast<int64_t>(NR) * (c + lane), c + lane < cend, own + kPitch<NR> * lane, a.err,
+                  polls);
     __syncwarp();
-#pragma unroll
-    for (int k = 0; k < 32; k++) fma_entry<NR>(static_cast<double>(lv[k]), own + NR * k, acc);
+    mma_tile(f, lv, own);
     __syncwarp();
 #pragma unroll
     for (int k = 0; k < 32; k++) lv[k] = lvn[k];
   }
-}
-
-// acc = the 32 x 32 block of the inverse at blk (entry (lane, c) at c * 33 +
-// lane) times the 32 entries at y.
-template <int NR>
-__device__ __forceinline__ void block_rows(const double *blk, const double *y, double (&acc)[NR]) {
-#pragma unroll
-  for (int k = 0; k < NR; k++) acc[k] = 0.0;
-#pragma unroll 8
-  for (int c = 0; c < 32; c++) fma_entry<NR>(blk[33 * c], y + NR * c, acc);
 }
 
 template <int NR, class T>
@@ -161,11 +314,12 @@ __device__ __noinline__ void fwd_slab_m(const FlowArgs<T> &a, FlowShared &S, con
                                         double *sm, uint32_t &phase) {
   const FlowFront &f   = I.item.f;
   const int        tid = threadIdx.x, warp = tid / 32, lane = tid % 32;
-  const int        row = tid / NR, v = tid % NR;  // the thread's output, tid < 32 NR
+  constexpr int    NP  = kPitch<NR>;
+  const int        row = tid / NR, v = tid % NR, at = NP * row + v;  // the thread's output, tid < 32 NR
   const long       polls = I.polls;
   const int        r0 = I.item.r0, s = r0 / kFlowSB, i = (r0 % kFlowSB) / 32;
   const bool       mine = row < I.item.nr, last = r0 + 32 >= f.w || i == 15;
-  double          *inv = sm, *yw = sm + kFlowInvSmem, *own = yw + 32 * NR * warp;
+  double          *inv = sm, *yw = sm + kFlowInvSmem, *own = yw + 32 * NP * warp;
   const uint32_t   bar = smem_addr(&S.bar);
   if (tid == 0) {
     const uint32_t bytes = (i + 1) * kFlowBlk * sizeof(double);
@@ -180,18 +334,17 @@ __device__ __noinline__ void fwd_slab_m(const FlowArgs<T> &a, FlowShared &S, con
     g.begin(a, f.zofs + r0 + row, a.z + v);
     zr = g.finish(a, a.z + v, a.x[v * a.n + f.col0 + r0 + row], polls);
   }
-  double acc[NR];
-#pragma unroll
-  for (int k = 0; k < NR; k++) acc[k] = 0.0;
+  Frag<NR> fr;
   if (s > 0) {
-    rows_apply_m<1, NR>(a, a.panel + f.panel, f.h, r0 + lane, lane < I.item.nr, s * kFlowSB,
-                        a.y + ((I.ticket % kMultiCopies) * a.n + f.col0) * NR, own, acc, polls);
-    put_entry<NR>(own + NR * lane, acc);
+    fr.zero();
+    rows_apply_m<1, NR>(a, a.panel + f.panel, f.h, r0, r0 + I.item.nr, s * kFlowSB,
+                        a.y + ((I.ticket % kMultiCopies) * a.n + f.col0) * NR, own, fr, polls);
+    fr.template put<false>(own);
     __syncthreads();
     if (row < 32) {
       double t[4] = {0.0, 0.0, 0.0, 0.0};
 #pragma unroll
-      for (int q = 0; q < 16; q++) t[q % 4] += yw[32 * NR * q + tid];
+      for (int q = 0; q < 16; q++) t[q % 4] += yw[32 * NP * q + at];
       zr -= (t[0] + t[1]) + (t[2] + t[3]);
     }
     __syncthreads();
@@ -199,25 +352,25 @@ __device__ __noinline__ void fwd_slab_m(const FlowArgs<T> &a, FlowShared &S, con
   double *yz = a.yz + static_cast<int64_t>(NR) * (f.col0 + s * kFlowSB);
   if (row < 32) {
     if (!last && I.publish) st_relaxed_f64(yz + 32 * NR * i + tid, zr);
-    yw[tid] = zr;  // the diagonal block's, for warp 0
+    yw[at] = zr;  // the diagonal block's, for warp 0
   }
   __syncthreads();
   bulk_wait(bar, phase, a.err);
   phase ^= 1;
   if (warp <= i) {
     const int j = warp == 0 ? i : warp - 1;
-    if (warp > 0) get_entry<NR>(yz + NR * (32 * j + lane), true, own + NR * lane, a.err, polls);
+    if (warp > 0) get_entry<NR>(yz + NR * (32 * j + lane), true, own + NP * lane, a.err, polls);
     __syncwarp();
-    block_rows<NR>(inv + j * kFlowBlk + lane, own, acc);
+    mma_inverse(fr, inv + j * kFlowBlk, own);
     __syncwarp();
-    put_entry<NR>(own + NR * lane, acc);
+    fr.template put<true>(own);
   }
   __syncthreads();
   if (mine) {
     double t[4] = {0.0, 0.0, 0.0, 0.0};
 #pragma unroll
     for (int q = 0; q < 16; q++)
-      if (q <= i) t[q % 4] += yw[32 * NR * q + tid];
+      if (q <= i) t[q % 4] += yw[32 * NP * q + at];
     const double  y = (t[0] + t[1]) + (t[2] + t[3]);
     const int64_t g = static_cast<int64_t>(NR) * (f.col0 + r0) + tid;
     if (I.publish) {
@@ -231,18 +384,16 @@ __device__ __noinline__ void fwd_slab_m(const FlowArgs<T> &a, FlowShared &S, con
 template <int NR, class T>
 __device__ __noinline__ void fwd_rows_m(const FlowArgs<T> &a, const FlowSlot &I, FlowSlot &N, double *sm) {
   const FlowFront &f   = I.item.f;
-  const int        tid = threadIdx.x, warp = tid / 32, lane = tid % 32;
+  const int        tid = threadIdx.x, warp = tid / 32;
   const long       polls = I.polls;
   const int        r0 = I.item.r0, nr = I.item.nr;
-  double          *yw = sm + kFlowInvSmem, *own = yw + 32 * NR * warp;
-  const int        rl = 32 * (warp % 4) + lane;
+  double          *yw = sm + kFlowInvSmem, *own = yw + 32 * kPitch<NR> * warp;
   flow_fetch(a, N);
-  double acc[NR];
-#pragma unroll
-  for (int k = 0; k < NR; k++) acc[k] = 0.0;
-  rows_apply_m<4, NR>(a, a.panel + f.panel, f.h, r0 + rl, rl < nr, f.w,
-                      a.y + ((I.ticket % kMultiCopies) * a.n + f.col0) * NR, own, acc, polls);
-  put_entry<NR>(own + NR * lane, acc);
+  Frag<NR> fr;
+  fr.zero();
+  rows_apply_m<4, NR>(a, a.panel + f.panel, f.h, r0 + 32 * (warp % 4), r0 + nr, f.w,
+                      a.y + ((I.ticket % kMultiCopies) * a.n + f.col0) * NR, own, fr, polls);
+  fr.template put<false>(own);
   // Output e: row e / NR, vector e % NR; its column quarters are 4 warps apart.
   constexpr int KO = NR / 4;
   Gather<NR>    g[KO];
@@ -256,8 +407,9 @@ __device__ __noinline__ void fwd_rows_m(const FlowArgs<T> &a, const FlowSlot &I,
   for (int m = 0; m < KO; m++) {
     const int e = tid + 512 * m;
     if (e / NR < nr) {
-      const double *p = yw + e;
-      const double  t = (p[0] + p[128 * NR]) + (p[256 * NR] + p[384 * NR]);
+      constexpr int NP = kPitch<NR>;
+      const double *p = yw + NP * (e / NR) + e % NR;
+      const double  t = (p[0] + p[128 * NP]) + (p[256 * NP] + p[384 * NP]);
       const double  u = g[m].finish(a, a.z + e % NR, 0.0, polls) - t;
       if (I.publish) st_relaxed_f64(a.z + NR * (f.zofs + r0) + e, u);
     }
@@ -271,8 +423,8 @@ __device__ __noinline__ void fwd_narrow_m(const FlowArgs<T> &a, FlowShared &S, c
   const int        tid = threadIdx.x, warp = tid / 32, lane = tid % 32;
   const int        w = f.w, nbw = (w + 31) / 32, nr = I.item.nr;
   const long       polls = I.polls;
-  constexpr int    KO = NR / 4;
-  double          *inv = sm, *zs = sm + kNarrowInv, *ys = zs + 128 * NR, *part = ys + 128 * NR;
+  constexpr int    KO = NR / 4, NP = kPitch<NR>;
+  double          *inv = sm, *zs = sm + kNarrowInv, *ys = zs + 128 * NP, *part = ys + 128 * NP;
   const uint32_t   bar = smem_addr(&S.bar);
   if (tid == 0) {
     const uint32_t bytes = nbw * (nbw + 1) / 2 * kFlowBlk * sizeof(double);
@@ -280,11 +432,11 @@ __device__ __noinline__ void fwd_narrow_m(const FlowArgs<T> &a, FlowShared &S, c
     bulk_get(inv, a.inv + f.inv, bytes, bar);
   }
   constexpr int kTile = 32 * RG;
-  const int     cq = warp / RG, rt = tid % kTile;
+  const int     cq = warp / RG, rw = 32 * (warp % RG);  // the warp's columns, rows of a tile
   const int64_t r0 = I.item.r0;
   const T      *P  = a.panel + f.panel;
   float         lv[32], lvn[32];
-  load_cols(lv, P, f.h, r0 + rt, rt < nr, 32 * cq, w);
+  load_frag(lv, P, f.h, r0 + rw, r0 + nr, 32 * cq, w);
   flow_fetch(a, N);
   {
     Gather<NR> g[KO];
@@ -297,50 +449,47 @@ __device__ __noinline__ void fwd_narrow_m(const FlowArgs<T> &a, FlowShared &S, c
     for (int m = 0; m < KO; m++) {
       const int e = tid + 512 * m;
       if (e < 128 * NR)
-        zs[e] = e < w * NR ? g[m].finish(a, a.z + e % NR, a.x[(e % NR) * a.n + f.col0 + e / NR], polls)
+        zs[NP * (e / NR) + e % NR] =
+            e < w * NR ? g[m].finish(a, a.z + e % NR, a.x[(e % NR) * a.n + f.col0 + e / NR], polls)
                            : 0.0;
     }
   }
   __syncthreads();
   bulk_wait(bar, phase, a.err);
   phase ^= 1;
-  {
-    // y = Inv z: thread (row tid % 128, vectors KO (tid / 128) ..)
-    const int i = tid % 128, vg = KO * (tid / 128), bi = i / 32;
-    double    y[KO];
+  // y = Inv z: warp 4 i + j takes block (i, j)
+  const int bi = warp / 4, bj = warp % 4;
+  Frag<NR>  fr;
+  if (bi < nbw && bj <= bi) {
+    mma_inverse(fr, inv + (bi * (bi + 1) / 2 + bj) * kFlowBlk, zs + 32 * NP * bj);
+    fr.template put<true>(part + NP * (128 * bj + 32 * bi));
+  }
+  __syncthreads();
 #pragma unroll
-    for (int k = 0; k < KO; k++) y[k] = 0.0;
-    if (bi < nbw)
-      for (int j = 0; j <= bi; j++) {
-        const double *blk = inv + (bi * (bi + 1) / 2 + j) * kFlowBlk + lane, *z = zs + 32 * NR * j + vg;
-#pragma unroll 8
-        for (int c = 0; c < 32; c++) {
-          const double l = blk[33 * c];
-#pragma unroll
-          for (int k = 0; k < KO; k++) y[k] += l * z[NR * c + k];
-        }
-      }
-#pragma unroll
-    for (int k = 0; k < KO; k++) {
-      ys[NR * i + vg + k] = i < w ? y[k] : 0.0;
-      if (i < w && r0 == w) a.f[static_cast<int64_t>(NR) * (f.col0 + i) + vg + k] = y[k];
-    }
+  for (int m = 0; m < KO; m++) {
+    const int e = tid + 512 * m, row = e / NR;
+    if (e >= 128 * NR) break;
+    double y = 0.0;
+    if (row < w)
+      for (int j = 0; j <= row / 32; j++) y += part[NP * (128 * j + row) + e % NR];
+    ys[NP * row + e % NR] = y;
+    if (row < w && r0 == w) a.f[static_cast<int64_t>(NR) * f.col0 + e] = y;
   }
   __syncthreads();
   for (int q = 0; q * kTile < nr; q++) {
-    const int rn = (q + 1) * kTile + rt;
-    if ((q + 1) * kTile < nr) load_cols(lvn, P, f.h, r0 + rn, rn < nr, 32 * cq, w);
-    double acc[NR];
-#pragma unroll
-    for (int k = 0; k < NR; k++) acc[k] = 0.0;
-#pragma unroll
-    for (int k = 0; k < 32; k++) fma_entry<NR>(static_cast<double>(lv[k]), ys + NR * (32 * cq + k), acc);
+    if ((q + 1) * kTile < nr) load_frag(lvn, P, f.h, r0 + (q + 1) * kTile + rw, r0 + nr, 32 * cq, w);
+    fr.zero();
+    mma_tile(fr, lv, ys + NP * 32 * cq);
+    double *out = part + NP * (kTile * cq + rw);
+    fr.template put<false>(out);
     if (RG == 16) {
-      // one tile; the thread's row: its children's values, then the result
+      // one tile; the lane's row: its children's values, then the result
+      __syncwarp();
+      const int rt = rw + lane;
       if (rt < nr) {
         double u[NR];
 #pragma unroll
-        for (int k = 0; k < NR; k++) u[k] = 0.0;
+        for (int k = 0; k < NR; k++) u[k] = -out[NP * lane + k];
         const int2 g = a.gfirst[f.zofs + r0 + rt];
         add_entry<NR>(a.z + static_cast<int64_t>(NR) * g.x, g.x >= 0, u, a.err, polls);
         if (g.y >= 0)
@@ -349,11 +498,10 @@ __device__ __noinline__ void fwd_narrow_m(const FlowArgs<T> &a, FlowShared &S, c
         if (I.publish) {
           double *z = a.z + NR * (f.zofs + r0 + rt);
 #pragma unroll
-          for (int k = 0; k < NR; k += 2) st_relaxed_2(z + k, u[k] - acc[k], u[k + 1] - acc[k + 1]);
+          for (int k = 0; k < NR; k += 2) st_relaxed_2(z + k, u[k], u[k + 1]);
         }
       }
     } else {
-      put_entry<NR>(part + NR * (128 * cq + rt), acc);
       Gather<NR> g[KO];
       const int  base = q * kTile * NR;  // output e of the item: row e / NR
 #pragma unroll
@@ -366,8 +514,8 @@ __device__ __noinline__ void fwd_narrow_m(const FlowArgs<T> &a, FlowShared &S, c
       for (int m = 0; m < KO; m++) {
         const int e = base + tid + 512 * m;
         if (e / NR < nr) {
-          const double *p = part + tid + 512 * m;
-          const double  t = (p[0] + p[128 * NR]) + (p[256 * NR] + p[384 * NR]);
+          const double *p = part + NP * (e / NR - q * kTile) + e % NR;
+          const double  t = (p[0] + p[128 * NP]) + (p[256 * NP] + p[384 * NP]);
           const double  u = g[m].finish(a, a.z + e % NR, 0.0, polls) - t;
           if (I.publish) st_relaxed_f64(a.z + NR * (f.zofs + r0) + e, u);
         }
@@ -504,74 +652,65 @@ __global__ void __launch_bounds__(kFlowThreads, 1) k_fwd_flow_m(const __grid_con
 // ---------------------------------------------------------------------------
 // Backward.
 
-// Sums over the lanes of K values each (K = 8, 16 or 32): lane l returns the
-// sum of value l / (32 / K).  At each of the first levels a lane keeps half of
-// its values and sends the other half.
-template <int K>
-__device__ __forceinline__ double reduce_lanes(double (&v)[K]) {
-  const unsigned full = 0xffffffffu;
-  const int      lane = threadIdx.x % 32;
-  int            o    = 16;
-#pragma unroll
-  for (int m = K / 2; m >= 1; m /= 2) {
-    const bool up = lane & o;
-#pragma unroll
-    for (int u = 0; u < m; u++) {
-      const double keep = up ? v[u + m] : v[u], send = up ? v[u] : v[u + m];
-      v[u] = keep + __shfl_xor_sync(full, send, o);
-    }
-    o /= 2;
-  }
-  for (; o >= 1; o /= 2) v[0] += __shfl_xor_sync(full, v[0], o);
-  return v[0];
-}
-
-// acc[NR j + k] += sum_i lv[j][i] x(lane + 32 i, k), the x values in shared
-// memory, a row every NR + 2 doubles (16-byte reads free of bank conflicts).
-template <int NR>
-__device__ __forceinline__ void tile_cols(const float (&lv)[2][16], const double *xs,
-                                          double (&acc)[2 * NR]) {
-  const int lane = threadIdx.x % 32;
-#pragma unroll 4
-  for (int i = 0; i < 16; i++) {
-    const double  l0 = static_cast<double>(lv[0][i]), l1 = static_cast<double>(lv[1][i]);
-    const double *x  = xs + (NR + 2) * (lane + 32 * i);
-#pragma unroll
-    for (int q = 0; q < NR; q += 2) {
-      const double2 v = *reinterpret_cast<const double2 *>(x + q);
-      acc[q] += l0 * v.x;
-      acc[q + 1] += l0 * v.y;
-      acc[NR + q] += l1 * v.x;
-      acc[NR + q + 1] += l1 * v.y;
-    }
-  }
-}
-
 // t(c, k) = sum_r L(r, c) x(r, k) over up to 512 rows below the block, for
-// columns [c0, cend): emit(c, k, t) by one lane a value.
+// columns [c0, cend), at most 128: emit(c, k, t) by one lane a value.  ncg = 1,
+// 2 or 4 groups of 32 columns by 16 / ncg groups of 32 ncg rows; the row groups
+// are then added through out: at once (512 entries), or, where 16 vectors leave
+// no room for that, pairwise (256 entries).
 template <int NR, class T, class Emit>
 __device__ __forceinline__ void chunk_cols_m(const FlowArgs<T> &a, const FlowFront &f, int64_t rb, int nr,
-                                             int c0, int cend, double *xs, long polls, FlowSlot &N,
-                                             Emit emit) {
-  const int tid = threadIdx.x, warp = tid / 32, lane = tid % 32;
-  const T  *P = a.panel + f.panel;
-  float     lv[2][16];
-  load_rows(lv, P, f.h, rb, nr, c0, cend);
+                                             int c0, int cend, double *xs, double *out, long polls,
+                                             FlowSlot &N, Emit emit) {
+  constexpr int NP  = kPitch<NR>;
+  const int     tid = threadIdx.x, warp = tid / 32;
+  const int     ncg = cend - c0 <= 32 ? 1 : cend - c0 <= 64 ? 2 : 4, cg = warp % ncg, rq = warp / ncg;
+  const T      *P   = a.panel + f.panel;
+  const int     c = c0 + 32 * cg, rw = 32 * ncg * rq;
+  float         lv[32], lvn[32];
+  load_frag_t(lv, P, f.h, rb + rw, rb + nr, c, cend);
   flow_fetch(a, N);
   const int row = tid < nr ? a.srows[f.rows + rb + tid] : -1;
   wait_gate(a, f.gate < 0 ? -1 : NR * f.gate, polls);
-  get_entry<NR>(a.xr + static_cast<int64_t>(NR) * row, row >= 0, xs + (NR + 2) * tid, a.err, polls);
+  get_entry<NR>(a.xr + static_cast<int64_t>(NR) * row, row >= 0, xs + NP * tid, a.err, polls);
   __syncthreads();
-  for (int c = c0; c < cend; c += 32) {
-    double acc[2 * NR];
+  Frag<NR> fr;
+  fr.zero();
+  for (int s = 0; s < ncg; s++) {
+    if (s + 1 < ncg) load_frag_t(lvn, P, f.h, rb + rw + 32 * (s + 1), rb + nr, c, cend);
+    mma_tile(fr, lv, xs + NP * (rw + 32 * s));
 #pragma unroll
-    for (int k = 0; k < 2 * NR; k++) acc[k] = 0.0;
-    tile_cols<NR>(lv, xs, acc);
-    if (c + 32 < cend) load_rows(lv, P, f.h, rb, nr, c + 32, cend);
-    const double t   = reduce_lanes<2 * NR>(acc);
-    constexpr int kL = 16 / NR;  // lanes a value
-    const int    e   = lane / kL, col = c + 2 * warp + e / NR;
-    if (lane % kL == 0 && col < cend) emit(col, e % NR, t);
+    for (int k = 0; k < 32; k++) lv[k] = lvn[k];
+  }
+  if (NR <= 8) {
+    fr.template put<false>(out + NP * 32 * warp);
+    __syncthreads();
+    for (int e = tid; e < 32 * ncg * NR; e += kFlowThreads) {
+      const int     col = c0 + e / NR;
+      const double *q   = out + NP * (e / NR) + e % NR;
+      double        t   = 0.0;
+      for (int g = 0; g < 16 / ncg; g++) t += q[NP * 32 * ncg * g];
+      if (col < cend) emit(col, e % NR, t);
+    }
+    return;
+  }
+  for (int half = 8 / ncg; half >= 1; half /= 2) {
+    if (rq >= half && rq < 2 * half) fr.template put<false>(out + NP * 32 * (warp - half * ncg));
+    __syncthreads();
+    if (rq < half) fr.add(out + NP * 32 * warp);
+    __syncthreads();
+  }
+  const int v = 2 * (threadIdx.x % 4);
+  if (rq == 0 && (NR >= 8 || v < 4)) {
+#pragma unroll
+    for (int o = 0; o < 4; o++) {
+      const int col = c + Frag<NR>::template row<false>(o);
+#pragma unroll
+      for (int n = 0; n < Frag<NR>::kN; n++)
+        if (col < cend) {
+          emit(col, 8 * n + v, fr.c[o][n][0]);
+          emit(col, 8 * n + v + 1, fr.c[o][n][1]);
+        }
+    }
   }
 }
 
@@ -582,7 +721,7 @@ __device__ __noinline__ void bwd_chunk_m(const FlowArgs<T> &a, const FlowSlot &I
   const int64_t    rb = f.w + static_cast<int64_t>(c) * kFlowChunk;
   const int        nr = static_cast<int>(min(static_cast<int64_t>(kFlowChunk), f.h - rb));
   double          *pp = a.part + NR * (f.part + static_cast<int64_t>(c) * f.w);
-  chunk_cols_m<NR>(a, f, rb, nr, I.item.r0, I.item.r0 + I.item.nr, sm + kFlowInvSmem, I.polls, N,
+  chunk_cols_m<NR>(a, f, rb, nr, I.item.r0, I.item.r0 + I.item.nr, sm + kFlowInvSmem, sm, I.polls, N,
                    [&](int col, int k, double t) { st_relaxed_f64(pp + NR * col + k, t); });
 }
 
@@ -608,11 +747,11 @@ template <int NR, class T>
 __device__ __noinline__ void bwd_narrow_m(const FlowArgs<T> &a, FlowShared &S, const FlowSlot &I,
                                           FlowSlot &N, double *sm, uint32_t &phase) {
   const FlowFront &f   = I.item.f;
-  const int        tid = threadIdx.x, lane = tid % 32;
+  const int        tid = threadIdx.x;
   const int        w = f.w, nbw = (w + 31) / 32;
   const long       polls = I.polls;
-  constexpr int    KO = NR / 4;
-  double          *inv = sm, *xs = sm + kNarrowInv, *vs = xs + 512 * (NR + 2);
+  constexpr int    KO = NR / 4, NP = kPitch<NR>;
+  double          *inv = sm, *xs = sm + kNarrowInv, *vs = xs + 512 * kPitch<NR>, *out = vs + 128 * kPitch<NR>;
   const uint32_t   bar = smem_addr(&S.bar);
   if (tid == 0) {
     const uint32_t bytes = nbw * (nbw + 1) / 2 * kFlowBlk * sizeof(double);
@@ -632,41 +771,42 @@ __device__ __noinline__ void bwd_narrow_m(const FlowArgs<T> &a, FlowShared &S, c
   }
   if (f.chunks > 0 || f.h == w) flow_fetch(a, N);
   if (f.chunks == 0 && f.h > w) {
-    chunk_cols_m<NR>(a, f, w, f.h - w, 0, w, xs, polls, N,
-                     [&](int col, int k, double t) { vs[NR * col + k] = t; });
+    chunk_cols_m<NR>(a, f, w, f.h - w, 0, w, xs, out, polls, N,
+                     [&](int col, int k, double t) { vs[NP * col + k] = t; });
     __syncthreads();
   }
 #pragma unroll
   for (int m = 0; m < KO; m++) {
     const int e = tid + 512 * m;
-    if (e < w * NR && f.h > w) v[m] -= f.chunks > 0 ? chunk_sum<NR>(a, f, e, polls) : vs[e];
+    if (e < w * NR && f.h > w) v[m] -= f.chunks > 0 ? chunk_sum<NR>(a, f, e, polls) : vs[NP * (e / NR) + e % NR];
   }
   __syncthreads();
 #pragma unroll
-  for (int m = 0; m < KO; m++)
-    if (tid + 512 * m < 128 * NR) vs[tid + 512 * m] = v[m];
+  for (int m = 0; m < KO; m++) {
+    const int e = tid + 512 * m;
+    if (e < 128 * NR) vs[NP * (e / NR) + e % NR] = v[m];
+  }
   __syncthreads();
   bulk_wait(bar, phase, a.err);
   phase ^= 1;
-  // x = Inv^T v: thread (column tid % 128, vectors KO (tid / 128) ..)
-  const int i = tid % 128, vg = KO * (tid / 128), bj = i / 32;
-  double    x[KO];
-#pragma unroll
-  for (int k = 0; k < KO; k++) x[k] = 0.0;
-  for (int b = bj; b < nbw; b++) {
-    const double *blk = inv + (b * (b + 1) / 2 + bj) * kFlowBlk + 33 * lane, *z = vs + 32 * NR * b + vg;
-#pragma unroll 8
-    for (int r = 0; r < 32; r++) {
-      const double l = blk[r];
-#pragma unroll
-      for (int k = 0; k < KO; k++) x[k] += l * z[NR * r + k];
-    }
+  // x = Inv^T v: warp b takes the columns 32 b .., all blocks below
+  const int b = tid / 32;
+  if (b < nbw) {
+    Frag<NR> fr;
+    fr.zero();
+    for (int i = b; i < nbw; i++)
+      mma_inverse_t(fr, inv + (i * (i + 1) / 2 + b) * kFlowBlk, vs + 32 * NP * i);
+    __syncwarp();
+    fr.template put<false>(xs + 32 * NP * b);
   }
-  if (i < w) {
+  __syncthreads();
 #pragma unroll
-    for (int k = 0; k < KO; k++) {
-      st_relaxed_f64(a.xr + static_cast<int64_t>(NR) * (f.col0 + i) + vg + k, x[k]);
-      a.x[(vg + k) * a.n + f.col0 + i] = x[k];
+  for (int m = 0; m < KO; m++) {
+    const int e = tid + 512 * m;
+    if (e < w * NR) {
+      const double x = xs[NP * (e / NR) + e % NR];
+      st_relaxed_f64(a.xr + static_cast<int64_t>(NR) * f.col0 + e, x);
+      a.x[(e % NR) * a.n + f.col0 + e / NR] = x;
     }
   }
 }
@@ -676,12 +816,13 @@ __device__ __noinline__ void bwd_slab_m(const FlowArgs<T> &a, FlowShared &S, con
                                         double *sm, uint32_t &phase) {
   const FlowFront &f   = I.item.f;
   const int        tid = threadIdx.x, warp = tid / 32, lane = tid % 32;
-  const int        col = tid / NR, vv = tid % NR;  // the thread's output, tid < 32 NR
+  constexpr int    NP  = kPitch<NR>;
+  const int        col = tid / NR, vv = tid % NR, at = NP * col + vv;  // the thread's output, tid < 32 NR
   const long       polls = I.polls;
   const int        w = f.w, k0 = I.item.r0, s = k0 / kFlowSB, j = (k0 % kFlowSB) / 32;
   const int        nsl = min(16, (w - s * kFlowSB + 31) / 32), nsb = (w + kFlowSB - 1) / kFlowSB;
   const bool       mine = col < I.item.nr;
-  double          *inv = sm, *xs = sm + kFlowInvSmem, *own = xs + 32 * NR * warp;
+  double          *inv = sm, *xs = sm + kFlowInvSmem, *own = xs + 32 * NP * warp;
   const uint32_t   bar = smem_addr(&S.bar);
   if (tid == 0) {
     bulk_expect(bar, (nsl - j) * kFlowBlk * sizeof(double));
@@ -694,9 +835,10 @@ __device__ __noinline__ void bwd_slab_m(const FlowArgs<T> &a, FlowShared &S, con
   const T      *P    = a.panel + f.panel;
   const double *xr   = a.xr + ((I.ticket % kMultiCopies) * a.n + f.col0) * NR;
   const int     cend = k0 + I.item.nr;
-  float         lv[2][16];
-  if (nsb - 1 > s) load_rows(lv, P, f.h, static_cast<int64_t>(nsb - 1) * kFlowSB,
-                             w - (nsb - 1) * kFlowSB, k0, cend);
+  // Tile R: the warp takes the rows 32 warp .. of super-block R.
+  const int64_t rw = 32 * warp;
+  float         lv[32], lvn[32];
+  if (nsb - 1 > s) load_frag_t(lv, P, f.h, (nsb - 1) * static_cast<int64_t>(kFlowSB) + rw, w, k0, cend);
   flow_fetch(a, N);
   double v = 0.0;
   if (mine) {
@@ -704,31 +846,34 @@ __device__ __noinline__ void bwd_slab_m(const FlowArgs<T> &a, FlowShared &S, con
     if (a.Dinv) v *= static_cast<double>(a.Dinv[f.col0 + k0 + col]);
     if (f.chunks > 0) v -= chunk_sum<NR>(a, f, NR * k0 + tid, polls);
   }
-  double acc[2 * NR];
-#pragma unroll
-  for (int k = 0; k < 2 * NR; k++) acc[k] = 0.0;
+  Frag<NR> fr;
+  fr.zero();
   for (int R = nsb - 1; R > s; R--) {
-    const int g = R * kFlowSB + tid;
-    get_entry<NR>(xr + static_cast<int64_t>(NR) * g, g < w, xs + (NR + 2) * tid, a.err, polls);
+    const int64_t rb = R * static_cast<int64_t>(kFlowSB) + rw;
+    if (R - 1 > s) load_frag_t(lvn, P, f.h, rb - kFlowSB, w, k0, cend);
+    get_entry<NR>(xr + NR * (rb + lane), rb + lane < w, own + NP * lane, a.err, polls);
+    __syncwarp();
+    mma_tile(fr, lv, own);
+    __syncwarp();
+#pragma unroll
+    for (int k = 0; k < 32; k++) lv[k] = lvn[k];
+  }
+  if (nsb - 1 > s) {
+    fr.template put<false>(own);
     __syncthreads();
-    tile_cols<NR>(lv, xs, acc);
-    if (R - 1 > s) load_rows(lv, P, f.h, static_cast<int64_t>(R - 1) * kFlowSB, kFlowSB, k0, cend);
+    if (col < 32) {
+      double t[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+      for (int q = 0; q < 16; q++) t[q % 4] += xs[32 * NP * q + at];
+      v -= (t[0] + t[1]) + (t[2] + t[3]);
+    }
     __syncthreads();
   }
-  // Sums of the warp's two columns, to the threads that own the outputs.
-  {
-    const double t   = reduce_lanes<2 * NR>(acc);
-    constexpr int kL = 16 / NR;
-    if (lane % kL == 0) xs[2 * NR * warp + lane / kL] = t;
-  }
-  __syncthreads();
-  if (col < 32) v -= xs[tid];
-  __syncthreads();
   double *xz = a.xz + static_cast<int64_t>(NR) * (f.col0 + s * kFlowSB);
   if (col < 32) {
     if (!mine) v = 0.0;
     if (j > 0 && mine) st_relaxed_f64(xz + 32 * NR * j + tid, v);
-    xs[tid] = v;  // the diagonal block's, for warp 0
+    xs[at] = v;  // the diagonal block's, for warp 0
   }
   __syncthreads();
   bulk_wait(bar, phase, a.err);
@@ -736,24 +881,20 @@ __device__ __noinline__ void bwd_slab_m(const FlowArgs<T> &a, FlowShared &S, con
   if (j + warp < nsl) {
     const int i = j + warp;
     if (warp > 0)
-      get_entry<NR>(xz + NR * (32 * i + lane), s * kFlowSB + 32 * i + lane < w, own + NR * lane, a.err,
+      get_entry<NR>(xz + NR * (32 * i + lane), s * kFlowSB + 32 * i + lane < w, own + NP * lane, a.err,
                     polls);
     __syncwarp();
-    double o[NR];
-#pragma unroll
-    for (int k = 0; k < NR; k++) o[k] = 0.0;
-    const double *blk = inv + warp * kFlowBlk + 33 * lane;
-#pragma unroll 8
-    for (int r = 0; r < 32; r++) fma_entry<NR>(blk[r], own + NR * r, o);
+    fr.zero();
+    mma_inverse_t(fr, inv + warp * kFlowBlk, own);
     __syncwarp();
-    put_entry<NR>(own + NR * lane, o);
+    fr.template put<false>(own);
   }
   __syncthreads();
   if (mine) {
     double t[4] = {0.0, 0.0, 0.0, 0.0};
 #pragma unroll
     for (int q = 0; q < 16; q++)
-      if (j + q < nsl) t[q % 4] += xs[32 * NR * q + tid];
+      if (j + q < nsl) t[q % 4] += xs[32 * NP * q + at];
     const double  x = (t[0] + t[1]) + (t[2] + t[3]);
     const int64_t g = static_cast<int64_t>(NR) * (f.col0 + k0) + tid;
 #pragma unroll
