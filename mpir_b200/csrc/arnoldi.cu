@@ -1,0 +1,574 @@
+// PrecondGmres (gmres_ir.hpp:636-741) on the device: the modified Gram-Schmidt
+// step, the Givens rotations and the stop tests, one launch per inner step.
+//
+// A step's k + 2 reductions depend on one another, and at these sizes each is
+// latency, not bandwidth: as separate launches (one per reduction, a copy of
+// the column to the host and a synchronisation for its rotations) a step of
+// k = 4 took about 40 us beside the preconditioner.  Here one thread-block
+// cluster per vector keeps w in registers and runs the whole step: a reduction
+// is a block reduction, one exchange through distributed shared memory and one
+// cluster barrier (about 1 us).  Systems of up to 8,192 unknowns take one CTA,
+// which needs neither; a cluster of 8 (16 from 65,536 on) covers the rest, with
+// the entries beyond its registers (512 threads x 16 a CTA) in global memory.
+// One thread applies the rotations and decides whether to go on; the kernels of
+// a step that is not taken return at once, so the host may queue the next step
+// before it knows.
+//
+// Measured outside the triangular solves: n = 1,280, 5 inner steps in two inner
+// loops, 0.46 ms a solve as separate launches, 0.15 here; n = 40,960 (8 CTAs), 7
+// steps in three, 0.9 -> 0.4 ms; three vectors of n = 40,951, 9 steps in three,
+// 1.3 -> 0.5 ms.
+//
+// Sums run in a fixed order (threads, warps, CTAs), so results are
+// reproducible.  Norms are sqrt of the sum of squares, or, where that sum is
+// not well inside the range of float64, the scaled form of Dnrm2
+// (ops.hpp:231-264).
+#include <cmath>
+
+#include "arnoldi.hpp"
+#include "common.cuh"
+
+namespace mpir {
+
+namespace {
+
+constexpr int kThreads = 512;
+constexpr int kRegs    = 16;  // entries of w a thread keeps
+constexpr int kWarps   = kThreads / 32;
+
+struct ArnoldiArgs {
+  int64_t    n, m, vs, block, stride;
+  double    *V, *state;
+  double     tol;
+  GmresMail *mail;
+};
+
+struct StateView {
+  GmresCtl *ctl;
+  double   *R, *c, *s, *g, *y, *col;
+  __device__ StateView(const ArnoldiArgs &a, int vec) {
+    double *p = a.state + vec * a.stride;
+    ctl       = reinterpret_cast<GmresCtl *>(p);
+    R         = p + 4;
+    c         = R + a.m * (a.m + 1) / 2;
+    s         = c + a.m;
+    g         = s + a.m;
+    y         = g + a.m + 1;
+    col       = y + a.m;
+  }
+};
+
+__device__ __forceinline__ uint32_t cluster_rank() {
+  uint32_t r;
+  asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ uint32_t cluster_size() {
+  uint32_t r;
+  asm("mov.u32 %0, %%cluster_nctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// One double into CTA `rank`'s copy of a shared variable.
+__device__ __forceinline__ void cluster_put(double *p, uint32_t rank, double v) {
+  uint32_t a = static_cast<uint32_t>(__cvta_generic_to_shared(p)), r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(rank));
+  asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(r), "d"(v) : "memory");
+}
+
+struct RedShared {
+  double warp[2][kWarps];
+  double slot[2][16][2];  // by the parity of the reduction, by CTA
+};
+
+// Sums (or, MAX, maxima) of a and b over the cluster, in every thread.
+template <bool MAX>
+struct Reducer {
+  RedShared &S;
+  int       &turn;
+  __device__ __forceinline__ static double op(double x, double y) { return MAX ? (x > y ? x : y) : x + y; }
+  __device__ __forceinline__ void run(double &a, double &b) {
+    const unsigned full = 0xffffffffu;
+    const int      warp = threadIdx.x / 32, lane = threadIdx.x % 32, C = cluster_size();
+    const int      t = turn & 1;
+    turn++;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      a = op(a, __shfl_xor_sync(full, a, o));
+      b = op(b, __shfl_xor_sync(full, b, o));
+    }
+    if (lane == 0) {
+      S.warp[0][warp] = a;
+      S.warp[1][warp] = b;
+    }
+    __syncthreads();
+    if (warp == 0) {
+      a = S.warp[0][lane % kWarps];
+      b = S.warp[1][lane % kWarps];
+#pragma unroll
+      for (int o = kWarps / 2; o > 0; o >>= 1) {
+        a = op(a, __shfl_xor_sync(full, a, o));
+        b = op(b, __shfl_xor_sync(full, b, o));
+      }
+      if (C == 1) {
+        if (lane == 0) {
+          S.slot[t][0][0] = a;
+          S.slot[t][0][1] = b;
+        }
+      } else if (lane < C) {
+        cluster_put(&S.slot[t][cluster_rank()][0], lane, a);
+        cluster_put(&S.slot[t][cluster_rank()][1], lane, b);
+      }
+    }
+    if (C == 1)
+      __syncthreads();
+    else
+      cluster_sync();
+    a = S.slot[t][0][0];
+    b = S.slot[t][0][1];
+    for (int r = 1; r < C; r++) {
+      a = op(a, S.slot[t][r][0]);
+      b = op(b, S.slot[t][r][1]);
+    }
+  }
+};
+
+// A vector spread over the cluster: entry j of a thread is (j C + rank) 512 +
+// tid; the first kRegs in registers, the rest in global memory.
+struct Spread {
+  int64_t n, i0, step;
+  __device__ Spread(int64_t n_) : n(n_) {
+    step = static_cast<int64_t>(cluster_size()) * kThreads;
+    i0   = static_cast<int64_t>(cluster_rank()) * kThreads + threadIdx.x;
+  }
+  __device__ __forceinline__ void load(double (&w)[kRegs], const double *p) const {
+#pragma unroll
+    for (int j = 0; j < kRegs; j++) w[j] = i0 + j * step < n ? p[i0 + j * step] : 0.0;
+  }
+  // f(i) for the entries beyond the registers.
+  template <class F>
+  __device__ __forceinline__ void rest(F f) const {
+#pragma unroll 4
+    for (int64_t i = i0 + kRegs * step; i < n; i += step) f(i);
+  }
+  template <class F>
+  __device__ __forceinline__ void regs(F f) const {
+#pragma unroll
+    for (int j = 0; j < kRegs; j++)
+      if (i0 + j * step < n) f(j, i0 + j * step);
+  }
+};
+
+// sqrt(ss), ss the sum of squares of w, or the scaled norm where ss has left
+// the range in which that is accurate.
+__device__ double safe_norm(double ss, const Spread &sp, const double (&w)[kRegs], const double *wg,
+                            RedShared &S, int &turn) {
+  if (ss > 1e-280 && ss < 1e280) return sqrt(ss);
+  if (!(ss == ss)) return ss;
+  double mx = 0.0, none = 0.0;
+#pragma unroll
+  for (int j = 0; j < kRegs; j++) mx = fmax(mx, fabs(w[j]));
+  sp.rest([&](int64_t i) { mx = fmax(mx, fabs(wg[i])); });
+  Reducer<true>{S, turn}.run(mx, none);
+  if (mx == 0.0 || !isfinite(mx)) return mx;
+  double q = 0.0;
+  none     = 0.0;
+#pragma unroll
+  for (int j = 0; j < kRegs; j++) q += (w[j] / mx) * (w[j] / mx);
+  sp.rest([&](int64_t i) { q += (wg[i] / mx) * (wg[i] / mx); });
+  Reducer<false>{S, turn}.run(q, none);
+  return mx * sqrt(q);
+}
+
+// A CTA of a cluster must not exit while another may still write to its shared
+// memory or wait for it.
+__device__ __forceinline__ void leave() {
+  if (cluster_size() > 1) cluster_sync();
+}
+
+__global__ void __launch_bounds__(kThreads)
+    k_gmres_begin(const ArnoldiArgs a, uint32_t act, const double *b, const VecFactors fac) {
+  __shared__ RedShared S;
+  int                  turn = 0;
+  const int            vec  = blockIdx.y;
+  StateView            st(a, vec);
+  const bool           lead = cluster_rank() == 0 && threadIdx.x == 0;
+  if (!(act >> vec & 1u)) {
+    if (lead) {
+      *st.ctl               = GmresCtl{0.0, 0, 0, 0, 0, {0, 0}};
+      a.mail->active[0][vec] = a.mail->active[1][vec] = 0;
+    }
+    return;
+  }
+  const Spread  sp(a.n);
+  const double  f  = fac.v[vec];
+  const double *bv = b + vec * a.vs;
+  double       *w0 = a.V + vec * a.vs, w[kRegs], ss = 0.0, none = 0.0;
+  sp.load(w, bv);
+#pragma unroll
+  for (int j = 0; j < kRegs; j++) {
+    w[j] *= f;
+    ss += w[j] * w[j];
+  }
+  sp.regs([&](int j, int64_t i) { w0[i] = w[j]; });
+  sp.rest([&](int64_t i) {
+    const double x = bv[i] * f;
+    w0[i]          = x;
+    ss += x * x;
+  });
+  Reducer<false>{S, turn}.run(ss, none);
+  const double rho = safe_norm(ss, sp, w, w0, S, turn);
+  if (lead) {
+    const int32_t go       = !(rho < a.tol);  // gmres_ir.hpp:655-657
+    *st.ctl                = GmresCtl{rho, 0, go, 0, go, {0, 0}};
+    a.mail->active[0][vec] = a.mail->active[1][vec] = go;
+  }
+  leave();
+}
+
+__global__ void __launch_bounds__(kThreads) k_gmres_first(const ArnoldiArgs a) {
+  __shared__ RedShared S;
+  int                  turn = 0;
+  const int            vec  = blockIdx.y;
+  StateView            st(a, vec);
+  if (st.ctl->active == 0) return;
+  const Spread sp(a.n);
+  double      *w0 = a.V + vec * a.vs, w[kRegs], ss = 0.0, none = 0.0;
+  sp.load(w, w0);
+#pragma unroll
+  for (int j = 0; j < kRegs; j++) ss += w[j] * w[j];
+  sp.rest([&](int64_t i) { ss += w0[i] * w0[i]; });
+  Reducer<false>{S, turn}.run(ss, none);
+  const double rho = safe_norm(ss, sp, w, w0, S, turn), f = 1 / rho;
+  sp.regs([&](int j, int64_t i) { w0[i] = w[j] * f; });
+  sp.rest([&](int64_t i) { w0[i] *= f; });
+  leave();  // every CTA has read the active flag
+  if (cluster_rank() == 0 && threadIdx.x == 0) {
+    st.g[0]         = rho;
+    st.ctl->rho     = rho;
+    st.ctl->active  = a.m > 0 && rho > a.tol;
+  }
+}
+
+// One inner step (gmres_ir.hpp:664-726): |w|, then for each basis vector v_j
+// h = w v_j and w -= h v_j, each pass summing for the next one (the loads of
+// v_{j+1} before its reduction); a second sweep where Brown and Hindmarsh's test
+// asks for it; w /= |w|; the rotations.
+__global__ void __launch_bounds__(kThreads) k_gmres_step(const ArnoldiArgs a, int64_t k) {
+  __shared__ RedShared S;
+  int                  turn = 0;
+  const int            vec  = blockIdx.y, lane = threadIdx.x % 32;
+  StateView            st(a, vec);
+  const bool           lead = cluster_rank() == 0 && threadIdx.x == 0;
+  if (st.ctl->active == 0) {
+    if (lead) a.mail->active[k & 1][vec] = 0;
+    return;
+  }
+  const Spread sp(a.n);
+  double      *V = a.V + vec * a.vs, *wg = V + (k + 1) * a.block;
+  double       w[kRegs], v[kRegs];
+  sp.load(w, wg);
+  sp.load(v, V);
+  double ss = 0.0, h = 0.0;
+#pragma unroll
+  for (int j = 0; j < kRegs; j++) {
+    ss += w[j] * w[j];
+    h += w[j] * v[j];
+  }
+  sp.rest([&](int64_t i) {
+    ss += wg[i] * wg[i];
+    h += wg[i] * V[i];
+  });
+  Reducer<false>{S, turn}.run(ss, h);
+  const double normav = safe_norm(ss, sp, w, wg, S, turn);
+  double       normw  = 0.0;
+  int32_t      reorth = 0;
+  for (int pass = 0;; pass++) {
+    for (int64_t j = 0; j <= k; j++) {
+      if (lead) st.col[j] = pass == 0 ? h : st.col[j] + h;
+      const double *vj = V + j * a.block, *vn = vj + a.block;
+      const double  hj = h;
+      const bool    more = j < k;
+#pragma unroll
+      for (int q = 0; q < kRegs; q++) w[q] -= v[q] * hj;
+      if (more) sp.load(v, vn);
+      double t = 0.0, none = 0.0;
+#pragma unroll
+      for (int q = 0; q < kRegs; q++) t += w[q] * (more ? v[q] : w[q]);
+      sp.rest([&](int64_t i) {
+        const double x = wg[i] - vj[i] * hj;
+        wg[i]          = x;
+        t += x * (more ? vn[i] : x);
+      });
+      Reducer<false>{S, turn}.run(t, none);
+      h = t;
+    }
+    normw = safe_norm(h, sp, w, wg, S, turn);
+    // Brown/Hindmarsh, gmres_ir.hpp:683
+    if (pass > 0 || !(normav + 0.001 * normw == normav)) break;
+    reorth = 1;
+    sp.load(v, V);
+    double t = 0.0, none = 0.0;
+#pragma unroll
+    for (int q = 0; q < kRegs; q++) t += w[q] * v[q];
+    sp.rest([&](int64_t i) { t += wg[i] * V[i]; });
+    Reducer<false>{S, turn}.run(t, none);
+    h = t;
+  }
+  const double f = normw != 0 ? 1 / normw : 1.0;
+  sp.regs([&](int j, int64_t i) { wg[i] = w[j] * f; });
+  sp.rest([&](int64_t i) { wg[i] *= f; });
+  leave();  // every CTA has read the active flag
+  if (cluster_rank() != 0 || threadIdx.x >= 32) return;
+  // The column's rotations, by one warp: 32 of them are loaded at a time, the
+  // chain over them runs in registers.
+  __syncwarp();
+  double       *R = st.R + k * (k + 1) / 2;
+  double        hj = __shfl_sync(0xffffffffu, lane == 0 ? st.col[0] : 0.0, 0);  // h(j, k) so far
+  for (int64_t j0 = 0; j0 < k; j0 += 32) {
+    const bool   ok = j0 + lane < k;
+    const double cj = ok ? st.c[j0 + lane] : 0.0, sj = ok ? st.s[j0 + lane] : 0.0;
+    const double hn = ok ? __ldcg(st.col + j0 + lane + 1) : 0.0;
+    double       out = 0.0;
+    const int    cnt = static_cast<int>(k - j0 < 32 ? k - j0 : 32);
+    for (int q = 0; q < cnt; q++) {
+      const double c1 = __shfl_sync(0xffffffffu, cj, q), s1 = __shfl_sync(0xffffffffu, sj, q);
+      const double h1 = __shfl_sync(0xffffffffu, hn, q);
+      const double w1 = c1 * hj - s1 * h1, w2 = s1 * hj + c1 * h1;
+      if (lane == q) out = w1;
+      hj = w2;
+    }
+    if (ok) R[j0 + lane] = out;
+  }
+  if (lane != 0) return;
+  // Dnrm2 of {h_kk, h_k+1,k}, walked last to first as ops.hpp:243 does.
+  double       scale = 0.0, ssq = 1.0;
+  const double pr[2] = {hj, normw};
+#pragma unroll
+  for (int q = 1; q >= 0; q--)
+    if (pr[q] != 0.0) {
+      const double x = fabs(pr[q]);
+      if (scale < x) {
+        ssq   = 1.0 + ssq * ((scale / x) * (scale / x));
+        scale = x;
+      } else {
+        ssq = ssq + ((x / scale) * (x / scale));
+      }
+    }
+  const double nu = scale * sqrt(ssq);
+  double       gk = st.g[k], gn = 0.0;
+  if (nu != 0) {
+    const double c = hj / nu, s = -normw / nu;
+    st.c[k] = c;
+    st.s[k] = s;
+    hj      = c * hj - s * normw;
+    gn      = s * gk;
+    gk      = c * gk;
+  } else {
+    st.c[k] = 0.0;
+    st.s[k] = 0.0;
+  }
+  R[k]           = hj;
+  st.g[k]        = gk;
+  st.g[k + 1]    = gn;
+  const double r = fabs(gn);
+  const int32_t go = k + 1 < a.m && r > a.tol;
+  st.ctl->rho    = r;
+  st.ctl->k      = static_cast<int32_t>(k + 1);
+  st.ctl->active = go;
+  st.ctl->reorth += reorth;
+  a.mail->active[k & 1][vec] = go;
+}
+
+__global__ void __launch_bounds__(kThreads)
+    k_gmres_end(const ArnoldiArgs a, uint32_t act, double *x, int update, const VecFactors fac,
+                unsigned long long *inf) {
+  __shared__ RedShared S;
+  int                  turn = 0;
+  const int            vec  = blockIdx.y, tid = threadIdx.x;
+  if (!(act >> vec & 1u)) return;
+  StateView     st(a, vec);
+  const int64_t k = st.ctl->k;
+  // y = R^{-1} g by columns, in the leading CTA.
+  if (cluster_rank() == 0) {
+    for (int64_t j = tid; j < k; j += kThreads) st.y[j] = st.g[j];
+    __syncthreads();
+    for (int64_t i = k - 1; i >= 0; i--) {
+      const double *R  = st.R + i * (i + 1) / 2;
+      const double  yi = st.y[i] / R[i];
+      __syncthreads();
+      for (int64_t j = tid; j <= i; j += kThreads) st.y[j] = j == i ? yi : st.y[j] - R[j] * yi;
+      __syncthreads();
+    }
+    if (tid == 0) {
+      a.mail->k[vec]      = static_cast<int32_t>(k);
+      a.mail->reorth[vec] = st.ctl->reorth;
+      a.mail->began[vec]  = st.ctl->began;
+    }
+  }
+  if (cluster_size() > 1)
+    cluster_sync();
+  else
+    __syncthreads();
+  const Spread  sp(a.n);
+  const double  f  = fac.v[vec];
+  const double *V  = a.V + vec * a.vs;
+  double       *xv = x + vec * a.vs, d[kRegs], dm = 0.0, xm = 0.0;
+#pragma unroll
+  for (int j = 0; j < kRegs; j++) d[j] = 0.0;
+  // (y is written by another CTA: not through the read-only path.)
+  for (int64_t j = 0; j < k; j++) {
+    const double  yj = __ldcg(st.y + j);
+    const double *vj = V + j * a.block;
+    sp.regs([&](int q, int64_t i) { d[q] += vj[i] * yj; });
+  }
+  auto put = [&](double dv, int64_t i) {  // gmres_ir.hpp:574-577
+    if (!update) {
+      xv[i] = dv;
+      return;
+    }
+    const double di = dv * f, xi = xv[i];
+    // NaN counts as above infinity, as in the max-norms of the vector kernels
+    dm    = fabs(di) > dm || !(di == di) ? fabs(di) : dm;
+    xm    = fabs(xi) > xm || !(xi == xi) ? fabs(xi) : xm;
+    xv[i] = xi + di;
+  };
+  sp.regs([&](int q, int64_t i) { put(d[q], i); });
+  sp.rest([&](int64_t i) {
+    double dv = 0.0;
+    for (int64_t j = 0; j < k; j++) dv += V[j * a.block + i] * __ldcg(st.y + j);
+    put(dv, i);
+  });
+  if (!update) return;
+  // max over the cluster on the bit patterns (the order of non-negative
+  // doubles, NaN above all)
+  {
+    const unsigned      full = 0xffffffffu;
+    unsigned long long  b0 = __double_as_longlong(dm), b1 = __double_as_longlong(xm);
+    __shared__ unsigned long long sb[2][kWarps];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      const unsigned long long c0 = __shfl_xor_sync(full, b0, o), c1 = __shfl_xor_sync(full, b1, o);
+      b0 = c0 > b0 ? c0 : b0;
+      b1 = c1 > b1 ? c1 : b1;
+    }
+    if (tid % 32 == 0) {
+      sb[0][tid / 32] = b0;
+      sb[1][tid / 32] = b1;
+    }
+    __syncthreads();
+    if (tid == 0) {
+      for (int q = 1; q < kWarps; q++) {
+        b0 = sb[0][q] > b0 ? sb[0][q] : b0;
+        b1 = sb[1][q] > b1 ? sb[1][q] : b1;
+      }
+      if (cluster_size() > 1) {
+        cluster_put(&S.slot[0][cluster_rank()][0], 0, __longlong_as_double(static_cast<long long>(b0)));
+        cluster_put(&S.slot[0][cluster_rank()][1], 0, __longlong_as_double(static_cast<long long>(b1)));
+      }
+    }
+    (void)turn;
+    if (cluster_size() > 1) cluster_sync();
+    if (cluster_rank() == 0 && tid == 0) {
+      if (cluster_size() > 1) {
+        b0 = b1 = 0;
+        for (uint32_t r = 0; r < cluster_size(); r++) {
+          const unsigned long long c0 = __double_as_longlong(S.slot[0][r][0]),
+                                   c1 = __double_as_longlong(S.slot[0][r][1]);
+          b0 = c0 > b0 ? c0 : b0;
+          b1 = c1 > b1 ? c1 : b1;
+        }
+      }
+      inf[8 * vec]     = 0;
+      inf[8 * vec + 1] = b0;
+      inf[8 * vec + 2] = b1;
+    }
+  }
+}
+
+ArnoldiArgs make_args(int64_t n, int64_t m, int64_t stride, double *V, int64_t block, double *state,
+                      double tol, GmresMail *mail) {
+  return ArnoldiArgs{n, m, n, block, stride, V, state, tol, mail};
+}
+
+// Launch on clusters of C CTAs, one per vector.
+template <class... K, class... A>
+void launch_cluster(void (*kernel)(K...), int C, int nb, cudaStream_t s, A &&...args) {
+  launch_add(1);
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim  = dim3(C, nb, 1);
+  cfg.blockDim = dim3(kThreads, 1, 1);
+  cfg.stream   = s;
+  cudaLaunchAttribute at{};
+  at.id               = cudaLaunchAttributeClusterDimension;
+  at.val.clusterDim.x = C;
+  at.val.clusterDim.y = 1;
+  at.val.clusterDim.z = 1;
+  cfg.attrs           = &at;
+  cfg.numAttrs        = 1;
+  MPIR_CUDA(cudaLaunchKernelEx(&cfg, kernel, static_cast<K>(args)...));
+}
+
+void allow_16() {
+  static const bool done = [] {
+    for (auto *f : {reinterpret_cast<const void *>(k_gmres_begin), reinterpret_cast<const void *>(k_gmres_first),
+                    reinterpret_cast<const void *>(k_gmres_step), reinterpret_cast<const void *>(k_gmres_end)})
+      MPIR_CUDA(cudaFuncSetAttribute(f, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    return true;
+  }();
+  (void)done;
+}
+
+}  // namespace
+
+Arnoldi::~Arnoldi() {
+  if (mail_) pinned_free(mail_, sizeof(GmresMail));
+}
+
+void Arnoldi::allocate(int64_t n, int64_t m, int vectors) {
+  n_       = n;
+  m_       = m;
+  vectors_ = vectors;
+  state_.resize(bytes_for(m, vectors));
+  if (!mail_) mail_ = static_cast<GmresMail *>(pinned_alloc(sizeof(GmresMail)));
+}
+
+const int32_t *Arnoldi::active() const {
+  return reinterpret_cast<const int32_t *>(state_.as<char>() + offsetof(GmresCtl, active));
+}
+
+// One CTA up to the entries its registers hold; 8 CTAs; 16 where that keeps
+// the vector in registers or nearly so.
+int Arnoldi::cluster() const {
+  constexpr int64_t cta = static_cast<int64_t>(kThreads) * kRegs;
+  return n_ <= cta ? 1 : n_ <= 8 * cta ? 8 : 16;
+}
+
+void Arnoldi::begin(int nb, uint32_t act, const double *b, const VecFactors &fac, double *V, double tol,
+                    cudaStream_t s) {
+  allow_16();
+  launch_cluster(k_gmres_begin, cluster(), nb, s,
+                 make_args(n_, m_, stride(m_), V, 0, state_.as<double>(), tol, mail_), act, b, fac);
+}
+
+void Arnoldi::first(int nb, double *V, double tol, cudaStream_t s) {
+  launch_cluster(k_gmres_first, cluster(), nb, s,
+                 make_args(n_, m_, stride(m_), V, 0, state_.as<double>(), tol, mail_));
+}
+
+void Arnoldi::step(int nb, int64_t j, double *V, int64_t block, double tol, cudaStream_t s) {
+  launch_cluster(k_gmres_step, cluster(), nb, s,
+                 make_args(n_, m_, stride(m_), V, block, state_.as<double>(), tol, mail_), j);
+}
+
+void Arnoldi::end(int nb, uint32_t act, const double *V, int64_t block, double *x, bool update,
+                  const VecFactors &scale, unsigned long long *inf, cudaStream_t s) {
+  launch_cluster(k_gmres_end, cluster(), nb, s,
+                 make_args(n_, m_, stride(m_), const_cast<double *>(V), block, state_.as<double>(), 0.0, mail_),
+                 act, x, update ? 1 : 0, scale, inf);
+}
+
+}  // namespace mpir

@@ -39,6 +39,10 @@ struct FlowArgs {
   int64_t  nmark;
   int32_t *ticket;
   int32_t *err;
+  // nactive flags active_stride apart (NULL: none): nothing is done when all
+  // are zero (the values stay as they are, for the next solve).
+  const int32_t *active;
+  int32_t        nactive, active_stride;
 };
 
 struct FlowSlot {
@@ -80,6 +84,15 @@ __device__ __forceinline__ void flow_fetch(const FlowArgs<T> &a, FlowSlot &S) {
   if (t < a.nitems && lane < kFlowItemWords)
     cp_async8(reinterpret_cast<double *>(&S.item) + lane,
               reinterpret_cast<const double *>(a.items + t) + lane);
+}
+
+// True when no vector is active: the kernel returns at once (no ticket taken,
+// no value marked).
+template <class T>
+__device__ __forceinline__ bool flow_idle(const FlowArgs<T> &a) {
+  int32_t on = a.active == nullptr;
+  for (int k = 0; k < a.nactive; k++) on |= a.active[k * a.active_stride];
+  return on == 0;
 }
 
 // The kernels' common loop: work(this slot, the next one) for every item.

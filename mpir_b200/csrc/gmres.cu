@@ -54,13 +54,17 @@ Solver::Solver(int uf_, int uw_, int ur_, int dev)
   stream_ = own_stream_;
   MPIR_CUDA(cudaEventCreate(&ev0_));
   MPIR_CUDA(cudaEventCreate(&ev1_));
+  for (cudaEvent_t &e : step_ev_) MPIR_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+  box_ = static_cast<HostBox *>(pinned_alloc(sizeof(HostBox)));
 }
 
 Solver::~Solver() {
   cudaSetDevice(device);
   if (own_stream_) cudaStreamSynchronize(own_stream_);
   if (stream_ && stream_ != own_stream_) cudaStreamSynchronize(stream_);
-  if (hpin_) pinned_free(hpin_, hpin_bytes_);
+  if (box_) pinned_free(box_, sizeof(HostBox));
+  for (cudaEvent_t e : step_ev_)
+    if (e) cudaEventDestroy(e);
   if (ev0_) cudaEventDestroy(ev0_);
   if (ev1_) cudaEventDestroy(ev1_);
   plan_.reset();
@@ -106,9 +110,7 @@ void Solver::adopt(std::shared_ptr<Plan> P) {
   num_.allocate(*plan_);
   num_.update_mode = update_mode_for(uf, update_engine);
   ws_.allocate(*plan_);
-  int sms = 148;
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-  vec_.allocate(n, sms);
+  vec_.allocate(n);
   vec_m_ = -1;
   // The batch buffers belong to the previous pattern.
   bw_  = 0;
@@ -121,12 +123,10 @@ void Solver::adopt(std::shared_ptr<Plan> P) {
 
 size_t Solver::device_bytes() const {
   size_t b = num_.device_bytes();
-  for (const DeviceBuffer *d : {&ws_.vals, &ws_.sync, &ws_.err,
-                                &mws_.vals, &mws_.sync, &mws_.err,
-                                &vec_.part, &vec_.count, &vec_.infbits, &vecb_.part, &vecb_.count,
-                                &vecb_.infbits, &V_, &bs_, &bp_, &ADp_, &x_, &r_, &t_, &d_, &hd_,
-                                &y_, &hb_, &hx_, &bV_, &bbs_, &bbp_, &bx_, &br_, &bt_, &bd_, &bhd_,
-                                &by_, &bfac_, &bact_, &bkq_, &bin_, &bout_})
+  b += ar_.bytes() + bar_.bytes();
+  for (const DeviceBuffer *d : {&ws_.vals, &ws_.sync, &ws_.err, &mws_.vals, &mws_.sync, &mws_.err,
+                                &vec_.infbits, &vecb_.infbits, &V_, &bs_, &bp_, &ADp_, &x_, &r_, &t_,
+                                &hb_, &hx_, &bV_, &bbs_, &bbp_, &bx_, &br_, &bin_, &bout_})
     b += d->bytes();
   return b;
 }
@@ -137,10 +137,10 @@ size_t Solver::bytes_for(const Plan &P, int64_t gmres_iter, int width, int uf) {
   size_t        b  = Numeric::bytes_for(P, uf == kBF16 ? 2 : uf == kF16 ? 3 : 1);
   // single-vector workspace and vectors
   b += SolveWorkspace::bytes_for(P);
-  b += (m + 1 + 10) * n * sizeof(double) + 2048 * sizeof(double);
+  b += (m + 1 + 8) * n * sizeof(double) + Arnoldi::bytes_for(m, 1);
   if (width > 1) {
     b += MultiSolveWorkspace::bytes_for(P, width);
-    b += (m + 1 + 8) * n * width * sizeof(double) + 2048 * width * sizeof(double);
+    b += (m + 1 + 6) * n * width * sizeof(double) + Arnoldi::bytes_for(m, width);
   }
   return b;
 }
@@ -156,11 +156,9 @@ void Solver::ensure_vectors() {
   x_.resize(vb);
   r_.resize(vb);
   t_.resize(vb);
-  d_.resize(vb);
   hb_.resize(vb);
   hx_.resize(vb);
-  hd_.resize(sizeof(double) * 2 * (m + 4));
-  y_.resize(sizeof(double) * (m + 1));
+  ar_.allocate(n, m, 1);
   vec_m_ = m;
 }
 
@@ -241,116 +239,51 @@ void Solver::set_wait_controls(int poll_log2, int withhold_item) {
   MPIR_CUDA(cudaStreamSynchronize(stream_));
 }
 
-// PrecondGmres, gmres_ir.hpp:636-741.
-void Solver::precond_gmres(const double *b, double *res, Report &st) {
-  const Plan   &P  = *plan_;
-  const int64_t n  = P.S.n;
-  cudaStream_t  s  = stream_;
-  gmres_iter       = std::min<int64_t>(gmres_iter, n);  // gmres_ir.hpp:643
-  const int64_t m  = gmres_iter;
-  double       *V  = V_.as<double>();
-  double       *hd = hd_.as<double>();
+void Solver::apply(int nb, int width, double *x, const ActiveFlags &act) {
+  if (width == 1)
+    ldlt_solve(*plan_, num_, x, ws_, stream_, kAllPhases, act);
+  else
+    ldlt_solve_multi(*plan_, num_, x, width, mws_, stream_, act);
+}
+
+// PrecondGmres, gmres_ir.hpp:636-741.  The host queues step j + 1 before it
+// knows whether step j was the last one (kernels of a step that is not taken
+// return at once), so the device never waits for the host.
+void Solver::inner(int nb, int width, uint32_t act, const double *b, const VecFactors &fac, double *V,
+                   Arnoldi &ar, VecOps &vo, double *x, bool update, const VecFactors &scale) {
+  const Plan    &P  = *plan_;
+  cudaStream_t   s  = stream_;
+  gmres_iter        = std::min<int64_t>(gmres_iter, P.S.n);  // gmres_ir.hpp:643
+  const int64_t  m  = gmres_iter, block = P.S.n * width;
   const int64_t *Kp = P.Kp.as<int64_t>();
   const int32_t *Kj = P.Kj.as<int32_t>();
   const double  *Kv = num_.Kval.as<double>();
-  MPIR_CUDA(cudaMemsetAsync(res, 0, n * sizeof(double), s));
-  auto read = [&](double *h, int first, int cnt) {
-    MPIR_CUDA(cudaMemcpyAsync(h, hd + first, cnt * sizeof(double), cudaMemcpyDeviceToHost, s));
-    MPIR_CUDA(cudaStreamSynchronize(s));
-  };
-  double rho;
-  vec_.mgs_pass(const_cast<double *>(b), nullptr, nullptr, nullptr, 1, hd, s);
-  read(&rho, 0, 1);
-  if (rho < tol) return;
-  MPIR_CUDA(cudaMemcpyAsync(V, b, n * sizeof(double), cudaMemcpyDeviceToDevice, s));
-  ldlt_solve(P, num_, V, ws_, s);
-  st.precond_applies++;
-  vec_.mgs_pass(V, nullptr, nullptr, nullptr, 1, hd, s);
-  read(&rho, 0, 1);
-  vec_.scale(V, 1 / rho, V, s);
+  const ActiveFlags on{ar.active(), nb, ar.active_stride()};
+  ar.begin(nb, act, b, fac, V, tol, s);
+  apply(nb, width, V, on);
+  ar.first(nb, V, tol, s);
+  for (int64_t j = 0; j < m; j++) {
+    double *w = V + (j + 1) * block;
+    vo.spmv(nb, Kp, Kj, Kv, w - block, w, s);
+    apply(nb, width, w, on);
+    ar.step(nb, j, V, block, tol, s);
+    MPIR_CUDA(cudaEventRecord(step_ev_[j & 1], s));
+    if (j == 0) continue;
+    MPIR_CUDA(cudaEventSynchronize(step_ev_[(j - 1) & 1]));
+    bool more = false;
+    for (int k = 0; k < nb; k++) more |= ar.mail().active[(j - 1) & 1][k] != 0;
+    if (!more) break;
+  }
+  ar.end(nb, act, V, block, x, update, scale, vo.infbits.as<unsigned long long>(), s);
+}
 
-  std::vector<double> H((m + 1) * std::max<int64_t>(m, 1), 0.0), g(m + 1, 0.0),
-      c(std::max<int64_t>(m, 1), 0.0), sn(std::max<int64_t>(m, 1), 0.0),
-      col(m + 3, 0.0);
-  auto h = [&](int64_t i, int64_t j) -> double & { return H[i * std::max<int64_t>(m, 1) + j]; };
-  g[0] = rho;
-  int64_t k;
-  for (k = 0; k < m && rho > tol; k++) {
-    double *vk = V + k * n, *w = V + (k + 1) * n;
-    vec_.spmv(Kp, Kj, Kv, vk, w, s);
-    st.spmv_count++;
-    ldlt_solve(P, num_, w, ws_, s);
-    st.precond_applies++;
-    double *hn = hd + (m + 2);  // normav
-    vec_.mgs_pass(w, nullptr, nullptr, nullptr, 1, hn, s);
-    vec_.mgs_pass(w, nullptr, nullptr, V, 0, hd, s);
-    for (int64_t j = 0; j <= k; j++)
-      vec_.mgs_pass(w, V + j * n, hd + j, j < k ? V + (j + 1) * n : nullptr, j < k ? 0 : 1,
-                    hd + j + 1, s);
-    // The column's k + 2 entries and normav (at m + 2) in one copy.
-    read(col.data(), 0, static_cast<int>(m + 3));
-    const double normav = col[m + 2];
-    for (int64_t j = 0; j <= k + 1; j++) h(j, k) = col[j];
-    const double normav2 = h(k + 1, k);
-    if (normav + 0.001 * normav2 == normav) {  // Brown/Hindmarsh, gmres_ir.hpp:683
-      st.reorth_count++;
-      double *h2 = hd + (m + 4);  // second bank is hd[m+4 .. 2m+8)
-      vec_.mgs_pass(w, nullptr, nullptr, V, 0, h2, s);
-      for (int64_t j = 0; j <= k; j++)
-        vec_.mgs_pass(w, V + j * n, h2 + j, j < k ? V + (j + 1) * n : nullptr, j < k ? 0 : 1,
-                      h2 + j + 1, s);
-      read(col.data(), static_cast<int>(m + 4), static_cast<int>(k + 2));
-      for (int64_t j = 0; j <= k; j++) h(j, k) += col[j];
-      h(k + 1, k) = col[k + 1];
-    }
-    if (h(k + 1, k) != 0) vec_.scale(w, 1 / h(k + 1, k), w, s);
-    for (int64_t j = 0; j < k; j++) {  // apply previous rotations
-      const double w1 = c[j] * h(j, k) - sn[j] * h(j + 1, k);
-      const double w2 = sn[j] * h(j, k) + c[j] * h(j + 1, k);
-      h(j, k)         = w1;
-      h(j + 1, k)     = w2;
-    }
-    // Dnrm2 of {h_kk, h_k+1,k}, walked last to first as ops.hpp:243 does.
-    double nu;
-    {
-      double scale = 0.0, ssq = 1.0;
-      const double pr[2] = {h(k, k), h(k + 1, k)};
-      for (int q = 1; q >= 0; q--)
-        if (pr[q] != 0.0) {
-          const double a = std::fabs(pr[q]);
-          if (scale < a) {
-            ssq   = 1.0 + ssq * ((scale / a) * (scale / a));
-            scale = a;
-          } else {
-            ssq = ssq + ((a / scale) * (a / scale));
-          }
-        }
-      nu = scale * std::sqrt(ssq);
-    }
-    if (nu != 0) {
-      c[k]            = h(k, k) / nu;
-      sn[k]           = -h(k + 1, k) / nu;
-      h(k, k)         = c[k] * h(k, k) - sn[k] * h(k + 1, k);
-      h(k + 1, k)     = 0.0;
-      const double w1 = c[k] * g[k] - sn[k] * g[k + 1];
-      const double w2 = sn[k] * g[k] + c[k] * g[k + 1];
-      g[k]            = w1;
-      g[k + 1]        = w2;
-    }
-    rho = std::fabs(g[k + 1]);
-  }
-  st.gmres_iterations += static_cast<int32_t>(k);
-  std::vector<double> y(std::max<int64_t>(k, 1), 0.0);
-  for (int64_t i = k; i-- > 0;) {
-    y[i] = g[i];
-    for (int64_t j = i + 1; j < k; j++) y[i] -= h(i, j) * y[j];
-    y[i] /= h(i, i);
-  }
-  if (k > 0) {
-    MPIR_CUDA(cudaMemcpyAsync(y_.as<double>(), y.data(), k * sizeof(double),
-                              cudaMemcpyHostToDevice, s));
-    vec_.combine(V, n, static_cast<int>(k), y_.as<double>(), res, s);
-    MPIR_CUDA(cudaStreamSynchronize(s));  // y lives on the host stack
+void Solver::count_inner(int nb, uint32_t act, const GmresMail &m, Report *st) {
+  for (int k = 0; k < nb; k++) {
+    if (!(act >> k & 1u) || !m.began[k]) continue;
+    st[k].precond_applies += 1 + m.k[k];
+    st[k].spmv_count += m.k[k];
+    st[k].gmres_iterations += m.k[k];
+    st[k].reorth_count += m.reorth[k];
   }
 }
 
@@ -369,27 +302,29 @@ int Solver::solve_device(const double *d_b, double *d_x, Report *rep) {
   const int64_t *Kp = P.Kp.as<int64_t>();
   const int32_t *Kj = P.Kj.as<int32_t>();
   const double  *Kv = num_.Kval.as<double>();
-  double *bs = bs_.as<double>(), *x = x_.as<double>(), *r = r_.as<double>(),
-         *t = t_.as<double>(), *d = d_.as<double>();
+  double *bs = bs_.as<double>(), *x = x_.as<double>(), *r = r_.as<double>();
   const bool dd = ur == kDD;
   if (n == 0) {
     if (rep) *rep = st;
     return kOk;
   }
-  vec_.rhs_in(P.perm.as<int64_t>(), num_.AD.as<double>(), d_b, bs, ADp_.as<double>(),
-              bp_.as<double>(), s);
-  double bs_inf;
-  vec_.read_inf(&bs_inf, 3, 1, s);
+  double    *inf = box_->inf;
+  VecFactors fac{}, one{};
+  one.v[0] = 1.0;
   const auto t_outer = std::chrono::steady_clock::now();
   auto       ms_since = [](std::chrono::steady_clock::time_point t0) {
     return std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0)
         .count();
   };
-  precond_gmres(bs, x, st);
-  vec_.residual(Kp, Kj, Kv, x, bs, r, dd, 0, s);
+  vec_.rhs_in(1, P.perm.as<int64_t>(), num_.AD.as<double>(), d_b, bs, ADp_.as<double>(),
+              bp_.as<double>(), s);
+  inner(1, 1, 1u, bs, one, V_.as<double>(), ar_, vec_, x, false, one);
+  vec_.residual(1, 1u, Kp, Kj, Kv, x, bs, r, dd, true, s);
+  vec_.read_inf(1, inf, s);
+  count_inner(1, 1u, ar_.mail(), &st);
   st.spmv_count++;
-  double r_inf;
-  vec_.read_inf(&r_inf, 0, 1, s);
+  const double bs_inf = inf[3];
+  double       r_inf  = inf[0];
   IrEvent ev;
   ev.initial_residual = r_inf;
   double r_prev = DBL_MAX, r_norm = r_inf / bs_inf;
@@ -405,16 +340,17 @@ int Solver::solve_device(const double *d_b, double *d_x, Report *rep) {
       st.stop_reason = 4;
       break;
     }
-    vec_.scale(r, 1.0 / scale, t, s);
     const auto t_inner = std::chrono::steady_clock::now();
-    precond_gmres(t, d, st);
-    vec_.ir_update(d, scale, x, s);
-    double nrm[2];
-    vec_.read_inf(nrm, 1, 2, s);
+    fac.v[0] = 1.0 / scale;
+    one.v[0] = scale;
+    inner(1, 1, 1u, r, fac, V_.as<double>(), ar_, vec_, x, true, one);
+    vec_.residual(1, 1u, Kp, Kj, Kv, x, bs, r, dd, false, s);
+    vec_.read_inf(1, inf, s);
+    count_inner(1, 1u, ar_.mail(), &st);
     const double inner_ms = ms_since(t_inner);
-    vec_.residual(Kp, Kj, Kv, x, bs, r, dd, 0, s);
+    const double nrm[2] = {inf[1], inf[2]};
     st.spmv_count++;
-    vec_.read_inf(&r_inf, 0, 1, s);
+    r_inf            = inf[0];
     r_norm           = r_inf / bs_inf;
     st.ir_iterations = static_cast<int32_t>(iter);
     ev.iterations.push_back({iter, r_norm, nrm[0], ms_since(t_outer), inner_ms});
@@ -433,24 +369,21 @@ int Solver::solve_device(const double *d_b, double *d_x, Report *rep) {
   ev.total_iterations = st.ir_iterations;
   ev.total_time_ms    = ms_since(t_outer);
   log_.push_back(std::move(ev));
-  vec_.sol_out(P.perm.as<int64_t>(), ADp_.as<double>(), x, d_x, s);
-  vec_.backward_terms(Kp, Kj, num_.Korig.as<double>(), x, ADp_.as<double>(),
-                      bp_.as<double>(), s);
-  double be[4];
-  vec_.read_inf(be, 4, 4, s);
-  const double den  = be[1] * be[2] + be[3];
-  st.backward_error = den > 0 ? be[0] / den : be[0];
+  vec_.sol_out(1, P.perm.as<int64_t>(), ADp_.as<double>(), x, d_x, s);
+  vec_.backward_terms(1, Kp, Kj, num_.Korig.as<double>(), x, ADp_.as<double>(), bp_.as<double>(), s);
   MPIR_CUDA(cudaEventRecord(ev1_, s));
-  MPIR_CUDA(cudaEventSynchronize(ev1_));
+  // The error word of a wait of the triangular solves that gave up (sticky).
+  MPIR_CUDA(cudaMemcpyAsync(&box_->err, ws_.err.as<void>(), sizeof box_->err, cudaMemcpyDeviceToHost, s));
+  vec_.read_inf(1, inf, s);
+  const double *be  = inf + 4;
+  const double  den = be[1] * be[2] + be[3];
+  st.backward_error = den > 0 ? be[0] / den : be[0];
   float ms = 0;
   MPIR_CUDA(cudaEventElapsedTime(&ms, ev0_, ev1_));
   st.solve_ms  = ms;
   st.factor_ms = last_factor_ms;
-  // A ready-flag wait of the triangular solves that gave up (sticky word).
-  int32_t wait_err = 0;
-  MPIR_CUDA(cudaMemcpy(&wait_err, ws_.err.as<void>(), sizeof wait_err, cudaMemcpyDeviceToHost));
-  if (wait_err != 0) {
-    device_zero(ws_.err.as<void>(), sizeof wait_err);
+  if (box_->err != 0) {
+    device_zero(ws_.err.as<void>(), sizeof(int32_t));
     st.status = -5;
     if (rep) *rep = st;
     return -5;
@@ -487,7 +420,7 @@ int Solver::luir_device(const double *d_b, double *d_x, int maxiter, Report *rep
   const double  *Kv = num_.Kval.as<double>();
   double *bs = bs_.as<double>(), *x = x_.as<double>(), *r = r_.as<double>(),
          *ADp = ADp_.as<double>();
-  vec_.rhs_in(P.perm.as<int64_t>(), num_.AD.as<double>(), d_b, bs, ADp, bp_.as<double>(), s);
+  vec_.rhs_in(1, P.perm.as<int64_t>(), num_.AD.as<double>(), d_b, bs, ADp, bp_.as<double>(), s);
   MPIR_CUDA(cudaMemcpyAsync(x, bs, n * sizeof(double), cudaMemcpyDeviceToDevice, s));
   vec_.round_to(uf, x, s);
   ldlt_solve(P, num_, x, ws_, s);
@@ -496,11 +429,11 @@ int Solver::luir_device(const double *d_b, double *d_x, int maxiter, Report *rep
   const double eps = eps_of(kF64);
   double       d0  = DBL_MAX;
   for (int it = 1; it <= maxiter; it++) {
-    vec_.residual(Kp, Kj, Kv, x, bs, r, false, 0, s);
+    vec_.residual(1, 1u, Kp, Kj, Kv, x, bs, r, false, true, s);
     st.spmv_count++;
     vec_.round_to(uf, r, s);
-    double rn;
-    vec_.read_inf(&rn, 0, 1, s);
+    vec_.read_inf(1, box_->inf, s);
+    const double rn = box_->inf[0];
     if (rn == 0.0) {
       st.stop_reason = 3;
       break;
@@ -515,8 +448,8 @@ int Solver::luir_device(const double *d_b, double *d_x, int maxiter, Report *rep
     st.precond_applies++;
     vec_.round_to(uf, r, s);
     vec_.ir_update(r, rn, x, s, ADp);
-    double nrm[2];
-    vec_.read_inf(nrm, 1, 2, s);
+    vec_.read_inf(1, box_->inf, s);
+    const double nrm[2] = {box_->inf[1], box_->inf[2]};
     st.ir_iterations = it;
     if (nrm[0] / nrm[1] <= 10 * eps) {
       st.stop_reason = 1;
@@ -528,10 +461,10 @@ int Solver::luir_device(const double *d_b, double *d_x, int maxiter, Report *rep
     }
     d0 = nrm[0];
   }
-  vec_.sol_out(P.perm.as<int64_t>(), ADp, x, d_x, s);
-  vec_.backward_terms(Kp, Kj, num_.Korig.as<double>(), x, ADp, bp_.as<double>(), s);
-  double be[4];
-  vec_.read_inf(be, 4, 4, s);
+  vec_.sol_out(1, P.perm.as<int64_t>(), ADp, x, d_x, s);
+  vec_.backward_terms(1, Kp, Kj, num_.Korig.as<double>(), x, ADp, bp_.as<double>(), s);
+  vec_.read_inf(1, box_->inf, s);
+  const double *be   = box_->inf + 4;
   const double den   = be[1] * be[2] + be[3];
   st.backward_error  = den > 0 ? be[0] / den : be[0];
   st.residual_norm   = be[3] > 0 ? be[0] / be[3] : be[0];  // |b - A x| / |b|
@@ -585,13 +518,13 @@ double Solver::residual(const double *b, const double *x, double *r, bool dd) {
   const double  *AD   = num_.AD.as<double>();
   MPIR_CUDA(cudaMemcpyAsync(hb_.as<void>(), b, n * sizeof(double), cudaMemcpyHostToDevice, s));
   MPIR_CUDA(cudaMemcpyAsync(hx_.as<void>(), x, n * sizeof(double), cudaMemcpyHostToDevice, s));
-  vec_.rhs_in(perm, AD, hx_.as<double>(), t_.as<double>(), nullptr, x_.as<double>(), s);
-  vec_.rhs_in(perm, AD, hb_.as<double>(), t_.as<double>(), nullptr, bp_.as<double>(), s);
-  vec_.residual(P.Kp.as<int64_t>(), P.Kj.as<int32_t>(), num_.Korig.as<double>(),
-                x_.as<double>(), bp_.as<double>(), r_.as<double>(), dd, 0, s);
-  double rinf = 0;
-  vec_.read_inf(&rinf, 0, 1, s);
-  vec_.sol_out(perm, nullptr, r_.as<double>(), hx_.as<double>(), s);
+  vec_.rhs_in(1, perm, AD, hx_.as<double>(), t_.as<double>(), nullptr, x_.as<double>(), s);
+  vec_.rhs_in(1, perm, AD, hb_.as<double>(), t_.as<double>(), nullptr, bp_.as<double>(), s);
+  vec_.residual(1, 1u, P.Kp.as<int64_t>(), P.Kj.as<int32_t>(), num_.Korig.as<double>(),
+                x_.as<double>(), bp_.as<double>(), r_.as<double>(), dd, true, s);
+  vec_.read_inf(1, box_->inf, s);
+  const double rinf = box_->inf[0];
+  vec_.sol_out(1, perm, nullptr, r_.as<double>(), hx_.as<double>(), s);
   MPIR_CUDA(cudaMemcpyAsync(r, hx_.as<void>(), n * sizeof(double), cudaMemcpyDeviceToHost, s));
   MPIR_CUDA(cudaStreamSynchronize(s));
   return rinf;

@@ -397,6 +397,7 @@ __global__ void __launch_bounds__(kFlowThreads, 1) k_fwd_flow(const __grid_const
   extern __shared__ __align__(128) double sm[];
   __shared__ __align__(16) FlowShared S;
   uint32_t phase = 0, wphase = 0;
+  if (flow_idle(a)) return;
   flow_loop(a, S, [&](const FlowSlot &I, FlowSlot &N) {
     switch (I.item.kind) {
       case kFlowWarps: fwd_warp(a, S, I, N, sm, wphase); break;
@@ -744,6 +745,7 @@ __global__ void __launch_bounds__(kFlowThreads, 1) k_bwd_flow(const __grid_const
   extern __shared__ __align__(128) double sm[];
   __shared__ __align__(16) FlowShared S;
   uint32_t phase = 0, wphase = 0;
+  if (flow_idle(a)) return;
   flow_loop(a, S, [&](const FlowSlot &I, FlowSlot &N) {
     switch (I.item.kind) {
       case kFlowWarps: bwd_warp(a, S, I, N, sm, wphase); break;
@@ -903,7 +905,7 @@ void SolveWorkspace::allocate(const Plan &P) {
 
 template <class T>
 static void ldlt_solve_t(const Plan &P, const Numeric &F, const T *pan, double *x,
-                         SolveWorkspace &ws, cudaStream_t s, int phases) {
+                         SolveWorkspace &ws, cudaStream_t s, int phases, const ActiveFlags &act) {
   const int64_t n = P.S.n;
   if (n == 0) return;
   KernelTimer      &kt = kernel_timer();
@@ -927,6 +929,9 @@ static void ldlt_solve_t(const Plan &P, const Numeric &F, const T *pan, double *
   a.xr    = a.part + P.flow_part_elems;
   a.xz    = a.xr + kFlowCopies * n;
   a.err   = ws.err.as<int32_t>();
+  a.active        = act.p;
+  a.nactive       = act.count;
+  a.active_stride = act.stride;
   static std::atomic<bool> attr{false};
   constexpr int            smem = kFlowSmem * sizeof(double);
   if (!attr) {
@@ -970,16 +975,16 @@ static void ldlt_solve_t(const Plan &P, const Numeric &F, const T *pan, double *
 }
 
 void ldlt_solve(const Plan &P, const Numeric &F, double *x, SolveWorkspace &ws,
-                cudaStream_t s, int phases) {
+                cudaStream_t s, int phases, const ActiveFlags &act) {
   switch (F.solve_prec()) {
     case 2:
-      ldlt_solve_t(P, F, F.panel16.as<__nv_bfloat16>(), x, ws, s, phases);
+      ldlt_solve_t(P, F, F.panel16.as<__nv_bfloat16>(), x, ws, s, phases, act);
       break;
     case 3:
-      ldlt_solve_t(P, F, F.panel16.as<__half>(), x, ws, s, phases);
+      ldlt_solve_t(P, F, F.panel16.as<__half>(), x, ws, s, phases, act);
       break;
     default:
-      ldlt_solve_t(P, F, F.panel.as<float>(), x, ws, s, phases);
+      ldlt_solve_t(P, F, F.panel.as<float>(), x, ws, s, phases, act);
   }
 }
 

@@ -21,13 +21,20 @@ struct SolveWorkspace {
   static size_t bytes_for(const Plan &P);
 };
 
+// Flags on the device, count of them stride apart: the full solve is left out
+// when all are zero (p NULL: never).
+struct ActiveFlags {
+  const int32_t *p     = nullptr;
+  int            count = 0, stride = 0;
+};
+
 // Phases of the solve, combinable as bits.
 enum SolvePhase : int { kForward = 1, kDiagonal = 2, kBackward = 4, kAllPhases = 7 };
 
 // x (permuted order, float64, device) <- (L D L^T)^{-1} x, or the phases
 // selected: (L+I)^{-1} x, Dinv .* x, (L+I)^{-T} x (qdldl.hpp:362-432).
 void ldlt_solve(const Plan &P, const Numeric &F, double *x, SolveWorkspace &ws,
-                cudaStream_t s, int phases = kAllPhases);
+                cudaStream_t s, int phases = kAllPhases, const ActiveFlags &act = ActiveFlags());
 
 // Workspace of the several-vector solves (solve_multi.cu) for one width, as
 // SolveWorkspace with nr values an entry.
@@ -46,7 +53,8 @@ int multi_width(int nrhs);
 // X (n x width, column-major, leading dimension n, permuted order, float64,
 // device) <- (L D L^T)^{-1} X, for all width columns at once (solve_multi.cu).
 void ldlt_solve_multi(const Plan &P, const Numeric &F, double *X, int width,
-                      MultiSolveWorkspace &ws, cudaStream_t s);
+                      MultiSolveWorkspace &ws, cudaStream_t s,
+                      const ActiveFlags &act = ActiveFlags());
 
 // QDLDL_solve (float32 factor, float64 x, host arrays) whose device data
 // lives in a fixed file-scope array instead of allocated memory; see

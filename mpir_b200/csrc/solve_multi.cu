@@ -633,6 +633,7 @@ __global__ void __launch_bounds__(kFlowThreads, 1) k_fwd_flow_m(const __grid_con
   extern __shared__ __align__(128) double sm[];
   __shared__ __align__(16) FlowShared S;
   uint32_t phase = 0, wphase = 0;
+  if (flow_idle(a)) return;
   flow_loop(a, S, [&](const FlowSlot &I, FlowSlot &N) {
     switch (I.item.kind) {
       case kFlowWarps: fwd_warp_m<NR>(a, S, I, N, sm, wphase); break;
@@ -995,6 +996,7 @@ __global__ void __launch_bounds__(kFlowThreads, 1) k_bwd_flow_m(const __grid_con
   extern __shared__ __align__(128) double sm[];
   __shared__ __align__(16) FlowShared S;
   uint32_t phase = 0, wphase = 0;
+  if (flow_idle(a)) return;
   flow_loop(a, S, [&](const FlowSlot &I, FlowSlot &N) {
     switch (I.item.kind) {
       case kFlowWarps: bwd_warp_m<NR>(a, S, I, N, sm, wphase); break;
@@ -1016,7 +1018,7 @@ struct MultiBuffers {
 
 template <int NR, class T>
 void solve_multi_nr(const Plan &P, const Numeric &F, const T *pan, double *X,
-                    MultiSolveWorkspace &ws, cudaStream_t s) {
+                    MultiSolveWorkspace &ws, cudaStream_t s, const ActiveFlags &act) {
   const int64_t      n = P.S.n;
   KernelTimer       &kt = kernel_timer();
   const MultiBuffers b(P);
@@ -1039,6 +1041,9 @@ void solve_multi_nr(const Plan &P, const Numeric &F, const T *pan, double *X,
   a.xr     = a.part + NR * P.flow_part_elems;
   a.xz     = a.xr + NR * kMultiCopies * n;
   a.err    = ws.err.as<int32_t>();
+  a.active        = act.p;
+  a.nactive       = act.count;
+  a.active_stride = act.stride;
   static std::atomic<bool> attr{false};  // idempotent; set once per process
   constexpr int            smem = kMultiSmem * sizeof(double);
   if (!attr) {
@@ -1094,16 +1099,16 @@ size_t MultiSolveWorkspace::bytes_for(const Plan &P, int width) {
 }
 
 void ldlt_solve_multi(const Plan &P, const Numeric &F, double *X, int width,
-                      MultiSolveWorkspace &ws, cudaStream_t s) {
+                      MultiSolveWorkspace &ws, cudaStream_t s, const ActiveFlags &act) {
   if (P.S.n == 0) return;
   if (ws.nr != width) throw std::logic_error("multi-vector workspace of another width");
   if (width != 4 && width != 8 && width != 16)
     throw std::invalid_argument("multi-vector solve width must be 4, 8 or 16");
   auto run = [&](auto *pan) {
     using T = std::remove_const_t<std::remove_pointer_t<decltype(pan)>>;
-    if (width == 4) solve_multi_nr<4, T>(P, F, pan, X, ws, s);
-    if (width == 8) solve_multi_nr<8, T>(P, F, pan, X, ws, s);
-    if (width == 16) solve_multi_nr<16, T>(P, F, pan, X, ws, s);
+    if (width == 4) solve_multi_nr<4, T>(P, F, pan, X, ws, s, act);
+    if (width == 8) solve_multi_nr<8, T>(P, F, pan, X, ws, s, act);
+    if (width == 16) solve_multi_nr<16, T>(P, F, pan, X, ws, s, act);
   };
   switch (F.solve_prec()) {
     case 2: run(F.panel16.as<const __nv_bfloat16>()); break;

@@ -6,6 +6,7 @@
 #include <vector>
 #include <stdexcept>
 
+#include "arnoldi.hpp"
 #include "engine.hpp"
 #include "solve.hpp"
 #include "vec.hpp"
@@ -95,7 +96,7 @@ class Solver {
   // device) <- (L D L^T)^{-1} X with the current factor: one vector by the
   // single-vector kernels, several by the several-vector kernels.
   void precond_device(int nrhs, double *d_X);
-  static constexpr int kMaxBatch = 16;
+  static constexpr int kMaxBatch = kMaxVectors;
   // The type the factor is computed and applied in (a double factor type is
   // served by the float32 factor).
   int applied_prec() const { return uf == kF64 ? kF32 : uf; }
@@ -136,44 +137,42 @@ class Solver {
   int64_t last_npos     = 0;
 
  private:
-  void precond_gmres(const double *b, double *res, Report &st);
   void ensure_vectors();
-  // Batched GMRES (gmres_batch.cu): vectors of the batch k*n apart inside
-  // blocks of width bw_ (n * bw_ doubles per block).
   void ensure_batch(int width);
-  void precond_gmres_batch(int nb, const double *b, double *res, std::vector<Report> &st,
-                           const std::vector<int32_t> &active);
-  void multi_apply(double *block);
+  // PrecondGmres (gmres_ir.hpp:636-741) for the vectors of act out of nb, n
+  // apart in blocks of width vectors (V: m + 1 blocks), b times fac on the
+  // right; its result is x, or (update) refines it (Arnoldi::end).  Queued up
+  // to the last step; the counts are added by count_inner once the stream has
+  // been waited for.
+  void inner(int nb, int width, uint32_t act, const double *b, const VecFactors &fac, double *V,
+             Arnoldi &ar, VecOps &vo, double *x, bool update, const VecFactors &scale);
+  static void count_inner(int nb, uint32_t act, const GmresMail &m, Report *st);
+  void apply(int nb, int width, double *x, const ActiveFlags &act);
 
   cudaStream_t          own_stream_ = nullptr, stream_ = nullptr;
   std::shared_ptr<Plan> plan_;
   Numeric               num_;
   SolveWorkspace        ws_;
   VecOps                vec_;
-  DeviceBuffer          V_, bs_, bp_, ADp_, x_, r_, t_, d_, hd_, y_, hb_, hx_;
+  Arnoldi               ar_;
+  DeviceBuffer          V_, bs_, bp_, ADp_, x_, r_, t_, hb_, hx_;
   int64_t               vec_m_ = -1;
-  // Batch state: width, basis and vectors, host staging of the per-vector
-  // scalars (pinned), the several-vector solve workspace.
+  // Batch state: width, basis and vectors, the several-vector solve workspace.
   int                   bw_ = 0;
   int64_t               bm_ = -1;
   VecOps                vecb_;
+  Arnoldi               bar_;
   MultiSolveWorkspace   mws_;
-  DeviceBuffer          bV_, bbs_, bbp_, bx_, br_, bt_, bd_, bhd_, by_, bfac_, bact_, bkq_, bin_,
-                        bout_, bpre_;
-  double               *hpin_ = nullptr;  // pinned host scalars (fac, y, act, kq)
-  size_t                hpin_bytes_ = 0;
-  static constexpr int  kStageSlots = 16;
-  int                   stage_next_ = 0;
-  // The next staging slot (2 * bw_ doubles) for an upload of per-vector
-  // scalars; slots are reused after kStageSlots uploads, and the batched
-  // solve synchronises its stream at least once in fewer uploads than that.
-  double *stage_slot() {
-    double *p   = hpin_ + static_cast<size_t>(stage_next_) * 2 * bw_;
-    stage_next_ = (stage_next_ + 1) % kStageSlots;
-    return p;
-  }
+  DeviceBuffer          bV_, bbs_, bbp_, bx_, br_, bin_, bout_;
+  // What a solve reads back (pinned): max-norm slots, the wait error word.
+  struct HostBox {
+    double  inf[8 * kMaxVectors];
+    int32_t err;
+  };
+  HostBox              *box_ = nullptr;
   int32_t               wait_ctl_[2] = {0, 0};  // SolveCtl words 1-2 (set_wait_controls)
   cudaEvent_t           ev0_ = nullptr, ev1_ = nullptr;
+  cudaEvent_t           step_ev_[2] = {nullptr, nullptr};  // inner steps, by parity
   std::vector<IrEvent>  log_;
 };
 

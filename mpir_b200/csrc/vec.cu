@@ -1,11 +1,8 @@
-// Vector kernels of the GMRES-IR loop: the symmetric SpMV and residual in
-// float64 or double-double (MatrixMultiply / VectorSubtract, ops.hpp:25-96),
-// norms (Dnrm2 / InfNrm, ops.hpp:231-329), dot products (ops.hpp:195-200),
-// the fused modified Gram-Schmidt passes of PrecondGmres
-// (gmres_ir.hpp:676-691) and the refinement update (gmres_ir.hpp:562-579).
-//
-// Sums and norms are two-stage reductions whose second stage adds the
-// per-block partials in block order, so results are reproducible.
+// Vector kernels around the GMRES steps (arnoldi.cu): the symmetric SpMV and
+// residual in float64 or double-double (MatrixMultiply / VectorSubtract,
+// ops.hpp:25-96), max-norms (InfNrm, ops.hpp:300-329), the gather and scatter
+// between the caller's order and the factor's, and the update of plain
+// refinement.
 #include <cfloat>
 #include <cmath>
 
@@ -16,8 +13,6 @@
 #include "vec.hpp"
 
 namespace mpir {
-
-constexpr int kRedThreads = 256;
 
 // ---------------------------------------------------------------------------
 // Double-double helpers (Knuth's TwoSum and the FMA form of Dekker's
@@ -75,16 +70,14 @@ __device__ __forceinline__ void warp_max_abs(unsigned long long *slot, double v,
 //
 // Batched form (all kernels below): blockIdx.y selects vector k of a batch,
 // the vectors k*vs apart, its max-norm slots at inf + 8k, and k is skipped
-// when act[k] == 0 (act NULL: every k).  One vector is gridDim.y == 1.
-__device__ __forceinline__ bool batch_skip(const int32_t *vact) {
-  return vact != nullptr && vact[blockIdx.y] == 0;
-}
+// unless bit k of vact is set.  One vector is gridDim.y == 1.
+__device__ __forceinline__ bool batch_skip(uint32_t vact) { return !(vact >> blockIdx.y & 1u); }
 
 template <int G, int MODE>
 __global__ void k_spmv(int64_t n, const int64_t *Kp, const int32_t *Kj,
                        const double *Kv, const double *x, const double *b,
                        double *y, unsigned long long *inf, int64_t vs,
-                       const int32_t *vact) {
+                       uint32_t vact) {
   if (batch_skip(vact)) return;
   x += blockIdx.y * vs;
   y += blockIdx.y * vs;
@@ -139,7 +132,7 @@ __global__ void k_backward_terms(int64_t n, const int64_t *Kp, const int32_t *Kj
                                  const double *Korig, const double *x,
                                  const double *ADp, const double *b,
                                  unsigned long long *inf, int64_t vs,
-                                 const int32_t *vact) {
+                                 uint32_t vact) {
   if (batch_skip(vact)) return;
   x += blockIdx.y * vs;
   b += blockIdx.y * vs;
@@ -167,179 +160,16 @@ __global__ void k_backward_terms(int64_t n, const int64_t *Kp, const int32_t *Kj
   warp_max_abs(inf + 3, lead ? b[row] : 0.0, lead);
 }
 
-// ---------------------------------------------------------------------------
-// Two-stage reductions.  Stage 1 writes one partial per block; the last block
-// to finish combines them in block order and resets the counter.
-__device__ __forceinline__ double block_sum(double v, double *sh) {
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
-  __syncthreads();
-  if (lane == 0) sh[warp] = v;
-  __syncthreads();
-  double t = 0.0;
-  if (threadIdx.x == 0)
-    for (int q = 0; q < (int)(blockDim.x / 32); q++) t += sh[q];
-  return t;
-}
-
-// LAPACK-style scaled sum of squares: the pair (scale, ssq) stands for
-// scale^2 * ssq.
-__device__ __forceinline__ void ssq_add(double &scale, double &ssq, double x) {
-  if (x != 0.0) {
-    const double a = fabs(x);
-    if (scale < a) {
-      ssq   = 1.0 + ssq * ((scale / a) * (scale / a));
-      scale = a;
-    } else {
-      ssq += (a / scale) * (a / scale);
-    }
-  }
-}
-__device__ __forceinline__ void ssq_merge(double &s1, double &q1, double s2, double q2) {
-  if (s2 == 0.0) return;
-  if (s1 == 0.0) {
-    s1 = s2;
-    q1 = q2;
-    return;
-  }
-  if (s1 >= s2) {
-    q1 += q2 * ((s2 / s1) * (s2 / s1));
-  } else {
-    q1 = q2 + q1 * ((s1 / s2) * (s1 / s2));
-    s1 = s2;
-  }
-}
-__device__ __forceinline__ void block_ssq(double &s, double &q, double *sh) {
-  for (int o = 16; o > 0; o >>= 1) {
-    const double s2 = __shfl_xor_sync(0xffffffffu, s, o);
-    const double q2 = __shfl_xor_sync(0xffffffffu, q, o);
-    ssq_merge(s, q, s2, q2);
-  }
-  const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
-  __syncthreads();
-  if (lane == 0) {
-    sh[2 * warp]     = s;
-    sh[2 * warp + 1] = q;
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    s = 0.0;
-    q = 1.0;
-    for (int w = 0; w < (int)(blockDim.x / 32); w++) ssq_merge(s, q, sh[2 * w], sh[2 * w + 1]);
-  }
-}
-
-// Finalisation helper: returns true in thread 0 of the last block.
-__device__ __forceinline__ bool last_block(unsigned int *count) {
-  __shared__ bool is_last;
-  __threadfence();
-  if (threadIdx.x == 0) is_last = atomicInc(count, gridDim.x) == gridDim.x - 1;
-  __syncthreads();
-  return is_last;
-}
-
-// MGS pass: w -= h * v (h read from *hsrc, skipped when hsrc is null), then
-// either dot(w, u) (mode 0) or ||w||_2 (mode 1) into *out.
-// Batched: vectors k*vs apart, h and out k*hs apart, scratch part + 2048 k
-// and count + k.
-__global__ void __launch_bounds__(kRedThreads)
-    k_mgs_pass(int64_t n, double *w, const double *v, const double *hsrc,
-               const double *u, int mode, double *part, unsigned int *count,
-               double *out, int64_t vs, int64_t hs, const int32_t *vact) {
-  __shared__ double sh[2 * kRedThreads / 32];
-  if (batch_skip(vact)) return;
-  {
-    const int64_t k = blockIdx.y;
-    w += k * vs;
-    if (v) v += k * vs;
-    if (u) u += k * vs;
-    if (hsrc) hsrc += k * hs;
-    out += k * hs;
-    part += 2048 * k;
-    count += k;
-  }
-  const double      h = hsrc ? *hsrc : 0.0;
-  double            acc = 0.0, sc = 0.0, sq = 1.0;
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
-       i += (int64_t)gridDim.x * blockDim.x) {
-    double wi = w[i];
-    if (hsrc) {
-      wi   = wi - v[i] * h;
-      w[i] = wi;
-    }
-    if (mode == 0)
-      acc += wi * u[i];
-    else
-      ssq_add(sc, sq, wi);
-  }
-  if (mode == 0) {
-    const double t = block_sum(acc, sh);
-    if (threadIdx.x == 0) part[blockIdx.x] = t;
-  } else {
-    block_ssq(sc, sq, sh);
-    if (threadIdx.x == 0) {
-      part[2 * blockIdx.x]     = sc;
-      part[2 * blockIdx.x + 1] = sq;
-    }
-  }
-  if (!last_block(count)) return;
-  // The last block adds the blocks' partials: thread j takes partials j,
-  // j + blockDim.x, ... in that order, then the fixed tree of the block
-  // reductions (the loads are independent, so none waits for another).
-  if (mode == 0) {
-    double t = 0.0;
-    for (unsigned b = threadIdx.x; b < gridDim.x; b += blockDim.x) t += __ldcg(part + b);
-    t = block_sum(t, sh);
-    if (threadIdx.x == 0) *out = t;
-  } else {
-    double s = 0.0, q = 1.0;
-    for (unsigned b = threadIdx.x; b < gridDim.x; b += blockDim.x)
-      ssq_merge(s, q, __ldcg(part + 2 * b), __ldcg(part + 2 * b + 1));
-    block_ssq(s, q, sh);
-    if (threadIdx.x == 0) *out = s * sqrt(q);
-  }
-  if (threadIdx.x == 0) *count = 0;
-}
-
-// y = a * x (a the host argument, or fac[k] for vector k when fac is given).
-__global__ void k_scale(int64_t n, const double *x, double a, double *y, int64_t vs,
-                        const double *fac, const int32_t *vact) {
-  if (batch_skip(vact)) return;
-  x += blockIdx.y * vs;
-  y += blockIdx.y * vs;
-  if (fac) a = fac[blockIdx.y];
+// y = a * x.
+__global__ void k_scale(int64_t n, const double *x, double a, double *y) {
   const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (i < n) y[i] = x[i] * a;
-}
-
-// res = sum_j V_j y_j for j < k (gmres_ir.hpp:735-739).
-// Batched: vector q's basis at V + q*vs (ldv apart), its coefficients at
-// y + q*ys and its count kq[q] (kq NULL: k for all).
-__global__ void k_combine(int64_t n, const double *V, int64_t ldv, int k,
-                          const double *y, double *res, int64_t vs, int64_t ys,
-                          const int32_t *kq, const int32_t *vact) {
-  if (batch_skip(vact)) return;
-  V += blockIdx.y * vs;
-  res += blockIdx.y * vs;
-  y += blockIdx.y * ys;
-  if (kq) k = kq[blockIdx.y];
-  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  double r = 0.0;
-  for (int j = 0; j < k; j++) r += V[j * ldv + i] * y[j];
-  res[i] = r;
 }
 
 // d *= scale; inf[0] = max|d|; inf[1] = max|x_old|; x += d
 // (gmres_ir.hpp:574-577).
 __global__ void k_ir_update(int64_t n, double *d, double scale, double *x,
-                            const double *w, unsigned long long *inf, int64_t vs,
-                            const double *fac, const int32_t *vact) {
-  if (batch_skip(vact)) return;
-  d += blockIdx.y * vs;
-  x += blockIdx.y * vs;
-  inf += 8 * blockIdx.y;
-  if (fac) scale = fac[blockIdx.y];
+                            const double *w, unsigned long long *inf) {
   const int64_t i   = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   const bool    act = i < n;
   double        di = 0.0, xi = 0.0, wi = 1.0;
@@ -407,154 +237,59 @@ static unsigned blocks_for(int64_t n, int t) {
   return static_cast<unsigned>(std::max<int64_t>(1, (n + t - 1) / t));
 }
 
-void VecOps::allocate(int64_t n_, int sms, int batch_) {
-  n       = n_;
-  batch   = std::max(batch_, 1);
-  nblocks = std::max(1, std::min<int>(2 * sms, static_cast<int>((n + kRedThreads - 1) / kRedThreads)));
-  part.resize(sizeof(double) * 2048 * batch);
-  count.resize(sizeof(unsigned int) * batch);
+void VecOps::allocate(int64_t n_, int batch_) {
+  n     = n_;
+  batch = std::max(batch_, 1);
   infbits.resize(sizeof(unsigned long long) * 8 * batch);
-  device_zero(count.as<void>(), sizeof(unsigned int) * batch);
 }
 
 // Zeroes slots [first, first + cnt) of banks 0 .. nb-1.
 static void clear_slots(unsigned long long *bits, int nb, int first, int cnt, cudaStream_t s) {
-  MPIR_CUDA(cudaMemset2DAsync(bits + first, 8 * sizeof(unsigned long long), 0,
-                              cnt * sizeof(unsigned long long), nb, s));
+  if (nb == 1)
+    MPIR_CUDA(cudaMemsetAsync(bits + first, 0, cnt * sizeof(unsigned long long), s));
+  else
+    MPIR_CUDA(cudaMemset2DAsync(bits + first, 8 * sizeof(unsigned long long), 0,
+                                cnt * sizeof(unsigned long long), nb, s));
 }
 
 static dim3 grid_b(int64_t work, int threads, int nb) {
   return dim3(blocks_for(work, threads), static_cast<unsigned>(nb), 1);
 }
 
-void VecOps::spmv_b(int nb, const int64_t *Kp, const int32_t *Kj, const double *Kv,
-                    const double *x, double *y, int64_t vs, const int32_t *act,
-                    cudaStream_t s) {
+constexpr uint32_t kAll = 0xffffffffu;
+
+void VecOps::spmv(int nb, const int64_t *Kp, const int32_t *Kj, const double *Kv, const double *x,
+                  double *y, cudaStream_t s) {
   constexpr int G = 8;
-  launch(k_spmv<G, 0>, grid_b(n * G, 256, nb), 256, 0, s, n, Kp, Kj, Kv, x, nullptr, y,
-         nullptr, vs, act);
+  launch(k_spmv<G, 0>, grid_b(n * G, 256, nb), 256, 0, s, n, Kp, Kj, Kv, x, nullptr, y, nullptr, n, kAll);
 }
 
-void VecOps::residual_b(int nb, const int64_t *Kp, const int32_t *Kj, const double *Kv,
-                        const double *x, const double *b, double *r, bool dd, int64_t vs,
-                        const int32_t *act, cudaStream_t s) {
-  constexpr int G = 8;
+void VecOps::residual(int nb, uint32_t act, const int64_t *Kp, const int32_t *Kj, const double *Kv,
+                      const double *x, const double *b, double *r, bool dd, bool clear, cudaStream_t s) {
+  constexpr int       G   = 8;
   unsigned long long *inf = infbits.as<unsigned long long>();
-  clear_slots(inf, nb, 0, 1, s);
-  if (dd)
-    launch(k_spmv<G, 2>, grid_b(n * G, 256, nb), 256, 0, s, n, Kp, Kj, Kv, x, b, r, inf, vs,
-           act);
-  else
-    launch(k_spmv<G, 1>, grid_b(n * G, 256, nb), 256, 0, s, n, Kp, Kj, Kv, x, b, r, inf, vs,
-           act);
+  if (clear) clear_slots(inf, nb, 0, 1, s);
+  launch(dd ? k_spmv<G, 2> : k_spmv<G, 1>, grid_b(n * G, 256, nb), 256, 0, s, n, Kp, Kj, Kv, x, b, r, inf, n,
+         act);
 }
 
-void VecOps::backward_terms_b(int nb, const int64_t *Kp, const int32_t *Kj, const double *Korig,
-                              const double *x, const double *ADp, const double *bp, int64_t vs,
-                              cudaStream_t s) {
-  constexpr int G = 8;
+void VecOps::backward_terms(int nb, const int64_t *Kp, const int32_t *Kj, const double *Korig,
+                            const double *x, const double *ADp, const double *bp, cudaStream_t s) {
+  constexpr int       G   = 8;
   unsigned long long *inf = infbits.as<unsigned long long>();
   clear_slots(inf, nb, 4, 4, s);
-  launch(k_backward_terms<G>, grid_b(n * G, 256, nb), 256, 0, s, n, Kp, Kj, Korig, x, ADp, bp,
-         inf + 4, vs, static_cast<const int32_t *>(nullptr));
-}
-
-void VecOps::mgs_pass_b(int nb, double *w, const double *v, const double *hsrc, const double *u,
-                        int mode, double *out, int64_t vs, int64_t hs, const int32_t *act,
-                        cudaStream_t s) {
-  launch(k_mgs_pass, dim3(nblocks, nb, 1), kRedThreads, 0, s, n, w, v, hsrc, u, mode,
-         part.as<double>(), count.as<unsigned int>(), out, vs, hs, act);
-}
-
-void VecOps::scale_b(int nb, const double *x, const double *fac, double *y, int64_t vs,
-                     const int32_t *act, cudaStream_t s) {
-  launch(k_scale, grid_b(n, 256, nb), 256, 0, s, n, x, 0.0, y, vs, fac, act);
-}
-
-void VecOps::combine_b(int nb, const double *V, int64_t ldv, const double *y, int64_t ys,
-                       const int32_t *kq, double *res, int64_t vs, const int32_t *act,
-                       cudaStream_t s) {
-  launch(k_combine, grid_b(n, 256, nb), 256, 0, s, n, V, ldv, 0, y, res, vs, ys, kq, act);
-}
-
-void VecOps::ir_update_b(int nb, double *d, const double *fac, double *x, int64_t vs,
-                         const int32_t *act, cudaStream_t s, const double *w) {
-  unsigned long long *inf = infbits.as<unsigned long long>();
-  clear_slots(inf, nb, 1, 2, s);
-  launch(k_ir_update, grid_b(n, 256, nb), 256, 0, s, n, d, 0.0, x, w, inf + 1, vs, fac, act);
-}
-
-void VecOps::rhs_in_b(int nb, const int64_t *perm, const double *AD, const double *b, double *bs,
-                      double *ADp, double *bp, int64_t vs, cudaStream_t s) {
-  unsigned long long *inf = infbits.as<unsigned long long>();
-  clear_slots(inf, nb, 3, 1, s);
-  launch(k_rhs_in, grid_b(n, 256, nb), 256, 0, s, n, perm, AD, b, bs, ADp, bp, inf + 3, vs);
-}
-
-void VecOps::sol_out_b(int nb, const int64_t *perm, const double *ADp, const double *x,
-                       double *out, int64_t vs, cudaStream_t s) {
-  launch(k_sol_out, grid_b(n, 256, nb), 256, 0, s, n, perm, ADp, x, out, vs);
-}
-
-void VecOps::read_inf_b(int nb, double *h, cudaStream_t s) {
-  static_assert(sizeof(double) == sizeof(unsigned long long), "bit copy");
-  MPIR_CUDA(cudaMemcpyAsync(h, infbits.as<void>(), nb * 8 * sizeof(double), cudaMemcpyDeviceToHost,
-                            s));
-  MPIR_CUDA(cudaStreamSynchronize(s));
-}
-
-void VecOps::spmv(const int64_t *Kp, const int32_t *Kj, const double *Kv,
-                  const double *x, double *y, cudaStream_t s) {
-  constexpr int G = 8;
-  launch(k_spmv<G, 0>, blocks_for(n * G, 256), 256, 0, s, n, Kp, Kj, Kv, x, nullptr, y, nullptr,
-         int64_t{0}, nullptr);
-}
-
-void VecOps::residual(const int64_t *Kp, const int32_t *Kj, const double *Kv,
-                      const double *x, const double *b, double *r, bool dd,
-                      int slot, cudaStream_t s) {
-  constexpr int G = 8;
-  unsigned long long *inf = infbits.as<unsigned long long>() + slot;
-  MPIR_CUDA(cudaMemsetAsync(inf, 0, sizeof(unsigned long long), s));
-  if (dd)
-    launch(k_spmv<G, 2>, blocks_for(n * G, 256), 256, 0, s, n, Kp, Kj, Kv, x, b, r, inf,
-           int64_t{0}, nullptr);
-  else
-    launch(k_spmv<G, 1>, blocks_for(n * G, 256), 256, 0, s, n, Kp, Kj, Kv, x, b, r, inf,
-           int64_t{0}, nullptr);
-}
-
-void VecOps::backward_terms(const int64_t *Kp, const int32_t *Kj, const double *Korig,
-                            const double *x, const double *ADp, const double *bp,
-                            cudaStream_t s) {
-  constexpr int G = 8;
-  unsigned long long *inf = infbits.as<unsigned long long>() + 4;
-  MPIR_CUDA(cudaMemsetAsync(inf, 0, 4 * sizeof(unsigned long long), s));
-  launch(k_backward_terms<G>, blocks_for(n * G, 256), 256, 0, s, n, Kp, Kj, Korig, x, ADp, bp, inf,
-         int64_t{0}, nullptr);
-}
-
-void VecOps::mgs_pass(double *w, const double *v, const double *hsrc, const double *u,
-                      int mode, double *out, cudaStream_t s) {
-  launch(k_mgs_pass, nblocks, kRedThreads, 0, s, n, w, v, hsrc, u, mode, part.as<double>(),
-         count.as<unsigned int>(), out, int64_t{0}, int64_t{0}, nullptr);
+  launch(k_backward_terms<G>, grid_b(n * G, 256, nb), 256, 0, s, n, Kp, Kj, Korig, x, ADp, bp, inf + 4, n,
+         kAll);
 }
 
 void VecOps::scale(const double *x, double a, double *y, cudaStream_t s) {
-  launch(k_scale, blocks_for(n, 256), 256, 0, s, n, x, a, y, int64_t{0}, nullptr, nullptr);
-}
-
-void VecOps::combine(const double *V, int64_t ldv, int k, const double *y, double *res,
-                     cudaStream_t s) {
-  launch(k_combine, blocks_for(n, 256), 256, 0, s, n, V, ldv, k, y, res, int64_t{0}, int64_t{0},
-         nullptr, nullptr);
+  launch(k_scale, blocks_for(n, 256), 256, 0, s, n, x, a, y);
 }
 
 void VecOps::ir_update(double *d, double scale, double *x, cudaStream_t s, const double *w) {
   unsigned long long *inf = infbits.as<unsigned long long>() + 1;
   MPIR_CUDA(cudaMemsetAsync(inf, 0, 2 * sizeof(unsigned long long), s));
-  launch(k_ir_update, blocks_for(n, 256), 256, 0, s, n, d, scale, x, w, inf, int64_t{0}, nullptr,
-         nullptr);
+  launch(k_ir_update, blocks_for(n, 256), 256, 0, s, n, d, scale, x, w, inf);
 }
 
 void VecOps::round_to(int prec, double *x, cudaStream_t s) {
@@ -562,28 +297,22 @@ void VecOps::round_to(int prec, double *x, cudaStream_t s) {
   launch(k_round_to, blocks_for(n, 256), 256, 0, s, n, prec, x);
 }
 
-void VecOps::rhs_in(const int64_t *perm, const double *AD, const double *b, double *bs,
+void VecOps::rhs_in(int nb, const int64_t *perm, const double *AD, const double *b, double *bs,
                     double *ADp, double *bp, cudaStream_t s) {
-  unsigned long long *inf = infbits.as<unsigned long long>() + 3;
-  MPIR_CUDA(cudaMemsetAsync(inf, 0, sizeof(unsigned long long), s));
-  launch(k_rhs_in, blocks_for(n, 256), 256, 0, s, n, perm, AD, b, bs, ADp, bp, inf, int64_t{0});
+  unsigned long long *inf = infbits.as<unsigned long long>();
+  clear_slots(inf, nb, 3, 1, s);
+  launch(k_rhs_in, grid_b(n, 256, nb), 256, 0, s, n, perm, AD, b, bs, ADp, bp, inf + 3, n);
 }
 
-void VecOps::sol_out(const int64_t *perm, const double *ADp, const double *x, double *out,
+void VecOps::sol_out(int nb, const int64_t *perm, const double *ADp, const double *x, double *out,
                      cudaStream_t s) {
-  launch(k_sol_out, blocks_for(n, 256), 256, 0, s, n, perm, ADp, x, out, int64_t{0});
+  launch(k_sol_out, grid_b(n, 256, nb), 256, 0, s, n, perm, ADp, x, out, n);
 }
 
-void VecOps::read_inf(double *h, int first, int cnt, cudaStream_t s) {
-  unsigned long long bits[8];
-  MPIR_CUDA(cudaMemcpyAsync(bits, infbits.as<unsigned long long>() + first,
-                            cnt * sizeof(unsigned long long), cudaMemcpyDeviceToHost, s));
+void VecOps::read_inf(int nb, double *h, cudaStream_t s) {
+  static_assert(sizeof(double) == sizeof(unsigned long long), "bit copy");
+  MPIR_CUDA(cudaMemcpyAsync(h, infbits.as<void>(), nb * 8 * sizeof(double), cudaMemcpyDeviceToHost, s));
   MPIR_CUDA(cudaStreamSynchronize(s));
-  for (int i = 0; i < cnt; i++) {
-    double v;
-    std::memcpy(&v, &bits[i], sizeof v);
-    h[i] = v;
-  }
 }
 
 }  // namespace mpir
