@@ -211,58 +211,134 @@ __global__ void __launch_bounds__(256)
 // the inverse X = L^{-1} of its unit-lower factor, right-looking by panels of
 // 32 columns in shared memory (row-major copies of the block and of X; the
 // block is padded with a unit diagonal up to a multiple of 32).  Panel p:
-//   A. warp 0 factors the 32 x 32 diagonal block: lane = row, the pivot
-//      column is broadcast by shuffles, F[i][j] -= (F[i][k] / d_k) F[j][k]
-//      (the reciprocal on this chain is the fast approximate one; D^{-1}
-//      itself is the correctly rounded 1 / d_k), then inverts its unit-lower
-//      factor by forward substitution (lane = column).  Meanwhile warps on
-//      the other three schedulers form T_pb = sum_{b <= c < p} L_pc X_cb for
-//      the blocks b < p of X's row block p;
-//   B. the rows below take their unscaled panel entries G = F X_pp^T
-//      (G = L D) and L = G D^{-1}, both kept transposed, while the warps
-//      without rows below finish X_pb = -X_pp T_pb;
-//   C. L goes into the block, and the columns right of the panel take the
-//      rank-32 update F[i][j] -= sum_k L[i][k] G[j][k] in 4 x 4 tiles.
-// One block-wide barrier per phase; nothing of X is left for after the loop.
-constexpr int kDiagLD = kNB + 1;  // Fs, Xs row stride (conflict-free columns)
-constexpr int kDiagLG = 36;       // Xd row stride (16-byte rows)
-constexpr int kDiagLT = 33;       // Ts row stride
-constexpr int kDiagSmemFloats =
-    2 * kNB * kDiagLD + 2 * 32 * kNB + 32 * kDiagLG + 3 * 32 * kDiagLT;
+//   A. warp 0 factors the 32 x 32 diagonal block (lane = row).  Its chain is
+//      one broadcast, one reciprocal (the fast approximate one; D^{-1} itself
+//      is the correctly rounded 1 / d_k), one product and one update a pivot;
+//      the rest of a pivot's update takes the column from shared memory one
+//      pivot later.  Every 8 pivots it signals a named barrier, and other
+//      warps take those pivots up while it goes on: up to two for the rows
+//      below (unscaled panel entries G = L D, kept transposed, then
+//      L = G D^{-1}) and one for X_pp (lane = column).  The other twelve warps do
+//      what the chain does not wait for, in 32 x 32 block products: the previous panel's update of the columns beyond this
+//      panel, X_{p-1,b} = -X_{p-1,p-1} T_{p-1,b}, the contributions
+//      T_ib += L_{i,p-1} X_{p-1,b} to the rows of X still to come (kept where
+//      X_ib will be), and the stores of what is final (in panel 0 they read
+//      the later panels' columns);
+//   B. the next panel's columns take this panel's update.
+// What bounds it: the chain of 128 pivots, and beside it the 128 bytes a cycle
+// that shared memory returns to registers (a broadcast value costs a warp as
+// much as 32 different ones), hence two rows a lane below the diagonal block
+// and 4 x 4 values a lane in the products.  One block of 128 columns: 35.0 us
+// with X_pp and G formed after the diagonal block, products of 4 x 2 and
+// everything written at the end; 28.4 us so (64 columns 17.5 -> 15.5, 32
+// columns 10 us both).  Two pivots a turn: no gain.
+constexpr int kDiagLD = kNB + 4;  // Fs, Xs row stride (16-byte rows, lane = row conflict-free)
+constexpr int kDiagSmemFloats = 2 * kNB * kDiagLD + 2 * 32 * kNB + 32 * 32;
 
-// Phase A of panel p for warp 0: the diagonal block at (c0, c0).  Kept out
-// of line: inlined into the kernel, whose other phases hold many registers,
-// its chain of shuffles is scheduled about 1.5x slower.
-__device__ __noinline__ void diag_panel(float *Fs, float *Xs, float *Xd, float *dinv_s,
-                                           int c0, int n, const StepDesc &d, float *D,
-                                           float *Dinv, float *packd, float *packs,
-                                           FactorStatus *st, int &npos) {
-  constexpr int LD = kDiagLD, LG = kDiagLG;
-  const int     lane = threadIdx.x % 32, r = c0 + lane;
-  float         a[32];
+__device__ __forceinline__ void bar_arrive(int id, int threads) {
+  __threadfence_block();
+  asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(threads) : "memory");
+}
+__device__ __forceinline__ void bar_wait(int id, int threads) {
+  asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
+}
+
+// Row r of 32 values starting at a 16-byte boundary.
+__device__ __forceinline__ void load_row32(float (&a)[32], const float *p) {
 #pragma unroll
-  for (int j = 0; j < 32; j++) a[j] = Fs[r * LD + c0 + j];
-  float piv = 1.0f;
+  for (int q = 0; q < 8; q++) {
+    const float4 v = reinterpret_cast<const float4 *>(p)[q];
+    a[4 * q]     = v.x;
+    a[4 * q + 1] = v.y;
+    a[4 * q + 2] = v.z;
+    a[4 * q + 3] = v.w;
+  }
+}
+__device__ __forceinline__ void store_quad(float *p, float x, float y, float z, float w) {
+  *reinterpret_cast<float4 *>(p) = make_float4(x, y, z, w);
+}
+// a[j] -= l col[j] for j > K of 32 (col: a broadcast row of shared memory).
+template <int K>
+__device__ __forceinline__ void update_row32(float (&a)[32], float l, const float *col) {
+#pragma unroll
+  for (int q = (K + 1) / 4; q < 8; q++) {
+    const float4 v = reinterpret_cast<const float4 *>(col)[q];
+    const float  f[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+    for (int u = 0; u < 4; u++)
+      if (4 * q + u > K) a[4 * q + u] -= l * f[u];
+  }
+}
+// f(integral constant k) for k = K0 .. K0 + 7.
+template <int K>
+struct Int {
+  static constexpr int v = K;
+};
+template <int K0, class F>
+__device__ __forceinline__ void each8(F f) {
+  f(Int<K0>{});
+  f(Int<K0 + 1>{});
+  f(Int<K0 + 2>{});
+  f(Int<K0 + 3>{});
+  f(Int<K0 + 4>{});
+  f(Int<K0 + 5>{});
+  f(Int<K0 + 6>{});
+  f(Int<K0 + 7>{});
+}
+
+// Phase A of panel p for warp 0: the diagonal block at (c0, c0).  Column k goes
+// to Gt (unscaled, at row c0 + lane) and Ld (scaled), its approximate reciprocal
+// pivot to dv_s.  The broadcasts that the next pivot waits for are issued
+// before the loads of this one's column.  nsync: threads of the chunk barriers.
+// Kept out of line: inlined into the kernel, whose other phases hold many
+// registers, its chain of shuffles is scheduled about 1.5x slower.
+__device__ __noinline__ void diag_panel(float *Fs, float *Gt, float *Ld, float *dv_s, int c0, int nsync,
+                                        int n, const StepDesc &d, float *D, float *Dinv, float *packd,
+                                        float *packs, FactorStatus *st, int &npos) {
+  constexpr unsigned full = 0xffffffffu;
+  const int          lane = threadIdx.x % 32, r = c0 + lane;
+  float             *g = Gt + c0;
+  float              a[32], fp[32], lp = 0.0f, piv = 1.0f;
+  load_row32(a, Fs + r * kDiagLD + c0);
+  float dk = __shfl_sync(full, a[0], 0), f1 = __shfl_sync(full, a[0], 1);
+  g[lane] = a[0];
 #pragma unroll
   for (int k = 0; k < 32; k++) {
-    const float dk = __shfl_sync(0xffffffffu, a[k], k);
     const float dv = __fdividef(1.0f, dk);
-    const float l  = a[k] * dv;  // L[r][k]
+    if (k > 0) {  // the previous pivot's update of the columns beyond k
 #pragma unroll
-    for (int j = 0; j < 32; j++) {
-      if (j > k) {
-        const float fjk = __shfl_sync(0xffffffffu, a[k], j);  // F[c0 + j][k]
-        if (j <= lane) a[j] -= l * fjk;
-      }
+      for (int j = 0; j < 32; j++)
+        if (j > k) a[j] -= lp * fp[j];
     }
-    if (lane > k) a[k] = l;
     if (lane == k) piv = dk;
-  }
-  const float pinv = 1.0f / piv;
+    const float l = a[k] * dv;  // L[r][k]
+    if (k < 31) {
+      a[k + 1] -= l * f1;
+      dk = __shfl_sync(full, a[k + 1], k + 1);
+      if (k < 30) f1 = __shfl_sync(full, a[k + 1], k + 2);
+      g[(k + 1) * kNB + lane] = a[k + 1];
+    }
+    Ld[32 * k + lane] = l;
+    if (lane == 0) dv_s[c0 + k] = dv;
+    __syncwarp();
 #pragma unroll
-  for (int j = 0; j < 32; j++) Fs[r * LD + c0 + j] = a[j];
-  dinv_s[r] = pinv;
+    for (int q = 0; q < 8; q++)
+      if (4 * q + 3 > k + 1) {
+        const float4 v = *reinterpret_cast<const float4 *>(g + k * kNB + 4 * q);
+        fp[4 * q]     = v.x;
+        fp[4 * q + 1] = v.y;
+        fp[4 * q + 2] = v.z;
+        fp[4 * q + 3] = v.w;
+      }
+    lp = l;
+    if (lane > k) a[k] = l;
+    if (k % 8 == 7) bar_arrive(1 + k / 8, nsync);
+  }
+#pragma unroll
+  for (int q = 0; q < 8; q++)
+    store_quad(Fs + r * kDiagLD + c0 + 4 * q, a[4 * q], a[4 * q + 1], a[4 * q + 2], a[4 * q + 3]);
   if (r < n) {
+    const float   pinv = 1.0f / piv;
     const int64_t cidx = (int64_t)d.col0 + d.kb + r;
     D[cidx]            = piv;
     Dinv[cidx]         = pinv;
@@ -272,20 +348,159 @@ __device__ __noinline__ void diag_panel(float *Fs, float *Xs, float *Xd, float *
     }
     note_pivot(st, static_cast<int32_t>(cidx), piv, &npos);
   }
-  __syncwarp();
-  // X of the diagonal block (lane = column)
-  float x[32];
+}
+
+// Phase A for R x 32 rows below the diagonal block (lane = rows r, r + 32, ..).
+template <int R>
+__device__ __noinline__ void diag_rows(float *Fs, float *Gt, const float *dv_s, int c0, int nsync, int r) {
+  const float *g   = Gt + c0;
+  const int    l8  = threadIdx.x % 8;
+  float       *row = Fs + r * kDiagLD + c0;
+  float        a[R][32];
 #pragma unroll
-  for (int ii = 0; ii < 32; ii++) {
-    float acc = 0.0f;
+  for (int v = 0; v < R; v++) load_row32(a[v], row + 32 * v * kDiagLD);
+  auto step = [&](auto kk) {
+    constexpr int k  = decltype(kk)::v;
+    const float   dv = dv_s[c0 + k];
+    float         l[R];
 #pragma unroll
-    for (int kk = 0; kk < ii; kk++) acc += Fs[(c0 + ii) * LD + c0 + kk] * x[kk];
-    x[ii] = ii == lane ? 1.0f : (ii > lane ? -acc : 0.0f);
+    for (int v = 0; v < R; v++) {
+      Gt[k * kNB + r + 32 * v] = a[v][k];
+      l[v]                     = a[v][k] * dv;
+    }
+#pragma unroll
+    for (int q = (k + 1) / 4; q < 8; q++) {
+      const float4 w    = reinterpret_cast<const float4 *>(g + k * kNB)[q];
+      const float  f[4] = {w.x, w.y, w.z, w.w};
+#pragma unroll
+      for (int u = 0; u < 4; u++)
+        if (4 * q + u > k) {
+#pragma unroll
+          for (int v = 0; v < R; v++) a[v][4 * q + u] -= l[v] * f[u];
+        }
+    }
+  };
+  // L of 8 columns (lane l8 of each 8 divides for column k0 + l8).
+  auto finish = [&](auto kk) {
+    constexpr int k0 = decltype(kk)::v;
+    const float   pv = 1.0f / g[(k0 + l8) * kNB + k0 + l8];
+#pragma unroll
+    for (int u = 0; u < 8; u++) {
+      const float pk = __shfl_sync(0xffffffffu, pv, u, 8);
+#pragma unroll
+      for (int v = 0; v < R; v++) a[v][k0 + u] *= pk;
+    }
+#pragma unroll
+    for (int v = 0; v < R; v++) {
+      float *p = row + 32 * v * kDiagLD + k0;
+      store_quad(p, a[v][k0], a[v][k0 + 1], a[v][k0 + 2], a[v][k0 + 3]);
+      store_quad(p + 4, a[v][k0 + 4], a[v][k0 + 5], a[v][k0 + 6], a[v][k0 + 7]);
+    }
+  };
+  bar_wait(1, nsync);
+  each8<0>(step);
+  finish(Int<0>{});
+  bar_wait(2, nsync);
+  each8<8>(step);
+  finish(Int<8>{});
+  bar_wait(3, nsync);
+  each8<16>(step);
+  finish(Int<16>{});
+  bar_wait(4, nsync);
+  each8<24>(step);
+  finish(Int<24>{});
+}
+
+// Phase A for X of the diagonal block (lane = column): x = L^{-1} e_lane.
+__device__ __noinline__ void diag_inverse(float *Xpp, const float *Ld, int nsync) {
+  const int lane = threadIdx.x % 32;
+  float     x[32];
+#pragma unroll
+  for (int i = 0; i < 32; i++) x[i] = i == lane ? 1.0f : 0.0f;
+  auto step = [&](auto kk) {
+    constexpr int k           = decltype(kk)::v;
+    Xpp[k * kDiagLD + lane] = x[k];
+    update_row32<k>(x, x[k], Ld + 32 * k);
+  };
+  bar_wait(1, nsync);
+  each8<0>(step);
+  bar_wait(2, nsync);
+  each8<8>(step);
+  bar_wait(3, nsync);
+  each8<16>(step);
+  bar_wait(4, nsync);
+  each8<24>(step);
+}
+
+// Half of C = (add ? C : 0) + sign A B, 32 x 32 blocks: 16 columns (half 0 or
+// 1) by one warp, a lane 4 x 4.  C may be B.
+__device__ __noinline__ void diag_product(const float *A, const float *B, int ldb, float *C, float sign,
+                                          bool add, int half) {
+  constexpr int LD   = kDiagLD;
+  const int     lane = threadIdx.x % 32, i0 = 4 * (lane / 4), j0 = 16 * half + 4 * (lane % 4);
+  float         acc[4][4] = {};
+  A += i0 * LD;
+  B += j0;
+  C += i0 * LD + j0;
+#pragma unroll 2
+  for (int k = 0; k < 32; k += 4) {
+    float4 b[4];
+#pragma unroll
+    for (int u = 0; u < 4; u++) b[u] = *reinterpret_cast<const float4 *>(B + (k + u) * ldb);
+#pragma unroll
+    for (int r = 0; r < 4; r++) {
+      const float4 f = *reinterpret_cast<const float4 *>(A + r * LD + k);
+      const float  a[4] = {f.x, f.y, f.z, f.w};
+#pragma unroll
+      for (int u = 0; u < 4; u++) {
+        acc[r][0] += a[u] * b[u].x;
+        acc[r][1] += a[u] * b[u].y;
+        acc[r][2] += a[u] * b[u].z;
+        acc[r][3] += a[u] * b[u].w;
+      }
+    }
   }
+  __syncwarp();
 #pragma unroll
-  for (int ii = 0; ii < 32; ii++) {
-    Xs[(c0 + ii) * LD + c0 + lane] = x[ii];
-    Xd[ii * LG + lane]             = x[ii];
+  for (int r = 0; r < 4; r++) {
+    float4 o = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    if (add) o = *reinterpret_cast<const float4 *>(C + r * LD);
+    store_quad(C + r * LD, o.x + sign * acc[r][0], o.y + sign * acc[r][1], o.z + sign * acc[r][2],
+               o.w + sign * acc[r][3]);
+  }
+}
+
+// Panel p's columns into the front (P, column stride h, n rows), by warp u of
+// nu: 4 columns a turn, lane = row.
+__device__ __noinline__ void diag_store_panel(float *P, int64_t h, int n, int nblk, const float *Fs, int p,
+                                              int u, int nu) {
+  const int lane = threadIdx.x % 32, cnt = 8 * (nblk - p);
+#pragma unroll 2
+  for (int e = u; e < cnt; e += nu) {
+    const int    i = 32 * (p + e / 8) + lane, j = 32 * p + 4 * (e % 8);
+    const float4 v = *reinterpret_cast<const float4 *>(Fs + i * kDiagLD + j);
+    float       *q = P + i + (int64_t)j * h;
+    const int    k = i < n ? i - j : -1;
+    if (k >= 0) q[0] = v.x;
+    if (k >= 1) q[h] = v.y;
+    if (k >= 2) q[2 * h] = v.z;
+    if (k >= 3) q[3 * h] = v.w;
+  }
+}
+// Row block x of X into Lv (blocks above the diagonal blocks, rows and columns
+// of the pad are zero), by warp u of nu.
+__device__ __noinline__ void diag_store_x(float *Lv, int n, int n32, const float *Xs, int x, int u, int nu) {
+  const int i = 32 * x + threadIdx.x % 32;
+#pragma unroll 2
+  for (int e = u; e < n32 / 4; e += nu) {
+    const int j = 4 * e, k = j < 32 * (x + 1) && i < n ? n - j : 0;
+    float4    v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    if (k > 0) v = *reinterpret_cast<const float4 *>(Xs + i * kDiagLD + j);
+    float *q   = Lv + i + j * kNB;
+    q[0]       = k > 0 ? v.x : 0.0f;
+    q[kNB]     = k > 1 ? v.y : 0.0f;
+    q[2 * kNB] = k > 2 ? v.z : 0.0f;
+    q[3 * kNB] = k > 3 ? v.w : 0.0f;
   }
 }
 
@@ -293,167 +508,113 @@ __global__ void __launch_bounds__(kDiagThreads)
     k_diag_block(const StepDesc *descs, float *panel, float *linv, float *D, float *Dinv,
                  float *packd, float *packs, FactorStatus *st) {
   static_assert(kDiagThreads == 4 * kNB, "diag kernel thread mapping");
-  constexpr int LD = kDiagLD, LG = kDiagLG, LT = kDiagLT;
+  constexpr int LD = kDiagLD;
   extern __shared__ __align__(16) float sm[];
-  float          *Fs = sm;             // the block, row-major
-  float          *Xs = Fs + kNB * LD;  // X, row-major
-  float          *Gt = Xs + kNB * LD;  // G^T of the current panel (rows below it)
-  float          *Lt = Gt + 32 * kNB;  // L^T of the current panel (rows below it)
-  float          *Xd = Lt + 32 * kNB;  // X of the current panel's diagonal block
-  float          *Ts = Xd + 32 * LG;   // T_pb, b < p
-  __shared__ float dinv_s[kNB];
+  float          *Fs = sm;                 // the block, row-major
+  float          *Xs = Fs + kNB * LD;      // X, row-major
+  float          *G2 = Xs + kNB * LD;      // G^T of two panels, by panel parity
+  float          *Ld = G2 + 2 * 32 * kNB;  // L^T of the current diagonal block
+  __shared__ float dv_s[kNB];
   const StepDesc   d    = descs[blockIdx.x];
   const int        n    = d.nbk;
   const int        nblk = (n + 31) / 32, n32 = 32 * nblk;
   const int64_t    h    = d.h;
   const int        tid = threadIdx.x, warp = tid / 32, lane = tid % 32;
-  const int        ri = tid % kNB, c = tid / kNB;
-  float           *P  = panel + d.panel + d.kb + (int64_t)d.kb * h;
+  float           *P = panel + d.panel + d.kb + (int64_t)d.kb * h, *Lv = linv + d.linv;
+  // Columns j .. j + 3 of row i (lower triangle, unit pad), as loads in flight.
+  auto quad = [&](int i, int j) {
+    const float *q  = P + i + (int64_t)j * h;
+    auto         at = [&](int u) {
+      return i >= j + u && i < n ? q[u * h] : (i == j + u ? 1.0f : 0.0f);
+    };
+    return make_float4(at(0), at(1), at(2), at(3));
+  };
   {
-    // Thread (ri, c): row ri, columns c + 4m; all loads in flight before the
-    // first store.
-    float v[32];
-#pragma unroll
-    for (int m = 0; m < 32; m++) {
-      const int j = c + 4 * m;
-      v[m] = (ri >= j && ri < n) ? P[ri + (int64_t)j * h] : (ri == j ? 1.0f : 0.0f);
+    const int i = tid % kNB, c = tid / kNB;
+    if (i < n32) {
+      const float4 v0 = quad(i, 4 * c), v1 = quad(i, 16 + 4 * c);
+      *reinterpret_cast<float4 *>(Fs + i * LD + 4 * c)      = v0;
+      *reinterpret_cast<float4 *>(Fs + i * LD + 16 + 4 * c) = v1;
+    } else {  // rows of X beyond the block
+      for (int j = c; j < n32; j += 4) Lv[i + j * kNB] = 0.0f;
     }
-#pragma unroll
-    for (int m = 0; m < 32; m++) Fs[ri * LD + c + 4 * m] = v[m];
   }
   __syncthreads();
   int npos = 0;
   for (int p = 0;; p++) {
-    const int c0 = 32 * p;
+    const int c0 = 32 * p, rest = nblk - 1 - p, nsync = 32 * (2 + (rest + 1) / 2);
+    float    *Gt = G2 + (p & 1) * 32 * kNB;
     // A.
     if (warp == 0) {
-      diag_panel(Fs, Xs, Xd, dinv_s, c0, n, d, D, Dinv, packd, packs, st, npos);
-    } else if (warp % 4 != 0) {
-      // T_pb (thread: rows 4 tr .. 4 tr + 3, columns 2 tc, 2 tc + 1 of block
-      // b); these warps share no scheduler with warp 0.
-      const int item = 32 * ((warp / 4) * 3 + warp % 4 - 1) + lane;
-      if (item < 128 * p) {
-        const int    b = item / 128, q = item % 128, tc = q % 16, tr = q / 16;
-        const float *Fr = Fs + (c0 + 4 * tr) * LD;
-        const float *Xc = Xs + 32 * b + 2 * tc;
-        float        acc[4][2] = {};
+      diag_panel(Fs, Gt, Ld, dv_s, c0, nsync, n, d, D, Dinv, packd, packs, st, npos);
+    } else if (warp == 1) {
+      if (rest >= 2)
+        diag_rows<2>(Fs, Gt, dv_s, c0, nsync, c0 + 32 + lane);
+      else if (rest == 1)
+        diag_rows<1>(Fs, Gt, dv_s, c0, nsync, c0 + 32 + lane);
+    } else if (warp == 2) {
+      if (rest == 3) diag_rows<1>(Fs, Gt, dv_s, c0, nsync, c0 + 96 + lane);
+    } else if (warp == 3) {
+      diag_inverse(Xs + c0 * LD + c0, Ld, nsync);
+    } else {
+      const int u = warp - 4, half = u % 2;
+      if (p == 0) {
+        // the later panels' columns: row blocks 1 .. nblk - 1, 8 quads a panel
+        const int nq = 4 * nblk * (nblk - 1);
 #pragma unroll 4
-        for (int k = 32 * b; k < c0; k++) {
-          const float x0 = Xc[k * LD], x1 = Xc[k * LD + 1];
-#pragma unroll
-          for (int rr = 0; rr < 4; rr++) {
-            const float f = Fr[rr * LD + k];
-            acc[rr][0] += f * x0;
-            acc[rr][1] += f * x1;
-          }
+        for (int e = u; e < nq; e += 12) {
+          const int b = e >= 24 ? 3 : e >= 8 ? 2 : 1, j = 32 + 4 * (e - 4 * b * (b - 1)), i = 32 * b + lane;
+          *reinterpret_cast<float4 *>(Fs + i * LD + j) = quad(i, j);
         }
-#pragma unroll
-        for (int rr = 0; rr < 4; rr++) {
-          Ts[b * 32 * LT + (4 * tr + rr) * LT + 2 * tc]     = acc[rr][0];
-          Ts[b * 32 * LT + (4 * tr + rr) * LT + 2 * tc + 1] = acc[rr][1];
+      } else {
+        // Half a block product a warp: p - 1 of X_{p-1,b}; the update of blocks
+        // (i, j), p < j <= i; T_{i,p-1}.  Then, with X_{p-1,b}, T_ib for b < p - 1.
+        const int    q = p - 1, nd = rest * (rest + 1) / 2, w = u / 2;
+        const float *Lq = Fs + 32 * q;  // L_{.,q}
+        if (w < q) {
+          float *X = Xs + 32 * q * LD + 32 * w;
+          diag_product(Xs + 32 * q * LD + 32 * q, X, LD, X, -1.0f, false, half);
+        } else if (w < q + nd) {
+          const int e = w - q, i = p + 1 + (e >= 1) + (e >= 3), j = p + 1 + e - (i - p - 1) * (i - p) / 2;
+          diag_product(Lq + 32 * i * LD, G2 + (q & 1) * 32 * kNB + 32 * j, kNB, Fs + 32 * i * LD + 32 * j,
+                       -1.0f, true, half);
+        } else if (w < q + nd + rest + 1) {
+          const int i = p + w - q - nd;
+          diag_product(Lq + 32 * i * LD, Xs + 32 * q * LD + 32 * q, LD, Xs + 32 * i * LD + 32 * q, 1.0f,
+                       false, half);
         }
+        diag_store_panel(P, h, n, nblk, Fs, q, 11 - u, 12);
+        bar_wait(5, 384);
+        const int e = 5 - w;
+        if (e < q * (rest + 1)) {
+          const int i = p + e / q, b = e % q;
+          diag_product(Lq + 32 * i * LD, Xs + 32 * q * LD + 32 * b, LD, Xs + 32 * i * LD + 32 * b, 1.0f, true,
+                       half);
+        }
+        diag_store_x(Lv, n, n32, Xs, q, u, 12);
       }
     }
     __syncthreads();
+    if (rest == 0) break;
     // B.
-    const bool below = c0 + 32 < n32;
-    if (ri >= c0 + 32 && ri < n32) {
-      // G = F X_pp^T (thread: row ri, columns c + 4t)
-      float f[32];
-#pragma unroll
-      for (int k = 0; k < 32; k++) f[k] = Fs[ri * LD + c0 + k];
-#pragma unroll
-      for (int t = 0; t < 8; t++) {
-        const int     jj  = c + 4 * t;
-        const float4 *xr  = reinterpret_cast<const float4 *>(Xd + jj * LG);
-        float         acc = 0.0f;
-#pragma unroll
-        for (int q = 0; q < 8; q++) {
-          const float4 xv = xr[q];
-          acc += f[4 * q] * xv.x;
-          acc += f[4 * q + 1] * xv.y;
-          acc += f[4 * q + 2] * xv.z;
-          acc += f[4 * q + 3] * xv.w;
-        }
-        Gt[jj * kNB + ri] = acc;
-        Lt[jj * kNB + ri] = acc * dinv_s[c0 + jj];
-      }
-    } else if (ri < c0 + 32 && p > 0) {
-      // X_pb = -X_pp T_pb (lane = column) on the warps without rows below.
-      const int u = (warp / 4) * (p + 1) + warp % 4, nu = 4 * (p + 1);
-      for (int e = u; e < 32 * p; e += nu) {
-        const int     b = e / 32, rr = e % 32;
-        const float4 *xr = reinterpret_cast<const float4 *>(Xd + rr * LG);
-        const float  *tb = Ts + b * 32 * LT + lane;
-        float         acc[4] = {};
-#pragma unroll
-        for (int q = 0; q < 8; q++) {
-          if (4 * q <= rr) {  // row rr of X_pp is zero right of rr
-            const float4 xv = xr[q];
-            acc[0] += xv.x * tb[(4 * q) * LT];
-            acc[1] += xv.y * tb[(4 * q + 1) * LT];
-            acc[2] += xv.z * tb[(4 * q + 2) * LT];
-            acc[3] += xv.w * tb[(4 * q + 3) * LT];
-          }
-        }
-        Xs[(c0 + rr) * LD + 32 * b + lane] = -((acc[0] + acc[1]) + (acc[2] + acc[3]));
-      }
-    }
-    if (!below) break;
-    __syncthreads();
-    // C. (the panel's L into the block; the update by 4 x 4 tiles of the
-    // lower triangle, row-major over the tiles)
-    if (ri >= c0 + 32 && ri < n32) {
-#pragma unroll
-      for (int t = 0; t < 8; t++) Fs[ri * LD + c0 + c + 4 * t] = Lt[(c + 4 * t) * kNB + ri];
-    }
-    {
-      const int mt = (n32 - c0 - 32) / 4, ntiles = mt * (mt + 1) / 2;
-      if (tid < ntiles) {
-        int ti = static_cast<int>((sqrtf(8.0f * tid + 1.0f) - 1.0f) * 0.5f);
-        if ((ti + 1) * (ti + 2) / 2 <= tid) ti++;
-        if (ti * (ti + 1) / 2 > tid) ti--;
-        const int tj = tid - ti * (ti + 1) / 2;
-        const int i0 = c0 + 32 + 4 * ti, j0 = c0 + 32 + 4 * tj;
-        float     acc[4][4] = {};
-#pragma unroll 8
-        for (int k = 0; k < 32; k++) {
-          const float4 lv = *reinterpret_cast<const float4 *>(Lt + k * kNB + i0);
-          const float4 gv = *reinterpret_cast<const float4 *>(Gt + k * kNB + j0);
-          const float  la[4] = {lv.x, lv.y, lv.z, lv.w}, ga[4] = {gv.x, gv.y, gv.z, gv.w};
-#pragma unroll
-          for (int r = 0; r < 4; r++)
-#pragma unroll
-            for (int s = 0; s < 4; s++) acc[r][s] += la[r] * ga[s];
-        }
-#pragma unroll
-        for (int r = 0; r < 4; r++)
-#pragma unroll
-          for (int s = 0; s < 4; s++)
-            if (j0 + s <= i0 + r) Fs[(i0 + r) * LD + j0 + s] -= acc[r][s];
-      }
+    if (warp < 2 * rest) {
+      const int i = c0 + 32 + 32 * (warp / 2);
+      diag_product(Fs + i * LD + c0, Gt + c0 + 32, kNB, Fs + i * LD + c0 + 32, -1.0f, true, warp % 2);
     }
     __syncthreads();
   }
   if (warp == 0) {
     npos = __reduce_add_sync(0xffffffffu, npos);
-    if (lane == 0 && npos > 0) atomicAdd(&st->npos, npos);
+    if (tid == 0 && npos > 0) atomicAdd(&st->npos, npos);
+  }
+  const int last = nblk - 1;
+  if (warp < 2 * last) {
+    float *X = Xs + 32 * last * LD + 32 * (warp / 2);
+    diag_product(Xs + 32 * last * LD + 32 * last, X, LD, X, -1.0f, false, warp % 2);
   }
   __syncthreads();
-  // The factor back into the panel (lower triangle) and X (blocks above the
-  // diagonal blocks are zero).
-#pragma unroll 4
-  for (int m = 0; m < 32; m++) {
-    const int j = c + 4 * m;
-    if (ri >= j && ri < n) P[ri + (int64_t)j * h] = Fs[ri * LD + j];
-  }
-  float *Lv = linv + d.linv;
-#pragma unroll 4
-  for (int m = 0; m < 32; m++) {
-    const int j = c + 4 * m;
-    if (j >= n32) break;
-    Lv[ri + j * kNB] = (ri < n && j < n && ri / 32 >= j / 32) ? Xs[ri * LD + j] : 0.0f;
-  }
+  diag_store_panel(P, h, n, nblk, Fs, last, warp, kDiagThreads / 32);
+  diag_store_x(Lv, n, n32, Xs, last, kDiagThreads / 32 - 1 - warp, kDiagThreads / 32);
 }
 
 // ---------------------------------------------------------------------------
