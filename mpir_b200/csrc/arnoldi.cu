@@ -191,6 +191,7 @@ __device__ __forceinline__ void leave() {
 
 __global__ void __launch_bounds__(kThreads)
     k_gmres_begin(const ArnoldiArgs a, uint32_t act, const double *b, const VecFactors fac) {
+  grid_wait();
   __shared__ RedShared S;
   int                  turn = 0;
   const int            vec  = blockIdx.y;
@@ -230,6 +231,7 @@ __global__ void __launch_bounds__(kThreads)
 }
 
 __global__ void __launch_bounds__(kThreads) k_gmres_first(const ArnoldiArgs a) {
+  grid_wait();
   __shared__ RedShared S;
   int                  turn = 0;
   const int            vec  = blockIdx.y;
@@ -258,6 +260,7 @@ __global__ void __launch_bounds__(kThreads) k_gmres_first(const ArnoldiArgs a) {
 // v_{j+1} before its reduction); a second sweep where Brown and Hindmarsh's test
 // asks for it; w /= |w|; the rotations.
 __global__ void __launch_bounds__(kThreads) k_gmres_step(const ArnoldiArgs a, int64_t k) {
+  grid_wait();
   __shared__ RedShared S;
   int                  turn = 0;
   const int            vec  = blockIdx.y, lane = threadIdx.x % 32;
@@ -386,6 +389,7 @@ __global__ void __launch_bounds__(kThreads) k_gmres_step(const ArnoldiArgs a, in
 __global__ void __launch_bounds__(kThreads)
     k_gmres_end(const ArnoldiArgs a, uint32_t act, double *x, int update, const VecFactors fac,
                 unsigned long long *inf) {
+  grid_wait();
   __shared__ RedShared S;
   int                  turn = 0;
   const int            vec  = blockIdx.y, tid = threadIdx.x;
@@ -494,24 +498,6 @@ ArnoldiArgs make_args(int64_t n, int64_t m, int64_t stride, double *V, int64_t b
   return ArnoldiArgs{n, m, n, block, stride, V, state, tol, mail};
 }
 
-// Launch on clusters of C CTAs, one per vector.
-template <class... K, class... A>
-void launch_cluster(void (*kernel)(K...), int C, int nb, cudaStream_t s, A &&...args) {
-  launch_add(1);
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim  = dim3(C, nb, 1);
-  cfg.blockDim = dim3(kThreads, 1, 1);
-  cfg.stream   = s;
-  cudaLaunchAttribute at{};
-  at.id               = cudaLaunchAttributeClusterDimension;
-  at.val.clusterDim.x = C;
-  at.val.clusterDim.y = 1;
-  at.val.clusterDim.z = 1;
-  cfg.attrs           = &at;
-  cfg.numAttrs        = 1;
-  MPIR_CUDA(cudaLaunchKernelEx(&cfg, kernel, static_cast<K>(args)...));
-}
-
 void allow_16() {
   static const bool done = [] {
     for (auto *f : {reinterpret_cast<const void *>(k_gmres_begin), reinterpret_cast<const void *>(k_gmres_first),
@@ -550,23 +536,23 @@ int Arnoldi::cluster() const {
 void Arnoldi::begin(int nb, uint32_t act, const double *b, const VecFactors &fac, double *V, double tol,
                     cudaStream_t s) {
   allow_16();
-  launch_cluster(k_gmres_begin, cluster(), nb, s,
+  launch_chained(n_, k_gmres_begin, cluster(), dim3(cluster(), nb, 1), kThreads, 0, s,
                  make_args(n_, m_, stride(m_), V, 0, state_.as<double>(), tol, mail_), act, b, fac);
 }
 
 void Arnoldi::first(int nb, double *V, double tol, cudaStream_t s) {
-  launch_cluster(k_gmres_first, cluster(), nb, s,
+  launch_chained(n_, k_gmres_first, cluster(), dim3(cluster(), nb, 1), kThreads, 0, s,
                  make_args(n_, m_, stride(m_), V, 0, state_.as<double>(), tol, mail_));
 }
 
 void Arnoldi::step(int nb, int64_t j, double *V, int64_t block, double tol, cudaStream_t s) {
-  launch_cluster(k_gmres_step, cluster(), nb, s,
+  launch_chained(n_, k_gmres_step, cluster(), dim3(cluster(), nb, 1), kThreads, 0, s,
                  make_args(n_, m_, stride(m_), V, block, state_.as<double>(), tol, mail_), j);
 }
 
 void Arnoldi::end(int nb, uint32_t act, const double *V, int64_t block, double *x, bool update,
                   const VecFactors &scale, unsigned long long *inf, cudaStream_t s) {
-  launch_cluster(k_gmres_end, cluster(), nb, s,
+  launch_chained(n_, k_gmres_end, cluster(), dim3(cluster(), nb, 1), kThreads, 0, s,
                  make_args(n_, m_, stride(m_), const_cast<double *>(V), block, state_.as<double>(), 0.0, mail_),
                  act, x, update ? 1 : 0, scale, inf);
 }

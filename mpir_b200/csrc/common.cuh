@@ -51,6 +51,42 @@ inline void launch(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem,
   kernel<<<grid, block, smem, s>>>(static_cast<KArgs>(args)...);
 }
 
+// Launch of a kernel whose first statement is grid_wait(), on clusters of
+// `cluster` blocks (in x) if more than one.  For systems of up to kChainedMax
+// unknowns (n) it overlaps the end of the kernel before it (programmatic
+// dependent launch), and the next one's launch may begin once every block here
+// has passed that statement.  The kernels of a solve are launched so: chains of
+// kernels of 5 to 50 us, each of which would wait for the one before to drain
+// and then for its own launch.  A solve took 7 % less at n = 1,280, 9 % at 2,160
+// and 2.4 % at 14,045; from n = 24,603 to 40,951 it took up to 1 % more.  The
+// factorization's kernels are not: inside its graph they took 3 to 8 % longer.
+constexpr int64_t kChainedMax = 20000;
+template <class... KArgs, class... Args>
+inline void launch_chained(int64_t n, void (*kernel)(KArgs...), int cluster, dim3 grid, dim3 block,
+                           size_t smem, cudaStream_t s, Args &&...args) {
+  launch_add(1);
+  cudaLaunchAttribute at[2] = {};
+  at[0].id                  = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x    = cluster;
+  at[0].val.clusterDim.y    = 1;
+  at[0].val.clusterDim.z    = 1;
+  at[1].id                  = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[1].val.programmaticStreamSerializationAllowed = n <= kChainedMax;
+  cudaLaunchConfig_t cfg    = {};
+  cfg.gridDim               = grid;
+  cfg.blockDim              = block;
+  cfg.dynamicSmemBytes      = smem;
+  cfg.stream                = s;
+  cfg.attrs                 = cluster > 1 ? at : at + 1;
+  cfg.numAttrs              = cluster > 1 ? 2 : 1;
+  MPIR_CUDA(cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...));
+}
+// Nothing that another kernel writes may be read, and nothing written, before
+// this.
+__device__ __forceinline__ void grid_wait() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
 
 // One block step of one front in the blocked dense partial factorization.
 // The front's panel is h x w column-major at `panel` (floats, relative to the

@@ -49,7 +49,9 @@ namespace mpir {
 // Shared memory (doubles): kFlowInvSmem, then 4,608 for vectors and partial sums.
 constexpr int kFlowSmem = kFlowInvSmem + 4608;
 
-__global__ void k_mark_pending(int64_t n, double *p) { flow_mark(p, n); }
+__global__ void k_mark_pending(int64_t n, double *p) {
+  flow_mark(p, n);
+}
 
 void flow_pending(double *p, int64_t n, cudaStream_t s) {
   launch(k_mark_pending, static_cast<unsigned>(std::min<int64_t>((n + 255) / 256, kSMs * 16)), 256, 0, s,
@@ -394,6 +396,7 @@ __device__ __noinline__ void fwd_warp(const FlowArgs<T> &a, FlowShared &S, const
 
 template <class T>
 __global__ void __launch_bounds__(kFlowThreads, 1) k_fwd_flow(const __grid_constant__ FlowArgs<T> a) {
+  grid_wait();
   extern __shared__ __align__(128) double sm[];
   __shared__ __align__(16) FlowShared S;
   uint32_t phase = 0, wphase = 0;
@@ -742,6 +745,7 @@ __device__ __noinline__ void bwd_warp(const FlowArgs<T> &a, FlowShared &S, const
 
 template <class T>
 __global__ void __launch_bounds__(kFlowThreads, 1) k_bwd_flow(const __grid_constant__ FlowArgs<T> a) {
+  grid_wait();
   extern __shared__ __align__(128) double sm[];
   __shared__ __align__(16) FlowShared S;
   uint32_t phase = 0, wphase = 0;
@@ -947,7 +951,7 @@ static void ldlt_solve_t(const Plan &P, const Numeric &F, const T *pan, double *
     a.mark   = bv;
     a.nmark  = b.bwd;
     a.ticket = ws.sync.as<int32_t>();
-    launch(k_fwd_flow<T>, std::min(P.nflow_fwd, kSMs), kFlowThreads, smem, s, a);
+    launch_chained(n, k_fwd_flow<T>, 1, std::min(P.nflow_fwd, kSMs), kFlowThreads, smem, s, a);
     ws.fwd_pending = false;
     ws.bwd_pending = true;
   }
@@ -967,7 +971,7 @@ static void ldlt_solve_t(const Plan &P, const Numeric &F, const T *pan, double *
   a.nmark  = b.fwd;
   a.Dinv   = (phases & kDiagonal) ? F.Dinv.as<float>() : nullptr;
   a.ticket = ws.sync.as<int32_t>() + 1;
-  launch(k_bwd_flow<T>, std::min(P.nflow_bwd, kSMs), kFlowThreads, smem, s, a);
+  launch_chained(n, k_bwd_flow<T>, 1, std::min(P.nflow_bwd, kSMs), kFlowThreads, smem, s, a);
   ws.bwd_pending = false;
   ws.fwd_pending = true;
   kt.end(s);

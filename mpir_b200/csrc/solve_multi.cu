@@ -630,6 +630,7 @@ __device__ __noinline__ void fwd_warp_m(const FlowArgs<T> &a, FlowShared &S, con
 
 template <int NR, class T>
 __global__ void __launch_bounds__(kFlowThreads, 1) k_fwd_flow_m(const __grid_constant__ FlowArgs<T> a) {
+  grid_wait();
   extern __shared__ __align__(128) double sm[];
   __shared__ __align__(16) FlowShared S;
   uint32_t phase = 0, wphase = 0;
@@ -993,6 +994,7 @@ __device__ __noinline__ void bwd_warp_m(const FlowArgs<T> &a, FlowShared &S, con
 
 template <int NR, class T>
 __global__ void __launch_bounds__(kFlowThreads, 1) k_bwd_flow_m(const __grid_constant__ FlowArgs<T> a) {
+  grid_wait();
   extern __shared__ __align__(128) double sm[];
   __shared__ __align__(16) FlowShared S;
   uint32_t phase = 0, wphase = 0;
@@ -1058,7 +1060,7 @@ void solve_multi_nr(const Plan &P, const Numeric &F, const T *pan, double *X,
   a.mark   = bv;
   a.nmark  = NR * b.bwd;
   a.ticket = ws.sync.as<int32_t>();
-  launch(k_fwd_flow_m<NR, T>, std::min(P.nflow_fwd, kSMs), kFlowThreads, smem, s, a);
+  launch_chained(n, k_fwd_flow_m<NR, T>, 1, std::min(P.nflow_fwd, kSMs), kFlowThreads, smem, s, a);
   kt.end(s);
   MPIR_CHECK_LAUNCH();
   kt.begin(kKcSolveBwd, s);
@@ -1068,7 +1070,7 @@ void solve_multi_nr(const Plan &P, const Numeric &F, const T *pan, double *X,
   a.nmark  = NR * b.fwd;
   a.Dinv   = F.Dinv.as<float>();
   a.ticket = ws.sync.as<int32_t>() + 1;
-  launch(k_bwd_flow_m<NR, T>, std::min(P.nflow_bwd, kSMs), kFlowThreads, smem, s, a);
+  launch_chained(n, k_bwd_flow_m<NR, T>, 1, std::min(P.nflow_bwd, kSMs), kFlowThreads, smem, s, a);
   ws.fwd_pending = true;
   kt.end(s);
   MPIR_CHECK_LAUNCH();

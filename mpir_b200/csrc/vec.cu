@@ -78,6 +78,7 @@ __global__ void k_spmv(int64_t n, const int64_t *Kp, const int32_t *Kj,
                        const double *Kv, const double *x, const double *b,
                        double *y, unsigned long long *inf, int64_t vs,
                        uint32_t vact) {
+  grid_wait();
   if (batch_skip(vact)) return;
   x += blockIdx.y * vs;
   y += blockIdx.y * vs;
@@ -133,6 +134,7 @@ __global__ void k_backward_terms(int64_t n, const int64_t *Kp, const int32_t *Kj
                                  const double *ADp, const double *b,
                                  unsigned long long *inf, int64_t vs,
                                  uint32_t vact) {
+  grid_wait();
   if (batch_skip(vact)) return;
   x += blockIdx.y * vs;
   b += blockIdx.y * vs;
@@ -203,6 +205,7 @@ __global__ void k_round_to(int64_t n, int prec, double *x) {
 __global__ void k_rhs_in(int64_t n, const int64_t *perm, const double *AD,
                          const double *b, double *bs, double *ADp, double *bp,
                          unsigned long long *inf, int64_t vs) {
+  grid_wait();
   b += blockIdx.y * vs;
   bs += blockIdx.y * vs;
   bp += blockIdx.y * vs;
@@ -225,6 +228,7 @@ __global__ void k_rhs_in(int64_t n, const int64_t *perm, const double *AD,
 // out[perm[i]] = x[i] * ADp[i] (ADp NULL: out[perm[i]] = x[i]).
 __global__ void k_sol_out(int64_t n, const int64_t *perm, const double *ADp,
                           const double *x, double *out, int64_t vs) {
+  grid_wait();
   x += blockIdx.y * vs;
   out += blockIdx.y * vs;
   const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
@@ -261,7 +265,8 @@ constexpr uint32_t kAll = 0xffffffffu;
 void VecOps::spmv(int nb, const int64_t *Kp, const int32_t *Kj, const double *Kv, const double *x,
                   double *y, cudaStream_t s) {
   constexpr int G = 8;
-  launch(k_spmv<G, 0>, grid_b(n * G, 256, nb), 256, 0, s, n, Kp, Kj, Kv, x, nullptr, y, nullptr, n, kAll);
+  launch_chained(n, k_spmv<G, 0>, 1, grid_b(n * G, 256, nb), 256, 0, s, n, Kp, Kj, Kv, x, nullptr, y, nullptr, n,
+                 kAll);
 }
 
 void VecOps::residual(int nb, uint32_t act, const int64_t *Kp, const int32_t *Kj, const double *Kv,
@@ -269,8 +274,8 @@ void VecOps::residual(int nb, uint32_t act, const int64_t *Kp, const int32_t *Kj
   constexpr int       G   = 8;
   unsigned long long *inf = infbits.as<unsigned long long>();
   if (clear) clear_slots(inf, nb, 0, 1, s);
-  launch(dd ? k_spmv<G, 2> : k_spmv<G, 1>, grid_b(n * G, 256, nb), 256, 0, s, n, Kp, Kj, Kv, x, b, r, inf, n,
-         act);
+  launch_chained(n, dd ? k_spmv<G, 2> : k_spmv<G, 1>, 1, grid_b(n * G, 256, nb), 256, 0, s, n, Kp, Kj, Kv, x, b,
+                 r, inf, n, act);
 }
 
 void VecOps::backward_terms(int nb, const int64_t *Kp, const int32_t *Kj, const double *Korig,
@@ -278,7 +283,7 @@ void VecOps::backward_terms(int nb, const int64_t *Kp, const int32_t *Kj, const 
   constexpr int       G   = 8;
   unsigned long long *inf = infbits.as<unsigned long long>();
   clear_slots(inf, nb, 4, 4, s);
-  launch(k_backward_terms<G>, grid_b(n * G, 256, nb), 256, 0, s, n, Kp, Kj, Korig, x, ADp, bp, inf + 4, n,
+  launch_chained(n, k_backward_terms<G>, 1, grid_b(n * G, 256, nb), 256, 0, s, n, Kp, Kj, Korig, x, ADp, bp, inf + 4, n,
          kAll);
 }
 
@@ -301,12 +306,12 @@ void VecOps::rhs_in(int nb, const int64_t *perm, const double *AD, const double 
                     double *ADp, double *bp, cudaStream_t s) {
   unsigned long long *inf = infbits.as<unsigned long long>();
   clear_slots(inf, nb, 3, 1, s);
-  launch(k_rhs_in, grid_b(n, 256, nb), 256, 0, s, n, perm, AD, b, bs, ADp, bp, inf + 3, n);
+  launch_chained(n, k_rhs_in, 1, grid_b(n, 256, nb), 256, 0, s, n, perm, AD, b, bs, ADp, bp, inf + 3, n);
 }
 
 void VecOps::sol_out(int nb, const int64_t *perm, const double *ADp, const double *x, double *out,
                      cudaStream_t s) {
-  launch(k_sol_out, grid_b(n, 256, nb), 256, 0, s, n, perm, ADp, x, out, n);
+  launch_chained(n, k_sol_out, 1, grid_b(n, 256, nb), 256, 0, s, n, perm, ADp, x, out, n);
 }
 
 void VecOps::read_inf(int nb, double *h, cudaStream_t s) {
