@@ -422,7 +422,7 @@ static int qdldl_solve_phases(int64_t n, const int64_t *Lp, const int64_t *Li, c
                                 cudaMemcpyHostToDevice, c->s));
       MPIR_CUDA(cudaMemcpyAsync(c->F->Dinv.as<void>(), dv.data(), n * sizeof(float),
                                 cudaMemcpyHostToDevice, c->s));
-      flow_invert(*c->P, *c->F, c->s);
+      flow_invert(*c->P, *c->F, kFlowAll, c->s);
       c->F->trim();  // the solves read L, Dinv and the block inverses only
       c->ws = std::make_unique<SolveWorkspace>();
       c->ws->allocate(*c->P);

@@ -127,6 +127,8 @@ class Plan {
   // directions, the strips of the block inverses, the rows' child contributions.
   DeviceBuffer flow_warp, flow_fwd, flow_bwd, flow_inv, flow_gfirst, flow_gmore;
   int32_t      nflow_fwd = 0, nflow_bwd = 0, nflow_inv = 0;
+  int32_t      nflow_inv_low = 0;      // those below the last level, first in flow_inv
+  bool         flow_warp_top = false;  // a warp-solved front in the last level
   int64_t      flow_part_elems = 0, flow_inv_elems = 0, flow_wpanel_total = 0;
   bool warp_solved(int64_t J) const { return S.w(J) <= kWarpSolveW && S.h(J) <= kWarpSolveH; }
   void build_flow();
@@ -240,8 +242,10 @@ class Numeric {
 
 // What the triangular solves read of a factor beyond its panels: the float64
 // inverses of the diagonal blocks and the panels of the warp-solved fronts
-// (solve.cu), once per factorization.
-void flow_invert(const Plan &P, Numeric &F, cudaStream_t s);
+// (solve.cu), once per factorization: those of the fronts below the last level,
+// of the last level, or all.
+enum FlowPart { kFlowLow, kFlowTop, kFlowAll };
+void flow_invert(const Plan &P, Numeric &F, FlowPart part, cudaStream_t s);
 // Tensor-core GemmProb updates from the packed fronts (mode 0 bfloat16,
 // 1 3xTF32, 2 float16).  packs = the sign(D) sqrt|D| array.
 void launch_gemm_tc(int mode, const GemmProb *probs, int nprob, int tiles, const float *pack,

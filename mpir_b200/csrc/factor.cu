@@ -1468,6 +1468,47 @@ void Numeric::run_graph(const Plan &P, const double *d_Ax, double eps, cudaStrea
   valid = true;
 }
 
+namespace {
+// A branch of the graph that a stream is recording: what is launched between
+// begin() and end() depends on what came before begin() only, and what follows
+// join() on both.
+class CaptureFork {
+ public:
+  explicit CaptureFork(cudaStream_t s) : s_(s) { capturing_ = query().first; }
+  bool capturing() const { return capturing_; }
+  bool forked() const { return !branch_.empty(); }
+  void begin() { main_ = query().second; }
+  void end() {
+    branch_ = query().second;
+    set(main_);
+  }
+  void join() {
+    if (!forked()) return;
+    std::vector<cudaGraphNode_t> all = query().second;
+    for (cudaGraphNode_t b : branch_)
+      if (std::find(all.begin(), all.end(), b) == all.end()) all.push_back(b);
+    set(all);
+  }
+
+ private:
+  std::pair<bool, std::vector<cudaGraphNode_t>> query() const {
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    const cudaGraphNode_t  *deps   = nullptr;
+    size_t                  n      = 0;
+    MPIR_CUDA(cudaStreamGetCaptureInfo(s_, &status, nullptr, nullptr, &deps, &n));
+    if (status != cudaStreamCaptureStatusActive) return {false, {}};
+    return {true, std::vector<cudaGraphNode_t>(deps, deps + n)};
+  }
+  void set(std::vector<cudaGraphNode_t> deps) {
+    MPIR_CUDA(cudaStreamUpdateCaptureDependencies(s_, deps.data(), deps.size(),
+                                                  cudaStreamSetCaptureDependencies));
+  }
+  cudaStream_t                 s_;
+  bool                         capturing_ = false;
+  std::vector<cudaGraphNode_t> main_, branch_;
+};
+}  // namespace
+
 void Numeric::run(const Plan &P, const double *d_Ax, double eps, cudaStream_t s) {
   if (!has_scratch) throw std::logic_error("factorization scratch released (ensure_scratch)");
   const Symbolic &S  = P.S;
@@ -1509,7 +1550,17 @@ void Numeric::run(const Plan &P, const double *d_Ax, double eps, cudaStream_t s)
                                    diag_smem));
     diag_attr = true;
   }
+  // Float64 inverses of the diagonal blocks for the triangular solves.  In a
+  // recorded graph those below the last level form a branch of their own beside
+  // it (its fronts are few and leave most of the chip idle; in a stream all of
+  // them follow the last level).
+  CaptureFork inverses(s);
   for (const LevelPlan &L : P.levels) {
+    if (&L == &P.levels.back() && inverses.capturing()) {
+      inverses.begin();
+      flow_invert(P, *this, kFlowLow, s);
+      inverses.end();
+    }
     // Children's update matrices into the fronts' panels (the update
     // matrices' own columns follow after the product that defines them).
     auto extend_add = [&](int phase) {
@@ -1580,9 +1631,9 @@ void Numeric::run(const Plan &P, const double *d_Ax, double eps, cudaStream_t s)
     extend_add(2);
     MPIR_CHECK_LAUNCH();
   }
-  // Float64 inverses of the diagonal blocks for the triangular solves.
   kt.begin(kKcDiag, s);
-  flow_invert(P, *this, s);
+  flow_invert(P, *this, inverses.forked() ? kFlowTop : kFlowAll, s);
+  inverses.join();
   kt.end(s);
   if (panel16.bytes() && S.panel_elems) {
     kt.begin(kKcScatter, s);

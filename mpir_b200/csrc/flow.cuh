@@ -71,7 +71,7 @@ constexpr int64_t flow_inv_blocks(int64_t w) {
   return full * kFlowTriSB + b * (b + 1) / 2;
 }
 
-// Strip of 8 columns of one super-block's inverse (k_flow_invert).
+// Strip of 16 columns of one super-block's inverse (k_flow_invert).
 struct FlowInvDesc {
   int64_t panel;  // panel offset of the super-block's (0, 0)
   int64_t inv;    // its inverse (doubles)

@@ -53,6 +53,10 @@ void Plan::build_flow() {
   host_.flow_gmore  = std::move(more);
   // Front descriptors; the inverses and the chunk partials of those that are
   // not solved by one warp.
+  std::vector<uint8_t> top(ns, 0);  // in the last level
+  if (S.nlevels > 0)
+    for (int64_t q = S.level_ptr[S.nlevels - 1]; q < S.level_ptr[S.nlevels]; q++) top[S.level_sup[q]] = 1;
+  std::vector<FlowInvDesc> inv_top;
   for (int64_t J = 0; J < ns; J++) {
     FlowFront    &f = fr[J];
     const int64_t w = S.w(J), h = S.h(J);
@@ -80,15 +84,17 @@ void Plan::build_flow() {
     if (warp_solved(J)) {
       f.inv = flow_wpanel_total;
       flow_wpanel_total += flow_wpanel_elems(f.w, f.h);
+      if (top[J]) flow_warp_top = true;
       continue;
     }
     f.inv = flow_inv_elems;
     flow_inv_elems += flow_inv_blocks(w) * kFlowBlk;
     for (int64_t s = 0; s * kFlowSB < w; s++) {
       const int32_t n = static_cast<int32_t>(std::min<int64_t>(kFlowSB, w - s * kFlowSB));
-      for (int32_t c = 0; c < n; c += 8)
-        inv.push_back(FlowInvDesc{f.panel + s * kFlowSB * (h + 1),
-                                  f.inv + s * kFlowTriSB * kFlowBlk, f.h, n, c, 0});
+      for (int32_t c = 0; c < n; c += 16)
+        (top[J] ? inv_top : inv)
+            .push_back(FlowInvDesc{f.panel + s * kFlowSB * (h + 1), f.inv + s * kFlowTriSB * kFlowBlk, f.h,
+                                   n, c, 0});
     }
     // The rows below a narrow block that fit one chunk are taken by the item
     // that solves the block.
@@ -99,21 +105,24 @@ void Plan::build_flow() {
     }
   }
   // Long strips first (a strip's work grows with the rows below it).
-  std::stable_sort(inv.begin(), inv.end(), [](const FlowInvDesc &a, const FlowInvDesc &b) {
-    return a.n - a.c0 > b.n - b.c0;
-  });
+  for (auto *v : {&inv, &inv_top})
+    std::stable_sort(v->begin(), v->end(), [](const FlowInvDesc &a, const FlowInvDesc &b) {
+      return a.n - a.c0 > b.n - b.c0;
+    });
+  nflow_inv_low = static_cast<int32_t>(inv.size());
+  inv.insert(inv.end(), inv_top.begin(), inv_top.end());
   // A level's warp-solved fronts, in groups that spread over the SMs and
   // whose panels fit the shared memory.
   auto warps = [&](std::vector<FlowItem> &out, size_t first, size_t count) {
     const size_t per = std::min<size_t>(kFlowWarpsPerItem, std::max<size_t>(1, (count + kSMs - 1) / kSMs));
     for (size_t q = first; q < first + count;) {
-      int64_t top = 0;
+      int64_t used = 0;
       size_t  e   = q;
       while (e < first + count && e - q < per) {
         const int64_t b = flow_wpanel_elems(warp[e].w, warp[e].h) * 8;
-        if (top + b > kFlowPanelSmem) break;
-        warp[e].part = top;
-        top += b;
+        if (used + b > kFlowPanelSmem) break;
+        warp[e].part = used;
+        used += b;
         e++;
       }
       out.push_back(FlowItem{FlowFront{}, kFlowWarps, static_cast<int32_t>(q),

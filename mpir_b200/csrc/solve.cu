@@ -768,68 +768,86 @@ __global__ void k_dscale(int64_t n, const float *Dinv, double *x) {
 
 // ---------------------------------------------------------------------------
 // Inverses of the diagonal super-blocks in float64 from the float32 factor,
-// once per factorization: a warp solves L X = E for two columns, by blocks of
-// 32 rows: the block's triangle (lane = row, the pivots' values by shuffle),
-// then the block's columns into the sums of the rows below (acc[q] belongs to
-// the q-th block from the current one).  Bound by the float32 -> float64
-// conversions (a quarter of the FMA rate), which is why a warp takes two
-// columns.
+// once per factorization: a CTA of four warps solves L X = E for 16 columns, by
+// blocks of 32 rows.  The block's triangle takes four columns a warp (lane =
+// row, the pivots' values by shuffle); the block's columns then go into the
+// sums of the rows below on the float64 matrix instructions, row block i on
+// warp i mod 4.  What bounds it is the chain of up to 16 blocks and the
+// float32 -> float64 conversions (24 cycles for a lone warp), which a fragment
+// shares among 16 columns.  A warp with two columns of its own and a
+// conversion for each use of L took 86 us for one block of 311 columns and 205
+// us at n = 24,603; it is 38 and 114 us so (with eight warps 45 and 148).
+constexpr int kInvCols  = 16;
+constexpr int kInvPitch = 20;  // conflict-free fragments
 __global__ void __launch_bounds__(128)
     k_flow_invert(const FlowInvDesc *descs, const float *panel, double *inv) {
-  __shared__ __align__(16) double xs[4][2][32];
+  __shared__ __align__(16) double xs[32 * kInvPitch];  // X of the block: row, column
+  __shared__ __align__(16) double as[32 * (kInvCols + 2)];  // its sum
   const FlowInvDesc d    = descs[blockIdx.x];
-  const int         warp = threadIdx.x / 32, lane = threadIdx.x % 32;
-  const int         n = d.n, nb = (n + 31) / 32, col = d.c0 + 2 * warp, j = col / 32;
+  const int         warp = threadIdx.x / 32, lane = threadIdx.x % 32, fr = lane / 4, fk = lane % 4;
+  const int         n = d.n, nb = (n + 31) / 32, col = d.c0 + 4 * warp, j = d.c0 / 32;
   const int64_t     h = d.h;
   const float      *P = panel + d.panel;
-  double            acc[16][2];
-#pragma unroll
-  for (int q = 0; q < 16; q++) acc[q][0] = acc[q][1] = 0.0;
+  double            acc[4][4][2][2] = {};  // row block 4 slot + warp, octet, column octet
   for (int i = j; i < nb; i++) {
     const int row = 32 * i + lane;
     float     l[32];
     load_cols(l, P, h, row, row < n, 32 * i, min(n, 32 * i + lane));
-    double v0 = (row == col && col < n ? 1.0 : 0.0) - acc[0][0];
-    double v1 = (row == col + 1 && col + 1 < n ? 1.0 : 0.0) - acc[0][1];
+#pragma unroll
+    for (int s = 0; s < 4; s++)
+      if (i == 4 * s + warp) {
+#pragma unroll
+        for (int m = 0; m < 4; m++)
+#pragma unroll
+          for (int q = 0; q < 2; q++)
+            *reinterpret_cast<double2 *>(as + (8 * m + fr) * (kInvCols + 2) + 8 * q + 2 * fk) =
+                make_double2(acc[s][m][q][0], acc[s][m][q][1]);
+      }
+    __syncthreads();
+    double v[4];
+#pragma unroll
+    for (int u = 0; u < 4; u++)
+      v[u] = (row == col + u && row < n ? 1.0 : 0.0) - as[lane * (kInvCols + 2) + 4 * warp + u];
 #pragma unroll
     for (int k = 0; k < 32; k++) {
-      const double x0 = __shfl_sync(0xffffffffu, v0, k), x1 = __shfl_sync(0xffffffffu, v1, k);
       const double lk = static_cast<double>(l[k]);
-      v0 -= lk * x0;
-      v1 -= lk * x1;
+#pragma unroll
+      for (int u = 0; u < 4; u++) v[u] -= lk * __shfl_sync(0xffffffffu, v[u], k);
     }
-    double *o = inv + d.inv + (static_cast<int64_t>(i) * (i + 1) / 2 + j) * kFlowBlk +
-                (col % 32) * 33 + lane;
-    o[0]  = v0;
-    o[33] = v1;
-    __syncwarp();
-    xs[warp][0][lane] = v0;
-    xs[warp][1][lane] = v1;
-    __syncwarp();
+    double *o = inv + d.inv + (static_cast<int64_t>(i) * (i + 1) / 2 + j) * kFlowBlk + (col % 32) * 33 + lane;
 #pragma unroll
-    for (int q = 1; q < 16; q++) {
-      if (i + q < nb) {
-        const int rq = 32 * (i + q) + lane;
-        load_cols(l, P, h, rq, rq < n, 32 * i, 32 * i + 32);
-        double s0 = 0.0, s1 = 0.0;
+    for (int u = 0; u < 4; u++) {
+      o[33 * u]                              = v[u];
+      xs[lane * kInvPitch + 4 * warp + u] = v[u];
+    }
+    __syncthreads();
+    if (i + 1 == nb) break;
+    double b[8][2];
 #pragma unroll
-        for (int k = 0; k < 32; k += 2) {
-          const double2 x0 = *reinterpret_cast<const double2 *>(&xs[warp][0][k]);
-          const double2 x1 = *reinterpret_cast<const double2 *>(&xs[warp][1][k]);
-          const double  la = static_cast<double>(l[k]), lb = static_cast<double>(l[k + 1]);
-          s0 += la * x0.x;
-          s1 += la * x1.x;
-          s0 += lb * x0.y;
-          s1 += lb * x1.y;
+    for (int t = 0; t < 8; t++)
+#pragma unroll
+      for (int q = 0; q < 2; q++) b[t][q] = xs[(4 * t + fk) * kInvPitch + 8 * q + fr];
+#pragma unroll
+    for (int s = 0; s < 4; s++) {
+      const int e = 4 * s + warp;
+      if (e <= i || e >= nb) continue;
+      const float *p = P + 32 * e + fr + (int64_t)(32 * i + fk) * h;
+#pragma unroll
+      for (int m = 0; m < 4; m++)
+#pragma unroll
+        for (int t = 0; t < 8; t++)
+          l[8 * m + t] = 32 * e + 8 * m + fr < n ? __ldg(p + 8 * m + 4 * t * h) : 0.0f;
+#pragma unroll
+      for (int m = 0; m < 4; m++)
+#pragma unroll
+        for (int t = 0; t < 8; t++) {
+          const double x = static_cast<double>(l[8 * m + t]);
+#pragma unroll
+          for (int q = 0; q < 2; q++)
+            asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+                : "+d"(acc[s][m][q][0]), "+d"(acc[s][m][q][1])
+                : "d"(x), "d"(b[t][q]));
         }
-        acc[q][0] += s0;
-        acc[q][1] += s1;
-      }
-    }
-#pragma unroll
-    for (int q = 0; q < 15; q++) {
-      acc[q][0] = acc[q + 1][0];
-      acc[q][1] = acc[q + 1][1];
     }
   }
 }
@@ -867,16 +885,19 @@ __global__ void __launch_bounds__(128)
   }
 }
 
-void flow_invert(const Plan &P, Numeric &F, cudaStream_t s) {
-  if (!P.host_.flow_warp.empty())
-    launch(k_flow_wpanel, static_cast<unsigned>((P.host_.flow_warp.size() + 3) / 4), 128, 0, s,
-           static_cast<const FlowFront *>(P.flow_warp.as<FlowFront>()),
-           static_cast<int>(P.host_.flow_warp.size()), static_cast<const float *>(F.panel.as<float>()),
-           F.wpanel.as<double>());
-  if (P.nflow_inv == 0) return;
-  launch(k_flow_invert, static_cast<unsigned>(P.nflow_inv), 128, 0, s,
-         static_cast<const FlowInvDesc *>(P.flow_inv.as<FlowInvDesc>()),
-         static_cast<const float *>(F.panel.as<float>()), F.inv64.as<double>());
+void flow_invert(const Plan &P, Numeric &F, FlowPart part, cudaStream_t s) {
+  // Warp-solved fronts: with the part that holds the last of them.
+  const int32_t nw = static_cast<int32_t>(P.host_.flow_warp.size());
+  if (nw > 0 && (part == kFlowAll || (part == kFlowTop) == P.flow_warp_top))
+    launch(k_flow_wpanel, static_cast<unsigned>((nw + 3) / 4), 128, 0, s,
+           static_cast<const FlowFront *>(P.flow_warp.as<FlowFront>()), nw,
+           static_cast<const float *>(F.panel.as<float>()), F.wpanel.as<double>());
+  const int32_t first = part == kFlowTop ? P.nflow_inv_low : 0;
+  const int32_t count = (part == kFlowLow ? P.nflow_inv_low : P.nflow_inv) - first;
+  if (count > 0)
+    launch(k_flow_invert, static_cast<unsigned>(count), 128, 0, s,
+           static_cast<const FlowInvDesc *>(P.flow_inv.as<FlowInvDesc>() + first),
+           static_cast<const float *>(F.panel.as<float>()), F.inv64.as<double>());
   MPIR_CHECK_LAUNCH();
 }
 
