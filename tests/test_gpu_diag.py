@@ -1,4 +1,4 @@
-"""Diagonal blocks of the factorization at the edges of their panels of 32.
+"""Diagonal blocks and small fronts of the factorization at the edges of their tiles.
 
 K has a dense leading block of w unknowns and one of 20, both coupled to a dense
 tail of 65 and not to each other; in natural order the first is a front of w
@@ -20,20 +20,21 @@ import mpir_b200 as mp
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("w", [33, 63, 64, 65, 95, 96, 97, 127, 128])
-def test_diagonal_block(w):
-    r, wb = 65, 20
-    n = w + wb + r
-    rng = np.random.default_rng(w)
+def _quasi_definite(n, seed):
+    rng = np.random.default_rng(seed)
     sign = np.where(np.arange(n) % 3 == 2, -1.0, 1.0)
     M = rng.standard_normal((n, 4 * n))
     M /= np.linalg.norm(M, axis=1)[:, None]
     C = M @ M.T
     A = rng.standard_normal((n, n)) / np.sqrt(n)
     K = np.where(np.equal.outer(sign, sign), np.outer(sign, sign) * C * sign[:, None], A + A.T)
-    K[:w, w:w + wb] = K[w:w + wb, :w] = 0.0
     K = K.astype(np.float32).astype(np.float64)
     K[np.arange(n), np.arange(n)] = sign
+    return K
+
+
+def _factor(K):
+    n = len(K)
     U = sp.csc_matrix(np.triu(K))
     U.sort_indices()
     solver = mp.GmresLDLIR()
@@ -44,7 +45,26 @@ def test_diagonal_block(w):
     cols = np.repeat(np.arange(n), np.diff(Lp))
     L = sp.csr_matrix((Lx.astype(np.float64), (Li, cols)), shape=(n, n)).toarray() + np.eye(n)
     solver.close()
-    L1, D1 = L[:w, :w], D[:w].astype(np.float64)
+    return L, D.astype(np.float64)
+
+
+@pytest.mark.parametrize("n", [1, 2, 7, 8, 9, 31, 32, 33, 63, 64])
+def test_small_front(n):
+    """One front in shared memory (at most 64 rows): the block's bound above."""
+    K = _quasi_definite(n, 100 + n)
+    L, D = _factor(K)
+    res = np.abs(K - (L * D) @ L.T)
+    assert (res <= 2 * (n + 10) * 2.0 ** -24 * ((np.abs(L) * np.abs(D)) @ np.abs(L.T))).all()
+
+
+@pytest.mark.parametrize("w", [33, 63, 64, 65, 95, 96, 97, 127, 128])
+def test_diagonal_block(w):
+    r, wb = 65, 20
+    n = w + wb + r
+    K = _quasi_definite(n, w)
+    K[:w, w:w + wb] = K[w:w + wb, :w] = 0.0
+    L, D = _factor(K)
+    L1, D1 = L[:w, :w], D[:w]
     u = 2.0 ** -24
     res = np.abs(K[:w, :w] - (L1 * D1) @ L1.T)
     assert (res <= 2 * (w + 10) * u * ((np.abs(L1) * np.abs(D1)) @ np.abs(L1.T))).all()
