@@ -98,6 +98,7 @@ struct LevelPlan {
   // factored, those of their update matrices [ea_begin[1], + ea_count[1])
   // after the products that define them.
   int32_t ea_begin[2] = {0, 0}, ea_count[2] = {0, 0};
+  int32_t ea_rows[2] = {0, 0};  // most parent rows of a chunk
   struct Step {
     int32_t begin, count, trsm_tiles, upd_tiles;
     // left-looking update of this block column before its diagonal block

@@ -72,3 +72,16 @@ def test_diagonal_block(w):
     LX = np.abs(sl.solve_triangular(L1, np.eye(w), lower=True).T) @ np.abs(L1.T)
     res = np.abs(F - (L[w + wb:, :w] * D1) @ L1.T)
     assert (res <= 4 * (w + 16) * u * (np.abs(F) @ LX @ LX)).all()
+
+
+@pytest.mark.parametrize("r", [255, 511, 512, 777, 1300])
+def test_extend_add_rows(r):
+    """Two dense blocks of 70 and 33 add to a dense tail of r (its rows split over
+    thread blocks from 512 on).  Products in three TF32 terms are within 17 u as
+    above, so the residual is within 4 (n + 16) u |L| |D| |L^T|."""
+    n = 103 + r
+    K = _quasi_definite(n, r)
+    K[:70, 70:103] = K[70:103, :70] = 0.0
+    L, D = _factor(K)
+    res = np.abs(K - (L * D) @ L.T)
+    assert (res <= 4 * (n + 16) * 2.0 ** -24 * ((np.abs(L) * np.abs(D)) @ np.abs(L.T))).all()
