@@ -108,24 +108,30 @@ class NestedDissection {
       return;
     }
     // Connected components.
-    std::vector<int32_t>              order, count;
-    std::vector<std::vector<int32_t>> comps;
+    std::vector<int32_t> order, count;
     reset_levels(S);
-    for (int32_t v : S) {
-      if (level_[v] >= 0) continue;
-      bfs(v, t, order, count);
-      comps.push_back(order);
-    }
-    if (comps.size() > 1) {
+    bfs(S[0], t, order, count);
+    if (order.size() < S.size()) {
+      std::vector<std::vector<int32_t>> comps(1, order);
+      for (int32_t v : S) {
+        if (level_[v] >= 0) continue;
+        bfs(v, t, order, count);
+        comps.push_back(order);
+      }
       for (auto &c : comps) split(c);
       return;
     }
-    // Pseudo-peripheral root.
+    // Pseudo-peripheral root; its search is the one made last, unless the
+    // iteration runs out.
     int32_t root = S[0];
-    int     ecc  = -1;
+    int     ecc  = -1, nl = static_cast<int>(count.size());
+    bool    searched = true;
     for (int it = 0; it < 6; it++) {
-      reset_levels(S);
-      const int nl = bfs(root, t, order, count);
+      if (it > 0) {
+        reset_levels(S);
+        nl = bfs(root, t, order, count);
+      }
+      searched = true;
       if (nl - 1 <= ecc) break;
       ecc          = nl - 1;
       int32_t best = -1;
@@ -134,10 +140,13 @@ class NestedDissection {
         if (level_[v] != nl - 1) break;
         if (best < 0 || g_.deg(v) < g_.deg(best)) best = v;
       }
-      root = best;
+      searched = best == root;
+      root     = best;
     }
-    reset_levels(S);
-    const int nl = bfs(root, t, order, count);
+    if (!searched) {
+      reset_levels(S);
+      nl = bfs(root, t, order, count);
+    }
     if (nl < 3) {  // no level separates: keep as one block
       out_->insert(out_->end(), S.begin(), S.end());
       return;
@@ -633,6 +642,10 @@ int analyze(int64_t n, const int64_t *Ap, const int64_t *Ai,
   std::vector<std::vector<int32_t>> R(ns);
   std::vector<int64_t>              mark(n, -1);
   std::vector<std::vector<int32_t>> kids(ns);
+  std::vector<int32_t>              both;
+  // Children's sets are sorted: up to this many are merged one after another
+  // (a merge touches what is there already again), more are collected and sorted.
+  constexpr size_t kMaxUnions = 8;
   for (int64_t J = 0; J < ns; J++) {
     const int64_t last = S.sfirst[J + 1] - 1;
     if (parent[last] >= 0) kids[col2sup[parent[last]]].push_back(static_cast<int32_t>(J));
@@ -648,16 +661,26 @@ int analyze(int64_t n, const int64_t *Ap, const int64_t *Ai,
           out.push_back(static_cast<int32_t>(r));
         }
       }
-    for (int32_t C : kids[J]) {
-      for (int32_t r : R[C])
-        if (r >= l && mark[r] != J) {
-          mark[r] = J;
-          out.push_back(r);
-        }
-      std::vector<int32_t>().swap(R[C]);  // children are done with
-      R[C].clear();
-    }
     std::sort(out.begin(), out.end());
+    if (kids[J].size() <= kMaxUnions) {
+      for (int32_t C : kids[J]) {
+        const auto rb = std::lower_bound(R[C].begin(), R[C].end(), static_cast<int32_t>(l));
+        both.resize(out.size() + (R[C].end() - rb));
+        both.resize(std::set_union(out.begin(), out.end(), rb, R[C].end(), both.begin()) - both.begin());
+        out.swap(both);
+        std::vector<int32_t>().swap(R[C]);  // children are done with
+      }
+    } else {
+      for (int32_t C : kids[J]) {
+        for (int32_t r : R[C])
+          if (r >= l && mark[r] != J) {
+            mark[r] = J;
+            out.push_back(r);
+          }
+        std::vector<int32_t>().swap(R[C]);
+      }
+      std::sort(out.begin(), out.end());
+    }
     if (S.Lnz[l - 1] != static_cast<int64_t>(out.size())) {
       err = "internal: supernode structure disagrees with column counts";
       return kBadArgument;
@@ -708,23 +731,10 @@ int analyze(int64_t n, const int64_t *Ap, const int64_t *Ai,
   S.Kj.resize(S.Kp[n]);
   S.Ksrc.resize(S.Kp[n]);
   {
-    // Fill column by column in permuted order so each row's columns ascend.
+    // Row r: the columns c < r, from the permuted upper column r, then the
+    // columns c >= r from the upper columns in order: each row's columns
+    // ascend (duplicates in the caller's order).
     std::vector<int64_t> fill(S.Kp.begin(), S.Kp.end() - 1);
-    for (int64_t c = 0; c < n; c++) {
-      // entries of permuted column c: (r, c) for r <= c from Ci and (r, c)
-      // for r > c from the transpose; visit both in ascending row order.
-      for (int64_t q = S.Cp[c]; q < S.Cp[c + 1]; q++) {
-        const int64_t r   = S.Ci[q];
-        const int64_t dst = fill[r]++;
-        S.Kj[dst]         = static_cast<int32_t>(c);
-        S.Ksrc[dst]       = S.Csrc[q];
-      }
-    }
-    // Lower part: row r gets column c < r from the permuted upper column r.
-    // The pass above put (r, c) with r <= c; now add (c', r') transposes.
-    // Rows are filled in increasing column order because the pass above
-    // visits columns in increasing order and the transposes below are added
-    // afterwards; sort each row to restore ascending columns.
     for (int64_t c = 0; c < n; c++)
       for (int64_t q = S.Cp[c]; q < S.Cp[c + 1]; q++) {
         const int64_t r = S.Ci[q];
@@ -733,17 +743,12 @@ int analyze(int64_t n, const int64_t *Ap, const int64_t *Ai,
         S.Kj[dst]         = static_cast<int32_t>(r);
         S.Ksrc[dst]       = S.Csrc[q];
       }
-    std::vector<std::pair<int32_t, int64_t>> tmp;
-    for (int64_t i = 0; i < n; i++) {
-      const int64_t b = S.Kp[i], e = S.Kp[i + 1];
-      tmp.resize(e - b);
-      for (int64_t q = b; q < e; q++) tmp[q - b] = {S.Kj[q], S.Ksrc[q]};
-      std::sort(tmp.begin(), tmp.end());
-      for (int64_t q = b; q < e; q++) {
-        S.Kj[q]   = tmp[q - b].first;
-        S.Ksrc[q] = tmp[q - b].second;
+    for (int64_t c = 0; c < n; c++)
+      for (int64_t q = S.Cp[c]; q < S.Cp[c + 1]; q++) {
+        const int64_t dst = fill[S.Ci[q]]++;
+        S.Kj[dst]         = static_cast<int32_t>(c);
+        S.Ksrc[dst]       = S.Csrc[q];
       }
-    }
   }
   return kOk;
 }
