@@ -268,10 +268,10 @@ __global__ void __launch_bounds__(256, 5)
 //      one broadcast, one reciprocal (the fast approximate one; D^{-1} itself
 //      is the correctly rounded 1 / d_k), one product and one update a pivot;
 //      the rest of a pivot's update takes the column from shared memory one
-//      pivot later.  Every 8 pivots it signals a named barrier, and other
-//      warps take those pivots up while it goes on: up to two for the rows
-//      below (unscaled panel entries G = L D, kept transposed, then
-//      L = G D^{-1}) and one for X_pp (lane = column).  The other twelve warps do
+//      pivot later.  Every 8 pivots it signals a named barrier, and a warp
+//      forms X_pp (lane = column) from them while it goes on; up to two more
+//      follow that one with the rows below, eight columns at a time
+//      (G = F X_pp^T = L D, kept transposed, then L = G D^{-1}).  The other twelve warps do
 //      what the chain does not wait for, in 32 x 32 block products: the previous panel's update of the columns beyond this
 //      panel, X_{p-1,b} = -X_{p-1,p-1} T_{p-1,b}, the contributions
 //      T_ib += L_{i,p-1} X_{p-1,b} to the rows of X still to come (kept where
@@ -281,10 +281,12 @@ __global__ void __launch_bounds__(256, 5)
 // What bounds it: the chain of 128 pivots, and beside it the 128 bytes a cycle
 // that shared memory returns to registers (a broadcast value costs a warp as
 // much as 32 different ones), hence two rows a lane below the diagonal block
-// and 4 x 4 values a lane in the products.  One block of 128 columns: 35.0 us
-// with X_pp and G formed after the diagonal block, products of 4 x 2 and
-// everything written at the end; 28.4 us so (64 columns 17.5 -> 15.5, 32
-// columns 10 us both).  Two pivots a turn: no gain.
+// and 4 x 4 values a lane in the products.  Every sum is taken in the order of
+// the kernel before this one (its results bit for bit): 35.0 us for a block of
+// 128 columns there, with X_pp and G formed after the diagonal block and
+// everything written at the end, 29.8 us here (32 columns 10 us both).  Rows
+// below by substitution beside the pivots instead of through X_pp: 28.4 us, but
+// other roundings.  Two pivots a turn: no gain.
 constexpr int kDiagLD = kNB + 4;  // Fs, Xs row stride (16-byte rows, lane = row conflict-free)
 constexpr int kDiagSmemFloats = 2 * kNB * kDiagLD + 2 * 32 * kNB + 32 * 32;
 
@@ -340,13 +342,14 @@ __device__ __forceinline__ void each8(F f) {
 }
 
 // Phase A of panel p for warp 0: the diagonal block at (c0, c0).  Column k goes
-// to Gt (unscaled, at row c0 + lane) and Ld (scaled), its approximate reciprocal
-// pivot to dv_s.  The broadcasts that the next pivot waits for are issued
-// before the loads of this one's column.  nsync: threads of the chunk barriers.
-// Kept out of line: inlined into the kernel, whose other phases hold many
+// to Gt (unscaled, at row c0 + lane) and Ld (scaled).  The broadcasts that the
+// next pivot waits for are issued before the loads of this one's column.  (Pivot
+// 0's update of column 30 is rounded twice: so it came out of the compiler in
+// the kernel before this one, and factors stay the same to the last bit.)  Kept
+// out of line: inlined into the kernel, whose other phases hold many
 // registers, its chain of shuffles is scheduled about 1.5x slower.
-__device__ __noinline__ void diag_panel(float *Fs, float *Gt, float *Ld, float *dv_s, int c0, int nsync,
-                                        int n, const StepDesc &d, float *D, float *Dinv, float *packd,
+__device__ __noinline__ void diag_panel(float *Fs, float *Gt, float *Ld, int c0, int n,
+                                        const StepDesc &d, float *D, float *Dinv, float *packd,
                                         float *packs, FactorStatus *st, int &npos) {
   constexpr unsigned full = 0xffffffffu;
   const int          lane = threadIdx.x % 32, r = c0 + lane;
@@ -361,7 +364,7 @@ __device__ __noinline__ void diag_panel(float *Fs, float *Gt, float *Ld, float *
     if (k > 0) {  // the previous pivot's update of the columns beyond k
 #pragma unroll
       for (int j = 0; j < 32; j++)
-        if (j > k) a[j] -= lp * fp[j];
+        if (j > k) a[j] = k == 1 && j == 30 ? __fsub_rn(a[j], __fmul_rn(lp, fp[j])) : a[j] - lp * fp[j];
     }
     if (lane == k) piv = dk;
     const float l = a[k] * dv;  // L[r][k]
@@ -372,7 +375,6 @@ __device__ __noinline__ void diag_panel(float *Fs, float *Gt, float *Ld, float *
       g[(k + 1) * kNB + lane] = a[k + 1];
     }
     Ld[32 * k + lane] = l;
-    if (lane == 0) dv_s[c0 + k] = dv;
     __syncwarp();
 #pragma unroll
     for (int q = 0; q < 8; q++)
@@ -385,7 +387,7 @@ __device__ __noinline__ void diag_panel(float *Fs, float *Gt, float *Ld, float *
       }
     lp = l;
     if (lane > k) a[k] = l;
-    if (k % 8 == 7) bar_arrive(1 + k / 8, nsync);
+    if (k % 8 == 7) bar_arrive(1 + k / 8, 64);
   }
 #pragma unroll
   for (int q = 0; q < 8; q++)
@@ -403,98 +405,117 @@ __device__ __noinline__ void diag_panel(float *Fs, float *Gt, float *Ld, float *
   }
 }
 
-// Phase A for R x 32 rows below the diagonal block (lane = rows r, r + 32, ..).
+// Phase A for R x 32 rows below the diagonal block (lane = rows r, r + 32, ..):
+// G = F X_pp^T, L = G D^{-1}, eight columns (rows of X_pp) at a time as the
+// inverse's warp finishes them.
 template <int R>
-__device__ __noinline__ void diag_rows(float *Fs, float *Gt, const float *dv_s, int c0, int nsync, int r) {
+__device__ __noinline__ void diag_rows(float *Fs, float *Gt, const float *Xpp, int c0, int nsync, int r) {
   const float *g   = Gt + c0;
   const int    l8  = threadIdx.x % 8;
   float       *row = Fs + r * kDiagLD + c0;
-  float        a[R][32];
+  float        f[R][32], out[R][8];
 #pragma unroll
-  for (int v = 0; v < R; v++) load_row32(a[v], row + 32 * v * kDiagLD);
-  auto step = [&](auto kk) {
-    constexpr int k  = decltype(kk)::v;
-    const float   dv = dv_s[c0 + k];
-    float         l[R];
+  for (int v = 0; v < R; v++) load_row32(f[v], row + 32 * v * kDiagLD);
+  auto column = [&](auto jc) {
+    constexpr int j = decltype(jc)::v;
+    float         acc[R];
 #pragma unroll
-    for (int v = 0; v < R; v++) {
-      Gt[k * kNB + r + 32 * v] = a[v][k];
-      l[v]                     = a[v][k] * dv;
+    for (int v = 0; v < R; v++) acc[v] = 0.0f;
+#pragma unroll
+    for (int q = 0; q <= j / 4; q++) {  // row j of X_pp is zero right of j
+      const float4 x = reinterpret_cast<const float4 *>(Xpp + j * kDiagLD)[q];
+#pragma unroll
+      for (int v = 0; v < R; v++) {
+        acc[v] += f[v][4 * q] * x.x;
+        acc[v] += f[v][4 * q + 1] * x.y;
+        acc[v] += f[v][4 * q + 2] * x.z;
+        acc[v] += f[v][4 * q + 3] * x.w;
+      }
     }
 #pragma unroll
-    for (int q = (k + 1) / 4; q < 8; q++) {
-      const float4 w    = reinterpret_cast<const float4 *>(g + k * kNB)[q];
-      const float  f[4] = {w.x, w.y, w.z, w.w};
-#pragma unroll
-      for (int u = 0; u < 4; u++)
-        if (4 * q + u > k) {
-#pragma unroll
-          for (int v = 0; v < R; v++) a[v][4 * q + u] -= l[v] * f[u];
-        }
+    for (int v = 0; v < R; v++) {
+      Gt[j * kNB + r + 32 * v] = acc[v];
+      out[v][j % 8]            = acc[v];
     }
   };
   // L of 8 columns (lane l8 of each 8 divides for column k0 + l8).
-  auto finish = [&](auto kk) {
-    constexpr int k0 = decltype(kk)::v;
-    const float   pv = 1.0f / g[(k0 + l8) * kNB + k0 + l8];
+  auto finish = [&](int k0) {
+    const float pv = 1.0f / g[(k0 + l8) * kNB + k0 + l8];
 #pragma unroll
     for (int u = 0; u < 8; u++) {
       const float pk = __shfl_sync(0xffffffffu, pv, u, 8);
 #pragma unroll
-      for (int v = 0; v < R; v++) a[v][k0 + u] *= pk;
+      for (int v = 0; v < R; v++) out[v][u] *= pk;
     }
 #pragma unroll
     for (int v = 0; v < R; v++) {
       float *p = row + 32 * v * kDiagLD + k0;
-      store_quad(p, a[v][k0], a[v][k0 + 1], a[v][k0 + 2], a[v][k0 + 3]);
-      store_quad(p + 4, a[v][k0 + 4], a[v][k0 + 5], a[v][k0 + 6], a[v][k0 + 7]);
+      store_quad(p, out[v][0], out[v][1], out[v][2], out[v][3]);
+      store_quad(p + 4, out[v][4], out[v][5], out[v][6], out[v][7]);
     }
   };
-  bar_wait(1, nsync);
-  each8<0>(step);
-  finish(Int<0>{});
-  bar_wait(2, nsync);
-  each8<8>(step);
-  finish(Int<8>{});
-  bar_wait(3, nsync);
-  each8<16>(step);
-  finish(Int<16>{});
-  bar_wait(4, nsync);
-  each8<24>(step);
-  finish(Int<24>{});
+  bar_wait(6, nsync);
+  each8<0>(column);
+  finish(0);
+  bar_wait(7, nsync);
+  each8<8>(column);
+  finish(8);
+  bar_wait(8, nsync);
+  each8<16>(column);
+  finish(16);
+  bar_wait(9, nsync);
+  each8<24>(column);
+  finish(24);
 }
 
-// Phase A for X of the diagonal block (lane = column): x = L^{-1} e_lane.
+// Phase A for X of the diagonal block (lane = column): x = L^{-1} e_lane.  Row k
+// is final at pivot k; nsync: threads of the barriers that hand eight rows on.
 __device__ __noinline__ void diag_inverse(float *Xpp, const float *Ld, int nsync) {
   const int lane = threadIdx.x % 32;
   float     x[32];
 #pragma unroll
   for (int i = 0; i < 32; i++) x[i] = i == lane ? 1.0f : 0.0f;
   auto step = [&](auto kk) {
-    constexpr int k           = decltype(kk)::v;
+    constexpr int k         = decltype(kk)::v;
     Xpp[k * kDiagLD + lane] = x[k];
     update_row32<k>(x, x[k], Ld + 32 * k);
   };
-  bar_wait(1, nsync);
+  bar_wait(1, 64);
   each8<0>(step);
-  bar_wait(2, nsync);
+  if (nsync > 32) bar_arrive(6, nsync);
+  bar_wait(2, 64);
   each8<8>(step);
-  bar_wait(3, nsync);
+  if (nsync > 32) bar_arrive(7, nsync);
+  bar_wait(3, 64);
   each8<16>(step);
-  bar_wait(4, nsync);
+  if (nsync > 32) bar_arrive(8, nsync);
+  bar_wait(4, 64);
   each8<24>(step);
+  if (nsync > 32) bar_arrive(9, nsync);
 }
 
-// Half of C = (add ? C : 0) + sign A B, 32 x 32 blocks: 16 columns (half 0 or
-// 1) by one warp, a lane 4 x 4.  C may be B.
-__device__ __noinline__ void diag_product(const float *A, const float *B, int ldb, float *C, float sign,
-                                          bool add, int half) {
-  constexpr int LD   = kDiagLD;
+// Half of a 32 x 32 block product: 16 columns (half 0 or 1) by one warp, a lane
+// 4 x 4.  kSub: C -= A B.  kFirst, kNext: C = A B, C += A B, one sum over both.
+// kNeg: C = -A B in four sums (terms k mod 4); C may be B.
+enum DiagMode { kSub, kFirst, kNext, kNeg };
+template <DiagMode MODE>
+__device__ __noinline__ void diag_product(const float *A, const float *B, int ldb, float *C, int half) {
+  constexpr int LD = kDiagLD, S = MODE == kNeg ? 4 : 1;
   const int     lane = threadIdx.x % 32, i0 = 4 * (lane / 4), j0 = 16 * half + 4 * (lane % 4);
-  float         acc[4][4] = {};
+  float         acc[S][4][4] = {};
   A += i0 * LD;
   B += j0;
   C += i0 * LD + j0;
+  if (MODE == kNext) {
+#pragma unroll
+    for (int r = 0; r < 4; r++) {
+      const float4 o = *reinterpret_cast<const float4 *>(C + r * LD);
+      acc[0][r][0] = o.x;
+      acc[0][r][1] = o.y;
+      acc[0][r][2] = o.z;
+      acc[0][r][3] = o.w;
+    }
+  }
 #pragma unroll 2
   for (int k = 0; k < 32; k += 4) {
     float4 b[4];
@@ -506,20 +527,29 @@ __device__ __noinline__ void diag_product(const float *A, const float *B, int ld
       const float  a[4] = {f.x, f.y, f.z, f.w};
 #pragma unroll
       for (int u = 0; u < 4; u++) {
-        acc[r][0] += a[u] * b[u].x;
-        acc[r][1] += a[u] * b[u].y;
-        acc[r][2] += a[u] * b[u].z;
-        acc[r][3] += a[u] * b[u].w;
+        acc[u % S][r][0] += a[u] * b[u].x;
+        acc[u % S][r][1] += a[u] * b[u].y;
+        acc[u % S][r][2] += a[u] * b[u].z;
+        acc[u % S][r][3] += a[u] * b[u].w;
       }
     }
   }
   __syncwarp();
 #pragma unroll
   for (int r = 0; r < 4; r++) {
-    float4 o = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    if (add) o = *reinterpret_cast<const float4 *>(C + r * LD);
-    store_quad(C + r * LD, o.x + sign * acc[r][0], o.y + sign * acc[r][1], o.z + sign * acc[r][2],
-               o.w + sign * acc[r][3]);
+    float o[4];
+#pragma unroll
+    for (int s = 0; s < 4; s++)
+      o[s] = MODE == kNeg ? -((acc[0][r][s] + acc[1 % S][r][s]) + (acc[2 % S][r][s] + acc[3 % S][r][s]))
+                          : acc[0][r][s];
+    if (MODE == kSub) {
+      const float4 c = *reinterpret_cast<const float4 *>(C + r * LD);
+      o[0] = c.x - o[0];
+      o[1] = c.y - o[1];
+      o[2] = c.z - o[2];
+      o[3] = c.w - o[3];
+    }
+    store_quad(C + r * LD, o[0], o[1], o[2], o[3]);
   }
 }
 
@@ -567,7 +597,6 @@ __global__ void __launch_bounds__(kDiagThreads)
   float          *Xs = Fs + kNB * LD;      // X, row-major
   float          *G2 = Xs + kNB * LD;      // G^T of two panels, by panel parity
   float          *Ld = G2 + 2 * 32 * kNB;  // L^T of the current diagonal block
-  __shared__ float dv_s[kNB];
   const StepDesc   d    = descs[blockIdx.x];
   const int        n    = d.nbk;
   const int        nblk = (n + 31) / 32, n32 = 32 * nblk;
@@ -595,20 +624,20 @@ __global__ void __launch_bounds__(kDiagThreads)
   __syncthreads();
   int npos = 0;
   for (int p = 0;; p++) {
-    const int c0 = 32 * p, rest = nblk - 1 - p, nsync = 32 * (2 + (rest + 1) / 2);
-    float    *Gt = G2 + (p & 1) * 32 * kNB;
+    const int c0 = 32 * p, rest = nblk - 1 - p, nsync = 32 * (1 + (rest + 1) / 2);
+    float    *Gt = G2 + (p & 1) * 32 * kNB, *Xpp = Xs + c0 * LD + c0;
     // A.
     if (warp == 0) {
-      diag_panel(Fs, Gt, Ld, dv_s, c0, nsync, n, d, D, Dinv, packd, packs, st, npos);
+      diag_panel(Fs, Gt, Ld, c0, n, d, D, Dinv, packd, packs, st, npos);
     } else if (warp == 1) {
       if (rest >= 2)
-        diag_rows<2>(Fs, Gt, dv_s, c0, nsync, c0 + 32 + lane);
+        diag_rows<2>(Fs, Gt, Xpp, c0, nsync, c0 + 32 + lane);
       else if (rest == 1)
-        diag_rows<1>(Fs, Gt, dv_s, c0, nsync, c0 + 32 + lane);
+        diag_rows<1>(Fs, Gt, Xpp, c0, nsync, c0 + 32 + lane);
     } else if (warp == 2) {
-      if (rest == 3) diag_rows<1>(Fs, Gt, dv_s, c0, nsync, c0 + 96 + lane);
+      if (rest == 3) diag_rows<1>(Fs, Gt, Xpp, c0, nsync, c0 + 96 + lane);
     } else if (warp == 3) {
-      diag_inverse(Xs + c0 * LD + c0, Ld, nsync);
+      diag_inverse(Xpp, Ld, nsync);
     } else {
       const int u = warp - 4, half = u % 2;
       if (p == 0) {
@@ -626,23 +655,23 @@ __global__ void __launch_bounds__(kDiagThreads)
         const float *Lq = Fs + 32 * q;  // L_{.,q}
         if (w < q) {
           float *X = Xs + 32 * q * LD + 32 * w;
-          diag_product(Xs + 32 * q * LD + 32 * q, X, LD, X, -1.0f, false, half);
+          diag_product<kNeg>(Xs + 32 * q * LD + 32 * q, X, LD, X, half);
         } else if (w < q + nd) {
           const int e = w - q, i = p + 1 + (e >= 1) + (e >= 3), j = p + 1 + e - (i - p - 1) * (i - p) / 2;
-          diag_product(Lq + 32 * i * LD, G2 + (q & 1) * 32 * kNB + 32 * j, kNB, Fs + 32 * i * LD + 32 * j,
-                       -1.0f, true, half);
+          diag_product<kSub>(Lq + 32 * i * LD, G2 + (q & 1) * 32 * kNB + 32 * j, kNB,
+                             Fs + 32 * i * LD + 32 * j, half);
         } else if (w < q + nd + rest + 1) {
           const int i = p + w - q - nd;
-          diag_product(Lq + 32 * i * LD, Xs + 32 * q * LD + 32 * q, LD, Xs + 32 * i * LD + 32 * q, 1.0f,
-                       false, half);
+          diag_product<kFirst>(Lq + 32 * i * LD, Xs + 32 * q * LD + 32 * q, LD, Xs + 32 * i * LD + 32 * q,
+                               half);
         }
         diag_store_panel(P, h, n, nblk, Fs, q, 11 - u, 12);
         bar_wait(5, 384);
         const int e = 5 - w;
         if (e < q * (rest + 1)) {
           const int i = p + e / q, b = e % q;
-          diag_product(Lq + 32 * i * LD, Xs + 32 * q * LD + 32 * b, LD, Xs + 32 * i * LD + 32 * b, 1.0f, true,
-                       half);
+          diag_product<kNext>(Lq + 32 * i * LD, Xs + 32 * q * LD + 32 * b, LD, Xs + 32 * i * LD + 32 * b,
+                              half);
         }
         diag_store_x(Lv, n, n32, Xs, q, u, 12);
       }
@@ -652,7 +681,7 @@ __global__ void __launch_bounds__(kDiagThreads)
     // B.
     if (warp < 2 * rest) {
       const int i = c0 + 32 + 32 * (warp / 2);
-      diag_product(Fs + i * LD + c0, Gt + c0 + 32, kNB, Fs + i * LD + c0 + 32, -1.0f, true, warp % 2);
+      diag_product<kSub>(Fs + i * LD + c0, Gt + c0 + 32, kNB, Fs + i * LD + c0 + 32, warp % 2);
     }
     __syncthreads();
   }
@@ -663,7 +692,7 @@ __global__ void __launch_bounds__(kDiagThreads)
   const int last = nblk - 1;
   if (warp < 2 * last) {
     float *X = Xs + 32 * last * LD + 32 * (warp / 2);
-    diag_product(Xs + 32 * last * LD + 32 * last, X, LD, X, -1.0f, false, warp % 2);
+    diag_product<kNeg>(Xs + 32 * last * LD + 32 * last, X, LD, X, warp % 2);
   }
   __syncthreads();
   diag_store_panel(P, h, n, nblk, Fs, last, warp, kDiagThreads / 32);
