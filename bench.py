@@ -593,8 +593,8 @@ def roofline_from_classes(info, kt, applies, uf, grid=None):
     dom_s = cls_ms[dom] / 1e3
     achieved = amount / dom_s if dom_s > 0 else float("nan")
     names = {"trailing_update": "k_gemm_tc (tensor-core updates) + k_split_reduce",
-             "solve_forward": "k_fwd_fronts / k_fwd_small",
-             "solve_backward": "k_bwd_fronts / k_bwd_chunks / k_bwd_small"}
+             "solve_forward": "k_fwd_flow",
+             "solve_backward": "k_bwd_flow"}
     solve_ms = cls_ms.get("solve_forward", 0) + cls_ms.get("solve_backward", 0)
     solve_gbs = (2 * applies * info["panel_read_bytes"] / 1e9) / (solve_ms / 1e3) if solve_ms else None
     return {"bound": bound, "kernel": names.get(dom, dom), "class": dom, "achieved": achieved,

@@ -1,8 +1,8 @@
 // GMRES-IR on the device: GmresLDLIR::Solve (gmres_ir.hpp:536-634) and
 // PrecondGmres (gmres_ir.hpp:636-741) with the supernodal LDL^T factor as the
 // left preconditioner.  Vectors and the Arnoldi basis are float64 in the
-// permuted order; the host keeps the small Hessenberg least-squares problem
-// and its Givens rotations, reading back one column of H per inner step.
+// permuted order; the inner steps run on the device (arnoldi.cu), the
+// refinement's stop tests on the host.
 #include <cfloat>
 #include <chrono>
 #include <cstdio>

@@ -21,31 +21,22 @@ __device__ __forceinline__ void cp_async8(double *dst, const double *src) {
                    static_cast<uint32_t>(__cvta_generic_to_shared(dst))),
                "l"(src) : "memory");
 }
-__device__ __forceinline__ void cp_async16(double *dst, const double *src) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(
-                   static_cast<uint32_t>(__cvta_generic_to_shared(dst))),
-               "l"(src) : "memory");
-}
 __device__ __forceinline__ void cp_async_wait_all() {
   asm volatile("cp.async.wait_all;" ::: "memory");
 }
 
-// Block results go from the CTA that computes them to the CTAs that wait on
-// them through the ready buffer: each entry holds the pending marker (a
-// signalling NaN, which no arithmetic produces) until its value is stored,
-// and a waiting lane polls its own entry at GPU scope, so the value is its
-// own ready signal (no flag, no fence, no second load).  The producer stores
-// kReadyCopies copies; the warps of the ~150 CTAs that wait for the same
-// block poll different copies.  A wait gives up after a bounded number of
-// polls (about a second by default), sets the sticky error word and returns
-// 0; it looks at that word every 64 polls, so one failure ends the launch
-// quickly.
+// Values go from the CTA that computes them to the CTAs that wait on them
+// through memory that holds the pending marker (a signalling NaN, which no
+// arithmetic produces) until a value is stored: a waiting lane polls its own
+// entry at GPU scope, so the value is its own ready signal (no flag, no fence,
+// no second load).  A wait gives up after a bounded number of polls (about a
+// second by default), sets the sticky error word and returns 0; it looks at
+// that word every 64 polls, so one failure ends the launch quickly.
 //
 // The control words beside the error word (SolveCtl) let a test make a wait
 // run out on purpose: a smaller poll limit, and one work item whose block
 // result is never published.  Both are read once per CTA with its ticket.
 constexpr unsigned long long kPending = 0x7ff0deadbeef0001ull;
-constexpr int kReadyCopies = 16;
 constexpr long kDefaultPolls = 1L << 22;
 struct SolveCtl {
   int32_t err;        // sticky: 1 once a bounded wait gave up
