@@ -498,14 +498,11 @@ ArnoldiArgs make_args(int64_t n, int64_t m, int64_t stride, double *V, int64_t b
   return ArnoldiArgs{n, m, n, block, stride, V, state, tol, mail};
 }
 
-void allow_16() {
-  static const bool done = [] {
-    for (auto *f : {reinterpret_cast<const void *>(k_gmres_begin), reinterpret_cast<const void *>(k_gmres_first),
-                    reinterpret_cast<const void *>(k_gmres_step), reinterpret_cast<const void *>(k_gmres_end)})
-      MPIR_CUDA(cudaFuncSetAttribute(f, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-    return true;
-  }();
-  (void)done;
+// Clusters of more than 8 CTAs have to be allowed, on each device.
+void allow_large_clusters() {
+  for (auto *f : {reinterpret_cast<const void *>(k_gmres_begin), reinterpret_cast<const void *>(k_gmres_first),
+                  reinterpret_cast<const void *>(k_gmres_step), reinterpret_cast<const void *>(k_gmres_end)})
+    MPIR_CUDA(cudaFuncSetAttribute(f, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
 }
 
 }  // namespace
@@ -519,6 +516,7 @@ void Arnoldi::allocate(int64_t n, int64_t m, int vectors) {
   m_       = m;
   vectors_ = vectors;
   state_.resize(bytes_for(m, vectors));
+  if (cluster() > 8) allow_large_clusters();
   if (!mail_) mail_ = static_cast<GmresMail *>(pinned_alloc(sizeof(GmresMail)));
 }
 
@@ -535,7 +533,6 @@ int Arnoldi::cluster() const {
 
 void Arnoldi::begin(int nb, uint32_t act, const double *b, const VecFactors &fac, double *V, double tol,
                     cudaStream_t s) {
-  allow_16();
   launch_chained(n_, k_gmres_begin, cluster(), dim3(cluster(), nb, 1), kThreads, 0, s,
                  make_args(n_, m_, stride(m_), V, 0, state_.as<double>(), tol, mail_), act, b, fac);
 }
