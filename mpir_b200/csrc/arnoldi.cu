@@ -68,9 +68,21 @@ __device__ __forceinline__ uint32_t cluster_size() {
   asm("mov.u32 %0, %%cluster_nctarank;" : "=r"(r));
   return r;
 }
+// (Not the .aligned forms: a warp's lanes may come here from a loop that they
+// left at different turns.)
 __device__ __forceinline__ void cluster_sync() {
-  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+  asm volatile("barrier.cluster.arrive.release;" ::: "memory");
+  asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+}
+// A CTA's shared memory exists for the others of its cluster only once it is
+// known to have started: arrive at the start, wait before the first
+// cluster_put (the vectors' first loads lie in between).  Nothing is handed
+// over, so the arrival orders no memory.
+__device__ __forceinline__ void cluster_arrive() {
+  if (cluster_size() > 1) asm volatile("barrier.cluster.arrive.relaxed;" ::: "memory");
+}
+__device__ __forceinline__ void cluster_wait() {
+  if (cluster_size() > 1) asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
 }
 // One double into CTA `rank`'s copy of a shared variable.
 __device__ __forceinline__ void cluster_put(double *p, uint32_t rank, double v) {
@@ -204,6 +216,7 @@ __global__ void __launch_bounds__(kThreads)
     }
     return;
   }
+  cluster_arrive();
   const Spread  sp(a.n);
   const double  f  = fac.v[vec];
   const double *bv = b + vec * a.vs;
@@ -220,6 +233,7 @@ __global__ void __launch_bounds__(kThreads)
     w0[i]          = x;
     ss += x * x;
   });
+  cluster_wait();
   Reducer<false>{S, turn}.run(ss, none);
   const double rho = safe_norm(ss, sp, w, w0, S, turn);
   if (lead) {
@@ -237,12 +251,14 @@ __global__ void __launch_bounds__(kThreads) k_gmres_first(const ArnoldiArgs a) {
   const int            vec  = blockIdx.y;
   StateView            st(a, vec);
   if (st.ctl->active == 0) return;
+  cluster_arrive();
   const Spread sp(a.n);
   double      *w0 = a.V + vec * a.vs, w[kRegs], ss = 0.0, none = 0.0;
   sp.load(w, w0);
 #pragma unroll
   for (int j = 0; j < kRegs; j++) ss += w[j] * w[j];
   sp.rest([&](int64_t i) { ss += w0[i] * w0[i]; });
+  cluster_wait();
   Reducer<false>{S, turn}.run(ss, none);
   const double rho = safe_norm(ss, sp, w, w0, S, turn), f = 1 / rho;
   sp.regs([&](int j, int64_t i) { w0[i] = w[j] * f; });
@@ -270,6 +286,7 @@ __global__ void __launch_bounds__(kThreads) k_gmres_step(const ArnoldiArgs a, in
     if (lead) a.mail->active[k & 1][vec] = 0;
     return;
   }
+  cluster_arrive();
   const Spread sp(a.n);
   double      *V = a.V + vec * a.vs, *wg = V + (k + 1) * a.block;
   double       w[kRegs], v[kRegs];
@@ -285,6 +302,7 @@ __global__ void __launch_bounds__(kThreads) k_gmres_step(const ArnoldiArgs a, in
     ss += wg[i] * wg[i];
     h += wg[i] * V[i];
   });
+  cluster_wait();
   Reducer<false>{S, turn}.run(ss, h);
   const double normav = safe_norm(ss, sp, w, wg, S, turn);
   double       normw  = 0.0;
