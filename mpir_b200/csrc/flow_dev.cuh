@@ -96,7 +96,10 @@ __device__ __forceinline__ bool flow_idle(const FlowArgs<T> &a) {
 }
 
 // The kernels' common loop: work(this slot, the next one) for every item.
-template <class T, class Work>
+// kStores: an item's ordinary stores may lie where the next one's bulk copies
+// go.  Those copies are of the async proxy, which a barrier alone does not
+// order after the stores.
+template <bool kStores, class T, class Work>
 __device__ __forceinline__ void flow_loop(const FlowArgs<T> &a, FlowShared &S, Work work) {
   if (threadIdx.x <= kFlowWarpsPerItem) {
     const uint32_t b = smem_addr(threadIdx.x == 0 ? &S.bar : &S.wbar[threadIdx.x - 1]);
@@ -109,6 +112,7 @@ __device__ __forceinline__ void flow_loop(const FlowArgs<T> &a, FlowShared &S, W
   for (int k = 0; S.slot[k & 1].ticket < a.nitems; k++) {
     work(S.slot[k & 1], S.slot[(k + 1) & 1]);
     cp_async_wait_all();
+    if (kStores) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     __syncthreads();
   }
 }

@@ -46,7 +46,8 @@
 
 namespace mpir {
 
-// Shared memory (doubles): kFlowInvSmem, then 4,608 for vectors and partial sums.
+// Shared memory (doubles): kFlowInvSmem, written by bulk copies only, then 4,608
+// for vectors and partial sums.
 constexpr int kFlowSmem = kFlowInvSmem + 4608;
 
 __global__ void k_mark_pending(int64_t n, double *p) {
@@ -401,7 +402,7 @@ __global__ void __launch_bounds__(kFlowThreads, 1) k_fwd_flow(const __grid_const
   __shared__ __align__(16) FlowShared S;
   uint32_t phase = 0, wphase = 0;
   if (flow_idle(a)) return;
-  flow_loop(a, S, [&](const FlowSlot &I, FlowSlot &N) {
+  flow_loop<false>(a, S, [&](const FlowSlot &I, FlowSlot &N) {
     switch (I.item.kind) {
       case kFlowWarps: fwd_warp(a, S, I, N, sm, wphase); break;
       case kFwdNarrow:
@@ -750,7 +751,7 @@ __global__ void __launch_bounds__(kFlowThreads, 1) k_bwd_flow(const __grid_const
   __shared__ __align__(16) FlowShared S;
   uint32_t phase = 0, wphase = 0;
   if (flow_idle(a)) return;
-  flow_loop(a, S, [&](const FlowSlot &I, FlowSlot &N) {
+  flow_loop<false>(a, S, [&](const FlowSlot &I, FlowSlot &N) {
     switch (I.item.kind) {
       case kFlowWarps: bwd_warp(a, S, I, N, sm, wphase); break;
       case kBwdChunk: bwd_chunk(a, I, N, sm); break;

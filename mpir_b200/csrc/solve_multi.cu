@@ -635,7 +635,7 @@ __global__ void __launch_bounds__(kFlowThreads, 1) k_fwd_flow_m(const __grid_con
   __shared__ __align__(16) FlowShared S;
   uint32_t phase = 0, wphase = 0;
   if (flow_idle(a)) return;
-  flow_loop(a, S, [&](const FlowSlot &I, FlowSlot &N) {
+  flow_loop<true>(a, S, [&](const FlowSlot &I, FlowSlot &N) {
     switch (I.item.kind) {
       case kFlowWarps: fwd_warp_m<NR>(a, S, I, N, sm, wphase); break;
       case kFwdNarrow:
@@ -999,7 +999,7 @@ __global__ void __launch_bounds__(kFlowThreads, 1) k_bwd_flow_m(const __grid_con
   __shared__ __align__(16) FlowShared S;
   uint32_t phase = 0, wphase = 0;
   if (flow_idle(a)) return;
-  flow_loop(a, S, [&](const FlowSlot &I, FlowSlot &N) {
+  flow_loop<true>(a, S, [&](const FlowSlot &I, FlowSlot &N) {
     switch (I.item.kind) {
       case kFlowWarps: bwd_warp_m<NR>(a, S, I, N, sm, wphase); break;
       case kBwdChunk: bwd_chunk_m<NR>(a, I, N, sm); break;

@@ -2,7 +2,9 @@
 
 Shared memory of another block of a cluster may be written only after a cluster
 barrier has shown that the block has started (CUDA programming guide,
-distributed shared memory)."""
+distributed shared memory).  Bulk copies write shared memory through the async
+proxy: ordinary stores to the same bytes come before them only with a proxy
+fence by the storing threads (PTX ISA, async proxy)."""
 import os
 import re
 
@@ -36,3 +38,21 @@ def test_cluster_stores_follow_a_barrier():
         first = min(m.start() for m in re.finditer(r"Reducer<|cluster_put\(|safe_norm\(", body))
         before = body[:first]
         assert re.search(r"cluster_sync\(\)|cluster_arrive\(\)[\s\S]*cluster_wait\(\)", before), name
+
+
+def test_bulk_copies_follow_a_proxy_fence():
+    """The several-vector solves store vectors and partial sums inside the area of the
+    inverse blocks; the single-vector ones keep theirs behind it (then no fence is needed)."""
+    (_, loop), = _bodies(_source("flow_dev.cuh"), r"\b(flow_loop)\(")
+    body = loop[loop.index("work("):]
+    assert re.search(r"if \(kStores\) asm volatile\(\"fence\.proxy\.async\.shared::cta;\"[^;]*;[^;]*"
+                     r"__syncthreads\(\)", body)
+    for name, head, kinds in (("solve_multi.cu", r"\b(k_(?:fwd|bwd)_flow_m)\(const", {"true"}),
+                              ("solve.cu", r"\b(k_(?:fwd|bwd)_flow)\(const", {"false"})):
+        kernels = _bodies(_source(name), head)
+        assert len(kernels) == 2
+        assert {re.search(r"flow_loop<(\w+)>", b).group(1) for _, b in kernels} == kinds
+    single = _source("solve.cu")
+    stored = re.findall(r"\*\s*(\w+)\s*=\s*sm(\s*\+\s*kFlowInvSmem)?", single)
+    assert stored and all(at or v == "inv" for v, at in stored)
+    assert not re.search(r"\b(?:inv|blk|M)\[[^\]]*\]\s*[-+]?=[^=]", single[:single.index("k_flow_invert(")])
