@@ -3,8 +3,11 @@
 #include <cuda_runtime.h>
 
 #include <cstdint>
+#include <initializer_list>
 #include <stdexcept>
 #include <string>
+
+#include "per_device.hpp"
 
 namespace mpir {
 
@@ -22,6 +25,17 @@ struct CudaError : std::runtime_error {
   } while (0)
 
 #define MPIR_CHECK_LAUNCH() MPIR_CUDA(cudaGetLastError())
+
+// Allows the kernels `bytes` of dynamic shared memory on the current device (the
+// attribute belongs to a kernel on one device).
+inline void allow_smem(OncePerDevice &once, int bytes, std::initializer_list<const void *> kernels) {
+  int d = 0;
+  MPIR_CUDA(cudaGetDevice(&d));
+  once.run(d, [&] {
+    for (const void *k : kernels)
+      MPIR_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+  });
+}
 
 // Host-side count of kernel launches issued by this library (read by the
 // benchmark for its launch figure); safe from several host threads.  While a

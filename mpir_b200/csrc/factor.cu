@@ -1619,20 +1619,11 @@ void Numeric::run(const Plan &P, const double *d_Ax, double eps, cudaStream_t s)
     return e != nullptr && std::string(e) == "simt";
   }();
   const bool trsm_tc = update_mode >= 0 && !trsm_simt_env;
-  static std::atomic<bool> trsm_attr{false};
-  const int     trsm_smem = kBM * (kBN + 1) * sizeof(float);
-  if (!trsm_attr) {
-    MPIR_CUDA(cudaFuncSetAttribute(k_step_gemm<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   trsm_smem));
-    trsm_attr = true;
-  }
-  static std::atomic<bool> diag_attr{false};
-  const int     diag_smem = kDiagSmemFloats * sizeof(float);
-  if (!diag_attr) {
-    MPIR_CUDA(cudaFuncSetAttribute(k_diag_block, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   diag_smem));
-    diag_attr = true;
-  }
+  static OncePerDevice trsm_attr, diag_attr;
+  const int            trsm_smem = kBM * (kBN + 1) * sizeof(float);
+  const int            diag_smem = kDiagSmemFloats * sizeof(float);
+  allow_smem(trsm_attr, trsm_smem, {reinterpret_cast<const void *>(k_step_gemm<true>)});
+  allow_smem(diag_attr, diag_smem, {reinterpret_cast<const void *>(k_diag_block)});
   // Float64 inverses of the diagonal blocks for the triangular solves.  In a
   // recorded graph those below the last level form a branch of their own beside
   // it (its fronts are few and leave most of the chip idle; in a stream all of

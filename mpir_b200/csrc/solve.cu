@@ -958,13 +958,9 @@ static void ldlt_solve_t(const Plan &P, const Numeric &F, const T *pan, double *
   a.active        = act.p;
   a.nactive       = act.count;
   a.active_stride = act.stride;
-  static std::atomic<bool> attr{false};
-  constexpr int            smem = kFlowSmem * sizeof(double);
-  if (!attr) {
-    MPIR_CUDA(cudaFuncSetAttribute(k_fwd_flow<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    MPIR_CUDA(cudaFuncSetAttribute(k_bwd_flow<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    attr = true;
-  }
+  static OncePerDevice attr;
+  constexpr int        smem = kFlowSmem * sizeof(double);
+  allow_smem(attr, smem, {reinterpret_cast<const void *>(k_fwd_flow<T>), reinterpret_cast<const void *>(k_bwd_flow<T>)});
   kt.begin(kKcSolveFwd, s);
   if (phases & kForward) {
     if (!ws.fwd_pending) flow_pending(fv, b.fwd, s);

@@ -27,7 +27,6 @@
 // n = 40,951: 0.44 ms (1.50; 0.44), for which half of each product is unused.
 // Per vector the sums inside an item run in another order than in the
 // single-vector kernels, so results agree with NR single solves to rounding.
-#include <atomic>
 #include <algorithm>
 #include <type_traits>
 
@@ -1046,13 +1045,10 @@ void solve_multi_nr(const Plan &P, const Numeric &F, const T *pan, double *X,
   a.active        = act.p;
   a.nactive       = act.count;
   a.active_stride = act.stride;
-  static std::atomic<bool> attr{false};  // idempotent; set once per process
-  constexpr int            smem = kMultiSmem * sizeof(double);
-  if (!attr) {
-    MPIR_CUDA(cudaFuncSetAttribute(k_fwd_flow_m<NR, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    MPIR_CUDA(cudaFuncSetAttribute(k_bwd_flow_m<NR, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    attr = true;
-  }
+  static OncePerDevice attr;
+  constexpr int        smem = kMultiSmem * sizeof(double);
+  allow_smem(attr, smem,
+             {reinterpret_cast<const void *>(k_fwd_flow_m<NR, T>), reinterpret_cast<const void *>(k_bwd_flow_m<NR, T>)});
   kt.begin(kKcSolveFwd, s);
   if (!ws.fwd_pending) flow_pending(fv, NR * b.fwd, s);
   a.items  = P.flow_fwd.as<FlowItem>();

@@ -35,7 +35,6 @@
 // Every mbarrier wait is bounded; on expiry the kernel records a timeout in
 // the factor status, stops issuing work, waits (bounded) for its own copies
 // and MMAs, frees its tensor memory and returns.
-#include <atomic>
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
@@ -867,12 +866,8 @@ __global__ void __launch_bounds__(256, 1)
 void launch_trsm_tc(const StepDesc *descs, int ndesc, int tiles, float *panel, const float *linv,
                     const float *Dinv, float *pack, FactorStatus *st, cudaStream_t s) {
   if (tiles <= 0) return;
-  static std::atomic<bool> attr{false};
-  if (!attr) {
-    MPIR_CUDA(cudaFuncSetAttribute(k_trsm_tc, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   static_cast<int>(tc::kTrsmSmem)));
-    attr = true;
-  }
+  static OncePerDevice attr;
+  allow_smem(attr, static_cast<int>(tc::kTrsmSmem), {reinterpret_cast<const void *>(k_trsm_tc)});
   launch(k_trsm_tc, tiles, 256, tc::kTrsmSmem, s, descs, ndesc, panel, linv, Dinv, pack, st);
 }
 
@@ -881,13 +876,9 @@ static void launch_mode(const GemmProb *probs, int nprob, int units, const float
                         const float *packd, const float *packs, const float *bconv,
                         float *panel, float *uarena, float *ws, FactorStatus *st,
                         cudaStream_t s) {
-  static std::atomic<bool> attr{false};
-  const int   smem = tc_gemm_smem_bytes(MODE);
-  if (!attr) {
-    MPIR_CUDA(cudaFuncSetAttribute(k_gemm_tc<MODE>,
-                                   cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    attr = true;
-  }
+  static OncePerDevice attr;
+  const int            smem = tc_gemm_smem_bytes(MODE);
+  allow_smem(attr, smem, {reinterpret_cast<const void *>(k_gemm_tc<MODE>)});
   const int grid = std::min(units, kSMs * tc_ctas_per_sm());
   launch(k_gemm_tc<MODE>, grid, tc::kThreads, smem, s, probs, nprob, units, pack, packd, packs,
          MODE == 1 ? bconv : nullptr, panel, uarena, ws, st);
