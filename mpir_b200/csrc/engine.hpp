@@ -163,8 +163,8 @@ class Plan {
     std::vector<FlowFront>   flow_warp;
     std::vector<FlowItem>    flow_fwd, flow_bwd;
     std::vector<FlowInvDesc> flow_inv;
-    std::vector<int2>        flow_gfirst;
-    std::vector<int32_t>     flow_gmore;
+    std::vector<FlowGather>  flow_gfirst;
+    std::vector<uint32_t>    flow_gmore;
   } host_;
   bool is_large(int64_t J) const { return S.h(J) > kSmallFront; }
   // Packed-front geometry (PackedFront): first packed row of the

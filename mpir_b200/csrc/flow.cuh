@@ -1,8 +1,27 @@
 // Tables and device helpers of the dataflow triangular solves (solve.cu).
 #pragma once
 #include <cstdint>
+#include <stdexcept>
 
 namespace mpir {
+
+// Entries of the front vectors are numbered in 32 bits without a sign (half of
+// what 64 would have a row's gather read); kFlowNone is no entry.  2^32 of them
+// do not fit the device: an entry takes 24 bytes in the front vectors, FlowGather
+// and the row indices and 12 a column in the float32 and float64 panels, and a
+// front has two columns (merged with its last child, at least) or is a leaf, whose
+// entries are the matrix's, at 88 bytes each: 206 GB of 192.
+constexpr uint32_t kFlowNone = 0xffffffffu;
+inline uint32_t    flow_entry(int64_t i) {
+  if (i < 0 || i >= static_cast<int64_t>(kFlowNone))
+    throw std::invalid_argument("front vectors of more than 2^32 entries");
+  return static_cast<uint32_t>(i);
+}
+// A row's child contributions: the first one's entry, and where the others lie
+// in the list of further ones (their number, then their entries).
+struct alignas(8) FlowGather {
+  uint32_t first, more;
+};
 
 // One front in the triangular solves.
 struct FlowFront {

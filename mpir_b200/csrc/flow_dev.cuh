@@ -23,8 +23,8 @@ struct FlowArgs {
   const FlowFront *warps;
   const T         *panel;
   const double    *inv, *wpanel;
-  const int2      *gfirst;
-  const int32_t   *gmore;
+  const FlowGather *gfirst;
+  const uint32_t   *gmore;
   const int32_t   *srows;
   const float     *Dinv;  // backward: f .* Dinv is its right-hand side (NULL: f)
   int64_t          n;
@@ -160,45 +160,46 @@ __device__ __forceinline__ double take_value(unsigned long long raw, const doubl
 // NR vectors are at NR i; z points at the vector's own of entry 0.
 template <int NR>
 struct Gather {
-  int2               g = {-1, -1};
+  FlowGather         g = {kFlowNone, kFlowNone};
   unsigned long long r0 = 0;
   template <class T>
   __device__ __forceinline__ void begin(const FlowArgs<T> &a, int64_t row, const double *z) {
     g = a.gfirst[row];
-    if (g.x >= 0) r0 = ld_relaxed_u64(z + static_cast<int64_t>(NR) * g.x);
+    if (g.first != kFlowNone) r0 = ld_relaxed_u64(z + static_cast<int64_t>(NR) * g.first);
   }
   template <class T>
   __device__ __forceinline__ double finish(const FlowArgs<T> &a, const double *z, double zr,
                                            long polls) {
-    if (g.x >= 0) zr += take_value(r0, z + static_cast<int64_t>(NR) * g.x, a.err, polls);
-    if (g.y < 0) return zr;
-    const int32_t *m = a.gmore + g.y + 1;
-    const int      n = m[-1];
-    for (int q = 0; q < n; q += 4) {
-      int                idx[4];
+    if (g.first != kFlowNone)
+      zr += take_value(r0, z + static_cast<int64_t>(NR) * g.first, a.err, polls);
+    if (g.more == kFlowNone) return zr;
+    const uint32_t *m = a.gmore + g.more + 1;
+    const uint32_t  n = m[-1];
+    for (uint32_t q = 0; q < n; q += 4) {
+      uint32_t           idx[4];
       unsigned long long raw[4];
 #pragma unroll
-      for (int u = 0; u < 4; u++) idx[u] = q + u < n ? m[q + u] : -1;
+      for (int u = 0; u < 4; u++) idx[u] = q + u < n ? m[q + u] : kFlowNone;
 #pragma unroll
       for (int u = 0; u < 4; u++)
-        raw[u] = idx[u] >= 0 ? ld_relaxed_u64(z + static_cast<int64_t>(NR) * idx[u]) : 0ull;
+        raw[u] = idx[u] != kFlowNone ? ld_relaxed_u64(z + static_cast<int64_t>(NR) * idx[u]) : 0ull;
 #pragma unroll
       for (int u = 0; u < 4; u++)
-        if (idx[u] >= 0)
+        if (idx[u] != kFlowNone)
           zr += take_value(raw[u], z + static_cast<int64_t>(NR) * idx[u], a.err, polls);
     }
     return zr;
   }
 };
 
-// z[t] += the value at v + ix[t] (ix < 0: none), all of them polled together.
+// z[t] += the value at v + ix[t] (kFlowNone: none), all of them polled together.
 template <int K>
-__device__ __forceinline__ void add_values(const double *v, const int (&ix)[K], double (&z)[K],
+__device__ __forceinline__ void add_values(const double *v, const uint32_t (&ix)[K], double (&z)[K],
                                            int32_t *err, long polls) {
   unsigned need = 0;
 #pragma unroll
   for (int t = 0; t < K; t++)
-    if (ix[t] >= 0) need |= 1u << t;
+    if (ix[t] != kFlowNone) need |= 1u << t;
   for (long it = 0; need != 0; it++) {
     unsigned long long raw[K];
 #pragma unroll
@@ -259,7 +260,7 @@ __device__ __forceinline__ void load_rows(float (&d)[2][16], const T *P, int64_t
 // that alone: all lanes polling their own entries from the start took enough
 // of L2 to triple the time of a level (n = 1,280: 12 to 16 us a level).
 template <class T>
-__device__ __forceinline__ void wait_gate(const FlowArgs<T> &a, int gate, long polls) {
+__device__ __forceinline__ void wait_gate(const FlowArgs<T> &a, int64_t gate, long polls) {
   if (gate >= 0 && threadIdx.x % 32 == 0) wait_value(a.xr + gate, a.err, polls);
   __syncwarp();
 }

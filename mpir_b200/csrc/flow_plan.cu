@@ -18,11 +18,9 @@ void Plan::build_flow() {
   // Child contributions of every front's rows (row i of front J at zofs[J] + i):
   // the first child's beside the row, the others' after their count, in child
   // order (the forward solves add them in this order).
-  // (The entries of the solve workspace are counted in 32 bits: 2^31 of them
-  // are 17 GB of front vectors, of systems whose fronts would not fit.)
-  if (S.z_elems > INT32_MAX) throw std::invalid_argument("front vectors of more than 2^31 entries");
-  std::vector<int32_t> more, cnt, src;
-  std::vector<int2>    first(S.z_elems, int2{-1, -1});
+  flow_entry(S.z_elems);
+  std::vector<uint32_t>   more, cnt, src;
+  std::vector<FlowGather> first(S.z_elems, FlowGather{kFlowNone, kFlowNone});
   for (int64_t J = 0; J < ns; J++) {
     const int64_t h = S.h(J);
     cnt.assign(h + 1, 0);
@@ -35,15 +33,15 @@ void Plan::build_flow() {
     for (int64_t c = S.child_ptr[J]; c < S.child_ptr[J + 1]; c++) {
       const int64_t C = S.child_list[c], wc = S.w(C);
       for (int64_t a = wc; a < S.h(C); a++)
-        src[cnt[S.srel[S.srowptr[C] + a]]++] = static_cast<int32_t>(S.zofs[C] + a);
+        src[cnt[S.srel[S.srowptr[C] + a]]++] = flow_entry(S.zofs[C] + a);
     }
     // cnt[i] is now the end of row i
     for (int64_t i = 0; i < h; i++) {
-      const int32_t e = i > 0 ? cnt[i - 1] : 0, n = cnt[i] - e;
-      int2         &g = first[S.zofs[J] + i];
-      if (n > 0) g.x = src[e];
+      const uint32_t e = i > 0 ? cnt[i - 1] : 0, n = cnt[i] - e;
+      FlowGather    &g = first[S.zofs[J] + i];
+      if (n > 0) g.first = src[e];
       if (n > 1) {
-        g.y = static_cast<int32_t>(more.size());
+        g.more = flow_entry(static_cast<int64_t>(more.size()));
         more.push_back(n - 1);
         more.insert(more.end(), src.begin() + e + 1, src.begin() + e + n);
       }

@@ -337,32 +337,32 @@ __device__ __noinline__ void fwd_warp(const FlowArgs<T> &a, FlowShared &S, const
   const double   *M   = warp_panel(a, f, sm, bar) + lane;
   double         *zs  = sm + kFlowInvSmem + 64 * warp, *ys = zs + 32;
   constexpr int   RT = kWarpSolveH / 32;
-  int             ix[RT], more[RT];
+  uint32_t        ix[RT], more[RT];
   double          z[RT];
 #pragma unroll
   for (int t = 0; t < RT; t++) {
-    int2 g = {-1, -1};
+    FlowGather g = {kFlowNone, kFlowNone};
     if (lane + 32 * t < h) g = a.gfirst[f.zofs + lane + 32 * t];
-    ix[t]   = g.x;
-    more[t] = g.y;
+    ix[t]   = g.first;
+    more[t] = g.more;
     z[t]    = 0.0;
   }
   if (lane < w) z[0] = a.x[f.col0 + lane];
   flow_fetch(a, N);
   add_values<RT>(a.z, ix, z, a.err, polls);
   // the rows with further children: their lists, one entry of each at a time
-  int  n[RT];
-  bool any = false;
+  uint32_t n[RT];
+  bool     any = false;
 #pragma unroll
   for (int t = 0; t < RT; t++) {
-    n[t] = more[t] >= 0 ? a.gmore[more[t]] : 0;
+    n[t] = more[t] != kFlowNone ? a.gmore[more[t]] : 0;
     any |= n[t] > 0;
   }
-  for (int q = 0; __any_sync(0xffffffffu, any); q++) {
+  for (uint32_t q = 0; __any_sync(0xffffffffu, any); q++) {
     any = false;
 #pragma unroll
     for (int t = 0; t < RT; t++) {
-      ix[t] = q < n[t] ? a.gmore[more[t] + 1 + q] : -1;
+      ix[t] = q < n[t] ? a.gmore[static_cast<int64_t>(more[t]) + 1 + q] : kFlowNone;
       any |= q + 1 < n[t];
     }
     add_values<RT>(a.z, ix, z, a.err, polls);
@@ -697,11 +697,11 @@ __device__ __noinline__ void bwd_warp(const FlowArgs<T> &a, FlowShared &S, const
     if (a.Dinv) v *= static_cast<double>(a.Dinv[f.col0 + lane]);
   }
   {
-    int    gi[RT];
-    double xv[RT];
+    uint32_t gi[RT];
+    double   xv[RT];
 #pragma unroll
     for (int t = 0; t < RT; t++) {
-      gi[t] = lane + 32 * t < nr ? a.srows[f.rows + w + lane + 32 * t] : -1;
+      gi[t] = lane + 32 * t < nr ? static_cast<uint32_t>(a.srows[f.rows + w + lane + 32 * t]) : kFlowNone;
       xv[t] = 0.0;
     }
     flow_fetch(a, N);
@@ -942,8 +942,8 @@ static void ldlt_solve_t(const Plan &P, const Numeric &F, const T *pan, double *
   a.panel = pan;
   a.inv   = F.inv64.as<double>();
   a.wpanel = F.wpanel.as<double>();
-  a.gfirst = P.flow_gfirst.as<int2>();
-  a.gmore  = P.flow_gmore.as<int32_t>();
+  a.gfirst = P.flow_gfirst.as<FlowGather>();
+  a.gmore  = P.flow_gmore.as<uint32_t>();
   a.srows = P.srows.as<int32_t>();
   a.n     = n;
   a.x     = x;

@@ -489,11 +489,13 @@ __device__ __noinline__ void fwd_narrow_m(const FlowArgs<T> &a, FlowShared &S, c
         double u[NR];
 #pragma unroll
         for (int k = 0; k < NR; k++) u[k] = -out[NP * lane + k];
-        const int2 g = a.gfirst[f.zofs + r0 + rt];
-        add_entry<NR>(a.z + static_cast<int64_t>(NR) * g.x, g.x >= 0, u, a.err, polls);
-        if (g.y >= 0)
-          for (int e = 1, n = a.gmore[g.y]; e <= n; e++)
-            add_entry<NR>(a.z + static_cast<int64_t>(NR) * a.gmore[g.y + e], true, u, a.err, polls);
+        const FlowGather g = a.gfirst[f.zofs + r0 + rt];
+        add_entry<NR>(a.z + static_cast<int64_t>(NR) * g.first, g.first != kFlowNone, u, a.err, polls);
+        if (g.more != kFlowNone) {
+          const uint32_t *m = a.gmore + g.more;
+          for (uint32_t e = 1, n = m[0]; e <= n; e++)
+            add_entry<NR>(a.z + static_cast<int64_t>(NR) * m[e], true, u, a.err, polls);
+        }
         if (I.publish) {
           double *z = a.z + NR * (f.zofs + r0 + rt);
 #pragma unroll
@@ -551,14 +553,14 @@ __device__ __noinline__ void fwd_warp_m(const FlowArgs<T> &a, FlowShared &S, con
     const int       w = f.w, h = f.h, ld = h | 1;
     const double   *M = sm + f.part / 8 + lane;
     double          z[RT][2];
-    int2            g[RT];
+    FlowGather      g[RT];
     bool            more = false;
 #pragma unroll
     for (int t = 0; t < RT; t++) {
-      g[t] = make_int2(-1, -1);
+      g[t] = FlowGather{kFlowNone, kFlowNone};
       if (lane + 32 * t < h) g[t] = a.gfirst[f.zofs + lane + 32 * t];
       z[t][0] = z[t][1] = 0.0;
-      more |= g[t].y >= 0;
+      more |= g[t].more != kFlowNone;
     }
     if (lane < w) {
       z[0][0] = a.x[vg * a.n + f.col0 + lane];
@@ -568,13 +570,13 @@ __device__ __noinline__ void fwd_warp_m(const FlowArgs<T> &a, FlowShared &S, con
     unsigned need = 0;
 #pragma unroll
     for (int t = 0; t < RT; t++)
-      if (g[t].x >= 0) need |= 1u << t;
+      if (g[t].first != kFlowNone) need |= 1u << t;
     for (long it = 0; need != 0; it++) {
       V2 raw[RT];
 #pragma unroll
       for (int t = 0; t < RT; t++) {
         raw[t] = V2{kPending, kPending};
-        if (need >> t & 1u) raw[t] = ld_relaxed_2(a.z + static_cast<int64_t>(NR) * g[t].x + vg);
+        if (need >> t & 1u) raw[t] = ld_relaxed_2(a.z + static_cast<int64_t>(NR) * g[t].first + vg);
       }
 #pragma unroll
       for (int t = 0; t < RT; t++)
@@ -595,9 +597,11 @@ __device__ __noinline__ void fwd_warp_m(const FlowArgs<T> &a, FlowShared &S, con
     if (more) {
 #pragma unroll
       for (int t = 0; t < RT; t++)
-        if (g[t].y >= 0)
-          for (int e = 1, n = a.gmore[g[t].y]; e <= n; e++)
-            add_entry<2>(a.z + static_cast<int64_t>(NR) * a.gmore[g[t].y + e] + vg, true, z[t], a.err, polls);
+        if (g[t].more != kFlowNone) {
+          const uint32_t *m = a.gmore + g[t].more;
+          for (uint32_t e = 1, n = m[0]; e <= n; e++)
+            add_entry<2>(a.z + static_cast<int64_t>(NR) * m[e] + vg, true, z[t], a.err, polls);
+        }
     }
     put_entry<2>(zs + 2 * lane, z[0]);
     __syncwarp();
@@ -671,7 +675,7 @@ __device__ __forceinline__ void chunk_cols_m(const FlowArgs<T> &a, const FlowFro
   load_frag_t(lv, P, f.h, rb + rw, rb + nr, c, cend);
   flow_fetch(a, N);
   const int row = tid < nr ? a.srows[f.rows + rb + tid] : -1;
-  wait_gate(a, f.gate < 0 ? -1 : NR * f.gate, polls);
+  wait_gate(a, f.gate < 0 ? -1 : static_cast<int64_t>(NR) * f.gate, polls);
   get_entry<NR>(a.xr + static_cast<int64_t>(NR) * row, row >= 0, xs + NP * tid, a.err, polls);
   __syncthreads();
   Frag<NR> fr;
@@ -931,7 +935,7 @@ __device__ __noinline__ void bwd_warp_m(const FlowArgs<T> &a, FlowShared &S, con
         gi[t]    = lane + 32 * t < nr ? a.srows[f.rows + w + lane + 32 * t] : -1;
         xv[t][0] = xv[t][1] = 0.0;
       }
-      wait_gate(a, f.gate < 0 ? -1 : NR * f.gate, polls);
+      wait_gate(a, f.gate < 0 ? -1 : static_cast<int64_t>(NR) * f.gate, polls);
       unsigned need = 0;
 #pragma unroll
       for (int t = 0; t < RT; t++)
@@ -1029,8 +1033,8 @@ void solve_multi_nr(const Plan &P, const Numeric &F, const T *pan, double *X,
   a.panel  = pan;
   a.inv    = F.inv64.as<double>();
   a.wpanel = F.wpanel.as<double>();
-  a.gfirst = P.flow_gfirst.as<int2>();
-  a.gmore  = P.flow_gmore.as<int32_t>();
+  a.gfirst = P.flow_gfirst.as<FlowGather>();
+  a.gmore  = P.flow_gmore.as<uint32_t>();
   a.srows  = P.srows.as<int32_t>();
   a.n      = n;
   a.x      = X;
