@@ -409,8 +409,7 @@ __global__ void __launch_bounds__(kThreads)
                 unsigned long long *inf) {
   grid_wait();
   __shared__ RedShared S;
-  int                  turn = 0;
-  const int            vec  = blockIdx.y, tid = threadIdx.x;
+  const int            vec = blockIdx.y, tid = threadIdx.x;
   if (!(act >> vec & 1u)) return;
   StateView     st(a, vec);
   const int64_t k = st.ctl->k;
@@ -492,7 +491,6 @@ __global__ void __launch_bounds__(kThreads)
         cluster_put(&S.slot[0][cluster_rank()][1], 0, __longlong_as_double(static_cast<long long>(b1)));
       }
     }
-    (void)turn;
     if (cluster_size() > 1) cluster_sync();
     if (cluster_rank() == 0 && tid == 0) {
       if (cluster_size() > 1) {
@@ -530,9 +528,8 @@ Arnoldi::~Arnoldi() {
 }
 
 void Arnoldi::allocate(int64_t n, int64_t m, int vectors) {
-  n_       = n;
-  m_       = m;
-  vectors_ = vectors;
+  n_ = n;
+  m_ = m;
   state_.resize(bytes_for(m, vectors));
   if (cluster() > 8) allow_large_clusters();
   if (!mail_) mail_ = static_cast<GmresMail *>(pinned_alloc(sizeof(GmresMail)));

@@ -69,7 +69,6 @@ class Arnoldi {
   }
   int          cluster() const;
   int64_t      n_ = 0, m_ = 0;
-  int          vectors_ = 0;
   DeviceBuffer state_;
   GmresMail   *mail_ = nullptr;
 };

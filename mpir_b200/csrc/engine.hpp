@@ -120,10 +120,10 @@ class Plan {
   double                 update_flops = 0, trsm_flops = 0, panel_read_bytes = 0;
   // Pattern arrays on the device.
   DeviceBuffer amap, arow, acol, diag_pos, Kp, Kj, Ksrc;
-  DeviceBuffer sfirst, srowptr, srows, srel, slofs, uofs, zofs, child_ptr,
+  DeviceBuffer sfirst, srowptr, srows, srel, slofs, uofs, child_ptr,
       child_list, perm;
   DeviceBuffer ea_chunks, ea_hits;  // EaChunk / EaHit, see LevelPlan::ea_begin
-  DeviceBuffer small_list, large_list, steps, ea_tasks, gemm_probs;
+  DeviceBuffer small_list, steps, ea_tasks, gemm_probs;
   // Triangular solves (flow.cuh): warp-solved fronts, the work items of the two
   // directions, the strips of the block inverses, the rows' child contributions.
   DeviceBuffer flow_warp, flow_fwd, flow_bwd, flow_inv, flow_gfirst, flow_gmore;

@@ -1353,7 +1353,7 @@ size_t Plan::upload_bytes() const {
   auto b = [](const auto &v) { return v.size() * sizeof(v[0]); };
   return b(S.amap) + b(S.arow) + b(S.acol) + b(S.diag_pos) + b(S.Kp) + b(S.Kj) + b(S.Ksrc) +
          b(S.sfirst) + b(S.srowptr) + b(S.srows) + b(S.srel) + b(S.slofs) + b(S.uofs) +
-         b(S.zofs) + b(S.child_ptr) + b(S.child_list) + b(S.perm) + b(h_small) + b(h_large) +
+         b(S.child_ptr) + b(S.child_list) + b(S.perm) + b(h_small) +
          b(host_.descs) + b(host_.tasks) + b(host_.chunks) + b(host_.hits) + b(host_.probs) +
          b(host_.flow_warp) + b(host_.flow_fwd) + b(host_.flow_bwd) + b(host_.flow_inv) +
          b(host_.flow_gfirst) + b(host_.flow_gmore);
@@ -1374,12 +1374,10 @@ void Plan::upload_all(cudaStream_t s) {
   srel       = upload(S.srel, s);
   slofs      = upload(S.slofs, s);
   uofs       = upload(S.uofs, s);
-  zofs       = upload(S.zofs, s);
   child_ptr  = upload(S.child_ptr, s);
   child_list = upload(S.child_list, s);
   perm       = upload(S.perm, s);
   small_list = upload(h_small, s);
-  large_list = upload(h_large, s);
   steps      = upload(host_.descs, s);
   ea_tasks   = upload(host_.tasks, s);
   ea_chunks  = upload(host_.chunks, s);
@@ -1399,8 +1397,8 @@ void Plan::upload_all(cudaStream_t s) {
 void Plan::release_device() {
   for (DeviceBuffer *d :
        {&amap, &arow, &acol, &diag_pos, &Kp, &Kj, &Ksrc, &sfirst, &srowptr, &srows, &srel,
-        &slofs, &uofs, &zofs, &child_ptr, &child_list, &perm, &ea_chunks, &ea_hits, &small_list,
-        &large_list, &steps, &ea_tasks, &gemm_probs, &flow_warp, &flow_fwd,
+        &slofs, &uofs, &child_ptr, &child_list, &perm, &ea_chunks, &ea_hits, &small_list,
+        &steps, &ea_tasks, &gemm_probs, &flow_warp, &flow_fwd,
         &flow_bwd, &flow_inv, &flow_gfirst, &flow_gmore})
     d->release();
   on_device = false;
@@ -1476,8 +1474,8 @@ size_t Plan::device_bytes() const {
   size_t b = 0;
   for (const DeviceBuffer *d :
        {&amap, &arow, &acol, &diag_pos, &Kp, &Kj, &Ksrc, &sfirst, &srowptr, &srows, &srel,
-        &slofs, &uofs, &zofs, &child_ptr, &child_list, &perm, &ea_chunks, &ea_hits, &small_list,
-        &large_list, &steps, &ea_tasks, &gemm_probs, &flow_warp, &flow_fwd,
+        &slofs, &uofs, &child_ptr, &child_list, &perm, &ea_chunks, &ea_hits, &small_list,
+        &steps, &ea_tasks, &gemm_probs, &flow_warp, &flow_fwd,
         &flow_bwd, &flow_inv, &flow_gfirst, &flow_gmore})
     b += d->bytes();
   return b;
