@@ -95,7 +95,15 @@ int Solver::analyze(int64_t n, const int64_t *Ap, const int64_t *Ai,
 void Solver::adopt(std::shared_ptr<Plan> P) {
   MPIR_CUDA(cudaSetDevice(device));
   const int64_t n = P->S.n;
-  plan_ = std::move(P);
+  // (No plan, and no vectors, until all of this solver's memory is there: what
+  // an allocation that fails leaves behind is not taken for complete.)
+  plan_.reset();
+  num_.valid = false;
+  vec_m_     = -1;
+  // The batch buffers belong to the previous pattern.
+  bw_  = 0;
+  bm_  = -1;
+  mws_ = MultiSolveWorkspace{};
   // The bfloat16 tier keeps L in bfloat16 for the solves.  The float16 tier
   // does not: float16's range (largest finite 65504) cannot hold the L of
   // these scaled quasi-definite systems, whose entries reach 1/delta-sized
@@ -104,21 +112,17 @@ void Solver::adopt(std::shared_ptr<Plan> P) {
   if (num_.store_prec == 2) {
     // The 16-bit copy sits beside the float32 panels during factorization;
     // where both do not fit, the solves read the float32 panels instead.
-    if (Numeric::bytes_for(*plan_, 2) > device_free_bytes(device) / 100 * 97)
+    if (Numeric::bytes_for(*P, 2) > device_free_bytes(device) / 100 * 97)
       num_.store_prec = 1;
   }
-  num_.allocate(*plan_);
+  num_.allocate(*P);
   num_.update_mode = update_mode_for(uf, update_engine);
-  ws_.allocate(*plan_);
+  ws_.allocate(*P);
   vec_.allocate(n);
-  vec_m_ = -1;
-  // The batch buffers belong to the previous pattern.
-  bw_  = 0;
-  bm_  = -1;
-  mws_ = MultiSolveWorkspace{};
   if (wait_ctl_[0] || wait_ctl_[1])
     MPIR_CUDA(cudaMemcpy(ws_.err.as<int32_t>() + 1, wait_ctl_, sizeof wait_ctl_,
                          cudaMemcpyHostToDevice));
+  plan_ = std::move(P);
 }
 
 size_t Solver::device_bytes() const {
@@ -148,6 +152,7 @@ size_t Solver::bytes_for(const Plan &P, int64_t gmres_iter, int width, int uf) {
 void Solver::ensure_vectors() {
   const int64_t n = plan_->S.n, m = std::max<int64_t>(std::min(gmres_iter, n), 1);
   if (vec_m_ == m) return;
+  vec_m_ = -1;  // until all of it is there
   const size_t vb = std::max<int64_t>(n, 1) * sizeof(double);
   V_.resize(vb * (m + 1));
   bs_.resize(vb);

@@ -41,6 +41,7 @@ void Solver::ensure_batch(int width) {
   ensure_vectors();
   const int64_t n = plan_->S.n, m = std::max<int64_t>(std::min(gmres_iter, n), 1);
   if (bw_ == width && bm_ == m) return;
+  bw_ = 0;  // until all of it is there
   const size_t blk = static_cast<size_t>(std::max<int64_t>(n, 1)) * width * sizeof(double);
   bV_.resize(blk * (m + 1));
   bbs_.resize(blk);

@@ -1086,13 +1086,14 @@ int multi_width(int nrhs) {
 
 void MultiSolveWorkspace::allocate(const Plan &P, int width) {
   const MultiBuffers b(P);
-  nr          = width;
+  nr          = 0;  // until all of it is there
   fwd_pending = false;
   vals.resize(std::max<int64_t>((b.fwd + b.bwd + P.S.n) * width, 1) * sizeof(double));
   sync.resize(4 * sizeof(int32_t));
   device_zero(sync.as<void>(), sync.bytes());
   err.resize(sizeof(SolveCtl));
   device_zero(err.as<void>(), sizeof(SolveCtl));
+  nr = width;
 }
 
 size_t MultiSolveWorkspace::bytes_for(const Plan &P, int width) {
