@@ -570,6 +570,12 @@ def run_reference(args):
     rank, world, _ = dist_env()
     if rank != 0:
         return
+    import oracle
+    if not oracle.have_reference():
+        print(json.dumps({"impl": "reference", "unavailable":
+                          "the reference's compiled harness (oracle/_ref/libmpir_ref.so) is not there; "
+                          "it is built where the reference's headers are"}), flush=True)
+        return
     {"small2d": ref_small2d, "grid3d": ref_grid3d, "stream": ref_stream}.get(
         args.config, lambda a: print(json.dumps(
             {"impl": "reference", "unavailable": f"no reference arm for --config {a.config}; "
