@@ -61,7 +61,7 @@ class Arnoldi {
   // Active flags on the device (int32, active_stride() apart) for kernels that
   // are skipped when no vector is active.
   const int32_t *active() const;
-  int            active_stride() const { return static_cast<int>(stride(m_) * 2); }
+  int64_t        active_stride() const { return stride(m_) * 2; }
 
  private:
   static int64_t stride(int64_t m) {

@@ -42,7 +42,8 @@ struct FlowArgs {
   // nactive flags active_stride apart (NULL: none): nothing is done when all
   // are zero (the values stay as they are, for the next solve).
   const int32_t *active;
-  int32_t        nactive, active_stride;
+  int32_t        nactive;
+  int64_t        active_stride;
 };
 
 struct FlowSlot {

@@ -24,8 +24,9 @@ struct SolveWorkspace {
 // Flags on the device, count of them stride apart: the full solve is left out
 // when all are zero (p NULL: never).
 struct ActiveFlags {
-  const int32_t *p     = nullptr;
-  int            count = 0, stride = 0;
+  const int32_t *p      = nullptr;
+  int            count  = 0;
+  int64_t        stride = 0;
 };
 
 // Phases of the solve, combinable as bits.

@@ -7,7 +7,7 @@ import numpy as np
 import pytest
 
 import mpir_b200 as mp
-from test_gpu_arnoldi import _system
+from test_gpu_arnoldi import _backward, _system
 
 pytestmark = pytest.mark.gpu
 
@@ -27,4 +27,19 @@ def test_solver_after_refused_allocation(nrhs, steps):
         solve()
     solver.SetMaxGmresIterations(10)
     np.testing.assert_array_equal(np.array(solve()), X)
+    solver.close()
+
+
+def test_many_steps_for_sixteen_vectors():
+    """12,000 steps: the vectors' states lie 1.4e8 words apart, the last one's flag past 2^31."""
+    n = 12100
+    K, Ap, Ai, Ax = _system(n)
+    solver = mp.GmresLDLIR()
+    solver.SetMaxGmresIterations(12000)
+    solver.analyze(Ap, Ai, Ax)
+    assert solver.factor(Ax) == 0
+    B = np.random.default_rng(8).standard_normal((16, n))
+    X = solver.SolveBatch(B)
+    for x, b in zip(X, B):
+        assert _backward(K, x, b) <= 3.6e-15
     solver.close()
