@@ -37,7 +37,7 @@ constexpr int kRegs    = 16;  // entries of w a thread keeps
 constexpr int kWarps   = kThreads / 32;
 
 struct ArnoldiArgs {
-  int64_t    n, m, vs, block, stride;
+  int64_t    n, m, cap, vs, block, stride;  // steps allowed, laid out
   double    *V, *state;
   double     tol;
   GmresMail *mail;
@@ -46,16 +46,16 @@ struct ArnoldiArgs {
 struct StateView {
   GmresCtl *ctl;
   double   *R, *c, *s, *g, *y, *col;
-  __device__ StateView(const ArnoldiArgs &a, int vec) {
-    double *p = a.state + vec * a.stride;
-    ctl       = reinterpret_cast<GmresCtl *>(p);
-    R         = p + 4;
-    c         = R + a.m * (a.m + 1) / 2;
-    s         = c + a.m;
-    g         = s + a.m;
-    y         = g + a.m + 1;
-    col       = y + a.m;
+  __host__ __device__ StateView(double *p, int64_t cap) {
+    ctl = reinterpret_cast<GmresCtl *>(p);
+    R   = p + 4;
+    c   = R + cap * (cap + 1) / 2;
+    s   = c + cap;
+    g   = s + cap;
+    y   = g + cap + 1;
+    col = y + cap;
   }
+  __device__ StateView(const ArnoldiArgs &a, int vec) : StateView(a.state + vec * a.stride, a.cap) {}
 };
 
 __device__ __forceinline__ uint32_t cluster_rank() {
@@ -509,9 +509,9 @@ __global__ void __launch_bounds__(kThreads)
   }
 }
 
-ArnoldiArgs make_args(int64_t n, int64_t m, int64_t stride, double *V, int64_t block, double *state,
+ArnoldiArgs make_args(int64_t n, int64_t m, int64_t cap, int64_t stride, double *V, int64_t block, double *state,
                       double tol, GmresMail *mail) {
-  return ArnoldiArgs{n, m, n, block, stride, V, state, tol, mail};
+  return ArnoldiArgs{n, m, cap, n, block, stride, V, state, tol, mail};
 }
 
 // Clusters of more than 8 CTAs have to be allowed, on each device.
@@ -528,11 +528,33 @@ Arnoldi::~Arnoldi() {
 }
 
 void Arnoldi::allocate(int64_t n, int64_t m, int vectors) {
-  n_ = n;
-  m_ = m;
+  n_       = n;
+  m_       = m;
+  cap_     = std::min(m, kSteps);
+  vectors_ = vectors;
   state_.resize(bytes_for(m, vectors));
   if (cluster() > 8) allow_large_clusters();
   if (!mail_) mail_ = static_cast<GmresMail *>(pinned_alloc(sizeof(GmresMail)));
+}
+
+void Arnoldi::reserve(int nb, int64_t steps, cudaStream_t s) {
+  if (steps <= cap_) return;
+  const int64_t cap = std::min(m_, std::max(steps, 2 * cap_));
+  DeviceBuffer  next(stride(cap) * vectors_ * sizeof(double));
+  for (int k = 0; k < nb; k++) {
+    const StateView from(state_.as<double>() + k * stride(cap_), cap_), to(next.as<double>() + k * stride(cap), cap);
+    auto            copy = [&](void *dst, const void *src, int64_t n) {
+      MPIR_CUDA(cudaMemcpyAsync(dst, src, n * sizeof(double), cudaMemcpyDeviceToDevice, s));
+    };
+    copy(to.ctl, from.ctl, from.R - reinterpret_cast<double *>(from.ctl));
+    copy(to.R, from.R, cap_ * (cap_ + 1) / 2);
+    copy(to.c, from.c, cap_);
+    copy(to.s, from.s, cap_);
+    copy(to.g, from.g, cap_ + 1);
+  }
+  MPIR_CUDA(cudaStreamSynchronize(s));
+  state_ = std::move(next);
+  cap_   = cap;
 }
 
 const int32_t *Arnoldi::active() const {
@@ -549,23 +571,23 @@ int Arnoldi::cluster() const {
 void Arnoldi::begin(int nb, uint32_t act, const double *b, const VecFactors &fac, double *V, double tol,
                     cudaStream_t s) {
   launch_chained(n_, k_gmres_begin, cluster(), dim3(cluster(), nb, 1), kThreads, 0, s,
-                 make_args(n_, m_, stride(m_), V, 0, state_.as<double>(), tol, mail_), act, b, fac);
+                 make_args(n_, m_, cap_, stride(cap_), V, 0, state_.as<double>(), tol, mail_), act, b, fac);
 }
 
 void Arnoldi::first(int nb, double *V, double tol, cudaStream_t s) {
   launch_chained(n_, k_gmres_first, cluster(), dim3(cluster(), nb, 1), kThreads, 0, s,
-                 make_args(n_, m_, stride(m_), V, 0, state_.as<double>(), tol, mail_));
+                 make_args(n_, m_, cap_, stride(cap_), V, 0, state_.as<double>(), tol, mail_));
 }
 
 void Arnoldi::step(int nb, int64_t j, double *V, int64_t block, double tol, cudaStream_t s) {
   launch_chained(n_, k_gmres_step, cluster(), dim3(cluster(), nb, 1), kThreads, 0, s,
-                 make_args(n_, m_, stride(m_), V, block, state_.as<double>(), tol, mail_), j);
+                 make_args(n_, m_, cap_, stride(cap_), V, block, state_.as<double>(), tol, mail_), j);
 }
 
 void Arnoldi::end(int nb, uint32_t act, const double *V, int64_t block, double *x, bool update,
                   const VecFactors &scale, unsigned long long *inf, cudaStream_t s) {
   launch_chained(n_, k_gmres_end, cluster(), dim3(cluster(), nb, 1), kThreads, 0, s,
-                 make_args(n_, m_, stride(m_), const_cast<double *>(V), block, state_.as<double>(), 0.0, mail_),
+                 make_args(n_, m_, cap_, stride(cap_), const_cast<double *>(V), block, state_.as<double>(), 0.0, mail_),
                  act, x, update ? 1 : 0, scale, inf);
 }
 

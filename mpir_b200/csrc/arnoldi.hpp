@@ -1,5 +1,6 @@
 // Device side of PrecondGmres (gmres_ir.hpp:636-741): arnoldi.cu.
 #pragma once
+#include <algorithm>
 #include <cstdint>
 
 #include "engine.hpp"
@@ -31,18 +32,27 @@ struct GmresMail {
 // The state of the vectors of a call: control words, the triangular factor R
 // of the Hessenberg matrix (column j's j + 1 entries at j (j + 1) / 2), the
 // rotations, their right-hand side and the solution of the least-squares
-// problem.
+// problem.  It is laid out for kSteps steps at first and grows with the steps that
+// are taken: a caller that allows n of them, as many as there can be, would have
+// n^2 / 2 values of R reserved.
 class Arnoldi {
  public:
   void   allocate(int64_t n, int64_t m, int vectors);
   size_t bytes() const { return state_.bytes(); }
-  static size_t bytes_for(int64_t m, int vectors) { return stride(m) * vectors * sizeof(double); }
+  static constexpr int64_t kSteps = 512;
+  // Bytes at first.
+  static size_t bytes_for(int64_t m, int vectors) {
+    return stride(std::min(m, kSteps)) * vectors * sizeof(double);
+  }
   ~Arnoldi();
   Arnoldi() = default;
   Arnoldi(const Arnoldi &)            = delete;
   Arnoldi &operator=(const Arnoldi &) = delete;
 
   // Vector k of every block at k * n; bit k of act: vector k takes part.
+  // Steps there is room for, and room for more (waits for the stream; the flags move).
+  int64_t room() const { return cap_; }
+  void    reserve(int nb, int64_t steps, cudaStream_t s);
   // begin:  V_0 = b fac, its norm against tol.
   void begin(int nb, uint32_t act, const double *b, const VecFactors &fac, double *V, double tol,
              cudaStream_t s);
@@ -61,14 +71,15 @@ class Arnoldi {
   // Active flags on the device (int32, active_stride() apart) for kernels that
   // are skipped when no vector is active.
   const int32_t *active() const;
-  int64_t        active_stride() const { return stride(m_) * 2; }
+  int64_t        active_stride() const { return stride(cap_) * 2; }
 
  private:
   static int64_t stride(int64_t m) {
     return (4 + m * (m + 1) / 2 + 2 * m + (m + 1) + m + (m + 2) + 1) / 2 * 2;
   }
   int          cluster() const;
-  int64_t      n_ = 0, m_ = 0;
+  int64_t      n_ = 0, m_ = 0, cap_ = 0;  // steps allowed, laid out
+  int          vectors_ = 0;
   DeviceBuffer state_;
   GmresMail   *mail_ = nullptr;
 };

@@ -263,21 +263,28 @@ void Solver::inner(int nb, int width, uint32_t act, const double *b, const VecFa
   const int64_t *Kp = P.Kp.as<int64_t>();
   const int32_t *Kj = P.Kj.as<int32_t>();
   const double  *Kv = num_.Kval.as<double>();
-  const ActiveFlags on{ar.active(), nb, ar.active_stride()};
+  ActiveFlags    on{ar.active(), nb, ar.active_stride()};
   ar.begin(nb, act, b, fac, V, tol, s);
   apply(nb, width, V, on);
   ar.first(nb, V, tol, s);
+  auto goes_on = [&](int64_t j) {  // after step j
+    MPIR_CUDA(cudaEventSynchronize(step_ev_[j & 1]));
+    bool more = false;
+    for (int k = 0; k < nb; k++) more |= ar.mail().active[j & 1][k] != 0;
+    return more;
+  };
   for (int64_t j = 0; j < m; j++) {
     double *w = V + (j + 1) * block;
+    if (j == ar.room()) {  // (a step that needs more memory is taken for sure)
+      if (!goes_on(j - 1)) break;
+      ar.reserve(nb, j + 1, s);
+      on = ActiveFlags{ar.active(), nb, ar.active_stride()};
+    }
     vo.spmv(nb, Kp, Kj, Kv, w - block, w, s);
     apply(nb, width, w, on);
     ar.step(nb, j, V, block, tol, s);
     MPIR_CUDA(cudaEventRecord(step_ev_[j & 1], s));
-    if (j == 0) continue;
-    MPIR_CUDA(cudaEventSynchronize(step_ev_[(j - 1) & 1]));
-    bool more = false;
-    for (int k = 0; k < nb; k++) more |= ar.mail().active[(j - 1) & 1][k] != 0;
-    if (!more) break;
+    if (j > 0 && !goes_on(j - 1)) break;
   }
   ar.end(nb, act, V, block, x, update, scale, vo.infbits.as<unsigned long long>(), s);
 }
