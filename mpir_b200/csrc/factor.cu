@@ -281,12 +281,12 @@ __global__ void __launch_bounds__(256, 5)
 // What bounds it: the chain of 128 pivots, and beside it the 128 bytes a cycle
 // that shared memory returns to registers (a broadcast value costs a warp as
 // much as 32 different ones), hence two rows a lane below the diagonal block
-// and 4 x 4 values a lane in the products.  Every sum is taken in the order of
-// the kernel before this one (its results bit for bit): 35.0 us for a block of
-// 128 columns there, with X_pp and G formed after the diagonal block and
-// everything written at the end, 29.8 us here (32 columns 10 us both).  Rows
-// below by substitution beside the pivots instead of through X_pp: 28.4 us, but
-// other roundings.  Two pivots a turn: no gain.
+// and 4 x 4 values a lane in the products.  A block of 128 columns takes 29.8
+// us, 35.0 with X_pp and G formed after the diagonal block and everything
+// written at the end (32 columns 10 us both); the sums run in the same order as
+// there.  Two pivots a turn: no gain.  Rows below by substitution beside the pivots
+// instead of through X_pp: 28.4 us, but L moves by as much as its own error (2e-7)
+// so, which the QDLDL functions pass on to their solution.
 constexpr int kDiagLD = kNB + 4;  // Fs, Xs row stride (16-byte rows, lane = row conflict-free)
 constexpr int kDiagSmemFloats = 2 * kNB * kDiagLD + 2 * 32 * kNB + 32 * 32;
 
@@ -343,11 +343,14 @@ __device__ __forceinline__ void each8(F f) {
 
 // Phase A of panel p for warp 0: the diagonal block at (c0, c0).  Column k goes
 // to Gt (unscaled, at row c0 + lane) and Ld (scaled).  The broadcasts that the
-// next pivot waits for are issued before the loads of this one's column.  (Pivot
-// 0's update of column 30 is rounded twice: so it came out of the compiler in
-// the kernel before this one, and factors stay the same to the last bit.)  Kept
-// out of line: inlined into the kernel, whose other phases hold many
-// registers, its chain of shuffles is scheduled about 1.5x slower.
+// next pivot waits for are issued before the loads of this one's column.  The
+// updates' roundings are written out, whatever a compiler would fuse.  Pivot 0's
+// update of column 30 alone is rounded twice, which is no better, but how
+// factors have been rounded so far: with one rounding the QDLDL functions'
+// unrefined solution moved by up to 5e-7 on one value set in five, at the same
+// distance from float64.  Kept out of line: inlined into the kernel, whose
+// other phases hold many registers, its chain of shuffles is scheduled about 1.5x
+// slower.
 __device__ __noinline__ void diag_panel(float *Fs, float *Gt, float *Ld, int c0, int n,
                                         const StepDesc &d, float *D, float *Dinv, float *packd,
                                         float *packs, FactorStatus *st, int &npos) {
@@ -364,7 +367,8 @@ __device__ __noinline__ void diag_panel(float *Fs, float *Gt, float *Ld, int c0,
     if (k > 0) {  // the previous pivot's update of the columns beyond k
 #pragma unroll
       for (int j = 0; j < 32; j++)
-        if (j > k) a[j] = k == 1 && j == 30 ? __fsub_rn(a[j], __fmul_rn(lp, fp[j])) : a[j] - lp * fp[j];
+        if (j > k)
+          a[j] = k == 1 && j == 30 ? __fsub_rn(a[j], __fmul_rn(lp, fp[j])) : __fmaf_rn(-lp, fp[j], a[j]);
     }
     if (lane == k) piv = dk;
     const float l = a[k] * dv;  // L[r][k]
