@@ -10,9 +10,10 @@
 // cluster barrier (about 1 us).  Systems of up to 8,192 unknowns take one CTA,
 // which needs neither; a cluster of 8 (16 from 65,536 on) covers the rest, with
 // the entries beyond its registers (512 threads x 16 a CTA) in global memory.
-// One thread applies the rotations and decides whether to go on; the kernels of
-// a step that is not taken return at once, so the host may queue the next step
-// before it knows.
+// One thread applies the rotations and decides whether to go on; these kernels
+// and the solves of a step that is not taken return at once, so the host may
+// queue the next step before it knows (that step's SpMV does run, once an inner
+// loop: 8.5 us at n = 40,960).
 //
 // Measured outside the triangular solves: n = 1,280, 5 inner steps in two inner
 // loops, 0.46 ms a solve as separate launches, 0.15 here; n = 40,960 (8 CTAs), 7

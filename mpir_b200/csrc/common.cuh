@@ -71,9 +71,12 @@ inline void launch(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem,
 // dependent launch), and the next one's launch may begin once every block here
 // has passed that statement.  The kernels of a solve are launched so: chains of
 // kernels of 5 to 50 us, each of which would wait for the one before to drain
-// and then for its own launch.  A solve took 7 % less at n = 1,280, 9 % at 2,160
-// and 2.4 % at 14,045; from n = 24,603 to 40,951 it took up to 1 % more.  The
-// factorization's kernels are not: inside its graph they took 3 to 8 % longer.
+// and then for its own launch.  What decides is how long the kernels are, for
+// which n stands in here.  Below the line a pass took 7 % less at n = 1,280, 9 % at
+// 2,160, 3 % with 4 vectors at 5,120 and 2 to 5 % at 14,045.  Above it the two
+// are within the spread of a case's runs, on two boxes: 2.2 % less to 0.7 % more at
+// 24,603, 1.4 % less with 16 vectors at 20,480, the same with 3 at 40,951.  The
+// factorization's kernels are not launched so: in its graph they took 3 to 8 % longer.
 constexpr int64_t kChainedMax = 20000;
 template <class... KArgs, class... Args>
 inline void launch_chained(int64_t n, void (*kernel)(KArgs...), int cluster, dim3 grid, dim3 block,

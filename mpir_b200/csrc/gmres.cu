@@ -252,8 +252,8 @@ void Solver::apply(int nb, int width, double *x, const ActiveFlags &act) {
 }
 
 // PrecondGmres, gmres_ir.hpp:636-741.  The host queues step j + 1 before it
-// knows whether step j was the last one (kernels of a step that is not taken
-// return at once), so the device never waits for the host.
+// knows whether step j was the last one (the solve and the step of one that is
+// not taken return at once, its SpMV runs), so the device never waits for the host.
 void Solver::inner(int nb, int width, uint32_t act, const double *b, const VecFactors &fac, double *V,
                    Arnoldi &ar, VecOps &vo, double *x, bool update, const VecFactors &scale) {
   const Plan    &P  = *plan_;

@@ -28,9 +28,10 @@
 // CTA of 32 rows no longer fits in shared memory.
 //
 // Measured, one application (forward + backward, float32 factor), against the
-// solves by levels of 128-row blocks that this replaced: n = 1,280: 0.081 ms
-// (0.205); n = 2,160: 0.082 (0.231); n = 40,960: 0.41 (0.98), 283 MB of L read
-// twice at 1.4 TB/s; n = 138,240: 2.09 (3.04), 2.6 GB read twice at 2.5 TB/s.
+// solves by levels of 128-row blocks that this replaced (events around each
+// launch, both on one box): n = 1,280: 0.079 ms (0.183); n = 2,160: 0.088 (0.249);
+// n = 24,603: 0.26 (0.74); n = 40,960: 0.41 (0.98), 283 MB of L read twice at 1.4
+// TB/s; n = 138,240: 2.1 (3.1), 2.6 GB read twice at 2.5 TB/s.
 // Vectors are float64, the factor float32 or 16-bit (widened on load), as
 // QDLDL_solve with FACTPREC = float and XPREC = double.  Sums have a fixed
 // order, so results do not depend on scheduling.

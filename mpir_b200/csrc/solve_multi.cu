@@ -23,8 +23,8 @@
 // SM, twice per 512 columns of the chain).
 // Measured, one application, against the solves by levels that these replaced
 // and, in between, the same items with plain FMAs: 16 vectors at n = 20,480:
-// 0.48 ms (2.73; 0.64 to 0.78), 8 at n = 40,960: 0.76 ms (3.00; 0.95), 4 at
-// n = 40,951: 0.44 ms (1.50; 0.44), for which half of each product is unused.
+// 0.48 ms (2.73; 0.64 to 0.78), 8 at n = 40,960: 0.80 ms (2.99; 0.95), 4 at
+// n = 40,951: 0.46 ms (1.51; 0.44), for which half of each product is unused.
 // Per vector the sums inside an item run in another order than in the
 // single-vector kernels, so results agree with NR single solves to rounding.
 #include <algorithm>
