@@ -131,6 +131,7 @@ class Plan {
   int32_t      nflow_inv_low = 0;      // those below the last level, first in flow_inv
   bool         flow_warp_top = false;  // a warp-solved front in the last level
   int64_t      flow_part_elems = 0, flow_inv_elems = 0, flow_wpanel_total = 0;
+  int64_t      flow_z_elems = 0;  // front vectors, then the sums of kFwdSum items
   bool warp_solved(int64_t J) const { return S.w(J) <= kWarpSolveW && S.h(J) <= kWarpSolveH; }
   void build_flow();
   int64_t      ws_elems = 0;  // split-K partial tiles (floats)

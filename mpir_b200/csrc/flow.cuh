@@ -18,7 +18,11 @@ inline uint32_t    flow_entry(int64_t i) {
   return static_cast<uint32_t>(i);
 }
 // A row's child contributions: the first one's entry, and where the others lie
-// in the list of further ones (their number, then their entries).
+// in the list of further ones (their number, then their entries).  A row with
+// more than kFlowFan (a star's centre has one for each of its points) has sums of
+// kFlowFan of them instead, or sums of such sums, at most 8: entries behind the
+// front vectors, formed by kFwdSum items.
+constexpr int kFlowFan = 32;
 struct alignas(8) FlowGather {
   uint32_t first, more;
 };
@@ -58,6 +62,8 @@ enum FlowKind : int32_t {
                       // rows below it
   kFwdSlab,           // w > kFlowNarrow: 32 rows of the diagonal block
   kFwdRows,           // w > kFlowNarrow: 128 rows below the diagonal block
+  kFwdSum,            // nr <= 32 sums of kFlowFan contributions each, at zofs ..;
+                      // their sources lie one after another from gmore[rows] on
   kBwdChunk,          // up to 512 rows below the block x up to 128 columns
   kBwdNarrow,         // w <= kFlowNarrow: the whole diagonal block
   kBwdSlab,           // w > kFlowNarrow: 32 columns of the diagonal block

@@ -21,6 +21,21 @@ void Plan::build_flow() {
   flow_entry(S.z_elems);
   std::vector<uint32_t>   more, cnt, src;
   std::vector<FlowGather> first(S.z_elems, FlowGather{kFlowNone, kFlowNone});
+  // Sums, by level and by the depth of a sum of sums.
+  std::vector<std::vector<std::vector<FlowItem>>> sums(S.nlevels);
+  std::vector<int32_t>                            level;
+  std::vector<std::vector<uint32_t>>              lists;  // of a front's rows with many contributions
+  std::vector<int64_t>                            list_row;
+  flow_z_elems = S.z_elems;
+  auto put = [&](int64_t row, const uint32_t *e, uint32_t n) {
+    FlowGather &g = first[row];
+    if (n > 0) g.first = e[0];
+    if (n > 1) {
+      g.more = flow_entry(static_cast<int64_t>(more.size()));
+      more.push_back(n - 1);
+      more.insert(more.end(), e + 1, e + n);
+    }
+  };
   for (int64_t J = 0; J < ns; J++) {
     const int64_t h = S.h(J);
     cnt.assign(h + 1, 0);
@@ -38,14 +53,50 @@ void Plan::build_flow() {
     // cnt[i] is now the end of row i
     for (int64_t i = 0; i < h; i++) {
       const uint32_t e = i > 0 ? cnt[i - 1] : 0, n = cnt[i] - e;
-      FlowGather    &g = first[S.zofs[J] + i];
-      if (n > 0) g.first = src[e];
-      if (n > 1) {
-        g.more = flow_entry(static_cast<int64_t>(more.size()));
-        more.push_back(n - 1);
-        more.insert(more.end(), src.begin() + e + 1, src.begin() + e + n);
+      if (n <= kFlowFan) {
+        put(S.zofs[J] + i, src.data() + e, n);
+      } else {
+        lists.emplace_back(src.begin() + e, src.begin() + e + n);
+        list_row.push_back(S.zofs[J] + i);
       }
     }
+    if (lists.empty()) continue;
+    if (level.empty()) {
+      level.resize(ns);
+      for (int32_t t = 0; t < S.nlevels; t++)
+        for (int64_t q = S.level_ptr[t]; q < S.level_ptr[t + 1]; q++) level[S.level_sup[q]] = t;
+    }
+    auto &out = sums[level[J]];
+    bool  any = true;
+    for (size_t depth = 0; any; depth++) {
+      any               = false;
+      const int64_t z0  = flow_z_elems, m0 = static_cast<int64_t>(more.size());
+      for (auto &l : lists) {
+        if (l.size() <= (depth == 0 ? kFlowFan : 8)) continue;
+        std::vector<uint32_t> up;
+        for (size_t q = 0; q < l.size(); q += kFlowFan) {
+          const size_t n = std::min<size_t>(kFlowFan, l.size() - q);
+          more.insert(more.end(), l.begin() + q, l.begin() + q + n);
+          more.insert(more.end(), kFlowFan - n, kFlowNone);
+          up.push_back(flow_entry(flow_z_elems++));
+        }
+        l   = std::move(up);
+        any = true;
+      }
+      if (out.size() <= depth && any) out.resize(depth + 1);
+      for (int64_t z = z0; z < flow_z_elems; z += kFlowFan) {
+        FlowItem it{};
+        it.f.zofs = z;
+        it.f.rows = m0 + (z - z0) * kFlowFan;
+        it.kind   = kFwdSum;
+        it.nr     = static_cast<int32_t>(std::min<int64_t>(kFlowFan, flow_z_elems - z));
+        out[depth].push_back(it);
+      }
+    }
+    for (size_t q = 0; q < lists.size(); q++)
+      put(list_row[q], lists[q].data(), static_cast<uint32_t>(lists[q].size()));
+    lists.clear();
+    list_row.clear();
   }
   host_.flow_gfirst = std::move(first);
   host_.flow_gmore  = std::move(more);
@@ -132,12 +183,14 @@ void Plan::build_flow() {
     size_t first, count;
   };
   std::vector<Range> wr(S.nlevels);
-  // Forward, leaves first.  Within a level: the slabs of the wide fronts'
+  // Forward, leaves first.  Within a level: the sums of its rows with many
+  // contributions (a sum's sources first), the slabs of the wide fronts'
   // diagonal blocks (their chains start together), the narrow fronts, the
   // warp-solved fronts, then the rows below the wide blocks, which wait on
   // the slabs.  An item waits only on items before it.
   for (int32_t t = 0; t < S.nlevels; t++) {
     wr[t].first = warp.size();
+    for (const auto &s : sums[t]) fwd.insert(fwd.end(), s.begin(), s.end());
     std::vector<FlowItem> rows, narrow;
     // Rows of a narrow front's items: 512, less where the level would leave
     // SMs idle (w <= 32: always 512, a thread a row).

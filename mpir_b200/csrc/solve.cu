@@ -320,6 +320,27 @@ __device__ __forceinline__ void warp_columns(const double *M, int ld, int w, con
   }
 }
 
+// kFwdSum: 16 lanes a sum, two contributions a lane.  A thread alone, as for the
+// rows with few, took 2.2 ms for the 13,000 contributions of a star's centre, longer
+// than the levels' solves before (1.0 ms an application; 5.4 so).
+template <class T>
+__device__ __noinline__ void fwd_sum(const FlowArgs<T> &a, const FlowSlot &I, FlowSlot &N) {
+  const int tid = threadIdx.x, e = tid / 16, l = tid % 16;
+  uint32_t  ix[2] = {kFlowNone, kFlowNone};
+  if (e < I.item.nr) {
+    const uint32_t *m = a.gmore + I.item.f.rows + kFlowFan * e + 2 * l;
+    ix[0]             = m[0];
+    ix[1]             = m[1];
+  }
+  flow_fetch(a, N);
+  double z[2] = {0.0, 0.0};
+  add_values<2>(a.z, ix, z, a.err, I.polls);
+  double s = z[0] + z[1];
+#pragma unroll
+  for (int o = 8; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  if (l == 0 && e < I.item.nr && I.publish) st_relaxed_f64(a.z + I.item.f.zofs + e, s);
+}
+
 // kFlowWarps: one front of w <= 32, h <= 256 per warp; lane l holds rows
 // l + 32 t.  The rows' child contributions are polled together, one of each
 // row at a time; then y = Inv z, and the rows below less L y.
@@ -413,6 +434,7 @@ __global__ void __launch_bounds__(kFlowThreads, 1) k_fwd_flow(const __grid_const
           fwd_narrow<4>(a, S, I, N, sm, phase);
         break;
       case kFwdSlab: fwd_slab(a, S, I, N, sm, phase); break;
+      case kFwdSum: fwd_sum(a, I, N); break;
       default: fwd_rows(a, I, N, sm);
     }
   });
@@ -910,7 +932,7 @@ namespace {
 struct FlowBuffers {
   int64_t fwd, bwd;
   explicit FlowBuffers(const Plan &P)
-      : fwd(P.S.z_elems + (kFlowCopies + 1) * P.S.n),
+      : fwd(P.flow_z_elems + (kFlowCopies + 1) * P.S.n),
         bwd(P.flow_part_elems + (kFlowCopies + 1) * P.S.n) {}
 };
 }  // namespace
@@ -950,7 +972,7 @@ static void ldlt_solve_t(const Plan &P, const Numeric &F, const T *pan, double *
   a.x     = x;
   a.f     = (phases & kForward) ? bv + b.bwd : x;
   a.z     = fv;
-  a.y     = a.z + P.S.z_elems;
+  a.y     = a.z + P.flow_z_elems;
   a.yz    = a.y + kFlowCopies * n;
   a.part  = bv;
   a.xr    = a.part + P.flow_part_elems;

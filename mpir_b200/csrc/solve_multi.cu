@@ -528,6 +528,31 @@ __device__ __noinline__ void fwd_narrow_m(const FlowArgs<T> &a, FlowShared &S, c
   }
 }
 
+// kFwdSum: a thread a sum and vector, eight contributions at a time.
+template <int NR, class T>
+__device__ __noinline__ void fwd_sum_m(const FlowArgs<T> &a, const FlowSlot &I, FlowSlot &N) {
+  flow_fetch(a, N);
+  const int e = threadIdx.x / NR, v = threadIdx.x % NR;
+  if (e >= I.item.nr) return;
+  const uint32_t *m = a.gmore + I.item.f.rows + kFlowFan * e;
+  const double   *z = a.z + v;
+  double          s = 0.0;
+  for (int q = 0; q < kFlowFan; q += 8) {
+    uint32_t           idx[8];
+    unsigned long long raw[8];
+#pragma unroll
+    for (int u = 0; u < 8; u++) idx[u] = m[q + u];
+#pragma unroll
+    for (int u = 0; u < 8; u++)
+      raw[u] = idx[u] != kFlowNone ? ld_relaxed_u64(z + static_cast<int64_t>(NR) * idx[u]) : 0ull;
+#pragma unroll
+    for (int u = 0; u < 8; u++)
+      if (idx[u] != kFlowNone)
+        s += take_value(raw[u], z + static_cast<int64_t>(NR) * idx[u], a.err, I.polls);
+  }
+  if (I.publish) st_relaxed_f64(a.z + NR * (I.item.f.zofs + e) + v, s);
+}
+
 // The panels of an item's warp-solved fronts into shared memory: warp q starts
 // the copy of front q.
 template <class T>
@@ -648,6 +673,7 @@ __global__ void __launch_bounds__(kFlowThreads, 1) k_fwd_flow_m(const __grid_con
           fwd_narrow_m<4, NR>(a, S, I, N, sm, phase);
         break;
       case kFwdSlab: fwd_slab_m<NR>(a, S, I, N, sm, phase); break;
+      case kFwdSum: fwd_sum_m<NR>(a, I, N); break;
       default: fwd_rows_m<NR>(a, I, N, sm);
     }
   });
@@ -1017,7 +1043,7 @@ __global__ void __launch_bounds__(kFlowThreads, 1) k_bwd_flow_m(const __grid_con
 struct MultiBuffers {
   int64_t fwd, bwd;
   explicit MultiBuffers(const Plan &P)
-      : fwd(P.S.z_elems + (kMultiCopies + 1) * P.S.n),
+      : fwd(P.flow_z_elems + (kMultiCopies + 1) * P.S.n),
         bwd(P.flow_part_elems + (kMultiCopies + 1) * P.S.n) {}
 };
 
@@ -1040,7 +1066,7 @@ void solve_multi_nr(const Plan &P, const Numeric &F, const T *pan, double *X,
   a.x      = X;
   a.f      = bv + NR * b.bwd;
   a.z      = fv;
-  a.y      = a.z + NR * P.S.z_elems;
+  a.y      = a.z + NR * P.flow_z_elems;
   a.yz     = a.y + NR * kMultiCopies * n;
   a.part   = bv;
   a.xr     = a.part + NR * P.flow_part_elems;
