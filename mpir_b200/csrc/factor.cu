@@ -112,13 +112,27 @@ __global__ void __launch_bounds__(kSmallThreads)
     const int      rc = static_cast<int>(srowptr[C + 1] - srowptr[C]) - wc;
     const float   *U  = uarena + uofs[C];
     const int32_t *rl = srel + srowptr[C] + wc;
-    // (a child's rows are among the front's: rc <= h)
-    const int r0 = lane < rc ? rl[lane] : 0, r1 = lane + 32 < rc ? rl[lane + 32] : 0;
-    for (int b = warp; b < rc; b += kW) {
-      const int    rb = rl[b];
-      const float *Ub = U + (int64_t)b * rc;
-      if (lane >= b && lane < rc) F[r0][rb] += Ub[lane];
-      if (lane + 32 >= b && lane + 32 < rc) F[r1][rb] += Ub[lane + 32];
+    // (a child's rows are among the front's: rc <= h; two of the warp's columns
+    // are loaded before the first is added)
+    const int     r0 = lane < rc ? rl[lane] : 0, r1 = lane + 32 < rc ? rl[lane + 32] : 0;
+    constexpr int kCols = 2;
+    for (int b0 = warp; b0 < rc; b0 += kCols * kW) {
+      int   rb[kCols];
+      float u0[kCols], u1[kCols];
+#pragma unroll
+      for (int q = 0; q < kCols; q++) {
+        const int    b  = b0 + q * kW;
+        const float *Ub = U + (int64_t)b * rc;
+        rb[q] = b < rc ? rl[b] : 0;
+        u0[q] = lane >= b && lane < rc ? Ub[lane] : 0.0f;
+        u1[q] = lane + 32 >= b && lane + 32 < rc ? Ub[lane + 32] : 0.0f;
+      }
+#pragma unroll
+      for (int q = 0; q < kCols; q++) {
+        const int b = b0 + q * kW;
+        if (lane >= b && lane < rc) F[r0][rb[q]] += u0[q];
+        if (lane + 32 >= b && lane + 32 < rc) F[r1][rb[q]] += u1[q];
+      }
     }
     __syncthreads();
   }
