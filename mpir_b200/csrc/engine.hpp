@@ -128,6 +128,10 @@ class Plan {
   // directions, the strips of the block inverses, the rows' child contributions.
   DeviceBuffer flow_warp, flow_fwd, flow_bwd, flow_inv, flow_gfirst, flow_gmore;
   int32_t      nflow_fwd = 0, nflow_bwd = 0, nflow_inv = 0;
+  // The leaves with kernels of their own: fronts, and their items, the first of
+  // flow_fwd and the last of flow_bwd (none: 0).
+  DeviceBuffer flow_leaf;
+  int32_t      nflow_leaf = 0, nflow_leaf_fwd = 0, nflow_leaf_bwd = 0;
   int32_t      nflow_inv_low = 0;      // those below the last level, first in flow_inv
   bool         flow_warp_top = false;  // a warp-solved front in the last level
   int64_t      flow_part_elems = 0, flow_inv_elems = 0, flow_wpanel_total = 0;
@@ -161,7 +165,7 @@ class Plan {
     std::vector<EaChunk>    chunks;
     std::vector<EaHit>      hits;
     std::vector<GemmProb>   probs;
-    std::vector<FlowFront>   flow_warp;
+    std::vector<FlowFront>   flow_warp, flow_leaf;
     std::vector<FlowItem>    flow_fwd, flow_bwd;
     std::vector<FlowInvDesc> flow_inv;
     std::vector<FlowGather>  flow_gfirst;

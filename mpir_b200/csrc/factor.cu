@@ -1375,7 +1375,7 @@ size_t Plan::upload_bytes() const {
          b(S.sfirst) + b(S.srowptr) + b(S.srows) + b(S.srel) + b(S.slofs) + b(S.uofs) +
          b(S.child_ptr) + b(S.child_list) + b(S.perm) + b(h_small) +
          b(host_.descs) + b(host_.tasks) + b(host_.chunks) + b(host_.hits) + b(host_.probs) +
-         b(host_.flow_warp) + b(host_.flow_fwd) + b(host_.flow_bwd) + b(host_.flow_inv) +
+         b(host_.flow_warp) + b(host_.flow_leaf) + b(host_.flow_fwd) + b(host_.flow_bwd) + b(host_.flow_inv) +
          b(host_.flow_gfirst) + b(host_.flow_gmore);
 }
 
@@ -1404,6 +1404,7 @@ void Plan::upload_all(cudaStream_t s) {
   ea_hits    = upload(host_.hits, s);
   gemm_probs = upload(host_.probs, s);
   flow_warp    = upload(host_.flow_warp, s);
+  flow_leaf    = upload(host_.flow_leaf, s);
   flow_fwd     = upload(host_.flow_fwd, s);
   flow_bwd     = upload(host_.flow_bwd, s);
   flow_inv     = upload(host_.flow_inv, s);
@@ -1418,7 +1419,7 @@ void Plan::release_device() {
   for (DeviceBuffer *d :
        {&amap, &arow, &acol, &diag_pos, &Kp, &Kj, &Ksrc, &sfirst, &srowptr, &srows, &srel,
         &slofs, &uofs, &child_ptr, &child_list, &perm, &ea_chunks, &ea_hits, &small_list,
-        &steps, &ea_tasks, &gemm_probs, &flow_warp, &flow_fwd,
+        &steps, &ea_tasks, &gemm_probs, &flow_warp, &flow_leaf, &flow_fwd,
         &flow_bwd, &flow_inv, &flow_gfirst, &flow_gmore})
     d->release();
   on_device = false;
@@ -1495,7 +1496,7 @@ size_t Plan::device_bytes() const {
   for (const DeviceBuffer *d :
        {&amap, &arow, &acol, &diag_pos, &Kp, &Kj, &Ksrc, &sfirst, &srowptr, &srows, &srel,
         &slofs, &uofs, &child_ptr, &child_list, &perm, &ea_chunks, &ea_hits, &small_list,
-        &steps, &ea_tasks, &gemm_probs, &flow_warp, &flow_fwd,
+        &steps, &ea_tasks, &gemm_probs, &flow_warp, &flow_leaf, &flow_fwd,
         &flow_bwd, &flow_inv, &flow_gfirst, &flow_gmore})
     b += d->bytes();
   return b;

@@ -179,6 +179,32 @@ void Plan::build_flow() {
       q = e;
     }
   };
+  // Leaves of at most 64 rows, where there are many of them.
+  nflow_leaf = nflow_leaf_fwd = nflow_leaf_bwd = 0;
+  std::vector<FlowFront> leaf;
+  size_t                 leaf_warps = 0;  // the first of the warp-solved fronts
+  if (S.nlevels > 0) {
+    int64_t nw = 0, nn = 0;
+    for (int64_t q = S.level_ptr[0]; q < S.level_ptr[1]; q++) {
+      const int64_t J = S.level_sup[q];
+      if (!is_large(J)) (warp_solved(J) ? nw : nn)++;
+    }
+    if (nw / kFlowWarpsPerItem + nn >= kFlowLeafItems)
+      for (int64_t q = S.level_ptr[0]; q < S.level_ptr[1]; q++) {
+        const int64_t J = S.level_sup[q];
+        if (is_large(J)) continue;
+        leaf.push_back(fr[J]);
+        if (warp_solved(J))
+          warp.push_back(fr[J]);
+        else
+          fwd.push_back(FlowItem{fr[J], kFwdNarrow, fr[J].w, fr[J].h - fr[J].w, 0});
+      }
+    leaf_warps = warp.size();
+    warps(fwd, 0, leaf_warps);
+    nflow_leaf     = static_cast<int32_t>(leaf.size());
+    nflow_leaf_fwd = static_cast<int32_t>(fwd.size());
+  }
+  auto taken = [&](int64_t J, int32_t t) { return t == 0 && nflow_leaf > 0 && !is_large(J); };
   struct Range {
     size_t first, count;
   };
@@ -204,6 +230,7 @@ void Plan::build_flow() {
     for (int64_t q = S.level_ptr[t]; q < S.level_ptr[t + 1]; q++) {
       const int64_t    J = S.level_sup[q];
       const FlowFront &f = fr[J];
+      if (taken(J, t)) continue;
       if (warp_solved(J)) {
         warp.push_back(f);
       } else if (f.w <= kFlowNarrow) {
@@ -232,7 +259,7 @@ void Plan::build_flow() {
     for (int64_t q = S.level_ptr[t]; q < S.level_ptr[t + 1]; q++) {
       const int64_t    J = S.level_sup[q];
       const FlowFront &f = fr[J];
-      if (warp_solved(J)) continue;
+      if (warp_solved(J) || taken(J, t)) continue;
       for (int32_t c = 0; c < f.chunks; c++)
         for (int32_t k = 0; k < f.w; k += kFlowChunkC)
           bwd.push_back(FlowItem{f, kBwdChunk, k, std::min(kFlowChunkC, f.w - k), c});
@@ -245,10 +272,16 @@ void Plan::build_flow() {
     bwd.insert(bwd.end(), own.begin(), own.end());
     warps(bwd, wr[t].first, wr[t].count);
   }
+  const size_t others = bwd.size();
+  for (const FlowFront &f : leaf)
+    if (!(f.w <= kWarpSolveW && f.h <= kWarpSolveH)) bwd.push_back(FlowItem{f, kBwdNarrow, 0, f.w, 0});
+  warps(bwd, 0, leaf_warps);
+  nflow_leaf_bwd    = static_cast<int32_t>(bwd.size() - others);
   nflow_fwd         = static_cast<int32_t>(fwd.size());
   nflow_bwd         = static_cast<int32_t>(bwd.size());
   nflow_inv         = static_cast<int32_t>(inv.size());
   host_.flow_warp   = std::move(warp);
+  host_.flow_leaf   = std::move(leaf);
   host_.flow_fwd    = std::move(fwd);
   host_.flow_bwd    = std::move(bwd);
   host_.flow_inv    = std::move(inv);

@@ -35,8 +35,10 @@
 // Vectors are float64, the factor float32 or 16-bit (widened on load), as
 // QDLDL_solve with FACTPREC = float and XPREC = double.  Sums have a fixed
 // order, so results do not depend on scheduling.
+#include <algorithm>
 #include <atomic>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include "common.cuh"
@@ -785,6 +787,107 @@ __global__ void __launch_bounds__(kFlowThreads, 1) k_bwd_flow(const __grid_const
   flow_mark(a.mark, a.nmark);
 }
 
+// ---------------------------------------------------------------------------
+// Leaves of at most 64 rows (FlowFront, one warp each, lane = rows l and l + 32) by
+// substitution with the float32 panel, for one vector, before the forward and after
+// the backward data flow.  A front waits on nothing, so what bounds it is latency,
+// and 64 warps an SM hide it where 16 with their fronts staged in shared memory do
+// not.  One application by items, by levels before those, and so (ms): 10,000
+// blocks of 40 x 40 0.40, 0.14, 0.08; 100,000 of 4 x 4 0.22, 0.20, 0.11; 500,000 of one
+// 0.99, 0.69, 0.33; the leaves of a 2-D grid of n = 1.4 million 1.11, 2.00, 0.92.  At
+// the line (kFlowLeafItems) the items of a direction take about 70 us; below it two
+// more launches weigh as much as they save.
+constexpr int kLeafWarps = 8;
+__global__ void __launch_bounds__(32 * kLeafWarps)
+    k_fwd_leaf(const FlowFront *fronts, int count, const float *panel, const double *x, double *f,
+               double *z, const int32_t *active) {
+  grid_wait();
+  if (active && *active == 0) return;
+  const int lane = threadIdx.x % 32, q = blockIdx.x * kLeafWarps + threadIdx.x / 32;
+  if (q >= count) return;
+  const FlowFront fr = fronts[q];
+  const int       w = fr.w, h = fr.h, i1 = lane + 32;
+  const float    *P = panel + fr.panel;
+  double          z0 = lane < w ? x[fr.col0 + lane] : 0.0, z1 = i1 < w ? x[fr.col0 + i1] : 0.0;
+  float           c0[4], c1[4], n0[4], n1[4];
+  auto            load = [&](float(&a)[4], float(&b)[4], int k0) {
+#pragma unroll
+    for (int u = 0; u < 4; u++) {
+      const int k = k0 + u;
+      a[u]        = k < w && lane > k && lane < h ? P[lane + k * h] : 0.0f;
+      b[u]        = k < w && i1 > k && i1 < h ? P[i1 + k * h] : 0.0f;
+    }
+  };
+  load(c0, c1, 0);
+  for (int k0 = 0; k0 < w; k0 += 4) {
+    load(n0, n1, k0 + 4);
+#pragma unroll
+    for (int u = 0; u < 4; u++) {
+      const int k = k0 + u;
+      if (k >= w) break;
+      const double y = __shfl_sync(0xffffffffu, k < 32 ? z0 : z1, k % 32);
+      if (lane > k) z0 -= static_cast<double>(c0[u]) * y;
+      if (i1 > k) z1 -= static_cast<double>(c1[u]) * y;
+    }
+#pragma unroll
+    for (int u = 0; u < 4; u++) {
+      c0[u] = n0[u];
+      c1[u] = n1[u];
+    }
+  }
+  if (lane < h) (lane < w ? f + fr.col0 : z + fr.zofs)[lane] = z0;
+  if (i1 < h) (i1 < w ? f + fr.col0 : z + fr.zofs)[i1] = z1;
+}
+
+__global__ void __launch_bounds__(32 * kLeafWarps)
+    k_bwd_leaf(const FlowFront *fronts, int count, const float *panel, const int32_t *srows,
+               const float *Dinv, const double *f, double *x, const int32_t *active) {
+  grid_wait();
+  if (active && *active == 0) return;
+  const int lane = threadIdx.x % 32, q = blockIdx.x * kLeafWarps + threadIdx.x / 32;
+  if (q >= count) return;
+  const FlowFront fr = fronts[q];
+  const int       w = fr.w, h = fr.h, i1 = lane + 32;
+  const float    *P  = panel + fr.panel;
+  auto            at = [&](int i) {
+    if (i >= h) return 0.0;
+    if (i >= w) return x[srows[fr.rows + i]];
+    return Dinv ? f[fr.col0 + i] * static_cast<double>(Dinv[fr.col0 + i]) : f[fr.col0 + i];
+  };
+  double x0 = at(lane), x1 = at(i1);
+  float  c0[4], c1[4], n0[4], n1[4];
+  auto   load = [&](float(&a)[4], float(&b)[4], int k0) {  // columns k0, k0 - 1, ..
+#pragma unroll
+    for (int u = 0; u < 4; u++) {
+      const int k = k0 - u;
+      a[u]        = k >= 0 && lane > k && lane < h ? P[lane + k * h] : 0.0f;
+      b[u]        = k >= 0 && i1 > k && i1 < h ? P[i1 + k * h] : 0.0f;
+    }
+  };
+  load(c0, c1, w - 1);
+  for (int k0 = w - 1; k0 >= 0; k0 -= 4) {
+    load(n0, n1, k0 - 4);
+#pragma unroll
+    for (int u = 0; u < 4; u++) {
+      const int k = k0 - u;
+      if (k < 0) break;
+      double s = lane > k ? static_cast<double>(c0[u]) * x0 : 0.0;
+      if (i1 > k) s += static_cast<double>(c1[u]) * x1;
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+      if (lane == k) x0 -= s;
+      if (i1 == k) x1 -= s;
+    }
+#pragma unroll
+    for (int u = 0; u < 4; u++) {
+      c0[u] = n0[u];
+      c1[u] = n1[u];
+    }
+  }
+  if (lane < w) x[fr.col0 + lane] = x0;
+  if (i1 < w) x[fr.col0 + i1] = x1;
+}
+
 __global__ void k_dscale(int64_t n, const float *Dinv, double *x) {
   const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (i < n) x[i] *= static_cast<double>(Dinv[i]);
@@ -984,15 +1087,25 @@ static void ldlt_solve_t(const Plan &P, const Numeric &F, const T *pan, double *
   static OncePerDevice attr;
   constexpr int        smem = kFlowSmem * sizeof(double);
   allow_smem(attr, smem, {reinterpret_cast<const void *>(k_fwd_flow<T>), reinterpret_cast<const void *>(k_bwd_flow<T>)});
+  // (The 16-bit panels are left to the items, which take these fronts' float32 values.
+  // Beside the leaves' kernels there may be few items or none; the launch still marks
+  // all the values pending.)
+  const bool      leaf  = std::is_same<T, float>::value && P.nflow_leaf > 0;
+  const FlowFront *lf   = P.flow_leaf.as<FlowFront>();
+  const float     *lp   = F.panel.as<float>();
+  const unsigned   lgrid = static_cast<unsigned>((P.nflow_leaf + kLeafWarps - 1) / kLeafWarps);
   kt.begin(kKcSolveFwd, s);
   if (phases & kForward) {
     if (!ws.fwd_pending) flow_pending(fv, b.fwd, s);
-    a.items  = P.flow_fwd.as<FlowItem>();
-    a.nitems = P.nflow_fwd;
+    if (leaf)
+      launch_chained(n, k_fwd_leaf, 1, lgrid, 32 * kLeafWarps, 0, s, lf, P.nflow_leaf, lp, x, a.f, a.z, act.p);
+    const int32_t skip = leaf ? P.nflow_leaf_fwd : 0;
+    a.items  = P.flow_fwd.as<FlowItem>() + skip;
+    a.nitems = P.nflow_fwd - skip;
     a.mark   = bv;
     a.nmark  = b.bwd;
     a.ticket = ws.sync.as<int32_t>();
-    launch_chained(n, k_fwd_flow<T>, 1, std::min(P.nflow_fwd, kSMs), kFlowThreads, smem, s, a);
+    launch_chained(n, k_fwd_flow<T>, 1, leaf ? kSMs : std::min(a.nitems, kSMs), kFlowThreads, smem, s, a);
     ws.fwd_pending = false;
     ws.bwd_pending = true;
   }
@@ -1007,12 +1120,15 @@ static void ldlt_solve_t(const Plan &P, const Numeric &F, const T *pan, double *
   kt.begin(kKcSolveBwd, s);
   if (!ws.bwd_pending) flow_pending(bv, b.bwd, s);
   a.items  = P.flow_bwd.as<FlowItem>();
-  a.nitems = P.nflow_bwd;
+  a.nitems = P.nflow_bwd - (leaf ? P.nflow_leaf_bwd : 0);
   a.mark   = fv;
   a.nmark  = b.fwd;
   a.Dinv   = (phases & kDiagonal) ? F.Dinv.as<float>() : nullptr;
   a.ticket = ws.sync.as<int32_t>() + 1;
-  launch_chained(n, k_bwd_flow<T>, 1, std::min(P.nflow_bwd, kSMs), kFlowThreads, smem, s, a);
+  launch_chained(n, k_bwd_flow<T>, 1, leaf ? kSMs : std::min(a.nitems, kSMs), kFlowThreads, smem, s, a);
+  if (leaf)
+    launch_chained(n, k_bwd_leaf, 1, lgrid, 32 * kLeafWarps, 0, s, lf, P.nflow_leaf, lp, a.srows, a.Dinv, a.f, x,
+                   act.p);
   ws.bwd_pending = false;
   ws.fwd_pending = true;
   kt.end(s);
