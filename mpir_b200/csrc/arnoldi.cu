@@ -20,6 +20,14 @@
 // steps in three, 0.9 -> 0.4 ms; three vectors of n = 40,951, 9 steps in three,
 // 1.3 -> 0.5 ms.
 //
+// A cluster's 16 SMs read the basis at about 1.3 TB/s.  Up to four vectors of more
+// than 200,000 entries are therefore swept by the whole chip, one launch a basis
+// vector (k_wide_*), whose partial sums the next one adds up; the cluster keeps the
+// norms' slow cases, the second sweep and the rotations.  80 steps over up to 40
+// basis vectors, solves included, as separate reductions and updates, by a cluster
+// alone, so (ms): n = 200,000 32.6, 28.5, -; 327,680 44.8, 51.8, 39.3; 500,000 64.6, 82.3,
+// 56.8; 4 million 490, 784, 423.
+//
 // Sums run in a fixed order (threads, warps, CTAs), so results are
 // reproducible.  Norms are sqrt of the sum of squares, or, where that sum is
 // not well inside the range of float64, the scaled form of Dnrm2
@@ -42,7 +50,22 @@ struct ArnoldiArgs {
   double    *V, *state;
   double     tol;
   GmresMail *mail;
+  double    *wide;  // kWideStride a vector: WideScratch, partial sums (NULL: no chip-wide kernels)
 };
+
+// Vectors of more than kWideFrom entries, up to kWideVectors of them, are swept by
+// the whole chip (k_wide_*), one launch a basis vector, the others by a cluster each.
+constexpr int64_t kWideFrom    = 200000;
+constexpr int     kWideVectors = 4;
+constexpr int     kWideCtas    = 148;
+constexpr int     kWideStride  = 4 + 4 * kWideCtas;
+struct WideScratch {
+  double  ss;   // |w|^2 before the sweep
+  double  f;    // factor of k_wide_scale
+  int32_t odd;  // |w|^2 has left the range in which it is accurate: the step is the cluster's
+  int32_t pad[3];
+};
+static_assert(sizeof(WideScratch) == 32, "four doubles");
 
 struct StateView {
   GmresCtl *ctl;
@@ -196,6 +219,178 @@ __device__ double safe_norm(double ss, const Spread &sp, const double (&w)[kRegs
   return mx * sqrt(q);
 }
 
+// x = d, or x += d f with the largest |d f| and |x before| (gmres_ir.hpp:574-577).  NaN
+// counts as above infinity, as in the max-norms of the vector kernels.
+__device__ __forceinline__ void refine(double d, double f, int update, double &x, double &dm, double &xm) {
+  if (!update) {
+    x = d;
+    return;
+  }
+  const double di = d * f, xi = x;
+  dm = fabs(di) > dm || !(di == di) ? fabs(di) : dm;
+  xm = fabs(xi) > xm || !(xi == xi) ? fabs(xi) : xm;
+  x  = xi + di;
+}
+
+__device__ __forceinline__ WideScratch *wide_scratch(const ArnoldiArgs &a, int vec) {
+  return reinterpret_cast<WideScratch *>(a.wide + static_cast<int64_t>(kWideStride) * vec);
+}
+// The CTAs' partial sums `which` of launches of parity t; added in a fixed order, in
+// every thread.
+__device__ __forceinline__ double *wide_part(const ArnoldiArgs &a, int vec, int t, int which) {
+  return a.wide + static_cast<int64_t>(kWideStride) * vec + 4 + (2 * t + which) * kWideCtas;
+}
+__device__ __forceinline__ double wide_sum(const double *p) {
+  __shared__ double out;
+  if (threadIdx.x < 32) {
+    double s = 0.0;
+#pragma unroll
+    for (int q = 0; q < (kWideCtas + 31) / 32; q++) {
+      const int i = threadIdx.x + 32 * q;
+      s += i < kWideCtas ? __ldcg(p + i) : 0.0;
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if (threadIdx.x == 0) out = s;
+  }
+  __syncthreads();
+  const double s = out;
+  __syncthreads();
+  return s;
+}
+// The CTA's sum of v into its place.
+__device__ __forceinline__ void wide_store(double *p, double v) {
+  __shared__ double warp[kWarps];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  if (threadIdx.x % 32 == 0) warp[threadIdx.x / 32] = v;
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    v = threadIdx.x < kWarps ? warp[threadIdx.x] : 0.0;
+#pragma unroll
+    for (int o = kWarps / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    if (threadIdx.x == 0) p[blockIdx.x] = v;
+  }
+  __syncthreads();
+}
+// f(i) for the entries of one CTA of the chip.
+template <class F>
+__device__ __forceinline__ void wide_each(int64_t n, F f) {
+  constexpr int64_t step = static_cast<int64_t>(kWideCtas) * kThreads;
+#pragma unroll 4
+  for (int64_t i = blockIdx.x * static_cast<int64_t>(kThreads) + threadIdx.x; i < n; i += step) f(i);
+}
+
+// V_0 = b fac with |V_0|^2 (begin), or |V_0|^2 of what is there.
+__global__ void __launch_bounds__(kThreads)
+    k_wide_norm(const ArnoldiArgs a, uint32_t act, const double *b, const VecFactors fac) {
+  grid_wait();
+  const int vec = blockIdx.y;
+  if (b ? !(act >> vec & 1u) : StateView(a, vec).ctl->active == 0) return;
+  const double f  = fac.v[vec];
+  double      *w0 = a.V + vec * a.vs, ss = 0.0;
+  wide_each(a.n, [&](int64_t i) {
+    double x = w0[i];
+    if (b) {
+      x     = b[vec * a.vs + i] * f;
+      w0[i] = x;
+    }
+    ss += x * x;
+  });
+  wide_store(wide_part(a, vec, 0, 1), ss);
+}
+
+// Launch j = 0 .. k + 1 of step k: h_{j-1} from the launch before, w -= h_{j-1}
+// v_{j-1}, the partial sums of w v_j, in the last one of |w|^2 (in the first also).
+__global__ void __launch_bounds__(kThreads) k_wide_sweep(const ArnoldiArgs a, int64_t k, int64_t j) {
+  grid_wait();
+  const int    vec = blockIdx.y, t = j & 1;
+  StateView    st(a, vec);
+  WideScratch *sc = wide_scratch(a, vec);
+  if (st.ctl->active == 0 || (j > 1 && sc->odd)) return;
+  const bool lead = blockIdx.x == 0 && threadIdx.x == 0;
+  double     h = 0.0, s = 0.0, ss = 0.0;
+  if (j > 0) {
+    h = wide_sum(wide_part(a, vec, 1 - t, 0));
+    if (j == 1) {
+      ss             = wide_sum(wide_part(a, vec, 0, 1));
+      const bool odd = !(ss > 1e-280 && ss < 1e280);
+      if (lead) {
+        sc->ss  = ss;
+        sc->odd = odd;
+      }
+      if (odd) return;
+      ss = 0.0;
+    }
+    if (lead) st.col[j - 1] = h;
+  }
+  double       *V = a.V + vec * a.vs, *w = V + (k + 1) * a.block;
+  const double *vb = V + (j - 1) * a.block, *vj = V + j * a.block;
+  if (j == 0) {
+    wide_each(a.n, [&](int64_t i) {
+      const double x = w[i];
+      s += x * vj[i];
+      ss += x * x;
+    });
+    wide_store(wide_part(a, vec, 0, 1), ss);
+  } else if (j <= k) {
+    wide_each(a.n, [&](int64_t i) {
+      const double x = w[i] - vb[i] * h;
+      w[i]           = x;
+      s += x * vj[i];
+    });
+  } else {
+    wide_each(a.n, [&](int64_t i) {
+      const double x = w[i] - vb[i] * h;
+      w[i]           = x;
+      s += x * x;
+    });
+  }
+  wide_store(wide_part(a, vec, t, 0), s);
+}
+
+// V_j *= the factor that the step (or first) left.
+__global__ void __launch_bounds__(kThreads) k_wide_scale(const ArnoldiArgs a, int64_t j) {
+  grid_wait();
+  const int vec = blockIdx.y;
+  if (StateView(a, vec).ctl->active == 0) return;
+  const double f = wide_scratch(a, vec)->f;
+  double      *w = a.V + vec * a.vs + j * a.block;
+  wide_each(a.n, [&](int64_t i) { w[i] *= f; });
+}
+
+// The combination of the basis (k_gmres_end).
+__global__ void __launch_bounds__(kThreads)
+    k_wide_end(const ArnoldiArgs a, uint32_t act, double *x, int update, const VecFactors fac,
+               unsigned long long *inf) {
+  grid_wait();
+  const int vec = blockIdx.y;
+  if (!(act >> vec & 1u)) return;
+  const StateView st(a, vec);
+  const int64_t   k  = st.ctl->k;
+  const double    f  = fac.v[vec];
+  const double   *V  = a.V + vec * a.vs;
+  double         *xv = x + vec * a.vs, dm = 0.0, xm = 0.0;
+  wide_each(a.n, [&](int64_t i) {
+    double d = 0.0;
+#pragma unroll 4
+    for (int64_t j = 0; j < k; j++) d += V[j * a.block + i] * st.y[j];
+    refine(d, f, update, xv[i], dm, xm);
+  });
+  if (!update) return;
+  unsigned long long b0 = __double_as_longlong(dm), b1 = __double_as_longlong(xm);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const unsigned long long c0 = __shfl_xor_sync(0xffffffffu, b0, o), c1 = __shfl_xor_sync(0xffffffffu, b1, o);
+    b0 = c0 > b0 ? c0 : b0;
+    b1 = c1 > b1 ? c1 : b1;
+  }
+  if (threadIdx.x % 32 == 0) {
+    atomicMax(inf + 8 * vec + 1, b0);
+    atomicMax(inf + 8 * vec + 2, b1);
+  }
+}
+
 // A CTA of a cluster must not exit while another may still write to its shared
 // memory or wait for it.
 __device__ __forceinline__ void leave() {
@@ -222,20 +417,26 @@ __global__ void __launch_bounds__(kThreads)
   const double  f  = fac.v[vec];
   const double *bv = b + vec * a.vs;
   double       *w0 = a.V + vec * a.vs, w[kRegs], ss = 0.0, none = 0.0;
-  sp.load(w, bv);
+  if (a.wide) {
+    sp.load(w, w0);
+    ss = wide_sum(wide_part(a, vec, 0, 1));
+    cluster_wait();
+  } else {
+    sp.load(w, bv);
 #pragma unroll
-  for (int j = 0; j < kRegs; j++) {
-    w[j] *= f;
-    ss += w[j] * w[j];
+    for (int j = 0; j < kRegs; j++) {
+      w[j] *= f;
+      ss += w[j] * w[j];
+    }
+    sp.regs([&](int j, int64_t i) { w0[i] = w[j]; });
+    sp.rest([&](int64_t i) {
+      const double x = bv[i] * f;
+      w0[i]          = x;
+      ss += x * x;
+    });
+    cluster_wait();
+    Reducer<false>{S, turn}.run(ss, none);
   }
-  sp.regs([&](int j, int64_t i) { w0[i] = w[j]; });
-  sp.rest([&](int64_t i) {
-    const double x = bv[i] * f;
-    w0[i]          = x;
-    ss += x * x;
-  });
-  cluster_wait();
-  Reducer<false>{S, turn}.run(ss, none);
   const double rho = safe_norm(ss, sp, w, w0, S, turn);
   if (lead) {
     const int32_t go       = !(rho < a.tol);  // gmres_ir.hpp:655-657
@@ -256,14 +457,23 @@ __global__ void __launch_bounds__(kThreads) k_gmres_first(const ArnoldiArgs a) {
   const Spread sp(a.n);
   double      *w0 = a.V + vec * a.vs, w[kRegs], ss = 0.0, none = 0.0;
   sp.load(w, w0);
+  if (a.wide) {
+    ss = wide_sum(wide_part(a, vec, 0, 1));
+    cluster_wait();
+  } else {
 #pragma unroll
-  for (int j = 0; j < kRegs; j++) ss += w[j] * w[j];
-  sp.rest([&](int64_t i) { ss += w0[i] * w0[i]; });
-  cluster_wait();
-  Reducer<false>{S, turn}.run(ss, none);
+    for (int j = 0; j < kRegs; j++) ss += w[j] * w[j];
+    sp.rest([&](int64_t i) { ss += w0[i] * w0[i]; });
+    cluster_wait();
+    Reducer<false>{S, turn}.run(ss, none);
+  }
   const double rho = safe_norm(ss, sp, w, w0, S, turn), f = 1 / rho;
-  sp.regs([&](int j, int64_t i) { w0[i] = w[j] * f; });
-  sp.rest([&](int64_t i) { w0[i] *= f; });
+  if (a.wide) {
+    if (cluster_rank() == 0 && threadIdx.x == 0) wide_scratch(a, vec)->f = f;
+  } else {
+    sp.regs([&](int j, int64_t i) { w0[i] = w[j] * f; });
+    sp.rest([&](int64_t i) { w0[i] *= f; });
+  }
   leave();  // every CTA has read the active flag
   if (cluster_rank() == 0 && threadIdx.x == 0) {
     st.g[0]         = rho;
@@ -291,25 +501,33 @@ __global__ void __launch_bounds__(kThreads) k_gmres_step(const ArnoldiArgs a, in
   const Spread sp(a.n);
   double      *V = a.V + vec * a.vs, *wg = V + (k + 1) * a.block;
   double       w[kRegs], v[kRegs];
+  const bool   swept = a.wide && !wide_scratch(a, vec)->odd;  // pass 0 is done
   sp.load(w, wg);
-  sp.load(v, V);
   double ss = 0.0, h = 0.0;
+  if (swept) {
+    ss = wide_scratch(a, vec)->ss;
+    h  = wide_sum(wide_part(a, vec, (k + 1) & 1, 0));
+    cluster_wait();
+  } else {
+    sp.load(v, V);
 #pragma unroll
-  for (int j = 0; j < kRegs; j++) {
-    ss += w[j] * w[j];
-    h += w[j] * v[j];
+    for (int j = 0; j < kRegs; j++) {
+      ss += w[j] * w[j];
+      h += w[j] * v[j];
+    }
+    sp.rest([&](int64_t i) {
+      ss += wg[i] * wg[i];
+      h += wg[i] * V[i];
+    });
+    cluster_wait();
+    Reducer<false>{S, turn}.run(ss, h);
   }
-  sp.rest([&](int64_t i) {
-    ss += wg[i] * wg[i];
-    h += wg[i] * V[i];
-  });
-  cluster_wait();
-  Reducer<false>{S, turn}.run(ss, h);
+  // (Of a swept w, which is not what ss was summed of, ss is within the range.)
   const double normav = safe_norm(ss, sp, w, wg, S, turn);
   double       normw  = 0.0;
   int32_t      reorth = 0;
   for (int pass = 0;; pass++) {
-    for (int64_t j = 0; j <= k; j++) {
+    for (int64_t j = swept && pass == 0 ? k + 1 : 0; j <= k; j++) {
       if (lead) st.col[j] = pass == 0 ? h : st.col[j] + h;
       const double *vj = V + j * a.block, *vn = vj + a.block;
       const double  hj = h;
@@ -341,8 +559,13 @@ __global__ void __launch_bounds__(kThreads) k_gmres_step(const ArnoldiArgs a, in
     h = t;
   }
   const double f = normw != 0 ? 1 / normw : 1.0;
-  sp.regs([&](int j, int64_t i) { wg[i] = w[j] * f; });
-  sp.rest([&](int64_t i) { wg[i] *= f; });
+  if (a.wide) {  // scaled by k_wide_scale, where the loop goes on
+    if (lead) wide_scratch(a, vec)->f = f;
+    if (!swept || reorth) sp.regs([&](int j, int64_t i) { wg[i] = w[j]; });
+  } else {
+    sp.regs([&](int j, int64_t i) { wg[i] = w[j] * f; });
+    sp.rest([&](int64_t i) { wg[i] *= f; });
+  }
   leave();  // every CTA has read the active flag
   if (cluster_rank() != 0 || threadIdx.x >= 32) return;
   // The column's rotations, by one warp: 32 of them are loaded at a time, the
@@ -431,6 +654,10 @@ __global__ void __launch_bounds__(kThreads)
       a.mail->began[vec]  = st.ctl->began;
     }
   }
+  if (a.wide) {  // the rest is k_wide_end's
+    if (update && cluster_rank() == 0 && tid < 3) inf[8 * vec + tid] = 0;
+    return;
+  }
   if (cluster_size() > 1)
     cluster_sync();
   else
@@ -447,17 +674,7 @@ __global__ void __launch_bounds__(kThreads)
     const double *vj = V + j * a.block;
     sp.regs([&](int q, int64_t i) { d[q] += vj[i] * yj; });
   }
-  auto put = [&](double dv, int64_t i) {  // gmres_ir.hpp:574-577
-    if (!update) {
-      xv[i] = dv;
-      return;
-    }
-    const double di = dv * f, xi = xv[i];
-    // NaN counts as above infinity, as in the max-norms of the vector kernels
-    dm    = fabs(di) > dm || !(di == di) ? fabs(di) : dm;
-    xm    = fabs(xi) > xm || !(xi == xi) ? fabs(xi) : xm;
-    xv[i] = xi + di;
-  };
+  auto put = [&](double dv, int64_t i) { refine(dv, f, update, xv[i], dm, xm); };
   sp.regs([&](int q, int64_t i) { put(d[q], i); });
   sp.rest([&](int64_t i) {
     double dv = 0.0;
@@ -511,8 +728,8 @@ __global__ void __launch_bounds__(kThreads)
 }
 
 ArnoldiArgs make_args(int64_t n, int64_t m, int64_t cap, int64_t stride, double *V, int64_t block, double *state,
-                      double tol, GmresMail *mail) {
-  return ArnoldiArgs{n, m, cap, n, block, stride, V, state, tol, mail};
+                      double tol, GmresMail *mail, double *wide) {
+  return ArnoldiArgs{n, m, cap, n, block, stride, V, state, tol, mail, wide};
 }
 
 // Clusters of more than 8 CTAs have to be allowed, on each device.
@@ -535,6 +752,7 @@ void Arnoldi::allocate(int64_t n, int64_t m, int vectors) {
   vectors_ = vectors;
   state_.resize(bytes_for(m, vectors));
   if (cluster() > 8) allow_large_clusters();
+  wide_.resize(n_ > kWideFrom ? sizeof(double) * kWideStride * std::min(vectors, kWideVectors) : 0);
   if (!mail_) mail_ = static_cast<GmresMail *>(pinned_alloc(sizeof(GmresMail)));
 }
 
@@ -569,27 +787,44 @@ int Arnoldi::cluster() const {
   return n_ <= cta ? 1 : n_ <= 8 * cta ? 8 : 16;
 }
 
+bool Arnoldi::wide(int nb) const { return n_ > kWideFrom && nb <= kWideVectors; }
+
 void Arnoldi::begin(int nb, uint32_t act, const double *b, const VecFactors &fac, double *V, double tol,
                     cudaStream_t s) {
-  launch_chained(n_, k_gmres_begin, cluster(), dim3(cluster(), nb, 1), kThreads, 0, s,
-                 make_args(n_, m_, cap_, stride(cap_), V, 0, state_.as<double>(), tol, mail_), act, b, fac);
+  const ArnoldiArgs a = make_args(n_, m_, cap_, stride(cap_), V, 0, state_.as<double>(), tol, mail_,
+                                  wide(nb) ? wide_.as<double>() : nullptr);
+  if (a.wide)
+    launch_chained(0, k_wide_norm, 1, dim3(kWideCtas, nb, 1), kThreads, 0, s, a, act, b, fac);
+  launch_chained(n_, k_gmres_begin, cluster(), dim3(cluster(), nb, 1), kThreads, 0, s, a, act, b, fac);
 }
 
 void Arnoldi::first(int nb, double *V, double tol, cudaStream_t s) {
-  launch_chained(n_, k_gmres_first, cluster(), dim3(cluster(), nb, 1), kThreads, 0, s,
-                 make_args(n_, m_, cap_, stride(cap_), V, 0, state_.as<double>(), tol, mail_));
+  const ArnoldiArgs a = make_args(n_, m_, cap_, stride(cap_), V, 0, state_.as<double>(), tol, mail_,
+                                  wide(nb) ? wide_.as<double>() : nullptr);
+  if (a.wide)
+    launch_chained(0, k_wide_norm, 1, dim3(kWideCtas, nb, 1), kThreads, 0, s, a, 0u, nullptr, VecFactors{});
+  launch_chained(n_, k_gmres_first, cluster(), dim3(cluster(), nb, 1), kThreads, 0, s, a);
+  if (a.wide) launch_chained(0, k_wide_scale, 1, dim3(kWideCtas, nb, 1), kThreads, 0, s, a, 0);
 }
 
 void Arnoldi::step(int nb, int64_t j, double *V, int64_t block, double tol, cudaStream_t s) {
-  launch_chained(n_, k_gmres_step, cluster(), dim3(cluster(), nb, 1), kThreads, 0, s,
-                 make_args(n_, m_, cap_, stride(cap_), V, block, state_.as<double>(), tol, mail_), j);
+  const ArnoldiArgs a = make_args(n_, m_, cap_, stride(cap_), V, block, state_.as<double>(), tol, mail_,
+                                  wide(nb) ? wide_.as<double>() : nullptr);
+  if (a.wide)
+    for (int64_t q = 0; q <= j + 1; q++)
+      launch_chained(0, k_wide_sweep, 1, dim3(kWideCtas, nb, 1), kThreads, 0, s, a, j, q);
+  launch_chained(n_, k_gmres_step, cluster(), dim3(cluster(), nb, 1), kThreads, 0, s, a, j);
+  if (a.wide) launch_chained(0, k_wide_scale, 1, dim3(kWideCtas, nb, 1), kThreads, 0, s, a, j + 1);
 }
 
 void Arnoldi::end(int nb, uint32_t act, const double *V, int64_t block, double *x, bool update,
                   const VecFactors &scale, unsigned long long *inf, cudaStream_t s) {
-  launch_chained(n_, k_gmres_end, cluster(), dim3(cluster(), nb, 1), kThreads, 0, s,
-                 make_args(n_, m_, cap_, stride(cap_), const_cast<double *>(V), block, state_.as<double>(), 0.0, mail_),
-                 act, x, update ? 1 : 0, scale, inf);
+  const ArnoldiArgs a = make_args(n_, m_, cap_, stride(cap_), const_cast<double *>(V), block, state_.as<double>(), 0.0, mail_,
+                                  wide(nb) ? wide_.as<double>() : nullptr);
+  launch_chained(n_, k_gmres_end, cluster(), dim3(cluster(), nb, 1), kThreads, 0, s, a, act, x, update ? 1 : 0,
+                 scale, inf);
+  if (a.wide)
+    launch_chained(0, k_wide_end, 1, dim3(kWideCtas, nb, 1), kThreads, 0, s, a, act, x, update ? 1 : 0, scale, inf);
 }
 
 }  // namespace mpir

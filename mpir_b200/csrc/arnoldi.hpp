@@ -38,7 +38,7 @@ struct GmresMail {
 class Arnoldi {
  public:
   void   allocate(int64_t n, int64_t m, int vectors);
-  size_t bytes() const { return state_.bytes(); }
+  size_t bytes() const { return state_.bytes() + wide_.bytes(); }
   static constexpr int64_t kSteps = 512;
   // Bytes at first.
   static size_t bytes_for(int64_t m, int vectors) {
@@ -78,9 +78,10 @@ class Arnoldi {
     return (4 + m * (m + 1) / 2 + 2 * m + (m + 1) + m + (m + 2) + 1) / 2 * 2;
   }
   int          cluster() const;
+  bool         wide(int nb) const;  // swept by the whole chip
   int64_t      n_ = 0, m_ = 0, cap_ = 0;  // steps allowed, laid out
   int          vectors_ = 0;
-  DeviceBuffer state_;
+  DeviceBuffer state_, wide_;
   GmresMail   *mail_ = nullptr;
 };
 
