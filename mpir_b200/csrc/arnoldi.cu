@@ -397,6 +397,7 @@ __device__ __forceinline__ void leave() {
   if (cluster_size() > 1) cluster_sync();
 }
 
+template <bool WIDE>
 __global__ void __launch_bounds__(kThreads)
     k_gmres_begin(const ArnoldiArgs a, uint32_t act, const double *b, const VecFactors fac) {
   grid_wait();
@@ -417,7 +418,7 @@ __global__ void __launch_bounds__(kThreads)
   const double  f  = fac.v[vec];
   const double *bv = b + vec * a.vs;
   double       *w0 = a.V + vec * a.vs, w[kRegs], ss = 0.0, none = 0.0;
-  if (a.wide) {
+  if (WIDE) {
     sp.load(w, w0);
     ss = wide_sum(wide_part(a, vec, 0, 1));
     cluster_wait();
@@ -446,6 +447,7 @@ __global__ void __launch_bounds__(kThreads)
   leave();
 }
 
+template <bool WIDE>
 __global__ void __launch_bounds__(kThreads) k_gmres_first(const ArnoldiArgs a) {
   grid_wait();
   __shared__ RedShared S;
@@ -457,7 +459,7 @@ __global__ void __launch_bounds__(kThreads) k_gmres_first(const ArnoldiArgs a) {
   const Spread sp(a.n);
   double      *w0 = a.V + vec * a.vs, w[kRegs], ss = 0.0, none = 0.0;
   sp.load(w, w0);
-  if (a.wide) {
+  if (WIDE) {
     ss = wide_sum(wide_part(a, vec, 0, 1));
     cluster_wait();
   } else {
@@ -468,7 +470,7 @@ __global__ void __launch_bounds__(kThreads) k_gmres_first(const ArnoldiArgs a) {
     Reducer<false>{S, turn}.run(ss, none);
   }
   const double rho = safe_norm(ss, sp, w, w0, S, turn), f = 1 / rho;
-  if (a.wide) {
+  if (WIDE) {
     if (cluster_rank() == 0 && threadIdx.x == 0) wide_scratch(a, vec)->f = f;
   } else {
     sp.regs([&](int j, int64_t i) { w0[i] = w[j] * f; });
@@ -486,6 +488,7 @@ __global__ void __launch_bounds__(kThreads) k_gmres_first(const ArnoldiArgs a) {
 // h = w v_j and w -= h v_j, each pass summing for the next one (the loads of
 // v_{j+1} before its reduction); a second sweep where Brown and Hindmarsh's test
 // asks for it; w /= |w|; the rotations.
+template <bool WIDE>
 __global__ void __launch_bounds__(kThreads) k_gmres_step(const ArnoldiArgs a, int64_t k) {
   grid_wait();
   __shared__ RedShared S;
@@ -501,7 +504,7 @@ __global__ void __launch_bounds__(kThreads) k_gmres_step(const ArnoldiArgs a, in
   const Spread sp(a.n);
   double      *V = a.V + vec * a.vs, *wg = V + (k + 1) * a.block;
   double       w[kRegs], v[kRegs];
-  const bool   swept = a.wide && !wide_scratch(a, vec)->odd;  // pass 0 is done
+  const bool   swept = WIDE && !wide_scratch(a, vec)->odd;  // pass 0 is done
   sp.load(w, wg);
   double ss = 0.0, h = 0.0;
   if (swept) {
@@ -559,7 +562,7 @@ __global__ void __launch_bounds__(kThreads) k_gmres_step(const ArnoldiArgs a, in
     h = t;
   }
   const double f = normw != 0 ? 1 / normw : 1.0;
-  if (a.wide) {  // scaled by k_wide_scale, where the loop goes on
+  if (WIDE) {  // scaled by k_wide_scale, where the loop goes on
     if (lead) wide_scratch(a, vec)->f = f;
     if (!swept || reorth) sp.regs([&](int j, int64_t i) { wg[i] = w[j]; });
   } else {
@@ -628,6 +631,7 @@ __global__ void __launch_bounds__(kThreads) k_gmres_step(const ArnoldiArgs a, in
   a.mail->active[k & 1][vec] = go;
 }
 
+template <bool WIDE>
 __global__ void __launch_bounds__(kThreads)
     k_gmres_end(const ArnoldiArgs a, uint32_t act, double *x, int update, const VecFactors fac,
                 unsigned long long *inf) {
@@ -654,7 +658,7 @@ __global__ void __launch_bounds__(kThreads)
       a.mail->began[vec]  = st.ctl->began;
     }
   }
-  if (a.wide) {  // the rest is k_wide_end's
+  if (WIDE) {  // the rest is k_wide_end's
     if (update && cluster_rank() == 0 && tid < 3) inf[8 * vec + tid] = 0;
     return;
   }
@@ -734,8 +738,11 @@ ArnoldiArgs make_args(int64_t n, int64_t m, int64_t cap, int64_t stride, double 
 
 // Clusters of more than 8 CTAs have to be allowed, on each device.
 void allow_large_clusters() {
-  for (auto *f : {reinterpret_cast<const void *>(k_gmres_begin), reinterpret_cast<const void *>(k_gmres_first),
-                  reinterpret_cast<const void *>(k_gmres_step), reinterpret_cast<const void *>(k_gmres_end)})
+  for (auto *f :
+       {reinterpret_cast<const void *>(k_gmres_begin<false>), reinterpret_cast<const void *>(k_gmres_first<false>),
+        reinterpret_cast<const void *>(k_gmres_step<false>), reinterpret_cast<const void *>(k_gmres_end<false>),
+        reinterpret_cast<const void *>(k_gmres_begin<true>), reinterpret_cast<const void *>(k_gmres_first<true>),
+        reinterpret_cast<const void *>(k_gmres_step<true>), reinterpret_cast<const void *>(k_gmres_end<true>)})
     MPIR_CUDA(cudaFuncSetAttribute(f, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
 }
 
@@ -795,7 +802,7 @@ void Arnoldi::begin(int nb, uint32_t act, const double *b, const VecFactors &fac
                                   wide(nb) ? wide_.as<double>() : nullptr);
   if (a.wide)
     launch_chained(0, k_wide_norm, 1, dim3(kWideCtas, nb, 1), kThreads, 0, s, a, act, b, fac);
-  launch_chained(n_, k_gmres_begin, cluster(), dim3(cluster(), nb, 1), kThreads, 0, s, a, act, b, fac);
+  launch_chained(n_, a.wide ? k_gmres_begin<true> : k_gmres_begin<false>, cluster(), dim3(cluster(), nb, 1), kThreads, 0, s, a, act, b, fac);
 }
 
 void Arnoldi::first(int nb, double *V, double tol, cudaStream_t s) {
@@ -803,7 +810,7 @@ void Arnoldi::first(int nb, double *V, double tol, cudaStream_t s) {
                                   wide(nb) ? wide_.as<double>() : nullptr);
   if (a.wide)
     launch_chained(0, k_wide_norm, 1, dim3(kWideCtas, nb, 1), kThreads, 0, s, a, 0u, nullptr, VecFactors{});
-  launch_chained(n_, k_gmres_first, cluster(), dim3(cluster(), nb, 1), kThreads, 0, s, a);
+  launch_chained(n_, a.wide ? k_gmres_first<true> : k_gmres_first<false>, cluster(), dim3(cluster(), nb, 1), kThreads, 0, s, a);
   if (a.wide) launch_chained(0, k_wide_scale, 1, dim3(kWideCtas, nb, 1), kThreads, 0, s, a, 0);
 }
 
@@ -813,7 +820,7 @@ void Arnoldi::step(int nb, int64_t j, double *V, int64_t block, double tol, cuda
   if (a.wide)
     for (int64_t q = 0; q <= j + 1; q++)
       launch_chained(0, k_wide_sweep, 1, dim3(kWideCtas, nb, 1), kThreads, 0, s, a, j, q);
-  launch_chained(n_, k_gmres_step, cluster(), dim3(cluster(), nb, 1), kThreads, 0, s, a, j);
+  launch_chained(n_, a.wide ? k_gmres_step<true> : k_gmres_step<false>, cluster(), dim3(cluster(), nb, 1), kThreads, 0, s, a, j);
   if (a.wide) launch_chained(0, k_wide_scale, 1, dim3(kWideCtas, nb, 1), kThreads, 0, s, a, j + 1);
 }
 
@@ -821,7 +828,7 @@ void Arnoldi::end(int nb, uint32_t act, const double *V, int64_t block, double *
                   const VecFactors &scale, unsigned long long *inf, cudaStream_t s) {
   const ArnoldiArgs a = make_args(n_, m_, cap_, stride(cap_), const_cast<double *>(V), block, state_.as<double>(), 0.0, mail_,
                                   wide(nb) ? wide_.as<double>() : nullptr);
-  launch_chained(n_, k_gmres_end, cluster(), dim3(cluster(), nb, 1), kThreads, 0, s, a, act, x, update ? 1 : 0,
+  launch_chained(n_, a.wide ? k_gmres_end<true> : k_gmres_end<false>, cluster(), dim3(cluster(), nb, 1), kThreads, 0, s, a, act, x, update ? 1 : 0,
                  scale, inf);
   if (a.wide)
     launch_chained(0, k_wide_end, 1, dim3(kWideCtas, nb, 1), kThreads, 0, s, a, act, x, update ? 1 : 0, scale, inf);
