@@ -85,7 +85,7 @@ constexpr int kFlowChunkC = 128;  // columns of one
 constexpr int kFlowWarpsPerItem = 16;
 // From this many items of leaves of at most 64 rows on, the solves for one
 // vector take them by kernels of their own (k_fwd_leaf, k_bwd_leaf).
-constexpr int kFlowLeafItems = 32 * 148;
+constexpr int kFlowLeafItems = 6 * 148;
 constexpr int kFlowPanelSmem = 16 * kFlowBlk * 8;  // bytes for a kFlowWarps item's panels
 
 // Doubles of a warp-solved front's float64 panel (even: copied in 16-byte words).

@@ -793,10 +793,10 @@ __global__ void __launch_bounds__(kFlowThreads, 1) k_bwd_flow(const __grid_const
 // the backward data flow.  A front waits on nothing, so what bounds it is latency,
 // and 64 warps an SM hide it where 16 with their fronts staged in shared memory do
 // not.  One application by items, by levels before those, and so (ms): 10,000
-// blocks of 40 x 40 0.40, 0.14, 0.08; 100,000 of 4 x 4 0.22, 0.20, 0.11; 500,000 of one
-// 0.99, 0.69, 0.33; the leaves of a 2-D grid of n = 1.4 million 1.11, 2.00, 0.92.  At
-// the line (kFlowLeafItems) the items of a direction take about 70 us; below it two
-// more launches weigh as much as they save.
+// blocks of 40 x 40 0.40, 0.14, 0.08, 1,000 0.053, 0.043, 0.033; 100,000 of 4 x 4 0.22,
+// 0.20, 0.11; 500,000 of one 0.99, 0.69, 0.33; 2-D grids of n = 640,000 0.52, 1.11, 0.44 and
+// 250,000 0.25, 0.63, 0.24 (the line, kFlowLeafItems, where the items of a direction take
+// about 15 us; below it two more launches weigh as much as they save).
 constexpr int kLeafWarps = 8;
 __global__ void __launch_bounds__(32 * kLeafWarps)
     k_fwd_leaf(const FlowFront *fronts, int count, const float *panel, const double *x, double *f,

@@ -1,5 +1,5 @@
 """Triangular solves with many leaves of at most 64 rows, which one vector takes by
-kernels of their own (from 4,736 work items of them on, 16 leaves of up to 32 columns
+kernels of their own (from 888 work items of them on, 16 leaves of up to 32 columns
 an item), alone and below a common front, beside leaves that are larger.  Tolerance as
 in test_gpu_flow.py (dominant systems, blocks of at most 150)."""
 import numpy as np
@@ -36,11 +36,11 @@ def _system(sizes, top, large=0, seed=0):
 
 
 CASES = {
-    "narrow": lambda: _system([33 + k % 32 for k in range(4900)], 0),
-    "below_the_line": lambda: _system([33 + k % 32 for k in range(4600)], 0),
-    "with_rows": lambda: _system([33 + k % 12 for k in range(4900)], 20),
-    "tiny": lambda: _system([1 + k % 3 for k in range(78000)], 2, large=5),
-    "mixed": lambda: _system([1 + k % 64 for k in range(9000)], 0, large=7),
+    "narrow": lambda: _system([33 + k % 32 for k in range(950)], 0),
+    "below_the_line": lambda: _system([33 + k % 32 for k in range(880)], 0),
+    "with_rows": lambda: _system([33 + k % 12 for k in range(950)], 20),
+    "tiny": lambda: _system([1 + k % 3 for k in range(15000)], 2, large=5),
+    "mixed": lambda: _system([1 + k % 64 for k in range(1800)], 0, large=7),
 }
 
 
