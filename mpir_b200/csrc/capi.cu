@@ -109,12 +109,21 @@ static void export_csc(const Plan &P, const Numeric &F, cudaStream_t s,
   exact_pattern(S, Lp, Li);
   Lx.resize(Li.size());
   for (int64_t J = 0; J < S.ns; J++) {
-    const int64_t f = S.sfirst[J], l = S.sfirst[J + 1], h = S.h(J);
-    for (int64_t j = f; j < l; j++)
+    const int64_t  f = S.sfirst[J], l = S.sfirst[J + 1], w = l - f, h = S.h(J);
+    const int32_t *below = S.srows.data() + S.srowptr[J] + w, *end = S.srows.data() + S.srowptr[J + 1];
+    for (int64_t j = f; j < l; j++) {
+      const int32_t *q   = below;  // a column's rows ascend
+      const float   *col = pan.data() + S.slofs[J] + (j - f) * h;
       for (int64_t p = Lp[j]; p < Lp[j + 1]; p++) {
-        const int64_t lr = local_row(S, J, Li[p]);
-        Lx[p] = lr < 0 ? 0.0f : pan[S.slofs[J] + (j - f) * h + lr];
+        const int64_t r = Li[p];
+        if (r < l) {
+          Lx[p] = col[r - f];
+          continue;
+        }
+        while (q != end && *q < r) q++;
+        Lx[p] = q != end && *q == r ? col[w + (q - below)] : 0.0f;
       }
+    }
   }
 }
 

@@ -51,7 +51,8 @@ namespace mpir {
 
 // Shared memory (doubles): kFlowInvSmem, written by bulk copies only, then 4,608
 // for vectors and partial sums.
-constexpr int kFlowSmem = kFlowInvSmem + 4608;
+constexpr int kFlowSmem      = kFlowInvSmem + 4608;
+constexpr int kFlowSmemBytes = kFlowSmem * sizeof(double);
 
 __global__ void k_mark_pending(int64_t n, double *p) {
   flow_mark(p, n);
@@ -419,7 +420,9 @@ __device__ __noinline__ void fwd_warp(const FlowArgs<T> &a, FlowShared &S, const
   }
 }
 
-template <class T>
+// SUMS: of a plan with kFwdSum items (the others' kernel took 0.5 us longer with their
+// case in it).
+template <class T, bool SUMS>
 __global__ void __launch_bounds__(kFlowThreads, 1) k_fwd_flow(const __grid_constant__ FlowArgs<T> a) {
   grid_wait();
   extern __shared__ __align__(128) double sm[];
@@ -436,8 +439,11 @@ __global__ void __launch_bounds__(kFlowThreads, 1) k_fwd_flow(const __grid_const
           fwd_narrow<4>(a, S, I, N, sm, phase);
         break;
       case kFwdSlab: fwd_slab(a, S, I, N, sm, phase); break;
-      case kFwdSum: fwd_sum(a, I, N); break;
-      default: fwd_rows(a, I, N, sm);
+      default:
+        if (SUMS && I.item.kind == kFwdSum)
+          fwd_sum(a, I, N);
+        else
+          fwd_rows(a, I, N, sm);
     }
   });
   flow_mark(a.mark, a.nmark);
@@ -1053,6 +1059,17 @@ void SolveWorkspace::allocate(const Plan &P) {
   err.resize(sizeof(SolveCtl));
   device_zero(err.as<void>(), sizeof(SolveCtl));
   fwd_pending = bwd_pending = false;
+  static OncePerDevice attr;
+  allow_smem(attr, kFlowSmemBytes,
+             {reinterpret_cast<const void *>(k_fwd_flow<float, false>),
+              reinterpret_cast<const void *>(k_fwd_flow<float, true>),
+              reinterpret_cast<const void *>(k_fwd_flow<__half, false>),
+              reinterpret_cast<const void *>(k_fwd_flow<__half, true>),
+              reinterpret_cast<const void *>(k_fwd_flow<__nv_bfloat16, false>),
+              reinterpret_cast<const void *>(k_fwd_flow<__nv_bfloat16, true>),
+              reinterpret_cast<const void *>(k_bwd_flow<float>),
+              reinterpret_cast<const void *>(k_bwd_flow<__half>),
+              reinterpret_cast<const void *>(k_bwd_flow<__nv_bfloat16>)});
 }
 
 template <class T>
@@ -1084,9 +1101,7 @@ static void ldlt_solve_t(const Plan &P, const Numeric &F, const T *pan, double *
   a.active        = act.p;
   a.nactive       = act.count;
   a.active_stride = act.stride;
-  static OncePerDevice attr;
-  constexpr int        smem = kFlowSmem * sizeof(double);
-  allow_smem(attr, smem, {reinterpret_cast<const void *>(k_fwd_flow<T>), reinterpret_cast<const void *>(k_bwd_flow<T>)});
+  constexpr int smem = kFlowSmemBytes;
   // (The 16-bit panels are left to the items, which take these fronts' float32 values.
   // Beside the leaves' kernels there may be few items or none; the launch still marks
   // all the values pending.)
@@ -1105,7 +1120,8 @@ static void ldlt_solve_t(const Plan &P, const Numeric &F, const T *pan, double *
     a.mark   = bv;
     a.nmark  = b.bwd;
     a.ticket = ws.sync.as<int32_t>();
-    launch_chained(n, k_fwd_flow<T>, 1, leaf ? kSMs : std::min(a.nitems, kSMs), kFlowThreads, smem, s, a);
+    launch_chained(n, P.flow_z_elems > P.S.z_elems ? k_fwd_flow<T, true> : k_fwd_flow<T, false>, 1,
+                   leaf ? kSMs : std::min(a.nitems, kSMs), kFlowThreads, smem, s, a);
     ws.fwd_pending = false;
     ws.bwd_pending = true;
   }

@@ -1075,10 +1075,7 @@ void solve_multi_nr(const Plan &P, const Numeric &F, const T *pan, double *X,
   a.active        = act.p;
   a.nactive       = act.count;
   a.active_stride = act.stride;
-  static OncePerDevice attr;
-  constexpr int        smem = kMultiSmem * sizeof(double);
-  allow_smem(attr, smem,
-             {reinterpret_cast<const void *>(k_fwd_flow_m<NR, T>), reinterpret_cast<const void *>(k_bwd_flow_m<NR, T>)});
+  constexpr int smem = kMultiSmem * sizeof(double);
   kt.begin(kKcSolveFwd, s);
   if (!ws.fwd_pending) flow_pending(fv, NR * b.fwd, s);
   a.items  = P.flow_fwd.as<FlowItem>();
@@ -1102,6 +1099,17 @@ void solve_multi_nr(const Plan &P, const Numeric &F, const T *pan, double *X,
   MPIR_CHECK_LAUNCH();
 }
 
+template <int NR>
+void allow_multi() {
+  static OncePerDevice attr;
+  allow_smem(attr, kMultiSmem * sizeof(double),
+             {reinterpret_cast<const void *>(k_fwd_flow_m<NR, float>), reinterpret_cast<const void *>(k_bwd_flow_m<NR, float>),
+              reinterpret_cast<const void *>(k_fwd_flow_m<NR, __half>),
+              reinterpret_cast<const void *>(k_bwd_flow_m<NR, __half>),
+              reinterpret_cast<const void *>(k_fwd_flow_m<NR, __nv_bfloat16>),
+              reinterpret_cast<const void *>(k_bwd_flow_m<NR, __nv_bfloat16>)});
+}
+
 }  // namespace
 
 int multi_width(int nrhs) {
@@ -1119,6 +1127,9 @@ void MultiSolveWorkspace::allocate(const Plan &P, int width) {
   device_zero(sync.as<void>(), sync.bytes());
   err.resize(sizeof(SolveCtl));
   device_zero(err.as<void>(), sizeof(SolveCtl));
+  if (width == 4) allow_multi<4>();
+  if (width == 8) allow_multi<8>();
+  if (width == 16) allow_multi<16>();
   nr = width;
 }
 
