@@ -40,6 +40,7 @@ CASES = {
     "below_the_line": lambda: _system([33 + k % 32 for k in range(880)], 0),
     "with_rows": lambda: _system([33 + k % 12 for k in range(950)], 20),
     "tiny": lambda: _system([1 + k % 3 for k in range(15000)], 2, large=5),
+    "dependent_launches": lambda: _system([1] * 14600, 3),  # (n of at most 20,000)
     "mixed": lambda: _system([1 + k % 64 for k in range(1800)], 0, large=7),
 }
 
